@@ -19,6 +19,7 @@
 
 #include "abi_guard.h"
 #include "kernels.h"
+#include "modgemm.cuh"
 
 using rpa::dd;
 
@@ -34,14 +35,17 @@ struct DevBuf {
 // Device-memory accounting of one handle: bytes its workspace holds, and the cap a caller may set
 // (rpa_b200_set_workspace_limit; 0 = none).  Every workspace allocation of a call goes through
 // dev_alloc / dev_free below, which charge the handle whose call is running on this thread.
+// idle: buffers of the handle that hold nothing between calls and that the running call has not asked
+// for yet; an allocation that finds no room frees them and tries again.
 struct WorkspaceAccount {
   size_t used = 0;
   size_t limit = 0;
+  std::vector<DevBuf*> idle;
 };
 namespace {
 thread_local WorkspaceAccount* g_account = nullptr;
 
-cudaError_t dev_alloc(void** p, size_t bytes) {
+cudaError_t dev_alloc_once(void** p, size_t bytes) {
   WorkspaceAccount* a = g_account;
   if (a && a->limit && (bytes > a->limit || a->used > a->limit - bytes)) {
     *p = nullptr;
@@ -57,6 +61,20 @@ void dev_free(void* p, size_t bytes) {
   cudaFree(p);
   WorkspaceAccount* a = g_account;
   if (a) a->used = a->used > bytes ? a->used - bytes : 0;
+}
+
+cudaError_t dev_alloc(void** p, size_t bytes) {
+  cudaError_t e = dev_alloc_once(p, bytes);
+  WorkspaceAccount* a = g_account;
+  if (e != cudaErrorMemoryAllocation || !a || a->idle.empty()) return e;
+  cudaGetLastError();
+  for (DevBuf* b : a->idle) {
+    dev_free(b->p, b->bytes);
+    b->p = nullptr;
+    b->bytes = 0;
+  }
+  a->idle.clear();
+  return dev_alloc_once(p, bytes);
 }
 }  // namespace
 
@@ -143,6 +161,11 @@ namespace {
 
 const double kPi = 3.14159265358979323846;
 
+// Residue products (modgemm.cu) pay off from here on; below, the DMMA kernels are as fast.
+constexpr int kModMinNQ = 128;
+constexpr int64_t kModMinK = 128;
+constexpr size_t kModBudget = (size_t)4 << 30;  // device bytes of one group of residue planes
+
 int fail(rpa_b200_handle* h, int status, const char* fmt, ...) {
   if (h) {
     char buf[512];
@@ -186,6 +209,10 @@ int screen_result(rpa_b200_handle* h, const double* A, int64_t ld, int64_t rows,
 }
 
 cudaError_t ensure(DevBuf& b, size_t bytes) {
+  if (g_account) {
+    auto& idle = g_account->idle;
+    idle.erase(std::remove(idle.begin(), idle.end(), &b), idle.end());
+  }
   if (b.bytes >= bytes && b.p) return cudaSuccess;
   if (b.p) {
     dev_free(b.p, b.bytes);
@@ -401,6 +428,90 @@ int prepare_sync(rpa_b200_handle* h, int NQ, int kg, int64_t nov_part, int** out
   return RPA_OK;
 }
 
+// ---- FP64-accurate products on the int8 tensor cores (modgemm.cu)
+// Allocates workspace that the caller can do without: false (no error left behind) when the device or
+// the caller's workspace cap has no room for it.
+bool try_ensure(DevBuf& b, size_t bytes) {
+  if (ensure(b, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
+// Residues of one product, from operand planes already on the device (pa: rowsA rows, pb: rowsB rows of K).
+int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t planesA, int rowsA, int8_t* pb,
+                int64_t planesB, int rowsB, int64_t K, int nz, bool tri, uint8_t* out, int64_t ldo) {
+  const int64_t pitch = rpa::mod_pitch(K);
+  CUtensorMap mA, mB, mBh;
+  if (rpa::mod_map(h->encode, &mA, pa, K, rowsA, planesA, pitch, 128) != cudaSuccess ||
+      rpa::mod_map(h->encode, &mB, pb, K, rowsB, planesB, pitch, 256) != cudaSuccess ||
+      rpa::mod_map(h->encode, &mBh, pb, K, rowsB, planesB, pitch, 128) != cudaSuccess)
+    return fail(h, RPA_ERR_CUDA, "cuTensorMapEncodeTiled failed for residue planes");
+  RPA_CUDA(h, rpa::mod_plan(a, rowsA, rowsB, K, nz, tri));
+  a.zplanesA = planesA > rpa::kModCount ? rpa::kModCount : 0;
+  a.zplanesB = planesB > rpa::kModCount ? rpa::kModCount : 0;
+  a.out = out;
+  a.ldo = ldo;
+  a.out_plane = (int64_t)rowsA * ldo;
+  a.err = h->err_dev;
+  a.sync = nullptr;
+  a.sync_every = h->sync_every;
+  const int64_t words = rpa::mod_sync_words(a, h->num_sms);
+  if (words > 0) {
+    RPA_CUDA(h, ensure(h->syncBuf, (size_t)words * sizeof(int)));
+    RPA_CUDA(h, cudaMemsetAsync(h->syncBuf.p, 0, (size_t)words * sizeof(int), h->stream));
+    a.sync = static_cast<int*>(h->syncBuf.p);
+  }
+  RPA_CUDA(h, rpa::launch_modgemm(mA, mB, mBh, a, h->num_sms, h->stream));
+  return RPA_OK;
+}
+
+// FP64 form of Pi(u) (lower triangles into h->Pi) by residue products.  Returns 1 (nothing done) for
+// shapes where the DMMA kernel is the faster one, or without memory for the residue planes.
+int build_pi_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t ldR, double alpha) {
+  const int NQ = v.NQ;
+  const int64_t nov = v.nov;
+  if (NQ < kModMinNQ || nov < kModMinK) return 1;
+  const int64_t pitch = rpa::mod_pitch(nov), ldo = (NQ + 255) / 256 * 256;
+  const size_t perA = (size_t)rpa::kModCount * NQ * pitch, perC = (size_t)rpa::kModCount * NQ * ldo;
+  // a few GiB of planes per group keep the tensor cores busy and leave the memory to the other buffers
+  const int kg = (int)std::min<size_t>(std::min(v.K, rpa::kMaxKgLaunch), std::max<size_t>(1, kModBudget / (perA + perC)));
+  const int qt = (NQ + 31) / 32;
+  const int nsplit = (int)std::min<int64_t>((nov + 63) / 64, std::max(1, (4 * h->num_sms + qt - 1) / qt));
+  const size_t b_fac = (size_t)kg * nov * 8, b_part = (size_t)nsplit * kg * NQ * 8, b_expo = (size_t)kg * NQ * 4;
+  if (!try_ensure(h->Xhi, kg * perA) || !try_ensure(h->Xlo, kg * perC) ||
+      !try_ensure(h->diag_part, b_fac + b_part + b_expo)) {
+    release(h->Xhi);  // leave the DMMA form all the room it had
+    release(h->Xlo);
+    return 1;
+  }
+  double* fac = static_cast<double*>(h->diag_part.p);
+  double* part = fac + (size_t)kg * nov;
+  int* expo = reinterpret_cast<int*>(part + (size_t)nsplit * kg * NQ);
+  double* Pi = static_cast<double*>(h->Pi.p);
+  for (int g0 = 0; g0 < v.K; g0 += kg) {
+    const int n = std::min(kg, v.K - g0);
+    rpa::FreqGroup fg{};
+    fg.n = n;
+    for (int k = 0; k < n; ++k) fg.u2[k] = v.freqs[g0 + k] * v.freqs[g0 + k];
+    cudaEvent_t e0 = pool_event(h), e1 = pool_event(h), e2 = pool_event(h);
+    RPA_CUDA(h, cudaEventRecord(e0, h->stream));
+    int8_t* planes = static_cast<int8_t*>(h->Xhi.p);
+    RPA_CUDA(h, rpa::launch_mod_pi(Rd, ldR, NQ, nov, static_cast<const double*>(h->D.p), fg, alpha, fac, part, nsplit,
+                                   expo, planes, h->stream));
+    RPA_CUDA(h, cudaEventRecord(e1, h->stream));
+    h->split_ev.push_back({e0, e1});
+    rpa::ModGemmArgs a{};
+    int s = mod_product(h, a, planes, (int64_t)n * rpa::kModCount, NQ, planes, (int64_t)n * rpa::kModCount, NQ, nov, n,
+                        true, static_cast<uint8_t*>(h->Xlo.p), ldo);
+    if (s != RPA_OK) return s;
+    RPA_CUDA(h, rpa::launch_mod_crt_lower(a.out, a.out_plane, ldo, expo, NQ, n, Pi + (int64_t)g0 * NQ * NQ, NQ,
+                                          (int64_t)NQ * NQ, h->stream));
+    RPA_CUDA(h, cudaEventRecord(e2, h->stream));
+    h->tc_ev.push_back({e1, e2});
+  }
+  return RPA_OK;
+}
+
 int build_pi(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t ldR, double alpha, int64_t prec) {
   const int NQ = v.NQ;
   const int64_t nov = v.nov;
@@ -410,6 +521,8 @@ int build_pi(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t l
   double* Pi = static_cast<double*>(h->Pi.p);
   const double* D = static_cast<const double*>(h->D.p);
   if (prec == RPA_PREC_FP64) {
+    int ms = build_pi_mod(h, v, Rd, ldR, alpha);
+    if (ms != 1) return ms;
     rpa::DsyrkArgs a{};
     a.A = Rd;
     a.lda = ldR;
@@ -1030,6 +1143,7 @@ int begin_call(rpa_b200_handle* h) {
   if (!h) return RPA_ERR_INVALID_ARG;
   h->last_error.clear();
   g_account = &h->account;
+  h->account.idle = {&h->Xhi, &h->Xlo, &h->gY};
   h->pool_used = 0;
   h->split_ev.clear();
   h->tc_ev.clear();

@@ -1,0 +1,735 @@
+// FP64-accurate matrix products on the int8 tensor cores by residue arithmetic.
+//
+//   C(i, j) = sum_k a(i, k) b(j, k)
+//
+// The modular scheme of Ozaki, Uchino and Imamura ("Ozaki Scheme II: a GEMM-oriented emulation of
+// floating-point matrix multiplication using an integer modular technique", 2025): every row of a
+// and b is scaled by a power of two and rounded to integers a', b' whose 2-norms stay below
+// 2^58; |sum_k a' b'| is then below P / 2 for P the product of 15 pairwise coprime moduli <= 256
+// (Cauchy-Schwarz, so the bound holds for every input), and the exact integer product follows from
+// its 15 residues (Chinese remainder theorem).  Each residue is one int8 x int8 -> int32 matrix
+// product of tcgen05 (kind::i8), exact as long as K <= 65536 per accumulation.  The only errors
+// are the rounding of the operands (0.5 units of 2^-58 of the row norm) and one rounding of C, less
+// than a chain of K FP64 additions leaves (tests/test_gpu_modgemm.py compares both).
+//
+// On B200 the int8 pipe sustains 3.9 POP/s (random operands from shared memory, M 128 x N 256), so
+// 15 products cost what 260 TFLOP/s of FP64 would, against 37 TFLOP/s of the FP64 pipe.
+//
+//  * mod_cols_kernel: operands whose K index is contiguous (column-major K x rows)
+//  * mod_pi_kernel:   X_k(Q, ai) = sqrt(alpha c_k(ai)) R(Q, ai), transposed to ai-contiguous rows
+//  * modgemm_kernel:  residues of C, 15 int8 products per tile
+//  * mod_*crt*:       C from its residues
+#include <algorithm>
+#include <utility>
+
+#include "modgemm.cuh"
+
+namespace rpa {
+
+namespace {
+// ------------------------------------------------------------------ residues of the operands
+// For an integer x in (-2^63, 2^63): x + 2^63 has eight unsigned bytes b_j, and
+// x = sum_j b_j 256^j - 2^63 = sum_j b_j (256^j mod p) + (-2^63 mod p)   (mod p): two 4-way byte
+// dot products give a value v < 2^20 congruent to x.  v is reduced in FP32 (exact: v < 2^23): the
+// dot product starts from the bits of 1.5 * 2^23, so its result is the float 1.5 * 2^23 + v.
+template <int I>
+struct ModConst {
+  static constexpr uint32_t p = kModuli[I];
+  static constexpr uint32_t pw(int j) {
+    uint32_t r = 1;
+    for (int t = 0; t < j; ++t) r = (r * 256u) % p;
+    return p == 256u && j > 0 ? 0u : r;
+  }
+  static constexpr uint32_t wlo = pw(0) | pw(1) << 8 | pw(2) << 16 | pw(3) << 24;
+  static constexpr uint32_t whi = pw(4) | pw(5) << 8 | pw(6) << 16 | pw(7) << 24;
+  static constexpr uint32_t off = (p - (128u * pw(7)) % p) % p;  // -2^63 mod p
+  static constexpr uint32_t init = 0x4B400000u + off;
+};
+
+template <int I>
+__device__ __forceinline__ uint32_t mod_residue_bits(uint32_t lo, uint32_t hi) {
+  using M = ModConst<I>;
+  const float big = 12582912.0f;  // 1.5 * 2^23
+  const float f = __uint_as_float(__dp4a(lo, M::wlo, __dp4a(hi, M::whi, M::init)));
+  const float q = __fsub_rn(__fmaf_rn(__fsub_rn(f, big), 1.0f / (float)M::p, big), big);
+  // 1.5 * 2^23 + r, |r| <= p / 2 (+ 1): its low byte is r as a signed 8-bit integer
+  return __float_as_uint(__fmaf_rn(-(float)M::p, q, f));
+}
+
+// Residues of N (a multiple of 4) integers for modulus I, packed four to a word.
+template <int I, int N>
+__device__ __forceinline__ void mod_pack(const uint32_t (&lo)[N], const uint32_t (&hi)[N], uint32_t (&w)[N / 4]) {
+#pragma unroll
+  for (int t = 0; t < N / 4; ++t) {
+    const uint32_t a = mod_residue_bits<I>(lo[4 * t], hi[4 * t]), b = mod_residue_bits<I>(lo[4 * t + 1], hi[4 * t + 1]);
+    const uint32_t c = mod_residue_bits<I>(lo[4 * t + 2], hi[4 * t + 2]),
+                   d = mod_residue_bits<I>(lo[4 * t + 3], hi[4 * t + 3]);
+    w[t] = __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+  }
+}
+
+template <int N, class Store, int... I>
+__device__ __forceinline__ void mod_all(const uint32_t (&lo)[N], const uint32_t (&hi)[N], const Store& store,
+                                        std::integer_sequence<int, I...>) {
+  (
+      [&] {
+        uint32_t w[N / 4];
+        mod_pack<I, N>(lo, hi, w);
+        store(I, w);
+      }(),
+      ...);
+}
+
+__device__ __forceinline__ void to_words(double x, uint32_t& lo, uint32_t& hi) {
+  const unsigned long long u = (unsigned long long)__double2ll_rn(x) ^ 0x8000000000000000ull;
+  lo = (uint32_t)u;
+  hi = (uint32_t)(u >> 32);
+}
+
+// Columns of a column-major (K x rows) matrix: one warp per column, 8 consecutive k per lane.
+// S: column r starts at S + r * ld; expo[r]: its power of two.  shift is subtracted from the diagonal.
+__global__ void __launch_bounds__(256) mod_cols_kernel(const double* __restrict__ S, int64_t ld, int64_t strideS,
+                                                       int K, int64_t rows, int8_t* __restrict__ planes,
+                                                       int64_t pitch, int64_t plane_stride, int64_t strideP,
+                                                       int* __restrict__ expo, double shift) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const int z = blockIdx.y;
+  const double* col = S + (int64_t)z * strideS + r * ld;
+  double s2 = 0.0;
+  for (int k = lane; k < K; k += 32) {
+    const double x = col[k] - (k == r ? shift : 0.0);
+    s2 = fma(x, x, s2);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  const int e = mod_exponent(s2);
+  if (lane == 0) expo[(int64_t)z * rows + r] = e;
+  const double sc = mod_pow2(e);
+  int8_t* out = planes + (int64_t)z * strideP + r * pitch;
+  for (int k0 = 8 * lane; k0 < pitch; k0 += 256) {
+    uint32_t lo[8], hi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      to_words(k0 + i < K ? (col[k0 + i] - (k0 + i == r ? shift : 0.0)) * sc : 0.0, lo[i], hi[i]);
+    mod_all<8>(
+        lo, hi,
+        [&](int m, const uint32_t(&w)[2]) {
+          *reinterpret_cast<uint2*>(out + m * plane_stride + k0) = make_uint2(w[0], w[1]);
+        },
+        std::make_integer_sequence<int, kModCount>());
+  }
+}
+
+// fac[k * nov + ai] = sqrt(alpha D / (D^2 + u_k^2))
+__global__ void mod_chi_kernel(const double* __restrict__ D, int64_t nov, FreqGroup fg, double alpha,
+                               double* __restrict__ fac) {
+  const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= nov) return;
+  const double d = D[a];
+#pragma unroll
+  for (int k = 0; k < kMaxKgLaunch; ++k)
+    if (k < fg.n) fac[k * nov + a] = sqrt(alpha * d / fma(d, d, fg.u2[k]));
+}
+
+// part[split][k][Q] = sum over the split's ai of (fac_k R)^2: lane = Q, each warp 16 of the 128 ai of a
+// chunk; the squared factors wait in shared memory ([ai][k], broadcast reads).  Reading the factors
+// from global memory inside the sum took 2.46 ms at NQ 2048, 16384 ai, 16 frequencies.
+constexpr int kNormWarps = 8;
+__global__ void __launch_bounds__(256) mod_pi_norm_kernel(const double* __restrict__ R, int64_t ldR, int NQ,
+                                                          int64_t nov, const double* __restrict__ fac, int kg,
+                                                          int64_t per_split, double* __restrict__ part) {
+  __shared__ __align__(16) double sm[kNormWarps * kMaxKgLaunch * 32];  // factors, then the warps' sums
+  static_assert(128 * kMaxKgLaunch <= kNormWarps * kMaxKgLaunch * 32, "the factors fit");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q = blockIdx.x * 32 + lane;
+  const int64_t a0 = (int64_t)blockIdx.y * per_split, a1 = min(nov, a0 + per_split);
+  double s[kMaxKgLaunch];
+#pragma unroll
+  for (int k = 0; k < kMaxKgLaunch; ++k) s[k] = 0.0;
+  for (int64_t c = a0; c < a1; c += 128) {
+    double r[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int64_t a = c + warp * 16 + j;
+      r[j] = (q < NQ && a < a1) ? __ldg(R + q + ldR * a) : 0.0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 128 * kMaxKgLaunch; i += 256) {
+      const int k = i >> 7, j = i & 127;
+      const double f = (k < kg && c + j < a1) ? __ldg(fac + k * nov + c + j) : 0.0;
+      sm[j * kMaxKgLaunch + k] = f * f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const double r2 = r[j] * r[j];
+      const double2* f2 = reinterpret_cast<const double2*>(sm + (warp * 16 + j) * kMaxKgLaunch);
+#pragma unroll
+      for (int k = 0; k < kMaxKgLaunch / 2; ++k) {
+        const double2 f = f2[k];
+        s[2 * k] = fma(r2, f.x, s[2 * k]);
+        s[2 * k + 1] = fma(r2, f.y, s[2 * k + 1]);
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kMaxKgLaunch; ++k) sm[(warp * kMaxKgLaunch + k) * 32 + lane] = s[k];
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < kg * 32; idx += 256) {
+    const int k = idx >> 5, l = idx & 31;
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kNormWarps; ++w) t += sm[(w * kMaxKgLaunch + k) * 32 + l];
+    if (blockIdx.x * 32 + l < NQ) part[((int64_t)blockIdx.y * kg + k) * NQ + blockIdx.x * 32 + l] = t;
+  }
+}
+
+__global__ void mod_pi_expo_kernel(const double* __restrict__ part, int nsplit, int64_t n, int* __restrict__ expo) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s = 0.0;
+  for (int t = 0; t < nsplit; ++t) s += part[t * n + i];
+  expo[i] = mod_exponent(s);
+}
+
+// planes[(k, m)][Q][ai]: a CTA takes a 32 x 128 block of R (read with Q across the lanes, kept in
+// shared memory) and writes whole 128-byte lines, four ai per lane and one row per warp.  The lines
+// are what bounds the pass: with 16 ai of 32 different rows per warp the stores of 15 planes were
+// half sectors, and more CTAs per SM only made them slower (7.3 ms with one, 13.1 ms with three at
+// NQ 2048, 16384 ai, 16 frequencies).
+constexpr int kPiPitch = 128 + 4;
+constexpr size_t kModPiSmem = sizeof(double) * (32 * kPiPitch + kMaxKgLaunch * 128);
+__global__ void __launch_bounds__(256, 4) mod_pi_kernel(const double* __restrict__ R, int64_t ldR, int NQ, int64_t nov,
+                                                        const double* __restrict__ fac, int kg,
+                                                        const int* __restrict__ expo, int8_t* __restrict__ planes,
+                                                        int64_t pitch) {
+  extern __shared__ __align__(16) double mod_smem[];
+  double* rs = mod_smem;                  // [32 Q][kPiPitch]
+  double* fs = mod_smem + 32 * kPiPitch;  // [kg][128 ai]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q0 = blockIdx.x * 32;
+  const int64_t b0 = (int64_t)blockIdx.y * 128;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const int64_t a = b0 + warp + 8 * j;
+    rs[lane * kPiPitch + warp + 8 * j] = (q0 + lane < NQ && a < nov) ? __ldg(R + q0 + lane + ldR * a) : 0.0;
+  }
+  for (int i = threadIdx.x; i < kg * 128; i += 256) {
+    const int64_t a = b0 + (i & 127);
+    fs[i] = a < nov ? __ldg(fac + (i >> 7) * nov + a) : 0.0;
+  }
+  __syncthreads();
+  const int64_t plane_stride = (int64_t)NQ * pitch;
+  for (int i = warp; i < 32 * kg; i += 8) {
+    const int k = i >> 5, q = i & 31;
+    if (q0 + q >= NQ) continue;
+    const double sc = mod_pow2(expo[(int64_t)k * NQ + q0 + q]);
+    const double2* r2 = reinterpret_cast<const double2*>(rs + q * kPiPitch + 4 * lane);
+    const double2* f2 = reinterpret_cast<const double2*>(fs + k * 128 + 4 * lane);
+    const double2 ra = r2[0], rb = r2[1], fa = f2[0], fb = f2[1];
+    uint32_t lo[4], hi[4];
+    to_words((ra.x * fa.x) * sc, lo[0], hi[0]);
+    to_words((ra.y * fa.y) * sc, lo[1], hi[1]);
+    to_words((rb.x * fb.x) * sc, lo[2], hi[2]);
+    to_words((rb.y * fb.y) * sc, lo[3], hi[3]);
+    int8_t* out = planes + ((int64_t)k * kModCount * NQ + q0 + q) * pitch + b0 + 4 * lane;
+    mod_all<4>(
+        lo, hi, [&](int m, const uint32_t(&w)[1]) { *reinterpret_cast<uint32_t*>(out + m * plane_stride) = w[0]; },
+        std::make_integer_sequence<int, kModCount>());
+  }
+}
+
+// ------------------------------------------------------------------ the products
+constexpr int MG_TM = 128;   // rows of the first operand per tile (TMEM lanes): index j of C
+constexpr int MG_TN = 256;   // rows of the second operand per tile (TMEM columns): index i of C
+constexpr int MG_TK = 128;   // k bytes per stage (one 128-byte swizzle row)
+constexpr int MG_STAGES = 4;
+constexpr int MG_ABYTES = MG_TM * MG_TK;
+constexpr int MG_BBYTES = MG_TN * MG_TK;
+constexpr int MG_STAGE = MG_ABYTES + MG_BBYTES;  // 48 KB
+constexpr int MG_THREADS = 576;                  // producer, MMA issuer, 16 epilogue warps
+constexpr int MG_SMEM = MG_STAGES * MG_STAGE + 1024 + 256;
+constexpr int MG_SEG = 65536 / MG_TK;  // stages per exact int32 accumulation (|r| <= 128: 2^14 per term)
+
+// Instruction descriptor: kind::i8, A = B = signed 8-bit, D = signed 32-bit, both K-major, M x N.
+constexpr uint32_t idesc_s8_s32(int M, int N) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_s8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                       uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// Shared-memory descriptor, K-major operand, 128-byte swizzle: 8-row groups 1024 B apart.
+__device__ __forceinline__ uint64_t desc_k_sw128(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | (uint64_t)1u << 16 | (uint64_t)(1024u >> 4) << 32 | (uint64_t)1u << 46 |
+         (uint64_t)2u << 61;
+}
+
+struct MgUnit {
+  int z, m, j0, i0, ni;  // batch, modulus, first row of each operand, live columns (256 or 128)
+};
+
+__device__ __forceinline__ MgUnit mg_unit(int u, const ModGemmArgs& a) {
+  MgUnit x;
+  const int zm = u / a.ntiles, t = u - zm * a.ntiles;
+  x.z = zm / kModCount;
+  x.m = zm - x.z * kModCount;
+  int ti, tj;
+  if (a.tri) {  // ti-major: tile (ti, tj) with tj <= 2 ti + 1 (only i >= j is kept)
+    ti = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((ti + 1) * (ti + 2) <= t) ++ti;
+    while (ti * (ti + 1) > t) --ti;
+    tj = t - ti * (ti + 1);
+  } else {
+    tj = t / a.nti;
+    ti = t - tj * a.nti;
+  }
+  x.j0 = tj * MG_TM;
+  x.i0 = ti * MG_TN;
+  x.ni = MG_TN;
+  if (a.tri && tj == 2 * ti + 1) {  // the first 128 columns lie above the diagonal
+    x.i0 += MG_TM;
+    x.ni = MG_TM;
+  }
+  return x;
+}
+
+__device__ __forceinline__ bool mg_wait_count(const int* c, int target) {
+  for (uint32_t it = 0; it < (1u << 20); ++it) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(c) : "memory");
+    if (v >= target) return true;
+    __nanosleep(64);
+  }
+  return false;
+}
+
+__global__ void __launch_bounds__(MG_THREADS, 1)
+    modgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmBh, const ModGemmArgs a, const ModReduce red) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + MG_STAGES * MG_STAGE);
+  uint64_t* empty = full + MG_STAGES;
+  uint64_t* acc_full = empty + MG_STAGES;
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* drain = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < MG_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 16);
+    }
+    mbar_init(drain, 1);
+    fence_mbar_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ------------------------------------------------------------ producer
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
+      int stage = 0;
+      uint32_t phase = 0, issued = 0, issued_par = 0;
+      bool ok = true, sync_wait = true;
+      const int nmile = a.sync ? (a.nch + a.sync_every - 1) / a.sync_every : 0;
+      for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x) {
+        const MgUnit x = mg_unit(u, a);
+        const int pa = x.z * a.zplanesA + x.m, pb = x.z * a.zplanesB + x.m;
+        const int wave = (u - (int)blockIdx.x) / (int)gridDim.x;
+        const int members = min((int)gridDim.x, a.nunits - wave * (int)gridDim.x);
+        const CUtensorMap* mb = x.ni == MG_TN ? &tmB : &tmBh;
+        const uint32_t bytes = (uint32_t)(MG_TM + x.ni) * MG_TK;
+        for (int ch = 0; ch < a.nch; ++ch) {
+          if (a.sync && ch % a.sync_every == 0) {
+            const int mi = ch / a.sync_every;
+            int* row = a.sync + (int64_t)wave * nmile;
+            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(row + mi) : "memory");
+            if (sync_wait && mi >= 2) sync_wait = mg_wait_count(row + mi - 2, members);
+          }
+          if (!mbar_wait(&empty[stage], phase ^ 1u, a.err, kDevTimeoutTmaEmpty)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(&full[stage], bytes);
+          uint8_t* st = smem + stage * MG_STAGE;
+          tma_load_3d(st, &tmA, &full[stage], ch * MG_TK, x.j0, pa);
+          tma_load_3d(st + MG_ABYTES, mb, &full[stage], ch * MG_TK, x.i0, pb);
+          issued |= 1u << stage;
+          issued_par = (issued_par & ~(1u << stage)) | (phase << stage);
+          if (++stage == MG_STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      // no bulk copy may still be landing in shared memory at exit
+      for (int s = 0; s < MG_STAGES; ++s)
+        if (issued & (1u << s)) mbar_wait(&full[s], (issued_par >> s) & 1u, a.err, kDevTimeoutDrain);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // ------------------------------------------------------------ MMA issuer
+      int stage = 0, it = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x) {
+        const MgUnit x = mg_unit(u, a);
+        const uint32_t idesc = x.ni == MG_TN ? idesc_s8_s32(MG_TM, MG_TN) : idesc_s8_s32(MG_TM, MG_TM);
+        for (int c0 = 0; c0 < a.nch && ok; c0 += MG_SEG, ++it) {
+          const int b = it & 1;
+          if (!mbar_wait(&acc_empty[b], (uint32_t)((it >> 1) & 1) ^ 1u, a.err, kDevTimeoutAccEmpty)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d = tmem_base + (uint32_t)(b * MG_TN);
+          const int c1 = min(a.nch, c0 + MG_SEG);
+          for (int ch = c0; ch < c1; ++ch) {
+            if (!mbar_wait(&full[stage], phase, a.err, kDevTimeoutTmaFull)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(smem + stage * MG_STAGE), sb = sa + MG_ABYTES;
+#pragma unroll
+            for (int kk = 0; kk < MG_TK / 32; ++kk)
+              mma_s8(d, desc_k_sw128(sa + kk * 32), desc_k_sw128(sb + kk * 32), idesc,
+                     (ch > c0 || kk > 0) ? 1u : 0u);
+            tc_commit(&empty[stage]);
+            if (++stage == MG_STAGES) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+          if (!ok) break;
+          tc_commit(&acc_full[b]);
+        }
+      }
+      // every issued MMA must complete before TMEM is freed
+      tc_commit(drain);
+      mbar_wait(drain, 0, a.err, kDevTimeoutDrain);
+    }
+  } else {
+    // -------------------------------------------------------------- epilogue
+    // warp w: TMEM lanes 32 (w mod 4) .., accumulator columns 64 ((w - 2) / 4) .. + 63.  Residues
+    // r = acc mod p in [0, p], four to a word; a segment adds the previous segments' residue.
+    const int quarter = warp & 3;
+    const int col0 = ((warp - 2) >> 2) * 64;
+    int it = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x) {
+      const MgUnit x = mg_unit(u, a);
+      const int p = red.p[x.m];
+      const int mg = red.magic[x.m];
+      uint32_t w[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w[i] = 0;
+      for (int c0 = 0; c0 < a.nch; c0 += MG_SEG, ++it) {
+        const int b = it & 1;
+        if (!mbar_wait(&acc_full[b], (uint32_t)((it >> 1) & 1), a.err, kDevTimeoutAccFull)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (col0 < x.ni) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            float v[32];
+            tmem_ld_32x32b_x32(
+                tmem_base + (uint32_t)(b * MG_TN + col0 + half * 32) + ((uint32_t)(quarter * 32) << 16), v);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+              uint32_t r[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int acc = __float_as_int(v[4 * t + e]) + (int)((w[half * 8 + t] >> (8 * e)) & 255u);
+                r[e] = (uint32_t)(acc - (__mulhi(acc, mg) >> 6) * p);
+              }
+              w[half * 8 + t] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[b]);
+      }
+      if (!ok) break;
+      const int j = x.j0 + quarter * 32 + lane;
+      if (col0 < x.ni && j < a.rowsA) {
+        uint4* dst = reinterpret_cast<uint4*>(a.out + ((int64_t)x.z * kModCount + x.m) * a.out_plane +
+                                              (int64_t)j * a.ldo + x.i0 + col0);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) dst[t] = make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// ------------------------------------------------------------------ C from its residues
+// Lower triangles Pi_z(i, j), i >= j (column-major, ld NQ): four consecutive i per thread.
+__global__ void __launch_bounds__(256) mod_crt_lower_kernel(const uint8_t* __restrict__ res, int64_t plane,
+                                                            int64_t ldo, const ModCrt crt,
+                                                            const int* __restrict__ expo, int n,
+                                                            double* __restrict__ C, int64_t ldc, int64_t strideC) {
+  const int z = blockIdx.z, j = blockIdx.y;
+  const int i0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i0 + 3 < j || i0 >= n) return;
+  const uint8_t* src = res + (int64_t)z * kModCount * plane + (int64_t)j * ldo + i0;
+  double c[4];
+  mod_crt4(src, plane, crt, c);
+  const double sj = mod_pow2(-expo[(int64_t)z * n + j]);
+  double* dst = C + (int64_t)z * strideC + (int64_t)j * ldc;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    if (i >= j && i < n) dst[i] = c[e] * mod_pow2(-expo[(int64_t)z * n + i]) * sj;
+  }
+}
+
+// C(i, j) = alpha * (...) + beta C(i, j), column-major: four consecutive i per thread
+__global__ void __launch_bounds__(256) mod_crt_full_kernel(const uint8_t* __restrict__ res, int64_t plane, int64_t ldo,
+                                                           const ModCrt crt, const int* __restrict__ expo_i,
+                                                           const int* __restrict__ expo_j, int ni, int64_t nj,
+                                                           double* __restrict__ C, int64_t ldc, double alpha,
+                                                           double beta) {
+  const int i0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int64_t j = (int64_t)blockIdx.y + (int64_t)blockIdx.z * gridDim.y;
+  if (i0 >= ni || j >= nj) return;
+  double c[4];
+  mod_crt4(res + j * ldo + i0, plane, crt, c);
+  const double sj = alpha * mod_pow2(-expo_j[j]);
+  double* dst = C + j * ldc;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    if (i < ni) {
+      const double v = c[e] * mod_pow2(-expo_i[i]) * sj;
+      dst[i] = beta == 0.0 ? v : fma(beta, dst[i], v);
+    }
+  }
+}
+
+// Adjoint accumulation from the residues of M_k R, M_k = (1 + Pi_k)^-1 - 1 (grad_accum_kernel without
+// its Y_k): one warp per column ai, four consecutive q per lane.
+__global__ void __launch_bounds__(256) mod_grad_kernel(const double* __restrict__ R, int64_t ldR,
+                                                       const uint8_t* __restrict__ res, int64_t plane, int64_t ldo,
+                                                       const ModCrt crt, const int* __restrict__ expo_m,
+                                                       const int* __restrict__ expo_r, int NQ, int64_t nov,
+                                                       const double* __restrict__ D, const GradGroup gg,
+                                                       double* __restrict__ dR, int64_t lddR, double* __restrict__ dD,
+                                                       int first) {
+  const int64_t a = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (a >= nov) return;
+  const double d = D[a];
+  const double sr = mod_pow2(-expo_r[a]);
+  // lane k holds the two factors of frequency k
+  double cf = 0.0, df = 0.0;
+  if (lane < gg.n) {
+    const double den = fma(d, d, gg.u2[lane]);
+    cf = 2.0 * gg.alpha * gg.f[lane] * d / den * sr;
+    df = gg.alpha * gg.f[lane] * (gg.u2[lane] - d * d) / (den * den) * sr;
+  }
+  double dot = 0.0;
+  for (int qb = 0; qb < NQ; qb += 128) {  // every lane takes every step: the shuffles need the whole warp
+    const int q0 = qb + 4 * lane;
+    double r[4], g[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      r[e] = q0 + e < NQ ? R[q0 + e + ldR * a] : 0.0;
+      g[e] = first || q0 + e >= NQ ? 0.0 : dR[q0 + e + lddR * a];
+    }
+    for (int k = 0; k < gg.n; ++k) {
+      const double cfac = __shfl_sync(0xffffffffu, cf, k), dfac = __shfl_sync(0xffffffffu, df, k);
+      if (q0 >= NQ) continue;
+      double c[4];
+      mod_crt4(res + (int64_t)k * kModCount * plane + a * ldo + q0, plane, crt, c);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (q0 + e >= NQ) continue;
+        const double m = c[e] * mod_pow2(-expo_m[(int64_t)k * NQ + q0 + e]);
+        g[e] = fma(cfac, m, g[e]);
+        dot = fma(dfac * r[e], m, dot);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (q0 + e < NQ) dR[q0 + e + lddR * a] = g[e];
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, off);
+  if (lane == 0) dD[a] = (first ? 0.0 : dD[a]) + dot;
+}
+}  // namespace
+
+// ------------------------------------------------------------------ host side
+namespace {
+typedef unsigned __int128 u128;
+
+struct ModTables {
+  ModReduce red;
+  ModCrt crt;
+  ModTables() {
+    u128 P = 1;
+    for (int i = 0; i < kModCount; ++i) P *= kModuli[i];
+    int bits = 0;
+    for (u128 t = P; t; t >>= 1) ++bits;
+    const int L = bits - 41;  // high parts hold 41 bits, so that sum_i 255 hi_i stays below 2^53
+    const u128 low = ((u128)1 << L) - 1;
+    auto dbl = [](u128 x) { return (double)(uint64_t)(x >> 64) * 18446744073709551616.0 + (double)(uint64_t)x; };
+    for (int i = 0; i < kModCount; ++i) {
+      const uint32_t p = kModuli[i];
+      red.p[i] = (int)p;
+      red.magic[i] = (int)((1ull << 38) / p + (p == 256 ? 0 : 1));
+      const u128 Pi = P / p;
+      const uint32_t r = (uint32_t)(Pi % p);
+      uint32_t inv = 1;
+      while ((r * inv) % p != 1) ++inv;
+      const u128 W = Pi * inv;  // < P, = 1 mod p, = 0 mod the others
+      crt.whi[i] = dbl(W >> L << L);
+      crt.wlo[i] = dbl(W & low);
+    }
+    crt.phi = dbl(P >> L << L);
+    crt.plo = dbl(P & low);
+    crt.rp = 1.0 / dbl(P);
+  }
+};
+const ModTables& tables() {
+  static const ModTables t;
+  return t;
+}
+}  // namespace
+
+const ModCrt& mod_crt_tables() { return tables().crt; }
+
+cudaError_t mod_map(PFN_cuTensorMapEncodeTiled_v12000 encode, CUtensorMap* m, void* planes, int64_t K, int64_t rows,
+                    int64_t nplanes, int64_t pitch, int box_rows) {
+  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)nplanes};
+  cuuint64_t strides[2] = {(cuuint64_t)pitch, (cuuint64_t)(pitch * rows)};
+  cuuint32_t box[3] = {MG_TK, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, planes, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? cudaSuccess
+             : cudaErrorInvalidValue;
+}
+
+cudaError_t launch_mod_cols(const double* S, int64_t ld, int64_t strideS, int K, int64_t rows, int batch,
+                            int8_t* planes, int* expo, cudaStream_t stream, double shift) {
+  if (rows <= 0 || batch <= 0) return cudaSuccess;
+  const int64_t pitch = mod_pitch(K), plane = pitch * rows;
+  mod_cols_kernel<<<dim3((unsigned)((rows + 7) / 8), (unsigned)batch), 256, 0, stream>>>(
+      S, ld, strideS, K, rows, planes, pitch, plane, plane * kModCount, expo, shift);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, const double* D, const FreqGroup& fg,
+                          double alpha, double* fac, double* part, int nsplit, int* expo, int8_t* planes,
+                          cudaStream_t stream) {
+  const int64_t pitch = mod_pitch(nov);
+  mod_chi_kernel<<<(unsigned)((nov + 255) / 256), 256, 0, stream>>>(D, nov, fg, alpha, fac);
+  const int64_t per = (nov + nsplit - 1) / nsplit;
+  mod_pi_norm_kernel<<<dim3((unsigned)((NQ + 31) / 32), (unsigned)nsplit), 256, 0, stream>>>(R, ldR, NQ, nov, fac,
+                                                                                           fg.n, per, part);
+  const int64_t n = (int64_t)fg.n * NQ;
+  mod_pi_expo_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(part, nsplit, n, expo);
+  const cudaError_t e = cudaFuncSetAttribute(mod_pi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModPiSmem);
+  if (e != cudaSuccess) return e;
+  mod_pi_kernel<<<dim3((unsigned)((NQ + 31) / 32), (unsigned)((pitch + 127) / 128)), 256, kModPiSmem, stream>>>(
+      R, ldR, NQ, nov, fac, fg.n, expo, planes, pitch);
+  g_launches += 4;
+  return cudaGetLastError();
+}
+
+int64_t mod_sync_words(const ModGemmArgs& a, int num_sms) {
+  if (a.sync_every <= 0) return 0;
+  const int grid = std::min(a.nunits, num_sms);
+  return grid <= 0 ? 0 : (int64_t)((a.nunits + grid - 1) / grid) * ((a.nch + a.sync_every - 1) / a.sync_every);
+}
+
+cudaError_t mod_plan(ModGemmArgs& a, int rowsA, int rowsB, int64_t K, int nz, bool tri) {
+  a.rowsA = rowsA;
+  a.nch = (int)((K + MG_TK - 1) / MG_TK);
+  a.tri = tri ? 1 : 0;
+  a.nti = (rowsB + MG_TN - 1) / MG_TN;
+  const int ntj = (rowsA + MG_TM - 1) / MG_TM;
+  int64_t tiles = (int64_t)a.nti * ntj;
+  if (tri) {  // tiles (ti, tj <= min(2 ti + 1, ntj - 1)): the enumeration is ti-major, so the cut is at its end
+    tiles = (int64_t)a.nti * (a.nti + 1) - (2 * a.nti > ntj ? 1 : 0);
+  }
+  const int64_t units = tiles * kModCount * nz;
+  if (units > INT32_MAX) return cudaErrorInvalidValue;
+  a.ntiles = (int)tiles;
+  a.nunits = (int)units;
+  return cudaSuccess;
+}
+
+cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmBh,
+                           const ModGemmArgs& a, int num_sms, cudaStream_t stream) {
+  if (a.nunits <= 0) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(modgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM);
+  if (e != cudaSuccess) return e;
+  modgemm_kernel<<<std::min(a.nunits, num_sms), MG_THREADS, MG_SMEM, stream>>>(tmA, tmB, tmBh, a, tables().red);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_crt_lower(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo, int n, int batch,
+                                 double* C, int64_t ldc, int64_t strideC, cudaStream_t stream) {
+  mod_crt_lower_kernel<<<dim3((unsigned)((n + 1023) / 1024), (unsigned)n, (unsigned)batch), 256, 0, stream>>>(
+      res, plane, ldo, tables().crt, expo, n, C, ldc, strideC);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_crt_full(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo_i, const int* expo_j,
+                                int ni, int64_t nj, double* C, int64_t ldc, double alpha, double beta,
+                                cudaStream_t stream) {
+  if (ni <= 0 || nj <= 0) return cudaSuccess;
+  const int64_t gy = std::min<int64_t>(nj, 32768);
+  mod_crt_full_kernel<<<dim3((unsigned)((ni + 1023) / 1024), (unsigned)gy, (unsigned)((nj + gy - 1) / gy)), 256, 0,
+                        stream>>>(res, plane, ldo, tables().crt, expo_i, expo_j, ni, nj, C, ldc, alpha, beta);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_grad(const double* R, int64_t ldR, const uint8_t* res, int64_t plane, int64_t ldo,
+                            const int* expo_m, const int* expo_r, int NQ, int64_t nov, const double* D,
+                            const GradGroup& gg, double* dR, int64_t lddR, double* dD, bool first,
+                            cudaStream_t stream) {
+  mod_grad_kernel<<<(unsigned)((nov + 7) / 8), 256, 0, stream>>>(R, ldR, res, plane, ldo, tables().crt, expo_m, expo_r,
+                                                                 NQ, nov, D, gg, dR, lddR, dD, first ? 1 : 0);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
+}  // namespace rpa

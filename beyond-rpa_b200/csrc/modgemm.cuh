@@ -1,0 +1,108 @@
+// Residue-arithmetic products on the int8 tensor cores (modgemm.cu): moduli, scaling and the
+// Chinese-remainder step shared by the kernels that read residues.
+#pragma once
+#include "kernels.h"
+
+namespace rpa {
+
+// Fifteen pairwise coprime moduli (256 = 2^8, 255 = 3 5 17, 253 = 11 23, 247 = 13 19, 217 = 7 31,
+// the others prime): P = 2^117.8.
+constexpr int kModCount = 15;
+constexpr uint32_t kModuli[kModCount] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+
+// Rows are scaled to 2-norms in [2^57, 2^58): the product of two, < 2^116, stays well below P / 2
+// (the rounding of at most 2^20 entries adds less than 2^10 to a norm).
+constexpr int kModNormBits = 58;
+
+// Chinese remainder weights split in two doubles: the high parts (41 bits) add up exactly.
+struct ModCrt {
+  double whi[kModCount], wlo[kModCount];
+  double phi, plo, rp;  // P = phi + plo, 1 / P
+};
+struct ModReduce {
+  int p[kModCount];
+  int magic[kModCount];  // ceil(2^38 / p): (acc * magic) >> 38 = floor(acc / p) for |acc| <= 2^30 + 255
+};
+
+// Power of two (exponent) that brings a row of squared norm s2 to a norm in [2^57, 2^58).  A zero
+// row keeps 0; a norm that overflows returns a marker for which mod_pow2 is NaN, so the products
+// of such a row are NaN (as the FP64 sums would be non-finite).
+constexpr int kModNaNExpo = 1 << 20;
+__host__ __device__ __forceinline__ int mod_exponent(double s2) {
+  if (!(s2 > 0.0)) return s2 == 0.0 ? 0 : kModNaNExpo;
+  if (s2 > 1.7e308) return kModNaNExpo;
+  int e;
+  frexp(sqrt(s2) * (1.0 + 1e-9), &e);  // norm < 2^e
+  return kModNormBits - e;
+}
+__device__ __forceinline__ double mod_pow2(int e) {
+  if (e > 1000 || e < -1000) return __longlong_as_double(0x7FF8000000000000ll);
+  return __longlong_as_double((long long)(1023 + e) << 52);
+}
+
+// Integers from four neighbouring columns of residues (one byte each, planes apart), as doubles
+// rounded once: sum_i r_i W_i mod P in (-P/2, P/2).
+__device__ __forceinline__ void mod_crt4(const uint8_t* src, int64_t plane, const ModCrt& crt, double (&c)[4]) {
+  uint32_t w[kModCount];
+#pragma unroll
+  for (int m = 0; m < kModCount; ++m) w[m] = __ldg(reinterpret_cast<const uint32_t*>(src + m * plane));
+  double hi[4] = {0.0, 0.0, 0.0, 0.0}, lo[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int m = 0; m < kModCount; ++m) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      // 2^52 + r - 2^52: a byte to a double without the slow integer conversion
+      const double r = __hiloint2double(0x43300000, (int)((w[m] >> (8 * e)) & 255u)) - 4503599627370496.0;
+      hi[e] = fma(r, crt.whi[m], hi[e]);
+      lo[e] = fma(r, crt.wlo[m], lo[e]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const double q = rint((hi[e] + lo[e]) * crt.rp);
+    c[e] = fma(-q, crt.phi, hi[e]) + fma(-q, crt.plo, lo[e]);
+  }
+}
+
+inline int64_t mod_pitch(int64_t K) { return (K + 127) / 128 * 128; }
+
+// One launch: residues of C(i, j) = sum_k a(j, k) b(i, k) for nz batches, j < rowsA (lanes),
+// i < rowsB; tri: only the tiles that hold some i >= j.
+struct ModGemmArgs {
+  int rowsA;
+  int nch;  // 128-wide k chunks
+  int nti, ntiles, nunits, tri;
+  int zplanesA, zplanesB;  // planes between batches of each operand (0: shared)
+  uint8_t* out;            // [z][modulus][j][i], i contiguous
+  int64_t out_plane, ldo;  // bytes between planes; between j (a multiple of 256)
+  int* sync;               // optional wave milestones (zeroed, mod_sync_words ints)
+  int sync_every;
+  int* err;
+};
+
+const ModCrt& mod_crt_tables();
+cudaError_t mod_map(PFN_cuTensorMapEncodeTiled_v12000 encode, CUtensorMap* m, void* planes, int64_t K, int64_t rows,
+                    int64_t nplanes, int64_t pitch, int box_rows);
+// Residue planes [z][modulus][row][pitch] of the columns of S - shift * 1 (S: K x rows, column-major,
+// strideS apart).
+cudaError_t launch_mod_cols(const double* S, int64_t ld, int64_t strideS, int K, int64_t rows, int batch,
+                            int8_t* planes, int* expo, cudaStream_t stream, double shift = 0.0);
+// Residue planes [k][modulus][Q][pitch] of X_k; fac: fg.n * nov doubles, part: nsplit * fg.n * NQ.
+cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, const double* D, const FreqGroup& fg,
+                          double alpha, double* fac, double* part, int nsplit, int* expo, int8_t* planes,
+                          cudaStream_t stream);
+cudaError_t mod_plan(ModGemmArgs& a, int rowsA, int rowsB, int64_t K, int nz, bool tri);
+int64_t mod_sync_words(const ModGemmArgs& a, int num_sms);
+cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmBh,
+                           const ModGemmArgs& a, int num_sms, cudaStream_t stream);
+cudaError_t launch_mod_crt_lower(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo, int n, int batch,
+                                 double* C, int64_t ldc, int64_t strideC, cudaStream_t stream);
+cudaError_t launch_mod_crt_full(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo_i, const int* expo_j,
+                                int ni, int64_t nj, double* C, int64_t ldc, double alpha, double beta,
+                                cudaStream_t stream);
+// Adjoint accumulation (launch_grad_accum) from the residues of M_k R: [k][modulus][ai][q].
+cudaError_t launch_mod_grad(const double* R, int64_t ldR, const uint8_t* res, int64_t plane, int64_t ldo,
+                            const int* expo_m, const int* expo_r, int NQ, int64_t nov, const double* D,
+                            const GradGroup& gg, double* dR, int64_t lddR, double* dD, bool first,
+                            cudaStream_t stream);
+}  // namespace rpa
