@@ -284,6 +284,10 @@ cudaError_t launch_trsm_lower_left(const double* L, int64_t ldl, int64_t sL, dou
 // Batched backward substitution L_b^T X_b = B_b in place (L lower, column-major).
 cudaError_t launch_trsm_lower_trans_left(const double* L, int64_t ldl, int64_t sL, double* X, int64_t ldx,
                                          int64_t sX, int n, int ncols, int batch, cudaStream_t stream);
+// V_b = L_b^-1 (lower; the upper triangles zeroed), L_b as launch_cholesky_lower leaves it: the strict
+// upper triangles of its kCholNB-column diagonal blocks hold the transposed block inverses.
+cudaError_t launch_tri_inverse(const double* L, int64_t ldl, int64_t sL, double* V, int64_t ldv, int64_t sV, int n,
+                               int batch, cudaStream_t stream);
 // Adjoint of E_c for a group of <= 16 frequencies (f_k = w_k / 2pi).
 struct GradGroup {
   int n;

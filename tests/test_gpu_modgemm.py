@@ -1,4 +1,5 @@
-"""Residue products on the int8 tensor cores (modgemm.cu): the FP64 form of Pi(u) at the edges of their 128 x 256 tiles, 128-wide K chunks and frequency groups.
+"""Residue products on the int8 tensor cores (modgemm.cu): the FP64 form of Pi(u) and the adjoint's
+back-contraction, at the edges of their 128 x 256 tiles, 128-wide K chunks and frequency groups.
 
 Tolerances.  Operand rows are rounded to 2^-58 of their 2-norm, so an entry of Pi is off by at most
   0.5 sqrt(nov) 2^-57 2 ||X_Q|| ||X_P||  (rounding)  +  2^-53 |Pi_QP|  (one rounding of the result)
@@ -72,3 +73,27 @@ def test_pi_fp64_padded_columns_and_small_workspace(handle, pkg):
         h.set_workspace_limit(4 * 300 * 300 * 8 + 300 * 280 * 8 + (1 << 20))
         capped = h.pi_u(R, s.eps_o, s.eps_v, x, prec="fp64")
     assert np.max(np.abs(capped - ref) / norms(ref)) < 280 * 2.0 ** -53  # 280 sequential FP64 additions
+
+
+@pytest.mark.parametrize("nq,no,nv,k", [(127, 2, 64, 2), (128, 2, 64, 2), (193, 4, 33, 3), (257, 5, 77, 17), (321, 3, 64, 5)])
+def test_gradient_fp64(handle, nq, no, nv, k):
+    # dE/dR and dE/de against the FP64 oracle: 1 + Pi has eigenvalues in [1, 1.8], so inverse and
+    # products lose a few roundings of sqrt(NQ) terms; 1e-13 of the largest entry bounds both sides
+    s = O.make_system(nq, no, nv, nq + k, decay=nq / 8.0, lam0=0.8)
+    x, w = O.casimir_polder(k, 0.8)
+    ref = O.ec_grad(s.R, s.eps_o, s.eps_v, x, w)
+    ec, dR, dO, dV = handle.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")
+    for a, b in zip((dR, dO, dV), ref):
+        assert np.max(np.abs(a - b)) < 1e-13 * np.max(np.abs(b))
+
+
+def test_gradient_without_room_for_planes(pkg):
+    # a cap that holds the triangular solves' buffers but not the residue planes
+    s = O.make_system(160, 4, 60, 5, decay=20.0, lam0=0.8)
+    x, w = O.casimir_polder(3, 0.8)
+    ref = O.ec_grad(s.R, s.eps_o, s.eps_v, x, w)
+    with pkg.Handle(0) as h:
+        h.set_workspace_limit(3 << 20)
+        _, dR, dO, dV = h.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")
+    for a, b in zip((dR, dO, dV), ref):
+        assert np.max(np.abs(a - b)) < 1e-13 * np.max(np.abs(b))
