@@ -20,115 +20,199 @@ namespace {
 constexpr int NB = kCholNB;  // Cholesky block size (64)
 constexpr int NB2 = 256;     // outer block of the two-level schedule
 
-// Factor the NB x NB diagonal block of each matrix (blockDim = 256): thread (r, q) = (t / 4,
-// t % 4) keeps columns 16q .. 16q+15 of row r in registers; the column loop is unrolled by 16, so
-// every register index is static.  Step j (one barrier): every thread forms the pivot d_j itself
-// from what step j-1 published (the diagonal entry a_jj and l_{j,j-1}: d_j = a_jj - l_{j,j-1}^2,
-// the same FMA the entry's owner applies), and the owners of column j publish the whole column,
-// l_rj = a_rj / sqrt(d_j) below the pivot and zeros on and above it (double-buffered); every thread
-// then subtracts l_rj l_cj from all 16 of its entries without a branch: the zeros leave the
-// finished columns and the rows above the pivot unchanged, and entries above the diagonal (never
-// stored) take whatever they get.  A block smaller than NB (the last of a matrix) is padded with
-// the identity.  A non-positive or NaN pivot is replaced by 1 so that the factorization finishes,
-// and reported.
+// Factor the 64 x 64 diagonal block of each matrix and form the inverse W of its factor, one CTA of
+// four warps per matrix.  The block is a chain of 64 dependent pivots, so what counts is the latency
+// of one column and the size of the code: a loop over eight panels of eight columns.
+//  * warp 0 factors a panel, rows lane and lane + 32 in registers: a column costs a shuffle of the
+//    pivot, its reciprocal and one dependent FP64 operation, and no barrier;
+//  * the panel's products are subtracted from the rest of the block in 8 x 8 tiles on DMMA m8n8k4:
+//    warp 0 takes the next panel's columns and goes on to factor them, the other warps the rest;
+//  * W: the 8 x 8 diagonal blocks by substitution (64 threads), then W21 = -W22 (L21 W11) for blocks
+//    of 8, 16 and 32 on DMMA.
+// Per 64-column block on B200: 17.7 us (12 matrices) against 33.6 us for 256 threads with a CTA barrier per
+// column.  One warp with 32 columns in registers (a fully unrolled 64 KB of code) spent its time
+// fetching instructions: 25.7 us.
 //
-// The inverse W = L^-1 of the block is then formed by columns, right-looking: thread (c, q) holds
-// rows 16q .. 16q+15 of column c of W, the owner of row k scales it by 1 / L_kk and hands it to the
-// column's other three threads by a shuffle.  W is stored transposed in the block's strict upper
-// triangle, which the lower factorization never reads: W(k, c) at (c, k) for k > c.  The panel
-// solve below reads it there; the diagonal of W, 1 / L_cc, it recomputes from the pivots.
-constexpr int kPotrfThreads = 256;
-constexpr int kLP = NB + 4;  // skewed pitch: index m at m + m / 16, so the four column blocks of a
-                             // warp's rows fall in different banks
-__device__ __forceinline__ int sk(int m) { return m + (m >> 4); }
+// A block smaller than 64 (the last of a matrix) is padded with the identity.  A non-positive or NaN
+// pivot is replaced by 1 so that the factorization finishes, and reported.  W is stored transposed
+// in the block's strict upper triangle, which the lower factorization never reads: W(k, c) at (c, k)
+// for k > c.  The panel solve below reads it there; the diagonal of W, 1 / L_cc, it recomputes.
+constexpr int kPotrfThreads = 128;
+constexpr int kPC = 8;       // panel columns
+constexpr int kLP = NB + 4;  // column pitch of both arrays, [c][r]: DMMA fragment loads without conflicts
+constexpr size_t kPotrfSmem = sizeof(double) * (2 * NB * kLP + NB);
+
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// 1 / d and 1 / sqrt(d) to about an ulp.  The hardware estimates (error 2^-20 or better) take one
+// third-order Newton step each: with e = 1 - d r, 1 / d = r (1 + e + e^2 + ...); with e = 1 - d y^2,
+// 1 / sqrt(d) = y (1 + e / 2 + 3 e^2 / 8 + ...), the rest of both series being below 2^-60.  Only the
+// reciprocal is on the chain of pivots.  Pivots near the ends of the exponent range take the library
+// functions; one that is not positive counts as 1 and is reported.
+__device__ __forceinline__ void pivot_inverses(double& d, double& rd, double& ri, bool& bad) {
+  if (!(d > 1e-290 && d < 1e290)) {
+    if (!(d > 0.0)) {
+      bad = true;
+      d = 1.0;
+    }
+    rd = 1.0 / d;
+    ri = rsqrt(d);
+    return;
+  }
+  double r, y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  rd = fma(r * e, 1.0 + e, r);
+  const double g = fma(-d * y, y, 1.0);
+  ri = fma(y * g, fma(g, 0.375, 0.5), y);
+}
+
+// One warp: columns 8 p .. 8 p + 7 of the block at S ([c][r]), already updated by the panels before.
+__device__ __forceinline__ void factor_panel(double* S, double* inv, int p, bool& bad) {
+  const int lane = threadIdx.x & 31;
+  const bool low = p < NB / 2 / kPC;  // the pivot rows are rows `lane` (else rows lane + 32)
+  double* col = S + p * kPC * kLP + lane;
+  double x0[kPC], x1[kPC];
+#pragma unroll
+  for (int c = 0; c < kPC; ++c) {
+    x0[c] = col[c * kLP];
+    x1[c] = col[c * kLP + 32];
+  }
+  double v = low ? x0[0] : x1[0];
+#pragma unroll
+  for (int j = 0; j < kPC; ++j) {
+    const int row = p * kPC + j;
+    double d = __shfl_sync(0xffffffffu, v, row & 31), rd, ri;
+    const double xp = low ? x0[j] : x1[j];
+    pivot_inverses(d, rd, ri, bad);
+    // the next pivot, in its lane: a - x^2 / d
+    if (j + 1 < kPC) v = fma(-(xp * xp), rd, low ? x0[j + 1] : x1[j + 1]);
+    const double l0 = lane > row ? x0[j] * ri : 0.0, l1 = lane + 32 > row ? x1[j] * ri : 0.0;
+    const double lp = low ? l0 : l1;
+    col[j * kLP] = lane == row ? d * ri : l0;
+    col[j * kLP + 32] = lane + 32 == row ? d * ri : l1;
+    if (lane == 0) inv[row] = ri;
+#pragma unroll
+    for (int c = j + 1; c < kPC; ++c) {
+      const double lc = __shfl_sync(0xffffffffu, lp, (p * kPC + c) & 31);
+      x0[c] = fma(-l0, lc, x0[c]);
+      x1[c] = fma(-l1, lc, x1[c]);
+    }
+  }
+}
+
+// Row of 8 x 8 tiles at r0, tile columns c0, c0 + 8, ... (count of them): subtract the products of the
+// panel at P (columns of the same rows), one warp, four tiles in flight.
+__device__ __forceinline__ void update_tiles(double* S, const double* P, int r0, int c0, int rstep, int cstep,
+                                             int count) {
+  const int lane = threadIdx.x & 31, fr = lane >> 2, fk = lane & 3;
+  for (int q0 = 0; q0 < count; q0 += 4) {
+    double acc[4][2], af[4][2], bf[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (q0 + u >= count) continue;
+      const int r = r0 + (q0 + u) * rstep, c = c0 + (q0 + u) * cstep;
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        acc[u][v] = S[(c + 2 * fk + v) * kLP + r + fr];
+        af[u][v] = -P[(4 * v + fk) * kLP + r + fr];
+        bf[u][v] = P[(4 * v + fk) * kLP + c + fr];
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (q0 + u < count) dmma(acc[u][0], acc[u][1], af[u][v], bf[u][v]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (q0 + u >= count) continue;
+      double* C = S + (c0 + (q0 + u) * cstep + 2 * fk) * kLP + r0 + (q0 + u) * rstep + fr;
+      C[0] = acc[u][0];
+      C[kLP] = acc[u][1];
+    }
+  }
+}
 
 __device__ __forceinline__ void potrf_diag_body(double* Az, int64_t ld, int n, int j0, double* Ldz, int* err) {
-  __shared__ double col[2][kLP];
-  __shared__ double dnx[2];
-  __shared__ double LsT[NB][kLP];  // LsT[c][sk(r)] = L(r, c) below the diagonal, 0 elsewhere
-  __shared__ double inv[NB];
+  extern __shared__ __align__(16) double potrf_smem[];
+  double* S = potrf_smem;        // the block, then L; S(r, c) at S[c * kLP + r]
+  double* W = S + NB * kLP;      // L^-1, the same layout
+  double* inv = W + NB * kLP;    // 1 / L_rr
   const int nbe = min(NB, n - j0);
-  const int t = threadIdx.x;
-  const int r = t >> 2, q = t & 3;
-  double v[16];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int fr = lane >> 2, fk = lane & 3;  // fragment row (or column) and k of this lane
+  double* Ab = Az + j0 + ld * (int64_t)j0;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int c = 16 * q + i;
-    v[i] = (c <= r && r < nbe) ? Az[(int64_t)(j0 + r) + ld * (int64_t)(j0 + c)] : (c == r ? 1.0 : 0.0);
+  for (int i = 0; i < NB * NB / kPotrfThreads; ++i) {
+    const int r = t & (NB - 1), c = 2 * i + (t >> 6);
+    S[c * kLP + r] = (c <= r && r < nbe) ? Ab[r + ld * (int64_t)c] : (c == r ? 1.0 : 0.0);
   }
-  if (t == 0) dnx[1] = v[0];
   __syncthreads();
-  double dj = dnx[1];  // pivot of column 0
-  double piv = 1.0;
   bool bad = false;
-  for (int g = 0; g < 4; ++g) {
-#pragma unroll
-    for (int jj = 0; jj < 16; ++jj) {
-      const int j = 16 * g + jj;
-      const int buf = jj & 1;
-      double d = dj;
-      if (!(d > 0.0)) {  // the same value in every thread
-        bad = true;
-        d = 1.0;
-      }
-      // one reciprocal square root (1 ulp) instead of a square root and a division: the pivot
-      // chain is the kernel's critical path
-      const double ri = rsqrt(d);
-      if (q == g) {
-        double l = 0.0;
-        if (r == j) {
-          v[jj] = d * ri;
-          piv = v[jj];
-        } else if (r > j) {
-          v[jj] *= ri;
-          l = v[jj];
-        }
-        col[buf][sk(r)] = l;
-      }
-      if (r == j + 1 && q == ((j + 1) >> 4)) dnx[buf] = v[(jj + 1) & 15];
-      __syncthreads();
-      if (j + 1 < NB) {
-        const double l1 = col[buf][sk(j + 1)];
-        dj = fma(-l1, l1, dnx[buf]);
-      }
-      const double lr = col[buf][sk(r)];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = fma(-lr, col[buf][sk(16 * q + i)], v[i]);
+#pragma unroll 1
+  for (int p = 0; p < NB / kPC; ++p) {
+    // panel p - 1 is final.  Warp 0 updates panel p and factors it, the other warps update the columns
+    // right of it, row by row of tiles.
+    const double* P = S + (p - 1) * kPC * kLP;
+    const int first = p * kPC, nt = NB / kPC - p;
+    if (warp == 0) {
+      if (p > 0) update_tiles(S, P, first, first, 8, 0, nt);
+      __syncwarp();
+      factor_panel(S, inv, p, bad);
+    } else if (p > 0) {
+      for (int ti = nt - warp; ti >= 1; ti -= 3) update_tiles(S, P, first + 8 * ti, first + 8, 0, 8, ti);
     }
+    __syncthreads();
   }
   if (bad && t == 0) atomicCAS(err, 0, (int)kDevNotSPD);
+  if (t < NB) {  // column t & 7 of the inverse of diagonal block t >> 3, right-looking
+    const int b0 = t & ~7, c = t & 7;
+    double s[8];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int c = 16 * q + i;
-    LsT[c][sk(r)] = c < r ? v[i] : 0.0;
-    if (c <= r && r < nbe) Az[(int64_t)(j0 + r) + ld * (int64_t)(j0 + c)] = v[i];
-  }
-  if (q == (r >> 4)) {  // the owner of the diagonal entry
-    inv[r] = 1.0 / piv;
-    if (r < nbe) Ldz[j0 + r] = piv;
-  }
-  __syncthreads();
-  // column c = r of W: s[i] = W(16q + i, c), zero above the diagonal
-  const int lane = t & 31;
-  double s[16];
+    for (int k = 0; k < 8; ++k) s[k] = k == c ? 1.0 : 0.0;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) s[i] = (16 * q + i == r) ? 1.0 : 0.0;
-  for (int g = 0; g < 4; ++g) {
+    for (int k = 0; k < 8; ++k) {
+      const double w = s[k] * inv[b0 + k];
+      W[t * kLP + b0 + k] = w;  // zero above the diagonal
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      const int k = 16 * g + kk;
-      double wk = s[kk] * inv[k];
-      if (q == g) s[kk] = wk;
-      wk = __shfl_sync(0xffffffffu, wk, (lane & ~3) | g);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) s[i] = fma(-LsT[k][sk(16 * q + i)], wk, s[i]);
+      for (int m = k + 1; m < 8; ++m) s[m] = fma(-S[(b0 + k) * kLP + b0 + m], w, s[m]);
     }
   }
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int m = 16 * q + i;
-    if (m > r && m < nbe) Az[(int64_t)(j0 + r) + ld * (int64_t)(j0 + m)] = s[i];
+  __syncthreads();
+#pragma unroll 1
+  for (int h = 8; h < NB; h *= 2) {
+    const int th = h / 8, per = th * th;  // tiles of one h x h block
+    // T = L21 W11 of every pair of blocks, kept in the pair's (unused) upper right block of S
+#pragma unroll 1
+    for (int stage = 0; stage < 2; ++stage) {
+      for (int q = warp; q < NB / (2 * h) * per; q += 4) {
+        const int base = q / per * 2 * h, u = q % per, r0 = u / th * 8, c0 = u % th * 8;
+        // stage 0: A = L21, B = W11; stage 1: A = W22, B = T
+        const double* A = stage ? W + (base + h) * kLP + base + h : S + base * kLP + base + h;
+        const double* B = stage ? S + (base + h) * kLP + base : W + base * kLP + base;
+        double a0 = 0.0, a1 = 0.0;
+        // W11(k, c) = 0 for k < c and W22(r, k) = 0 for k > r (their blocks there are not stored)
+        for (int k = stage ? 0 : c0; k < (stage ? r0 + 8 : h); k += 4) dmma(a0, a1, A[(k + fk) * kLP + r0 + fr], B[(c0 + fr) * kLP + k + fk]);
+        double* C = stage ? W + (base + c0 + 2 * fk) * kLP + base + h + r0 + fr
+                          : S + (base + h + c0 + 2 * fk) * kLP + base + r0 + fr;
+        C[0] = stage ? -a0 : a0;
+        C[kLP] = stage ? -a1 : a1;
+      }
+      __syncthreads();
+    }
   }
+#pragma unroll 8
+  for (int i = 0; i < NB * NB / kPotrfThreads; ++i) {
+    const int r = t & (NB - 1), c = 2 * i + (t >> 6);
+    if (r < nbe && c < nbe) Ab[r + ld * (int64_t)c] = c <= r ? S[c * kLP + r] : W[r * kLP + c];
+  }
+  if (t < nbe) Ldz[j0 + t] = S[t * kLP + t];
 }
 
 __global__ void __launch_bounds__(kPotrfThreads) potrf_diag_kernel(double* A, int64_t ld, int64_t stride, int n,
@@ -154,12 +238,6 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
                : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
 
 __device__ __forceinline__ void trsm_panel_body(double* Az, int64_t ld, int n, int j0, int rblock, const double* Ldz) {
   extern __shared__ __align__(16) double trsm_smem[];
@@ -240,10 +318,14 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_varlen_kernel(const MatDesc
   trsm_panel_body(md.A, md.ld, md.n, j0, blockIdx.x, md.Ldiag);
 }
 
-// Shared-memory opt-in of the panel solve (> 48 KB), once per process.
-cudaError_t trsm_smem_optin() {
+// Shared-memory opt-in of the panel kernels (> 48 KB), once per process.
+cudaError_t panel_smem_optin() {
   static const cudaError_t e = [] {
     cudaError_t r = cudaFuncSetAttribute(trsm_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(potrf_varlen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem);
     if (r == cudaSuccess)
       r = cudaFuncSetAttribute(trsm_varlen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem);
     return r;
@@ -501,7 +583,7 @@ cudaError_t launch_cholesky_lower(double* A, int64_t ld, int64_t stride, int n, 
   if (!valid_logdet_plan(plan)) return cudaErrorInvalidValue;
   const int nb2 = plan.nb2;
   if (oz && (oz->S == 0 || oz->K != nb2)) oz = nullptr;
-  if (cudaError_t e0 = trsm_smem_optin()) return e0;
+  if (cudaError_t e0 = panel_smem_optin()) return e0;
   int obuf = 0;  // digit-plane buffer of the current outer block (alternates: the rest of block t's
                  // update may still read its planes while block t+1 is sliced)
   LookaheadState st{la, stream};
@@ -511,7 +593,7 @@ cudaError_t launch_cholesky_lower(double* A, int64_t ld, int64_t stride, int n, 
   for (int J0 = 0; J0 < n; J0 += nb2) {
     const int J1 = min(n, J0 + nb2);
     for (int j0 = J0; j0 < J1; j0 += NB) {
-      potrf_diag_kernel<<<nmat, kPotrfThreads, 0, S>>>(A, ld, stride, n, j0, Ldiag, err);
+      potrf_diag_kernel<<<nmat, kPotrfThreads, kPotrfSmem, S>>>(A, ld, stride, n, j0, Ldiag, err);
       ++g_launches;
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
@@ -563,7 +645,7 @@ cudaError_t launch_logdet_varlen(const MatDesc* mats, int nmat, int nmax, int* e
                                  const LogdetPlan& plan, const Lookahead* la) {
   if (nmat <= 0) return cudaSuccess;
   if (!valid_logdet_plan(plan)) return cudaErrorInvalidValue;
-  if (cudaError_t e0 = trsm_smem_optin()) return e0;
+  if (cudaError_t e0 = panel_smem_optin()) return e0;
   trace_shift_varlen_kernel<<<nmat, 256, 0, stream>>>(mats);
   ++g_launches;
   cudaError_t e = cudaGetLastError();
@@ -575,7 +657,7 @@ cudaError_t launch_logdet_varlen(const MatDesc* mats, int nmat, int nmax, int* e
   for (int J0 = 0; J0 < nmax; J0 += nb2) {
     const int J1 = std::min(nmax, J0 + nb2);
     for (int j0 = J0; j0 < J1; j0 += NB) {
-      potrf_varlen_kernel<<<nmat, kPotrfThreads, 0, S>>>(mats, j0, err);
+      potrf_varlen_kernel<<<nmat, kPotrfThreads, kPotrfSmem, S>>>(mats, j0, err);
       ++g_launches;
       const int below = nmax - j0 - NB;
       if (below <= 0) break;
