@@ -2561,7 +2561,7 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   RPA_CUDA(h, ensure(h->jX, (size_t)ng * no * 8));
   RPA_CUDA(h, ensure(h->jU, (size_t)nov * nt * 8));
   const size_t nvv = (size_t)nv * nv;
-  const size_t wwords = (size_t)nt + 3 * nvv + (size_t)nq * nv + 2 * (size_t)ng * nv + (size_t)nq + (size_t)ng +
+  const size_t wwords = (size_t)nt + 3 * nvv + (size_t)nq * nv + 2 * (size_t)ng * nv + ((size_t)nq + (size_t)ng) * no +
                         2 * nvv + 4 * nvv + 2 * nvv + 2 * (size_t)ng * nv + (size_t)nslot * rpa::kDotPartials + 64;
   RPA_CUDA(h, ensure(h->jWork, wwords * 8));
   double* w = static_cast<double*>(h->jWork.p);
@@ -2572,9 +2572,9 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   double* ZYXk = Vm + nvv;         // NQ x nv
   double* ZYXg = ZYXk + (size_t)nq * nv;  // NGrid x nv
   double* Wg = ZYXg + (size_t)ng * nv;    // NGrid x nv
-  double* zk = Wg + (size_t)ng * nv;      // NQ
-  double* zg = zk + nq;                   // NGrid
-  double* Gg = zg + ng;                   // G for 2g..2j (nv x nv)
+  double* zkj = Wg + (size_t)ng * nv;     // NQ x NOcc: the pairs of one j
+  double* zgj = zkj + (size_t)nq * no;    // NGrid x NOcc
+  double* Gg = zgj + (size_t)ng * no;     // G for 2g..2j (nv x nv)
   double* Gb = Gg + nvv;                  // G for 2b..2d
   double* Sm = Gb + nvv;                  // 4 S blocks (<= nv x nv each)
   double* QS = Sm + 4 * nvv;              // nv x 2 Nkj
@@ -2741,7 +2741,7 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
                                     cudaMemcpyDeviceToDevice, h->stream));
     }
   RPA_CUDA(h, ensure(h->jQS, (size_t)nv * maxcol * 2 * 8));
-  RPA_CUDA(h, ensure(h->jSK, (size_t)64 * nvv * 8));
+  RPA_CUDA(h, ensure(h->jSK, std::max((size_t)64 * nvv, (size_t)16 * std::max(nq, ng) * no) * 8));
   RPA_CUDA(h, ensure(h->jS, (size_t)4 * no * std::max<int64_t>(max_n * max_n, 1) * 8));
   RPA_CUDA(h, ensure(h->jD, (size_t)(8 * no + 8) * sizeof(rpa::GemmF64Args) + (size_t)(8 * no + 16) * sizeof(int)));
 
@@ -2850,15 +2850,22 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
     g1.kscale = xj;
     RPA_CUDA(h, G(g1));
     RPA_CUDA(h, G(gemm_g(ng, nv, nq, Zd, ldz, false, ZYXk, nq, false, ZYXg, ng)));
+    // ZXX(k) = sum_g Z(g, k) X(g, i) X(g, j) of every pair i >= j at once, and ZXX(g) = Z ZXX(k): one
+    // product each per j (as one-column products they kept 4 of 148 SMs busy for 80 us per pair)
+    auto narrow = [&](rpa::GemmF64Args g) {
+      g.splitk = (int)std::max<int64_t>(1, std::min<int64_t>({16, g.K / 64, 600 / std::max(1, rpa::gemm_f64_tiles(g))}));
+      g.work = static_cast<double*>(h->jSK.p);
+      return G(g);
+    };
+    rpa::GemmF64Args g2 = gemm_g(nq, no - j, ng, Zd, ldz, true, xj, ldx, false, zkj, nq);
+    g2.kscale = xj;
+    RPA_CUDA(h, narrow(g2));
+    RPA_CUDA(h, narrow(gemm_g(ng, no - j, nq, Zd, ldz, false, zkj, nq, false, zgj, ng)));
     for (int i = j; i < no; ++i, ++pair) {
       pair_ij.push_back({i, j});
       const double* xi = Xd + (int64_t)ldx * i;
-      // ZXX(k) = sum_g Z(g, k) X(g, i) X(g, j), its norm for the screening, ZXX(g) = Z ZXX(k)
-      rpa::GemmF64Args g2 = gemm_g(nq, 1, ng, Zd, ldz, true, xj, ng, false, zk, nq);
-      g2.kscale = xi;
-      RPA_CUDA(h, G(g2));
+      const double *zk = zkj + (size_t)nq * (i - j), *zg = zgj + (size_t)ng * (i - j);
       RPA_CUDA(h, rpa::launch_dot_partials(zk, nq, zk, nq, nq, 1, nullptr, slot(pair, 4), h->stream));
-      RPA_CUDA(h, G(gemm_g(ng, 1, nq, Zd, ldz, false, zk, nq, false, zg, ng)));
       // S1a, S1b of the pair (i, j)
       const int nij = pn[(size_t)i + (size_t)no * j];
       if (nij > 0) {
