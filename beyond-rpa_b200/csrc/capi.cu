@@ -92,6 +92,7 @@ struct rpa_b200_handle {
   // batched (many-instance) workspace: descriptors and per-batch results
   DevBuf bDesc, bRes;
   DevBuf gY, gD, gM;  // adjoint workspace
+  DevBuf mA, mB, mC, mE;  // FP64 products by residues: planes of both operands, residues, exponents
   DevBuf xM;      // MBPT3 exchange: NT x NT matrices, R U and U X
   DevBuf eW, eA, eZ;  // symmetric eigensolver workspace, input and eigenvector buffers
   DevBuf thZ, thXa, thXi, thYX, thR;  // THC factors, Khatri-Rao block, Cholesky vectors formed from them
@@ -462,6 +463,51 @@ int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t pla
     a.sync = static_cast<int*>(h->syncBuf.p);
   }
   RPA_CUDA(h, rpa::launch_modgemm(mA, mB, mBh, a, h->num_sms, h->stream));
+  return RPA_OK;
+}
+
+// One FP64 product on the FP64 tensor pipe, or by residues where that is the faster: the pipe's
+// 28 TFLOP/s against 15 int8 products at 2.4 POP/s, the conversion of both operands (3 TB/s of
+// planes), the residues of C written and read, and the extra launches.  1.2: the estimate's margin.
+bool mod_pays(int64_t M, int64_t N, int64_t K) {
+  const double flops = 2.0 * (double)M * (double)N * (double)K;
+  return M >= 128 && N >= 128 && K >= 128 &&
+         flops * (1.0 / 28e12 - 15.0 / 2.4e15) > 1.2 * (5e-12 * (double)(M + N) * (double)K + 1e-11 * (double)M * (double)N + 25e-6);
+}
+
+int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30) {
+  const bool plain = g.batch == 1 && g.splitk <= 1 && (!g.kscale || g.b_k == 1) && !g.rowscale && (g.a_m == 1 || g.a_k == 1) &&
+                     (g.b_n == 1 || g.b_k == 1);
+  if (plain && g.K <= INT32_MAX && mod_pays(g.M, g.N, g.K)) {
+    const size_t NM = rpa::kModCount;
+    const int64_t pitch = rpa::mod_pitch(g.K), ldo = ((int64_t)g.M + 255) / 256 * 256;
+    // C is formed in blocks of columns whose planes and residues fit the budget
+    const int64_t nmax = (int64_t)(budget / (NM * (size_t)(pitch + ldo))) / 128 * 128;
+    const int64_t nb = std::min<int64_t>(g.N, nmax);
+    if (nb >= std::min<int64_t>(g.N, 128) && try_ensure(h->mA, NM * g.M * (size_t)pitch) &&
+        try_ensure(h->mB, NM * nb * (size_t)pitch) && try_ensure(h->mC, NM * nb * (size_t)ldo) &&
+        try_ensure(h->mE, ((size_t)g.M + nb) * sizeof(int))) {
+      int8_t *pa = static_cast<int8_t*>(h->mA.p), *pb = static_cast<int8_t*>(h->mB.p);
+      int *ea = static_cast<int*>(h->mE.p), *eb = ea + g.M;
+      if (g.a_k == 1) RPA_CUDA(h, rpa::launch_mod_cols(g.A, g.a_m, 0, (int)g.K, g.M, 1, pa, ea, h->stream));
+      else RPA_CUDA(h, rpa::launch_mod_rows(g.A, g.a_k, g.M, g.K, pa, ea, h->stream));
+      for (int64_t n0 = 0; n0 < g.N; n0 += nb) {
+        const int64_t n = std::min<int64_t>(nb, g.N - n0);
+        if (g.b_k == 1)
+          RPA_CUDA(h, rpa::launch_mod_cols(g.B + n0 * g.b_n, g.b_n, 0, (int)g.K, n, 1, pb, eb, h->stream, 0.0,
+                                           g.kscale));
+        else RPA_CUDA(h, rpa::launch_mod_rows(g.B + n0, g.b_k, (int)n, g.K, pb, eb, h->stream));
+        rpa::ModGemmArgs a{};
+        if (int s = mod_product(h, a, pb, NM, (int)n, pa, NM, g.M, g.K, 1, false, static_cast<uint8_t*>(h->mC.p), ldo))
+          return s;
+        RPA_CUDA(h, rpa::launch_mod_crt_full(a.out, a.out_plane, ldo, ea, eb, g.M, n, g.C + n0 * g.ldc, g.ldc, g.alpha,
+                                             g.beta, h->stream));
+      }
+      return RPA_OK;
+    }
+    for (DevBuf* b : {&h->mA, &h->mB, &h->mC, &h->mE}) release(*b);
+  }
+  RPA_CUDA(h, rpa::launch_gemm_f64(g, h->stream));
   return RPA_OK;
 }
 
@@ -1042,7 +1088,7 @@ int apply_I(rpa_b200_handle* h, const T2Ctx& c, const double* M, int ncols, doub
     g.alpha = 1.0;
     g.beta = 0.0;
     g.batch = 1;
-    RPA_CUDA(h, rpa::launch_gemm_f64(g, h->stream));
+    if (int gs = gemm64(h, g)) return gs;
     rpa::GemmF64Args g2{};
     g2.M = (int)c.nov;
     g2.N = ncols;
@@ -1058,7 +1104,7 @@ int apply_I(rpa_b200_handle* h, const T2Ctx& c, const double* M, int ncols, doub
     g2.alpha = -1.0 / (4.0 * kPi);
     g2.beta = first ? 0.0 : 1.0;
     g2.batch = 1;
-    RPA_CUDA(h, rpa::launch_gemm_f64(g2, h->stream));
+    if (int gs = gemm64(h, g2)) return gs;
     first = false;
   }
   return RPA_OK;
@@ -1143,7 +1189,7 @@ int begin_call(rpa_b200_handle* h) {
   if (!h) return RPA_ERR_INVALID_ARG;
   h->last_error.clear();
   g_account = &h->account;
-  h->account.idle = {&h->Xhi, &h->Xlo, &h->gY, &h->gM};
+  h->account.idle = {&h->Xhi, &h->Xlo, &h->gY, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE};
   h->pool_used = 0;
   h->split_ev.clear();
   h->tc_ev.clear();
@@ -1261,7 +1307,7 @@ int rpa_b200_destroy(rpa_b200_handle* h) try {
   if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
   for (DevBuf* b : {&h->R, &h->D, &h->eps, &h->Xhi, &h->Xlo, &h->diag_part, &h->diag, &h->Pi, &h->Ldiag, &h->ddbuf,
                     &h->tZ, &h->tOm, &h->tIOm, &h->tP, &h->tS, &h->tV, &h->tT, &h->tTIT, &h->tVt, &h->tW, &h->tU,
-                    &h->tRU, &h->tSmall, &h->tPerm, &h->bDesc, &h->bRes, &h->gY, &h->gD, &h->gM,
+                    &h->tRU, &h->tSmall, &h->tPerm, &h->bDesc, &h->bRes, &h->gY, &h->gD, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE,
                     &h->xM, &h->eW, &h->eA, &h->eZ, &h->thZ, &h->thXa, &h->thXi, &h->thYX, &h->thR,
                     &h->jU, &h->jL, &h->jX, &h->jPno, &h->jWork,
                     &h->jPack, &h->jQS, &h->jS, &h->jD, &h->syncBuf,
@@ -1603,7 +1649,7 @@ int rpa_b200_dring_t2(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVir
   // S = IOm^T IOm, eigenvalues above the linear-dependency cutoff (771-795)
   double* S = static_cast<double*>(h->tS.p);
   double* Vs = static_cast<double*>(h->tV.p);
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn(G, G, nov, IOm, nov, IOm, nov, S, G), h->stream));
+  if (int gs = gemm64(h, gemm_tn(G, G, nov, IOm, nov, IOm, nov, S, G))) return gs;
   RPA_CUDA(h, rpa::launch_symmetrize_avg(S, G, G, h->stream));
   std::vector<double> sval;
   std::vector<int> sord;
@@ -1625,7 +1671,7 @@ int rpa_b200_dring_t2(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVir
   double* W = static_cast<double*>(h->tW.p);
   double* T = static_cast<double*>(h->tT.p);
   if ((s = gather(h, Vs, G, W, wcols, &wscale))) return s;
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn((int)nov, NT, G, IOm, nov, W, G, T, nov), h->stream));
+  if (int gs = gemm64(h, gemm_nn((int)nov, NT, G, IOm, nov, W, G, T, nov))) return gs;
   // Rayleigh-Ritz: TIT = T^T I T (rpa_CC_MIM_v5, 425-488), eigenpairs (797-808)
   double* IT = Om;  // guess vectors no longer needed
   if ((s = apply_I(h, c, T, NT, IT))) return s;
@@ -1633,7 +1679,7 @@ int rpa_b200_dring_t2(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVir
   RPA_CUDA(h, ensure(h->tVt, (size_t)NT * NT * 8));
   double* TIT = static_cast<double*>(h->tTIT.p);
   double* Vt = static_cast<double*>(h->tVt.p);
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn(NT, NT, nov, T, nov, IT, nov, TIT, NT), h->stream));
+  if (int gs = gemm64(h, gemm_tn(NT, NT, nov, T, nov, IT, nov, TIT, NT))) return gs;
   RPA_CUDA(h, rpa::launch_symmetrize_avg(TIT, NT, NT, h->stream));
   std::vector<double> aval;
   std::vector<int> aord;
@@ -1682,11 +1728,11 @@ int rpa_b200_dring_t2(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVir
   if ((s = gather(h, Vt, NT, W, tcols, nullptr))) return s;  // W reused: NT x keep
   RPA_CUDA(h, ensure(h->tU, (size_t)nov * keep * 8));
   double* Ud = static_cast<double*>(h->tU.p);
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn((int)nov, keep, NT, T, nov, W, NT, Ud, nov), h->stream));
+  if (int gs = gemm64(h, gemm_nn((int)nov, keep, NT, T, nov, W, NT, Ud, nov))) return gs;
   // EigRPA(mu) = 2 A_mu |R U_mu|^2 (rpa_T2_EigRPA, 987-1009)
   RPA_CUDA(h, ensure(h->tRU, (size_t)v.NQ * keep * 8));
   double* RU = static_cast<double*>(h->tRU.p);
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn(v.NQ, keep, nov, Rd, ldd, Ud, nov, RU, v.NQ), h->stream));
+  if (int gs = gemm64(h, gemm_nn(v.NQ, keep, nov, Rd, ldd, Ud, nov, RU, v.NQ))) return gs;
   double* nrm = static_cast<double*>(h->tSmall.p);
   RPA_CUDA(h, rpa::launch_col_sqnorm(RU, v.NQ, keep, v.NQ, nrm, h->stream));
   std::vector<double> n2(keep);
@@ -1928,12 +1974,12 @@ int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
   RPA_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
 
   // Ukl = (R U)^T (R U), Dkl = U^T diag(D) U, then the A, B and S matrices
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn((int)NQ, NT, nov, Rd, ldr, Ud, ldu, RU, NQ), h->stream));
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn(NT, NT, NQ, RU, NQ, RU, NQ, Ukl, NT), h->stream));
+  if (int gs = gemm64(h, gemm_nn((int)NQ, NT, nov, Rd, ldr, Ud, ldu, RU, NQ))) return gs;
+  if (int gs = gemm64(h, gemm_tn(NT, NT, NQ, RU, NQ, RU, NQ, Ukl, NT))) return gs;
   {
     rpa::GemmF64Args g = gemm_tn(NT, NT, nov, Ud, ldu, Ud, ldu, Dkl, NT);
     g.kscale = Dd;
-    RPA_CUDA(h, rpa::launch_gemm_f64(g, h->stream));
+    if (int gs = gemm64(h, g)) return gs;
   }
   RPA_CUDA(h, rpa::launch_mbpt3_build(Ukl, Dkl, Ad, NT, Am, Bm, Sm, h->stream));
   std::vector<double> mu;
@@ -1964,11 +2010,11 @@ int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
       rpa::GemmF64Args g1 = gemm_tn(NT, NT, NT, Bm, NT, Xd, NT, Res, NT);
       g1.alpha = -1.0;
       g1.beta = 1.0;
-      RPA_CUDA(h, rpa::launch_gemm_f64(g1, h->stream));
+      if (int gs = gemm64(h, g1)) return gs;
       rpa::GemmF64Args g2 = gemm_nn(NT, NT, NT, Xd, NT, Bm, NT, Res, NT);
       g2.alpha = -1.0;
       g2.beta = 1.0;
-      RPA_CUDA(h, rpa::launch_gemm_f64(g2, h->stream));
+      if (int gs = gemm64(h, g2)) return gs;
       if ((s = sqnorm(Res, r2))) return s;
       if (!std::isfinite(r2) || r2 > 1e4 * a2)
         return fail(h, RPA_ERR_NOT_CONVERGED, "MBPT3 Lyapunov iteration diverged (|res|/|A| = %.3e)",
@@ -1979,15 +2025,15 @@ int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
       }
     }
     // Y = Q^T Res Q / (mu_m + mu_n);  X += Q Y Q^T   (Sm and Ukl serve as scratch)
-    RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn(NT, NT, NT, Q, NT, Res, NT, Sm, NT), h->stream));
-    RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn(NT, NT, NT, Sm, NT, Q, NT, Ukl, NT), h->stream));
+    if (int gs = gemm64(h, gemm_tn(NT, NT, NT, Q, NT, Res, NT, Sm, NT))) return gs;
+    if (int gs = gemm64(h, gemm_nn(NT, NT, NT, Sm, NT, Q, NT, Ukl, NT))) return gs;
     RPA_CUDA(h, rpa::launch_lyap_scale(Ukl, mud, NT, bad, h->stream));
-    RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn(NT, NT, NT, Q, NT, Ukl, NT, Sm, NT), h->stream));
+    if (int gs = gemm64(h, gemm_nn(NT, NT, NT, Q, NT, Ukl, NT, Sm, NT))) return gs;
     rpa::GemmF64Args g3 = gemm_nn(NT, NT, NT, Sm, NT, Q, NT, Xd, NT);
     g3.b_k = NT;  // Q^T
     g3.b_n = 1;
     g3.beta = 1.0;
-    RPA_CUDA(h, rpa::launch_gemm_f64(g3, h->stream));
+    if (int gs = gemm64(h, g3)) return gs;
     if (it == 0) {
       int nbad = 0;
       RPA_CUDA(h, cudaMemcpyAsync(&nbad, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -2002,7 +2048,7 @@ int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
                 std::sqrt(r2 / a2));
 
   // Tr(XK): W_ij from U, W_ji from U X
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn((int)nov, NT, NT, Ud, ldu, Xd, NT, UX, nov), h->stream));
+  if (int gs = gemm64(h, gemm_nn((int)nov, NT, NT, Ud, ldu, Xd, NT, UX, nov))) return gs;
   RPA_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
   int64_t npart = 0;
   double split_sum = 0.0;
@@ -2159,10 +2205,10 @@ int rpa_b200_piu_basis(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVi
         RPA_CUDA(h, rpa::launch_fill_uniform(Q0, n, n, n, seed, h->stream));
       }
       // Yt = (Pi G0)^T = G0^T Pi
-      RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn(n, n, n, Q0, n, Pi, n, Yt, n), h->stream));
+      if (int gs = gemm64(h, gemm_tn(n, n, n, Q0, n, Pi, n, Yt, n))) return gs;
       for (int it = 0; it < 2; ++it) {
         if (it > 0)  // Yt <- Q^T Pi  (Y = Pi Q)
-          RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn(n, n, n, Gd, n, Pi, n, Yt, n), h->stream));
+          if (int gs = gemm64(h, gemm_nn(n, n, n, Gd, n, Pi, n, Yt, n))) return gs;
         // shifted CholeskyQR3 on the columns of Y = Yt^T (Fukaya, Kannan, Nakatsukasa, Zhang,
         // Yamamoto, SIAM J. Sci. Comput. 42 (2020) A477): the first pass factors Y^T Y +
         // 11 (n^2 + n(n+1)) u ||Y||_F^2 I, which succeeds for numerically rank-deficient Y; two
@@ -2172,7 +2218,7 @@ int rpa_b200_piu_basis(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVi
           rpa::GemmF64Args g = gemm_nn(n, n, n, Yt, n, Yt, n, S, n);  // S = Yt Yt^T
           g.b_k = n;
           g.b_n = 1;
-          RPA_CUDA(h, rpa::launch_gemm_f64(g, h->stream));
+          if (int gs = gemm64(h, g)) return gs;
           if (pass == 0) {
             double* red = static_cast<double*>(h->tSmall.p);
             RPA_CUDA(h, rpa::launch_offdiag(Yt, n, n, red, h->stream));  // red[0] + red[1] = ||Y||_F^2
@@ -2194,7 +2240,7 @@ int rpa_b200_piu_basis(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVi
         RPA_CUDA(h, cudaMemcpyAsync(Gd, Yt, nn * 8, cudaMemcpyDeviceToDevice, h->stream));  // Gd <- Q^T
       }
       // trace weights diag(Q^T Pi Q): T = Q^T Pi, rwr_p = sum_k T(p,k) Q^T(p,k)
-      RPA_CUDA(h, rpa::launch_gemm_f64(gemm_nn(n, n, n, Yt, n, Pi, n, S, n), h->stream));
+      if (int gs = gemm64(h, gemm_nn(n, n, n, Yt, n, Pi, n, S, n))) return gs;
       std::vector<double> Th(nn), Qh(nn);
       RPA_CUDA(h, cudaMemcpyAsync(Th.data(), S, nn * 8, cudaMemcpyDeviceToHost, h->stream));
       RPA_CUDA(h, cudaMemcpyAsync(Qh.data(), Yt, nn * 8, cudaMemcpyDeviceToHost, h->stream));
@@ -2269,7 +2315,7 @@ int rpa_b200_project_basis(rpa_b200_handle* h, int64_t NQ, int64_t NVecs, int64_
     ldo = NVecs;
   }
   RPA_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
-  RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn((int)NVecs, (int)nov, NQ, Gd, ldg, Rd, ldr, out, ldo), h->stream));
+  if (int gs = gemm64(h, gemm_tn((int)NVecs, (int)nov, NQ, Gd, ldg, Rd, ldr, out, ldo))) return gs;
   RPA_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
   RPA_CUDA(h, cudaEventRecord(h->ev[3], h->stream));
   if ((s = screen_result(h, out, ldo, NVecs, nov, "the projected Cholesky vectors"))) return s;
@@ -2312,9 +2358,8 @@ static int form_thc_r(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   for (int64_t i0 = 0; i0 < NOcc; i0 += ib) {
     const int64_t ni = std::min(ib, NOcc - i0);
     RPA_CUDA(h, rpa::launch_khatri_rao(Xad, ldxa, Xid, ldxi, (int)NGrid, (int)NVirt, (int)i0, (int)ni, YX, h->stream));
-    RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn((int)NQ, (int)(NVirt * ni), NGrid, Zd, ldz, YX, NGrid,
-                                             Rout + ldR * (i0 * NVirt), ldR),
-                                     h->stream));
+    if (int gs = gemm64(h, gemm_tn((int)NQ, (int)(NVirt * ni), NGrid, Zd, ldz, YX, NGrid,
+                                             Rout + ldR * (i0 * NVirt), ldR))) return gs;
   }
   return RPA_OK;
 }
@@ -2406,7 +2451,7 @@ int build_pi_thc(rpa_b200_handle* h, const Validated& v, int64_t NGrid, const do
     const bool first = a0 == 0, last = a0 + wp == nov;
     cudaEvent_t e0 = pool_event(h), e1 = pool_event(h), e2 = pool_event(h);
     RPA_CUDA(h, rpa::launch_khatri_rao_cols(Xad, ldxa, Xid, ldxi, (int)NGrid, (int)v.nv, a0, wp, YX, h->stream));
-    RPA_CUDA(h, rpa::launch_gemm_f64(gemm_tn(NQ, (int)wp, NGrid, Zd, ldz, YX, NGrid, Rp, NQ), h->stream));
+    if (int gs = gemm64(h, gemm_tn(NQ, (int)wp, NGrid, Zd, ldz, YX, NGrid, Rp, NQ), h->thc_piece_bytes / 2)) return gs;
     RPA_CUDA(h, rpa::launch_count_nonfinite(Rp, (int64_t)NQ * wp, h->count_dev, h->stream));
     const rpa::SplitPlan plan = rpa::plan_scale_split(NQ, wp, h->num_sms);
     RPA_CUDA(h, ensure(h->diag_part, (size_t)plan.nsplit * K * NQ * 8));
@@ -2589,13 +2634,13 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   RPA_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
   // occupied localisation: X <- X L, U(:, :, mu) <- U(:, :, mu) L
   if (Ld) {
-    RPA_CUDA(h, rpa::launch_gemm_f64(gemm_g(ng, no, no, Xd0, ldx0, false, Ld, ldl, false, Xd, ldx), h->stream));
+    if (int gs = gemm64(h, gemm_g(ng, no, no, Xd0, ldx0, false, Ld, ldl, false, Xd, ldx))) return gs;
     rpa::GemmF64Args g = gemm_g(nv, no, no, Ud0, nv, false, Ld, ldl, false, Ud, nv);
     g.batch = nt;
     g.sA = ldu0;
     g.sB = 0;
     g.sC = nov;
-    RPA_CUDA(h, rpa::launch_gemm_f64(g, h->stream));
+    if (int gs = gemm64(h, g)) return gs;
   } else {
     RPA_CUDA(h, cudaMemcpy2DAsync(Xd, (size_t)ng * 8, Xd0, (size_t)ldx0 * 8, (size_t)ng * 8, (size_t)no,
                                   cudaMemcpyDeviceToDevice, h->stream));
@@ -2606,7 +2651,7 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   double maxvabab = 0.0;
   if (BoysScreening) {
     RPA_CUDA(h, rpa::launch_hadamard(Yd, ldy, Yd, ldy, ng, nv, Wg, ng, h->stream));
-    RPA_CUDA(h, rpa::launch_gemm_f64(gemm_g(nq, nv, ng, Zd, ldz, true, Wg, ng, false, ZYXk, nq), h->stream));
+    if (int gs = gemm64(h, gemm_g(nq, nv, ng, Zd, ldz, true, Wg, ng, false, ZYXk, nq))) return gs;
     std::vector<double> zz((size_t)nq * nv);
     RPA_CUDA(h, cudaMemcpyAsync(zz.data(), ZYXk, zz.size() * 8, cudaMemcpyDeviceToHost, h->stream));
     RPA_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -2658,7 +2703,7 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
     rpa::GemmF64Args gm = gemm_g(nv, nv, nv, Tb, nv, false, Tb, nv, true, Mb, nv);
     gm.batch = nbat;
     gm.sA = gm.sB = gm.sC = (int64_t)nvv;
-    RPA_CUDA(h, rpa::launch_gemm_f64(gm, h->stream));
+    if (int gs = gemm64(h, gm)) return gs;
     std::vector<double> ev;
     bool conv = false;
     RPA_CUDA(h, rpa::syevd_batched(Mb, nv, nbat, Vb, h->eW.p, h->eW.bytes, ev, conv, h->stream));

@@ -87,24 +87,36 @@ __device__ __forceinline__ void to_words(double x, uint32_t& lo, uint32_t& hi) {
 }
 
 // Columns of a column-major (K x rows) matrix: one warp per column, 8 consecutive k per lane.
-// S: column r starts at S + r * ld; expo[r]: its power of two.  shift is subtracted from the diagonal.
+// S: column r starts at S + r * ld; expo[r]: its power of two.  shift is subtracted from the diagonal;
+// ks (optional) multiplies entry k of every column.
 __global__ void __launch_bounds__(256) mod_cols_kernel(const double* __restrict__ S, int64_t ld, int64_t strideS,
                                                        int K, int64_t rows, int8_t* __restrict__ planes,
                                                        int64_t pitch, int64_t plane_stride, int64_t strideP,
-                                                       int* __restrict__ expo, double shift) {
+                                                       int* __restrict__ expo, double shift,
+                                                       const double* __restrict__ ks) {
   const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
   const int z = blockIdx.y;
   const double* col = S + (int64_t)z * strideS + r * ld;
-  double s2 = 0.0;
-  for (int k = lane; k < K; k += 32) {
+  auto entry = [&](int k) {
     const double x = col[k] - (k == r ? shift : 0.0);
-    s2 = fma(x, x, s2);
-  }
+    return ks ? x * __ldg(ks + k) : x;
+  };
+  auto sum = [&](double f) {
+    double s2 = 0.0;
+    for (int k = lane; k < K; k += 32) {
+      const double x = entry(k) * f;
+      s2 = fma(x, x, s2);
+    }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  const int e = mod_exponent(s2);
+    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    return s2;
+  };
+  double s2 = sum(1.0);
+  const int sh = mod_needs_shift(s2);  // squares that overflow or vanish: sum them scaled (warp-uniform)
+  if (sh) s2 = sum(mod_pow2(sh));
+  const int e = mod_exponent(s2, sh);
   if (lane == 0) expo[(int64_t)z * rows + r] = e;
   const double sc = mod_pow2(e);
   int8_t* out = planes + (int64_t)z * strideP + r * pitch;
@@ -112,7 +124,7 @@ __global__ void __launch_bounds__(256) mod_cols_kernel(const double* __restrict_
     uint32_t lo[8], hi[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      to_words(k0 + i < K ? (col[k0 + i] - (k0 + i == r ? shift : 0.0)) * sc : 0.0, lo[i], hi[i]);
+      to_words(k0 + i < K ? entry(k0 + i) * sc : 0.0, lo[i], hi[i]);
     mod_all<8>(
         lo, hi,
         [&](int m, const uint32_t(&w)[2]) {
@@ -192,7 +204,42 @@ __global__ void mod_pi_expo_kernel(const double* __restrict__ part, int nsplit, 
   if (i >= n) return;
   double s = 0.0;
   for (int t = 0; t < nsplit; ++t) s += part[t * n + i];
-  expo[i] = mod_exponent(s);
+  expo[i] = mod_exponent(s, 0);
+}
+
+// expo[r] of the rows of a column-major (rows x K) matrix: lane = row, eight warps stride over k
+__global__ void __launch_bounds__(256) mod_row_norm_kernel(const double* __restrict__ S, int64_t ld, int rows,
+                                                           int64_t K, int* __restrict__ expo) {
+  __shared__ double red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
+  auto sum = [&](double f) {
+    double s0 = 0.0, s1 = 0.0;
+    int64_t k = warp;
+    for (; k + 8 < K; k += 16) {
+      const double x = r < rows ? S[r + ld * k] * f : 0.0, y = r < rows ? S[r + ld * (k + 8)] * f : 0.0;
+      s0 = fma(x, x, s0);
+      s1 = fma(y, y, s1);
+    }
+    if (k < K && r < rows) {
+      const double x = S[r + ld * k] * f;
+      s0 = fma(x, x, s0);
+    }
+    __syncthreads();
+    red[warp][lane] = s0 + s1;
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += red[w][lane];
+    return t;
+  };
+  double s2 = sum(1.0);
+  int shift = 0;
+  if (__syncthreads_or(mod_needs_shift(s2) != 0)) {  // squares that overflow or vanish: sum them scaled
+    shift = mod_needs_shift(s2);
+    s2 = sum(mod_pow2(shift));
+  }
+  if (warp == 0 && r < rows) expo[r] = mod_exponent(s2, shift);
 }
 
 // planes[(k, m)][Q][ai]: a CTA takes a 32 x 128 block of R (read with Q across the lanes, kept in
@@ -202,6 +249,8 @@ __global__ void mod_pi_expo_kernel(const double* __restrict__ part, int nsplit, 
 // NQ 2048, 16384 ai, 16 frequencies).
 constexpr int kPiPitch = 128 + 4;
 constexpr size_t kModPiSmem = sizeof(double) * (32 * kPiPitch + kMaxKgLaunch * 128);
+// kFac false: the rows of R itself (one set of planes, no factors).
+template <bool kFac>
 __global__ void __launch_bounds__(256, 4) mod_pi_kernel(const double* __restrict__ R, int64_t ldR, int NQ, int64_t nov,
                                                         const double* __restrict__ fac, int kg,
                                                         const int* __restrict__ expo, int8_t* __restrict__ planes,
@@ -217,9 +266,11 @@ __global__ void __launch_bounds__(256, 4) mod_pi_kernel(const double* __restrict
     const int64_t a = b0 + warp + 8 * j;
     rs[lane * kPiPitch + warp + 8 * j] = (q0 + lane < NQ && a < nov) ? __ldg(R + q0 + lane + ldR * a) : 0.0;
   }
-  for (int i = threadIdx.x; i < kg * 128; i += 256) {
-    const int64_t a = b0 + (i & 127);
-    fs[i] = a < nov ? __ldg(fac + (i >> 7) * nov + a) : 0.0;
+  if (kFac) {
+    for (int i = threadIdx.x; i < kg * 128; i += 256) {
+      const int64_t a = b0 + (i & 127);
+      fs[i] = a < nov ? __ldg(fac + (i >> 7) * nov + a) : 0.0;
+    }
   }
   __syncthreads();
   const int64_t plane_stride = (int64_t)NQ * pitch;
@@ -229,7 +280,8 @@ __global__ void __launch_bounds__(256, 4) mod_pi_kernel(const double* __restrict
     const double sc = mod_pow2(expo[(int64_t)k * NQ + q0 + q]);
     const double2* r2 = reinterpret_cast<const double2*>(rs + q * kPiPitch + 4 * lane);
     const double2* f2 = reinterpret_cast<const double2*>(fs + k * 128 + 4 * lane);
-    const double2 ra = r2[0], rb = r2[1], fa = f2[0], fb = f2[1];
+    const double2 one = make_double2(1.0, 1.0);
+    const double2 ra = r2[0], rb = r2[1], fa = kFac ? f2[0] : one, fb = kFac ? f2[1] : one;
     uint32_t lo[4], hi[4];
     to_words((ra.x * fa.x) * sc, lo[0], hi[0]);
     to_words((ra.y * fa.y) * sc, lo[1], hi[1]);
@@ -274,34 +326,53 @@ __device__ __forceinline__ uint64_t desc_k_sw128(uint32_t addr) {
          (uint64_t)2u << 61;
 }
 
+// One tile of one modulus: operand rows j0 .. (128 lanes) and i0 .. (ni columns) of planes pa and pb.
 struct MgUnit {
-  int z, m, j0, i0, ni;  // batch, modulus, first row of each operand, live columns (256 or 128)
+  int m, j0, i0, ni, pa, pb;
+  bool live;
+  uint8_t* out;  // residues of (j0, i0)
+  int nj;        // rows of the tile that are stored
 };
 
-__device__ __forceinline__ MgUnit mg_unit(int u, const ModGemmArgs& a) {
-  MgUnit x;
-  const int zm = u / a.ntiles, t = u - zm * a.ntiles;
-  x.z = zm / kModCount;
-  x.m = zm - x.z * kModCount;
-  int ti, tj;
-  if (a.tri) {  // ti-major: tile (ti, tj) with tj <= 2 ti + 1 (only i >= j is kept)
-    ti = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-    while ((ti + 1) * (ti + 2) <= t) ++ti;
-    while (ti * (ti + 1) > t) --ti;
-    tj = t - ti * (ti + 1);
-  } else {
-    tj = t / a.nti;
-    ti = t - tj * a.nti;
+// Persistent launch over (batch, modulus, tile), tiles of one plane next to one another.
+struct MgFull {
+  const CUtensorMap *mA, *mB, *mBh;
+  const ModGemmArgs& a;
+  __device__ __forceinline__ int begin() const { return blockIdx.x; }
+  __device__ __forceinline__ int end() const { return a.nunits; }
+  __device__ __forceinline__ int step() const { return gridDim.x; }
+  __device__ __forceinline__ int nch() const { return a.nch; }
+  __device__ __forceinline__ int64_t ldo() const { return a.ldo; }
+  __device__ __forceinline__ MgUnit get(int u) const {
+    MgUnit x;
+    const int zm = u / a.ntiles, t = u - zm * a.ntiles;
+    const int z = zm / kModCount;
+    x.m = zm - z * kModCount;
+    int ti, tj;
+    if (a.tri) {  // ti-major: tile (ti, tj) with tj <= 2 ti + 1 (only i >= j is kept)
+      ti = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+      while ((ti + 1) * (ti + 2) <= t) ++ti;
+      while (ti * (ti + 1) > t) --ti;
+      tj = t - ti * (ti + 1);
+    } else {
+      tj = t / a.nti;
+      ti = t - tj * a.nti;
+    }
+    x.j0 = tj * MG_TM;
+    x.i0 = ti * MG_TN;
+    x.ni = MG_TN;
+    if (a.tri && tj == 2 * ti + 1) {  // the first 128 columns lie above the diagonal
+      x.i0 += MG_TM;
+      x.ni = MG_TM;
+    }
+    x.pa = z * a.zplanesA + x.m;
+    x.pb = z * a.zplanesB + x.m;
+    x.live = true;
+    x.nj = a.rowsA - x.j0;
+    x.out = a.out + (int64_t)zm * a.out_plane + (int64_t)x.j0 * a.ldo + x.i0;
+    return x;
   }
-  x.j0 = tj * MG_TM;
-  x.i0 = ti * MG_TN;
-  x.ni = MG_TN;
-  if (a.tri && tj == 2 * ti + 1) {  // the first 128 columns lie above the diagonal
-    x.i0 += MG_TM;
-    x.ni = MG_TM;
-  }
-  return x;
-}
+};
 
 __device__ __forceinline__ bool mg_wait_count(const int* c, int target) {
   for (uint32_t it = 0; it < (1u << 20); ++it) {
@@ -313,9 +384,10 @@ __device__ __forceinline__ bool mg_wait_count(const int* c, int target) {
   return false;
 }
 
-__global__ void __launch_bounds__(MG_THREADS, 1)
-    modgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const __grid_constant__ CUtensorMap tmBh, const ModGemmArgs a, const ModReduce red) {
+template <class Src>
+__device__ __forceinline__ void modgemm_body(const Src& src, const CUtensorMap* tmA, const CUtensorMap* tmB,
+                                             const CUtensorMap* tmBh, int* sync, int sync_every, int* err,
+                                             const ModReduce& red) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + MG_STAGES * MG_STAGE);
@@ -347,34 +419,33 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
   if (warp == 0) {
     if (lane == 0) {
       // ------------------------------------------------------------ producer
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
+      tma_prefetch_desc(tmA);
+      tma_prefetch_desc(tmB);
       int stage = 0;
       uint32_t phase = 0, issued = 0, issued_par = 0;
       bool ok = true, sync_wait = true;
-      const int nmile = a.sync ? (a.nch + a.sync_every - 1) / a.sync_every : 0;
-      for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x) {
-        const MgUnit x = mg_unit(u, a);
-        const int pa = x.z * a.zplanesA + x.m, pb = x.z * a.zplanesB + x.m;
-        const int wave = (u - (int)blockIdx.x) / (int)gridDim.x;
-        const int members = min((int)gridDim.x, a.nunits - wave * (int)gridDim.x);
-        const CUtensorMap* mb = x.ni == MG_TN ? &tmB : &tmBh;
+      const int nmile = sync ? (src.nch() + sync_every - 1) / sync_every : 0;
+      for (int u = src.begin(); u < src.end() && ok; u += src.step()) {
+        const MgUnit x = src.get(u);
+        const int wave = sync ? (u - (int)blockIdx.x) / (int)gridDim.x : 0;
+        const int members = min((int)gridDim.x, src.end() - wave * (int)gridDim.x);
+        const CUtensorMap* mb = x.ni == MG_TN ? tmB : tmBh;
         const uint32_t bytes = (uint32_t)(MG_TM + x.ni) * MG_TK;
-        for (int ch = 0; ch < a.nch; ++ch) {
-          if (a.sync && ch % a.sync_every == 0) {
-            const int mi = ch / a.sync_every;
-            int* row = a.sync + (int64_t)wave * nmile;
+        for (int ch = 0; ch < src.nch(); ++ch) {
+          if (sync && ch % sync_every == 0) {
+            const int mi = ch / sync_every;
+            int* row = sync + (int64_t)wave * nmile;
             asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(row + mi) : "memory");
             if (sync_wait && mi >= 2) sync_wait = mg_wait_count(row + mi - 2, members);
           }
-          if (!mbar_wait(&empty[stage], phase ^ 1u, a.err, kDevTimeoutTmaEmpty)) {
+          if (!mbar_wait(&empty[stage], phase ^ 1u, err, kDevTimeoutTmaEmpty)) {
             ok = false;
             break;
           }
           mbar_arrive_expect_tx(&full[stage], bytes);
           uint8_t* st = smem + stage * MG_STAGE;
-          tma_load_3d(st, &tmA, &full[stage], ch * MG_TK, x.j0, pa);
-          tma_load_3d(st + MG_ABYTES, mb, &full[stage], ch * MG_TK, x.i0, pb);
+          tma_load_3d(st, tmA, &full[stage], ch * MG_TK, x.j0, x.pa);
+          tma_load_3d(st + MG_ABYTES, mb, &full[stage], ch * MG_TK, x.i0, x.pb);
           issued |= 1u << stage;
           issued_par = (issued_par & ~(1u << stage)) | (phase << stage);
           if (++stage == MG_STAGES) {
@@ -385,7 +456,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
       }
       // no bulk copy may still be landing in shared memory at exit
       for (int s = 0; s < MG_STAGES; ++s)
-        if (issued & (1u << s)) mbar_wait(&full[s], (issued_par >> s) & 1u, a.err, kDevTimeoutDrain);
+        if (issued & (1u << s)) mbar_wait(&full[s], (issued_par >> s) & 1u, err, kDevTimeoutDrain);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -393,20 +464,20 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
       int stage = 0, it = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x) {
-        const MgUnit x = mg_unit(u, a);
+      for (int u = src.begin(); u < src.end() && ok; u += src.step()) {
+        const MgUnit x = src.get(u);
         const uint32_t idesc = x.ni == MG_TN ? idesc_s8_s32(MG_TM, MG_TN) : idesc_s8_s32(MG_TM, MG_TM);
-        for (int c0 = 0; c0 < a.nch && ok; c0 += MG_SEG, ++it) {
+        for (int c0 = 0; c0 < src.nch() && ok; c0 += MG_SEG, ++it) {
           const int b = it & 1;
-          if (!mbar_wait(&acc_empty[b], (uint32_t)((it >> 1) & 1) ^ 1u, a.err, kDevTimeoutAccEmpty)) {
+          if (!mbar_wait(&acc_empty[b], (uint32_t)((it >> 1) & 1) ^ 1u, err, kDevTimeoutAccEmpty)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t d = tmem_base + (uint32_t)(b * MG_TN);
-          const int c1 = min(a.nch, c0 + MG_SEG);
+          const int c1 = min(src.nch(), c0 + MG_SEG);
           for (int ch = c0; ch < c1; ++ch) {
-            if (!mbar_wait(&full[stage], phase, a.err, kDevTimeoutTmaFull)) {
+            if (!mbar_wait(&full[stage], phase, err, kDevTimeoutTmaFull)) {
               ok = false;
               break;
             }
@@ -428,7 +499,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
       }
       // every issued MMA must complete before TMEM is freed
       tc_commit(drain);
-      mbar_wait(drain, 0, a.err, kDevTimeoutDrain);
+      mbar_wait(drain, 0, err, kDevTimeoutDrain);
     }
   } else {
     // -------------------------------------------------------------- epilogue
@@ -438,16 +509,16 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
     const int col0 = ((warp - 2) >> 2) * 64;
     int it = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x) {
-      const MgUnit x = mg_unit(u, a);
+    for (int u = src.begin(); u < src.end() && ok; u += src.step()) {
+      const MgUnit x = src.get(u);
       const int p = red.p[x.m];
       const int mg = red.magic[x.m];
       uint32_t w[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) w[i] = 0;
-      for (int c0 = 0; c0 < a.nch; c0 += MG_SEG, ++it) {
+      for (int c0 = 0; c0 < src.nch(); c0 += MG_SEG, ++it) {
         const int b = it & 1;
-        if (!mbar_wait(&acc_full[b], (uint32_t)((it >> 1) & 1), a.err, kDevTimeoutAccFull)) {
+        if (!mbar_wait(&acc_full[b], (uint32_t)((it >> 1) & 1), err, kDevTimeoutAccFull)) {
           ok = false;
           break;
         }
@@ -475,10 +546,9 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
         if (lane == 0) mbar_arrive(&acc_empty[b]);
       }
       if (!ok) break;
-      const int j = x.j0 + quarter * 32 + lane;
-      if (col0 < x.ni && j < a.rowsA) {
-        uint4* dst = reinterpret_cast<uint4*>(a.out + ((int64_t)x.z * kModCount + x.m) * a.out_plane +
-                                              (int64_t)j * a.ldo + x.i0 + col0);
+      const int j = quarter * 32 + lane;
+      if (col0 < x.ni && j < x.nj) {
+        uint4* dst = reinterpret_cast<uint4*>(x.out + (int64_t)j * src.ldo() + col0);
 #pragma unroll
         for (int t = 0; t < 4; ++t) dst[t] = make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
       }
@@ -490,6 +560,12 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+}
+
+__global__ void __launch_bounds__(MG_THREADS, 1)
+    modgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmBh, const ModGemmArgs a, const ModReduce red) {
+  modgemm_body(MgFull{&tmA, &tmB, &tmBh, a}, &tmA, &tmB, &tmBh, a.sync, a.sync_every, a.err, red);
 }
 
 // ------------------------------------------------------------------ C from its residues
@@ -643,11 +719,11 @@ cudaError_t mod_map(PFN_cuTensorMapEncodeTiled_v12000 encode, CUtensorMap* m, vo
 }
 
 cudaError_t launch_mod_cols(const double* S, int64_t ld, int64_t strideS, int K, int64_t rows, int batch,
-                            int8_t* planes, int* expo, cudaStream_t stream, double shift) {
+                            int8_t* planes, int* expo, cudaStream_t stream, double shift, const double* ks) {
   if (rows <= 0 || batch <= 0) return cudaSuccess;
   const int64_t pitch = mod_pitch(K), plane = pitch * rows;
   mod_cols_kernel<<<dim3((unsigned)((rows + 7) / 8), (unsigned)batch), 256, 0, stream>>>(
-      S, ld, strideS, K, rows, planes, pitch, plane, plane * kModCount, expo, shift);
+      S, ld, strideS, K, rows, planes, pitch, plane, plane * kModCount, expo, shift, ks);
   ++g_launches;
   return cudaGetLastError();
 }
@@ -662,11 +738,26 @@ cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, con
                                                                                            fg.n, per, part);
   const int64_t n = (int64_t)fg.n * NQ;
   mod_pi_expo_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(part, nsplit, n, expo);
-  const cudaError_t e = cudaFuncSetAttribute(mod_pi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModPiSmem);
+  const cudaError_t e =
+      cudaFuncSetAttribute(mod_pi_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModPiSmem);
   if (e != cudaSuccess) return e;
-  mod_pi_kernel<<<dim3((unsigned)((NQ + 31) / 32), (unsigned)((pitch + 127) / 128)), 256, kModPiSmem, stream>>>(
+  mod_pi_kernel<true><<<dim3((unsigned)((NQ + 31) / 32), (unsigned)((pitch + 127) / 128)), 256, kModPiSmem, stream>>>(
       R, ldR, NQ, nov, fac, fg.n, expo, planes, pitch);
   g_launches += 4;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, int8_t* planes, int* expo,
+                            cudaStream_t stream) {
+  if (rows <= 0) return cudaSuccess;
+  const int64_t pitch = mod_pitch(K);
+  const cudaError_t e =
+      cudaFuncSetAttribute(mod_pi_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModPiSmem);
+  if (e != cudaSuccess) return e;
+  mod_row_norm_kernel<<<(unsigned)((rows + 31) / 32), 256, 0, stream>>>(S, ld, rows, K, expo);
+  mod_pi_kernel<false><<<dim3((unsigned)((rows + 31) / 32), (unsigned)((pitch + 127) / 128)), 256,
+                         sizeof(double) * 32 * kPiPitch, stream>>>(S, ld, rows, K, nullptr, 1, expo, planes, pitch);
+  g_launches += 2;
   return cudaGetLastError();
 }
 

@@ -24,16 +24,22 @@ struct ModReduce {
   int magic[kModCount];  // ceil(2^38 / p): (acc * magic) >> 38 = floor(acc / p) for |acc| <= 2^30 + 255
 };
 
-// Power of two (exponent) that brings a row of squared norm s2 to a norm in [2^57, 2^58).  A zero
-// row keeps 0; a norm that overflows returns a marker for which mod_pow2 is NaN, so the products
-// of such a row are NaN (as the FP64 sums would be non-finite).
+// Power of two (exponent) that brings a row of norm sqrt(s2) / 2^shift to a norm in [2^57, 2^58).  A zero
+// row keeps 0.  A row with NaN or Inf returns a marker for which mod_pow2 is NaN, so its products are
+// NaN (as the FP64 sums would be non-finite).
 constexpr int kModNaNExpo = 1 << 20;
-__host__ __device__ __forceinline__ int mod_exponent(double s2) {
+__host__ __device__ __forceinline__ int mod_exponent(double s2, int shift) {
   if (!(s2 > 0.0)) return s2 == 0.0 ? 0 : kModNaNExpo;
   if (s2 > 1.7e308) return kModNaNExpo;
   int e;
   frexp(sqrt(s2) * (1.0 + 1e-9), &e);  // norm < 2^e
-  return kModNormBits - e;
+  e = kModNormBits - e + shift;
+  return e < -1000 ? -1000 : e > 1000 ? 1000 : e;
+}
+// Scaling (exponent) under which a sum of squares that overflowed or got lost in the denormals is
+// taken again; 0: the sum is fine.  (A sum that is zero because the row is stays zero.)
+__host__ __device__ __forceinline__ int mod_needs_shift(double s2) {
+  return s2 > 1e300 ? -600 : (s2 < 1e-290 ? 400 : 0);
 }
 __device__ __forceinline__ double mod_pow2(int e) {
   if (e > 1000 || e < -1000) return __longlong_as_double(0x7FF8000000000000ll);
@@ -84,9 +90,13 @@ const ModCrt& mod_crt_tables();
 cudaError_t mod_map(PFN_cuTensorMapEncodeTiled_v12000 encode, CUtensorMap* m, void* planes, int64_t K, int64_t rows,
                     int64_t nplanes, int64_t pitch, int box_rows);
 // Residue planes [z][modulus][row][pitch] of the columns of S - shift * 1 (S: K x rows, column-major,
-// strideS apart).
+// strideS apart), entry k times ks[k] when ks is given.
 cudaError_t launch_mod_cols(const double* S, int64_t ld, int64_t strideS, int K, int64_t rows, int batch,
-                            int8_t* planes, int* expo, cudaStream_t stream, double shift = 0.0);
+                            int8_t* planes, int* expo, cudaStream_t stream, double shift = 0.0,
+                            const double* ks = nullptr);
+// Residue planes [modulus][row][pitch] of the rows of S (rows x K, column-major).
+cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, int8_t* planes, int* expo,
+                            cudaStream_t stream);
 // Residue planes [k][modulus][Q][pitch] of X_k; fac: fg.n * nov doubles, part: nsplit * fg.n * NQ.
 cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, const double* D, const FreqGroup& fg,
                           double alpha, double* fac, double* part, int nsplit, int* expo, int8_t* planes,
