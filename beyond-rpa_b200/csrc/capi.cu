@@ -92,6 +92,10 @@ struct rpa_b200_handle {
   // batched (many-instance) workspace: descriptors and per-batch results
   DevBuf bDesc, bRes;
   DevBuf gY, gD, gM;  // adjoint workspace
+  // residue updates of the log-det (single systems): planes and residues, descriptors and what they describe
+  DevBuf mcBuf, mcDesc;
+  std::vector<rpa::ModMat> mc_mats;
+  DevBuf bMod;            // the same buffer of the batched log-det
   DevBuf mA, mB, mC, mE;  // FP64 products by residues: planes of both operands, residues, exponents
   DevBuf xM;      // MBPT3 exchange: NT x NT matrices, R U and U X
   DevBuf eW, eA, eZ;  // symmetric eigensolver workspace, input and eigenvector buffers
@@ -130,6 +134,7 @@ struct rpa_b200_handle {
     cudaStream_t stream;
     int nb2, tile_w;
     int oz;  // digits of the int8 trailing updates (0: DMMA)
+    const void* mod;  // descriptors of the residue updates (null: DMMA); their contents are the call's
     cudaGraphExec_t exec;
     int64_t launches;
   };
@@ -165,6 +170,12 @@ const double kPi = 3.14159265358979323846;
 // Residue products (modgemm.cu) pay off from here on; below, the DMMA kernels are as fast.
 constexpr int kModMinNQ = 128;
 constexpr int64_t kModMinK = 128;
+// Orders from which the log-det's trailing updates run by residues: one system (16 matrices) 1100 0.75
+// -> 0.72 ms, 1387 1.10 -> 1.00, 2048 2.47 -> 2.11, 4096 13.4 -> 8.8; batches, whose many small
+// matrices fill the FP64 pipe (60 matrices): 1280 2.21 -> 2.24, 1408 2.71 -> 2.74, 1792 4.89 -> 4.57,
+// 2304 9.45 -> 7.89.
+constexpr int kModCholMin = 1280;
+constexpr int kModCholMinBatch = 1536;
 constexpr size_t kModBudget = (size_t)4 << 30;  // device bytes of one group of residue planes
 
 int fail(rpa_b200_handle* h, int status, const char* fmt, ...) {
@@ -759,10 +770,41 @@ rpa::LogdetPlan plan_for(const rpa_b200_handle* h, int n) {
   return it != h->logdet_plans.end() ? it->second : rpa::default_logdet_plan();
 }
 
+// Descriptors of the residue updates for nmat matrices of order n at A (uploaded when they differ from
+// those on the device): {nullptr} for small orders or without memory (the updates stay on DMMA).
+int mod_chol_for(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, int nmat, rpa::ModChol* out) {
+  out->mats = nullptr;
+  if (n < kModCholMin || h->ozaki_slices) return RPA_OK;
+  size_t pb, rb;
+  const size_t per = rpa::mod_chol_bytes(n, 256, &pb, &rb);
+  if (!try_ensure(h->mcBuf, per * nmat) || !try_ensure(h->mcDesc, sizeof(rpa::ModMat) * nmat)) {
+    release(h->mcBuf);
+    h->mc_mats.clear();
+    return RPA_OK;
+  }
+  uint8_t* base = static_cast<uint8_t*>(h->mcBuf.p);
+  const auto& m = h->mc_mats;
+  const bool same = (int)m.size() == nmat && m[0].A == A && m[0].ld == ld && m[0].n == n &&
+                    reinterpret_cast<uint8_t*>(m[0].planes) == base && (nmat == 1 || m[1].A == A + stride);
+  if (!same) {
+    h->mc_mats.assign(nmat, rpa::ModMat{});
+    for (int z = 0; z < nmat; ++z)
+      if (rpa::mod_chol_fill(h->encode, h->mc_mats[z], A + (int64_t)z * stride, ld, n, 256, base + per * z) != cudaSuccess) {
+        h->mc_mats.clear();
+        return fail(h, RPA_ERR_CUDA, "cuTensorMapEncodeTiled failed for residue planes");
+      }
+    RPA_CUDA(h, cudaMemcpyAsync(h->mcDesc.p, h->mc_mats.data(), sizeof(rpa::ModMat) * nmat, cudaMemcpyHostToDevice,
+                                h->stream));
+  }
+  out->mats = static_cast<const rpa::ModMat*>(h->mcDesc.p);
+  return RPA_OK;
+}
+
 // Time every candidate on nmat matrices of orders <= nmax (device descriptors; contents are
 // overwritten with seeded SPD test matrices), two runs each (the first also loads the variant's
 // kernels), keep the fastest for the bucket of nmax.  ms (6 entries or null): each candidate's time.
-int tune_logdet_on(rpa_b200_handle* h, const rpa::MatDesc* dmats, int nmat, int nmax, double* ms) {
+int tune_logdet_on(rpa_b200_handle* h, const rpa::MatDesc* dmats, int nmat, int nmax, double* ms,
+                   const rpa::ModChol* mc = nullptr) {
   cudaEvent_t t0 = pool_event(h), t1 = pool_event(h);
   if (!t0 || !t1) return fail(h, RPA_ERR_CUDA, "event creation failed");
   int best = 0;
@@ -773,7 +815,7 @@ int tune_logdet_on(rpa_b200_handle* h, const rpa::MatDesc* dmats, int nmat, int 
       RPA_CUDA(h, rpa::launch_fill_spd_varlen(dmats, nmat, nmax, 0x5eedull + (uint64_t)rep, h->stream));
       RPA_CUDA(h, cudaEventRecord(t0, h->stream));
       RPA_CUDA(h, rpa::launch_logdet_varlen(dmats, nmat, nmax, h->err_dev, h->stream, kLogdetCands[c],
-                                            h->lookahead ? &h->la[0] : nullptr));
+                                            h->lookahead ? &h->la[0] : nullptr, mc));
       RPA_CUDA(h, cudaEventRecord(t1, h->stream));
       RPA_CUDA(h, cudaEventSynchronize(t1));
       RPA_CUDA(h, cudaEventElapsedTime(&t, t0, t1));
@@ -807,7 +849,9 @@ int tune_uniform(rpa_b200_handle* h, int n, int nmat, double* base, double* ms) 
     mats[z].ld_dd = mats[z].tr_dd + 2;
   }
   RPA_CUDA(h, cudaMemcpyAsync(dmats, mats.data(), sizeof(rpa::MatDesc) * nmat, cudaMemcpyHostToDevice, h->stream));
-  int s = tune_logdet_on(h, dmats, nmat, n, ms);
+  rpa::ModChol mc;
+  int s = mod_chol_for(h, base, n, (int64_t)n * n, n, nmat, &mc);
+  if (s == RPA_OK) s = tune_logdet_on(h, dmats, nmat, n, ms, &mc);
   RPA_CUDA(h, cudaStreamSynchronize(h->stream));  // mats must outlive its copy
   return s;
 }
@@ -873,8 +917,10 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
   if (int ts = tune_single(h, n, nmat)) return ts;
   const rpa::LogdetPlan plan = plan_for(h, n);
   const rpa::OzakiWork* oz = ozaki_for(h, n, nmat, plan);
+  rpa::ModChol mc;
+  if (int ms = mod_chol_for(h, A, ld, stride, n, nmat, &mc)) return ms;
   for (auto& g : h->chol_graphs) {
-    if (g.A == A && g.ld == ld && g.stride == stride && g.n == n && g.nmat == nmat && g.Ldiag == Ldiag &&
+    if (g.mod == mc.mats && g.A == A && g.ld == ld && g.stride == stride && g.n == n && g.nmat == nmat && g.Ldiag == Ldiag &&
         g.stream == h->stream && g.nb2 == plan.nb2 && g.tile_w == plan.tile_w && g.oz == (oz ? oz->S : 0)) {
       RPA_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
       rpa::g_launches += g.launches;
@@ -885,7 +931,7 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
   cudaGraph_t graph = nullptr;
   if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
     cudaError_t e = rpa::launch_cholesky_lower(A, ld, stride, n, nmat, Ldiag, h->err_dev, h->stream, plan,
-                                               h->lookahead ? &h->la[0] : nullptr, oz);
+                                               h->lookahead ? &h->la[0] : nullptr, oz, &mc);
     cudaError_t e2 = cudaStreamEndCapture(h->stream, &graph);
     const int64_t count = rpa::g_launches - before;
     rpa::g_launches = before;
@@ -898,7 +944,7 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
         h->chol_graphs.erase(h->chol_graphs.begin());
       }
       h->chol_graphs.push_back(
-          {A, ld, stride, n, nmat, Ldiag, h->stream, plan.nb2, plan.tile_w, oz ? oz->S : 0, exec, count});
+          {A, ld, stride, n, nmat, Ldiag, h->stream, plan.nb2, plan.tile_w, oz ? oz->S : 0, mc.mats, exec, count});
       RPA_CUDA(h, cudaGraphLaunch(exec, h->stream));
       rpa::g_launches += count;
       return RPA_OK;
@@ -909,7 +955,7 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
     cudaGetLastError();
   }
   // capture unavailable on this stream: launch the same kernels directly
-  RPA_CUDA(h, rpa::launch_cholesky_lower(A, ld, stride, n, nmat, Ldiag, h->err_dev, h->stream, plan, nullptr, oz));
+  RPA_CUDA(h, rpa::launch_cholesky_lower(A, ld, stride, n, nmat, Ldiag, h->err_dev, h->stream, plan, nullptr, oz, &mc));
   return RPA_OK;
 }
 
@@ -1189,7 +1235,7 @@ int begin_call(rpa_b200_handle* h) {
   if (!h) return RPA_ERR_INVALID_ARG;
   h->last_error.clear();
   g_account = &h->account;
-  h->account.idle = {&h->Xhi, &h->Xlo, &h->gY, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE};
+  h->account.idle = {&h->Xhi, &h->Xlo, &h->gY, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE, &h->mcBuf, &h->bMod};
   h->pool_used = 0;
   h->split_ev.clear();
   h->tc_ev.clear();
@@ -1307,7 +1353,7 @@ int rpa_b200_destroy(rpa_b200_handle* h) try {
   if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
   for (DevBuf* b : {&h->R, &h->D, &h->eps, &h->Xhi, &h->Xlo, &h->diag_part, &h->diag, &h->Pi, &h->Ldiag, &h->ddbuf,
                     &h->tZ, &h->tOm, &h->tIOm, &h->tP, &h->tS, &h->tV, &h->tT, &h->tTIT, &h->tVt, &h->tW, &h->tU,
-                    &h->tRU, &h->tSmall, &h->tPerm, &h->bDesc, &h->bRes, &h->gY, &h->gD, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE,
+                    &h->tRU, &h->tSmall, &h->tPerm, &h->bDesc, &h->bRes, &h->gY, &h->gD, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE, &h->mcBuf, &h->mcDesc, &h->bMod,
                     &h->xM, &h->eW, &h->eA, &h->eZ, &h->thZ, &h->thXa, &h->thXi, &h->thYX, &h->thR,
                     &h->jU, &h->jL, &h->jX, &h->jPno, &h->jWork,
                     &h->jPack, &h->jQS, &h->jS, &h->jD, &h->syncBuf,
@@ -3067,7 +3113,7 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
   struct Per {
     int64_t pitch;
     rpa::SplitPlan plan;
-    size_t xb, pib, smallb;
+    size_t xb, pib, smallb, modb;  // modb: planes and residues of the log-det updates, per frequency
   };
   std::vector<Per> per(n);
   for (int i = 0; i < n; ++i) {
@@ -3077,6 +3123,8 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
     per[i].xb = prec == RPA_PREC_SPLIT_BF16 ? (size_t)v[i].K * v[i].NQ * per[i].pitch * 2 : 0;  // each of hi, lo
     per[i].pib = (size_t)v[i].K * v[i].NQ * v[i].NQ * 8;
     per[i].smallb = (size_t)v[i].K * v[i].NQ * 8 * (2 + per[i].plan.nsplit) + 64 * (size_t)v[i].K;
+    size_t pb, rb;
+    per[i].modb = v[i].NQ >= kModCholMinBatch && !h->ozaki_slices ? rpa::mod_chol_bytes(v[i].NQ, 256, &pb, &rb) : 0;
   }
   if (prec == RPA_PREC_FP64) {  // the bf16 operands are not used: give their memory to Pi
     RPA_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -3086,14 +3134,14 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
   size_t freeB = 0, totalB = 0;
   RPA_CUDA(h, cudaMemGetInfo(&freeB, &totalB));
   // buffers that ensure() below may free and reallocate count as available
-  const size_t have = h->Xhi.bytes + h->Xlo.bytes + h->Pi.bytes + h->Ldiag.bytes;
+  const size_t have = h->Xhi.bytes + h->Xlo.bytes + h->Pi.bytes + h->Ldiag.bytes + h->bMod.bytes;
   const size_t budget = h->batch_bytes > 0 ? h->batch_bytes : (size_t)(0.6 * (double)(freeB + have));
   std::vector<std::pair<int, int>> batches;  // [b0, b1)
   {
     size_t acc = 0;
     int b0 = 0;
     for (int i = 0; i < n; ++i) {
-      const size_t need = 2 * per[i].xb + per[i].pib + per[i].smallb;
+      const size_t need = 2 * per[i].xb + per[i].pib + per[i].smallb + v[i].K * per[i].modb;
       if (i > b0 && acc + need > budget) {
         batches.push_back({b0, i});
         b0 = i;
@@ -3103,10 +3151,10 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
     }
     batches.push_back({b0, n});
   }
-  size_t maxX = 0, maxPi = 0, maxSmall = 0;
+  size_t maxX = 0, maxPi = 0, maxSmall = 0, maxMod = 0;
   std::vector<size_t> desc_off(batches.size() + 1, 0), res_off(batches.size() + 1, 0);
   for (size_t b = 0; b < batches.size(); ++b) {
-    size_t x = 0, pi = 0, sm = 0, units = 0, work = 0, mats = 0;
+    size_t x = 0, pi = 0, sm = 0, units = 0, work = 0, mats = 0, md = 0;
     for (int i = batches[b].first; i < batches[b].second; ++i) {
       x += per[i].xb;
       pi += per[i].pib;
@@ -3114,11 +3162,14 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
       units += (size_t)v[i].K * rpa::syrk_tc_blocks(v[i].NQ);
       work += (size_t)per[i].plan.qtiles * per[i].plan.nsplit;
       mats += (size_t)v[i].K;
+      md += v[i].K * per[i].modb;
     }
+    maxMod = std::max(maxMod, md);
     const int ni = batches[b].second - batches[b].first;
     const size_t desc = ((sizeof(rpa::SyrkInst) * ni + 255) / 256 + (sizeof(rpa::SplitJob) * ni + 255) / 256 +
                          (sizeof(int64_t) * (ni + 1) + 255) / 256 + (sizeof(uint4) * units + 255) / 256 +
-                         (sizeof(int4) * work + 255) / 256 + (sizeof(rpa::MatDesc) * mats + 255) / 256) *
+                         (sizeof(int4) * work + 255) / 256 + (sizeof(rpa::MatDesc) * mats + 255) / 256 +
+                         (sizeof(rpa::ModMat) * mats + 255) / 256) *
                         256;
     desc_off[b + 1] = desc_off[b] + desc;
     res_off[b + 1] = res_off[b] + mats * 4;  // tr_dd, ld_dd per matrix
@@ -3137,6 +3188,8 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
   RPA_CUDA(h, ensure(h->Ldiag, 2 * smallStride + 256));
   RPA_CUDA(h, ensure(h->bDesc, desc_off.back() + 256));
   RPA_CUDA(h, ensure(h->bRes, res_off.back() * 8 + 256));
+  // without room for the planes the log-det's updates stay on DMMA
+  const bool mod_ld = maxMod > 0 && try_ensure(h->bMod, maxMod);
 
   // wave-milestone counters of every batch's multi-instance SYRK, allocated once for the call
   std::vector<int64_t> sync_off(batches.size() + 1, 0);
@@ -3160,7 +3213,7 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
   mix((uint64_t)prec);
   mix((uint64_t)h->seg_chunks);
   for (void* p : {h->Xhi.p, h->Xlo.p, h->Pi.p, h->Ldiag.p, h->bDesc.p, h->bRes.p, h->D.p, h->syncBuf.p,
-                  (void*)h->stream})
+                  mod_ld ? h->bMod.p : nullptr, (void*)h->stream})
     mix((uint64_t)(uintptr_t)p);
   for (int i = 0; i < n; ++i) {
     mix((uint64_t)(uintptr_t)Rd[i]);
@@ -3196,6 +3249,7 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
       int first, count, nmax;  // matrices [first, first + count) of the batch's (bucket-sorted) list
       int tune_count, tune_nmax;  // the tuner's subset: the first tune_count of them
       double cost;                // sum of n^3
+      int nmin;                   // smallest order
     };
     struct BatchDev {
       rpa::SyrkInst* sinst = nullptr;
@@ -3208,6 +3262,7 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
       int ni = 0;
       int64_t offs_total = 0;
       rpa::MatDesc* mats = nullptr;
+      rpa::ModMat* mod = nullptr;  // residue-update descriptors, parallel to mats
       std::vector<Bucket> buckets;
       std::vector<rpa::DsyrkArgs> fp64;  // FP64 form: one scaled SYRK per instance
       int* msync = nullptr;
@@ -3311,10 +3366,11 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
                        [](const rpa::MatDesc& a, const rpa::MatDesc& c) { return plan_bucket(a.n) < plan_bucket(c.n); });
       for (int m = 0; m < (int)mats.size(); ++m) {
         if (dv.buckets.empty() || plan_bucket(mats[m].n) != plan_bucket(mats[dv.buckets.back().first].n))
-          dv.buckets.push_back({m, 0, 0, 0, 0, 0.0});
+          dv.buckets.push_back({m, 0, 0, 0, 0, 0.0, INT32_MAX});
         Bucket& bk = dv.buckets.back();
         ++bk.count;
         bk.nmax = std::max(bk.nmax, mats[m].n);
+        bk.nmin = std::min(bk.nmin, mats[m].n);
         bk.cost += std::pow((double)mats[m].n, 3);
         if (bk.tune_count < 128) {
           ++bk.tune_count;
@@ -3335,6 +3391,17 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
       dv.units = reinterpret_cast<uint4*>(put(units.data(), sizeof(uint4) * units.size()));
       dv.work = reinterpret_cast<int4*>(put(work.data(), sizeof(int4) * work.size()));
       dv.mats = reinterpret_cast<rpa::MatDesc*>(put(mats.data(), sizeof(rpa::MatDesc) * mats.size()));
+      std::vector<rpa::ModMat> mod(mod_ld ? mats.size() : 0);
+      size_t mo = 0;
+      for (size_t m = 0; m < mod.size(); ++m) {
+        if (mats[m].n < kModCholMinBatch) continue;
+        size_t pb, rb;
+        if (rpa::mod_chol_fill(h->encode, mod[m], mats[m].A, mats[m].ld, mats[m].n, 256,
+                               static_cast<uint8_t*>(h->bMod.p) + mo) != cudaSuccess)
+          return fail(h, RPA_ERR_CUDA, "cuTensorMapEncodeTiled failed for residue planes");
+        mo += rpa::mod_chol_bytes(mats[m].n, 256, &pb, &rb);
+      }
+      if (mod_ld) dv.mod = reinterpret_cast<rpa::ModMat*>(put(mod.data(), sizeof(rpa::ModMat) * mod.size()));
       RPA_CUDA(h, cudaGetLastError());
       RPA_CUDA(h, cudaStreamSynchronize(h->stream));  // host vectors must outlive their copies
       dv.nunits = (int)units.size();
@@ -3345,12 +3412,21 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
       dv.sync_words = sync_off[b + 1] - sync_off[b];
       dv.msync = dv.sync_words > 0 ? static_cast<int*>(h->syncBuf.p) + sync_off[b] : nullptr;
     }
+    // residue updates of a bucket: all of its orders have descriptors, or none is used
+    auto bucket_mod = [&](const BatchDev& dv, const Bucket& bk) {
+      rpa::ModChol mc;
+      if (dv.mod && bk.nmin >= kModCholMinBatch) mc.mats = dv.mod + bk.first;
+      return mc;
+    };
     // ---- tile plans of order buckets met for the first time, tuned on this call's own buffers
     if (h->autotune) {
       for (const BatchDev& dv : bd)
         for (const Bucket& bk : dv.buckets)
           if (!h->logdet_plans.count(plan_bucket(bk.nmax)))
-            if ((s = tune_logdet_on(h, dv.mats + bk.first, bk.tune_count, bk.tune_nmax, nullptr))) return s;
+          {
+            const rpa::ModChol mc = bucket_mod(dv, bk);
+            if ((s = tune_logdet_on(h, dv.mats + bk.first, bk.tune_count, bk.tune_nmax, nullptr, &mc))) return s;
+          }
       RPA_CUDA(h, cudaMemsetAsync(h->err_dev, 0, sizeof(int), h->stream));
     }
     // ---- one graph for the whole call.  Split form: batch b+1's scale/split pass (branch aux[0])
@@ -3389,8 +3465,9 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
       for (int i : order) {
         if (r != cudaSuccess) break;
         const Bucket& bk = dv.buckets[i];
+        const rpa::ModChol mc = bucket_mod(dv, bk);
         r = rpa::launch_logdet_varlen(dv.mats + bk.first, bk.count, bk.nmax, h->err_dev, br[branch[i]],
-                                      plan_for(h, bk.nmax), h->lookahead ? &h->la[branch[i]] : nullptr);
+                                      plan_for(h, bk.nmax), h->lookahead ? &h->la[branch[i]] : nullptr, &mc);
       }
       for (int j = 1; j < nbr && r == cudaSuccess; ++j) {
         r = cudaEventRecord(h->fork_ev[j], br[j]);

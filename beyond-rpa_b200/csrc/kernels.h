@@ -210,9 +210,18 @@ cudaError_t launch_ozaki_slices(const OzakiWork& w, int buf, const double* A, in
 cudaError_t launch_ozaki_update(const OzakiWork& w, int buf, double* A, int64_t ld, int64_t stride, int n, int nmat,
                                 int row0, int col0, int nrows, int ncols, int* err, int num_sms, cudaStream_t stream);
 
+// Trailing updates by residue products (modgemm.cuh): device descriptors of the same matrices in the
+// same order, or mats == nullptr.
+struct ModMat;
+struct ModChol {
+  const ModMat* mats = nullptr;
+};
+// Outer block of the factorization under residue updates: a multiple of 128, at most 256 (the residue
+// buffers hold that many columns); 0 when the plan's block is none.
+inline int mod_chol_block(int nb2) { return nb2 % 128 != 0 ? 0 : nb2 < 256 ? nb2 : 256; }
 cudaError_t launch_cholesky_lower(double* A, int64_t ld, int64_t stride, int n, int nmat, double* Ldiag, int* err,
                                   cudaStream_t stream, const LogdetPlan& plan, const Lookahead* la = nullptr,
-                                  const OzakiWork* oz = nullptr);
+                                  const OzakiWork* oz = nullptr, const ModChol* mc = nullptr);
 // tr[z] = sum_i A_z(i,i) (double-double, deterministic); then A_z(i,i) += 1.
 // If `diag` is non-null the diagonal is first overwritten with diag[z*n+i].
 cudaError_t launch_trace_shift(double* A, int64_t ld, int64_t stride, int n, int nmat, const double* diag,
@@ -395,7 +404,7 @@ struct MatDesc {
 };
 // trace_shift + blocked Cholesky + log sums for nmat matrices of orders <= nmax.
 cudaError_t launch_logdet_varlen(const MatDesc* mats, int nmat, int nmax, int* err, cudaStream_t stream,
-                                 const LogdetPlan& plan, const Lookahead* la = nullptr);
+                                 const LogdetPlan& plan, const Lookahead* la = nullptr, const ModChol* mc = nullptr);
 // Overwrite the lower triangles of the matrices with a seeded, strictly diagonally dominant
 // symmetric test matrix (unit diagonal, |off-diagonal row sums| < 1/2): the input of the tile tuner.
 // One SYRK step of the variable-size schedule: mode 0 panel update, mode 1 trailing update,

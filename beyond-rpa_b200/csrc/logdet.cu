@@ -12,7 +12,7 @@
 
 #include <cstdlib>
 
-#include "kernels.h"
+#include "modgemm.cuh"
 
 namespace rpa {
 
@@ -538,6 +538,7 @@ struct LookaheadState {
   }
   // before (a) of block t: (b) of block t-1 done; the panel of block t is final
   cudaError_t before_next_block() {
+    if (!la) return cudaSuccess;
     cudaError_t e = cudaSuccess;
     if (rest_pending) e = cudaStreamWaitEvent(S, la->ev[2], 0);
     if (e == cudaSuccess) e = cudaEventRecord(la->ev[1], S);
@@ -557,6 +558,22 @@ struct LookaheadState {
     return e;
   }
 };
+
+// Residue form of the rest of the update: instead of panel t from every column right of block t + 1, all
+// panels 0 .. t from block t + 2 only, which is then read and written once (K = J1).  At order 4096
+// the read-modify-write of the whole trailing matrix by every panel would bound it.  The waits are
+// those of the right-looking form: block t + 2 is complete before the panel of block t + 1, on the
+// critical stream, is subtracted from it.
+cudaError_t mod_rest(LookaheadState& st, const ModMat* mats, int nmat, int n, int J0, int J1, int J2, int nb2,
+                     int* err) {
+  if (n - J2 <= 0) return cudaSuccess;
+  cudaError_t e = st.la ? st.fork_rest() : cudaSuccess;
+  const cudaStream_t R = st.la ? st.la->rest : st.S;
+  if (e == cudaSuccess) e = launch_mod_chol_planes(mats, nmat, n, J2, J0, nb2, R);
+  if (e == cudaSuccess) e = launch_mod_chol_update(mats, nmat, n, J2, nb2, J1, err, R);
+  if (e == cudaSuccess && st.la) e = st.rest_done();
+  return e;
+}
 
 DsyrkArgs update_args(double* A, int64_t ld, int64_t stride, int nmat, int row0, int col0, int n, int ncols,
                       int kdim, int tile_w) {
@@ -579,11 +596,14 @@ DsyrkArgs update_args(double* A, int64_t ld, int64_t stride, int nmat, int row0,
 
 cudaError_t launch_cholesky_lower(double* A, int64_t ld, int64_t stride, int n, int nmat, double* Ldiag, int* err,
                                   cudaStream_t stream, const LogdetPlan& plan, const Lookahead* la,
-                                  const OzakiWork* oz) {
+                                  const OzakiWork* oz, const ModChol* mc) {
   if (!valid_logdet_plan(plan)) return cudaErrorInvalidValue;
-  const int nb2 = plan.nb2;
-  if (oz && (oz->S == 0 || oz->K != nb2)) oz = nullptr;
+  if (oz && (oz->S == 0 || oz->K != plan.nb2)) oz = nullptr;
+  const bool use_mod = !oz && mc && mc->mats && mod_chol_block(plan.nb2) > 0;
+  const int nb2 = use_mod ? mod_chol_block(plan.nb2) : plan.nb2;
   if (cudaError_t e0 = panel_smem_optin()) return e0;
+  if (use_mod)
+    if (cudaError_t e0 = launch_mod_chol_expo(mc->mats, nmat, n, stream)) return e0;
   int obuf = 0;  // digit-plane buffer of the current outer block (alternates: the rest of block t's
                  // update may still read its planes while block t+1 is sliced)
   LookaheadState st{la, stream};
@@ -611,6 +631,14 @@ cudaError_t launch_cholesky_lower(double* A, int64_t ld, int64_t stride, int n, 
     }
     const int trail = n - J1;
     if (trail <= 0) break;
+    if (use_mod) {
+      const int J2 = min(n, J1 + nb2);
+      if ((e = st.before_next_block()) != cudaSuccess) return e;
+      e = launch_dsyrk_lower(update_args(A, ld, stride, nmat, J1, J0, trail, J2 - J1, J1 - J0, plan.tile_w), S);
+      if (e == cudaSuccess) e = mod_rest(st, mc->mats, nmat, n, J0, J1, J2, nb2, err);
+      if (e != cudaSuccess) return e;
+      continue;
+    }
     // full-width panels take the int8 route; a narrower last panel (n not a multiple of nb2) stays on DMMA
     const bool use_oz = oz && J1 - J0 == oz->K;
     if (use_oz && (e = launch_ozaki_slices(*oz, obuf, A, ld, stride, n, nmat, J1, J0, S)) != cudaSuccess) return e;
@@ -642,7 +670,7 @@ cudaError_t launch_cholesky_lower(double* A, int64_t ld, int64_t stride, int n, 
 // every step is launched for the largest order and matrices that are already
 // finished (or too small for the step) leave at once.
 cudaError_t launch_logdet_varlen(const MatDesc* mats, int nmat, int nmax, int* err, cudaStream_t stream,
-                                 const LogdetPlan& plan, const Lookahead* la) {
+                                 const LogdetPlan& plan, const Lookahead* la, const ModChol* mc) {
   if (nmat <= 0) return cudaSuccess;
   if (!valid_logdet_plan(plan)) return cudaErrorInvalidValue;
   if (cudaError_t e0 = panel_smem_optin()) return e0;
@@ -650,7 +678,9 @@ cudaError_t launch_logdet_varlen(const MatDesc* mats, int nmat, int nmax, int* e
   ++g_launches;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const int nb2 = plan.nb2;
+  const bool use_mod = mc && mc->mats && mod_chol_block(plan.nb2) > 0;
+  const int nb2 = use_mod ? mod_chol_block(plan.nb2) : plan.nb2;
+  if (use_mod && (e = launch_mod_chol_expo(mc->mats, nmat, nmax, stream)) != cudaSuccess) return e;
   LookaheadState st{la, stream};
   if ((e = st.begin(stream)) != cudaSuccess) return e;
   const cudaStream_t S = st.S;
@@ -667,6 +697,13 @@ cudaError_t launch_logdet_varlen(const MatDesc* mats, int nmat, int nmax, int* e
       if (e != cudaSuccess) return e;
     }
     if (nmax - J1 <= 0) break;
+    if (use_mod) {
+      if ((e = st.before_next_block()) != cudaSuccess) return e;
+      e = launch_dsyrk_varlen(mats, nmat, 2, J0, 0, nb2, plan.tile_w, nmax, S);
+      if (e == cudaSuccess) e = mod_rest(st, mc->mats, nmat, nmax, J0, J1, J1 + nb2, nb2, err);
+      if (e != cudaSuccess) return e;
+      continue;
+    }
     if (!la) {
       e = launch_dsyrk_varlen(mats, nmat, 1, J0, 0, nb2, plan.tile_w, nmax, S);
       if (e != cudaSuccess) return e;

@@ -374,6 +374,42 @@ struct MgFull {
   }
 };
 
+// Block column of a batch of Cholesky factors: a CTA takes one tile of one matrix and a third of the
+// moduli.  CTAs live for microseconds, so that the launches of the critical path, on a stream of
+// higher priority, find SMs (a persistent launch would hold them all until its end).
+constexpr int MG_GROUPS = 3;
+struct MgChol {
+  const ModMat* mat;
+  const ModCholArgs& a;
+  int t, g;  // tile, third of the moduli
+  __device__ __forceinline__ int begin() const { return g * (kModCount / MG_GROUPS); }
+  __device__ __forceinline__ int end() const { return (g + 1) * (kModCount / MG_GROUPS); }
+  __device__ __forceinline__ int step() const { return 1; }
+  __device__ __forceinline__ int nch() const { return a.K / MG_TK; }
+  __device__ __forceinline__ int64_t ldo() const { return mat->ldo; }
+  __device__ __forceinline__ bool any() const {
+    const int tj = t % a.ntj, ti = t / a.ntj;
+    return a.col0 + tj * MG_TM < mat->n && a.col0 + ti * MG_TN < mat->n && tj <= 2 * ti + 1 && (tj == 0 || a.col0 + ti * MG_TN + (tj == 2 * ti + 1 ? MG_TM : 0) < mat->n);
+  }
+  __device__ __forceinline__ MgUnit get(int m) const {
+    MgUnit x;
+    const int tj = t % a.ntj, ti = t / a.ntj;
+    x.m = x.pa = x.pb = m;
+    x.ni = MG_TN;
+    int i0 = ti * MG_TN;
+    if (tj == 2 * ti + 1) {
+      i0 += MG_TM;
+      x.ni = MG_TM;
+    }
+    x.j0 = a.col0 + tj * MG_TM;
+    x.i0 = a.col0 + i0;
+    x.live = true;
+    x.nj = min(MG_TM, min(a.nb, mat->n - a.col0) - tj * MG_TM);
+    x.out = mat->res + (int64_t)m * a.nb * mat->ldo + (int64_t)(tj * MG_TM) * mat->ldo + i0;
+    return x;
+  }
+};
+
 __device__ __forceinline__ bool mg_wait_count(const int* c, int target) {
   for (uint32_t it = 0; it < (1u << 20); ++it) {
     int v;
@@ -566,6 +602,67 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
     modgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmBh, const ModGemmArgs a, const ModReduce red) {
   modgemm_body(MgFull{&tmA, &tmB, &tmBh, a}, &tmA, &tmB, &tmBh, a.sync, a.sync_every, a.err, red);
+}
+
+__global__ void __launch_bounds__(MG_THREADS, 1)
+    modgemm_chol_kernel(const ModMat* __restrict__ mats, const ModCholArgs a, const ModReduce red) {
+  const ModMat* mat = mats + blockIdx.y;
+  MgChol src{mat, a, (int)blockIdx.x / MG_GROUPS, (int)blockIdx.x % MG_GROUPS};
+  if (!src.any()) return;  // CTA-uniform
+  modgemm_body(src, &mat->mA, &mat->mB, &mat->mA, nullptr, 1, a.err, red);
+}
+
+// Power of two of every row of a Cholesky factor, known beforehand: ||L_i||^2 = A_ii.
+__global__ void mod_chol_expo_kernel(const ModMat* __restrict__ mats) {
+  const ModMat& m = mats[blockIdx.y];
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < m.n) m.expo[i] = mod_exponent(m.A[i + m.ld * (int64_t)i], 0);
+}
+
+// Planes of columns c0 .. c0 + nb - 1 (nb a multiple of 128), rows row0 .. n - 1, of the factors: the
+// block transposition of mod_pi_kernel.
+__global__ void __launch_bounds__(256, 4) mod_chol_planes_kernel(const ModMat* __restrict__ mats, int row0, int c0) {
+  __shared__ __align__(16) double rs[32 * kPiPitch];
+  const ModMat& m = mats[blockIdx.z];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q0 = row0 + blockIdx.x * 32, b0 = c0 + blockIdx.y * 128;
+  if (q0 >= m.n) return;
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    rs[lane * kPiPitch + warp + 8 * j] = q0 + lane < m.n ? m.A[q0 + lane + m.ld * (int64_t)(b0 + warp + 8 * j)] : 0.0;
+  __syncthreads();
+  const int64_t plane_stride = (int64_t)m.n * m.pitch;
+  for (int q = warp; q < 32 && q0 + q < m.n; q += 8) {
+    const double sc = mod_pow2(m.expo[q0 + q]);
+    const double2* r2 = reinterpret_cast<const double2*>(rs + q * kPiPitch + 4 * lane);
+    const double2 ra = r2[0], rb = r2[1];
+    uint32_t lo[4], hi[4];
+    to_words(ra.x * sc, lo[0], hi[0]);
+    to_words(ra.y * sc, lo[1], hi[1]);
+    to_words(rb.x * sc, lo[2], hi[2]);
+    to_words(rb.y * sc, lo[3], hi[3]);
+    int8_t* out = m.planes + (int64_t)(q0 + q) * m.pitch + b0 + 4 * lane;
+    mod_all<4>(
+        lo, hi, [&](int k, const uint32_t(&w)[1]) { *reinterpret_cast<uint32_t*>(out + k * plane_stride) = w[0]; },
+        std::make_integer_sequence<int, kModCount>());
+  }
+}
+
+// A(i, j) -= (sum_k L(i, k) L(j, k)) for the block column at col0, from its residues.
+__global__ void __launch_bounds__(256) mod_chol_crt_kernel(const ModMat* __restrict__ mats, int col0, int nb,
+                                                           const ModCrt crt) {
+  const ModMat& m = mats[blockIdx.z];
+  const int j = blockIdx.y, i0 = 4 * (int)(blockIdx.x * 256 + threadIdx.x);  // relative to col0
+  if (col0 + j >= m.n || col0 + i0 >= m.n || i0 + 3 < j) return;
+  double c[4];
+  mod_crt4(m.res + (int64_t)j * m.ldo + i0, (int64_t)nb * m.ldo, crt, c);
+  const double sj = mod_pow2(-m.expo[col0 + j]);
+  double* dst = m.A + col0 + m.ld * (int64_t)(col0 + j);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    if (i >= j && col0 + i < m.n) dst[i] -= c[e] * mod_pow2(-m.expo[col0 + i]) * sj;
+  }
 }
 
 // ------------------------------------------------------------------ C from its residues
@@ -820,6 +917,63 @@ cudaError_t launch_mod_grad(const double* R, int64_t ldR, const uint8_t* res, in
   mod_grad_kernel<<<(unsigned)((nov + 7) / 8), 256, 0, stream>>>(R, ldR, res, plane, ldo, tables().crt, expo_m, expo_r,
                                                                  NQ, nov, D, gg, dR, lddR, dD, first ? 1 : 0);
   ++g_launches;
+  return cudaGetLastError();
+}
+
+size_t mod_chol_bytes(int n, int nb, size_t* planes, size_t* res) {
+  *planes = (size_t)kModCount * n * (size_t)mod_pitch(n);
+  *res = (size_t)kModCount * nb * (size_t)((n + 255) / 256 * 256);
+  return *planes + *res + ((size_t)n * sizeof(int) + 255) / 256 * 256;
+}
+
+cudaError_t mod_chol_fill(PFN_cuTensorMapEncodeTiled_v12000 encode, ModMat& m, double* A, int64_t ld, int n, int nb,
+                          uint8_t* base) {
+  size_t pb, rb;
+  mod_chol_bytes(n, nb, &pb, &rb);
+  m.A = A;
+  m.ld = ld;
+  m.n = n;
+  m.pitch = (int)mod_pitch(n);
+  m.ldo = (n + 255) / 256 * 256;
+  m.planes = reinterpret_cast<int8_t*>(base);
+  m.res = base + pb;
+  m.expo = reinterpret_cast<int*>(base + pb + rb);
+  cudaError_t e = mod_map(encode, &m.mA, m.planes, n, n, kModCount, m.pitch, MG_TM);
+  return e == cudaSuccess ? mod_map(encode, &m.mB, m.planes, n, n, kModCount, m.pitch, MG_TN) : e;
+}
+
+cudaError_t launch_mod_chol_expo(const ModMat* mats, int nmat, int nmax, cudaStream_t stream) {
+  mod_chol_expo_kernel<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)nmat), 256, 0, stream>>>(mats);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_chol_planes(const ModMat* mats, int nmat, int nmax, int row0, int c0, int nb,
+                                   cudaStream_t stream) {
+  if (row0 >= nmax) return cudaSuccess;
+  mod_chol_planes_kernel<<<dim3((unsigned)((nmax - row0 + 31) / 32), (unsigned)(nb / 128), (unsigned)nmat), 256, 0,
+                           stream>>>(mats, row0, c0);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_chol_update(const ModMat* mats, int nmat, int nmax, int col0, int nb, int K, int* err,
+                                   cudaStream_t stream) {
+  if (col0 >= nmax || K <= 0) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(modgemm_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM);
+  if (e != cudaSuccess) return e;
+  ModCholArgs a;
+  a.col0 = col0;
+  a.nb = nb;
+  a.K = K;
+  a.ntj = nb / MG_TM;
+  a.err = err;
+  const int rows = nmax - col0, nti = (rows + MG_TN - 1) / MG_TN;
+  modgemm_chol_kernel<<<dim3((unsigned)(nti * a.ntj * MG_GROUPS), (unsigned)nmat), MG_THREADS, MG_SMEM, stream>>>(
+      mats, a, tables().red);
+  mod_chol_crt_kernel<<<dim3((unsigned)((rows + 1023) / 1024), (unsigned)std::min(nb, rows), (unsigned)nmat), 256, 0,
+                        stream>>>(mats, col0, nb, tables().crt);
+  g_launches += 2;
   return cudaGetLastError();
 }
 

@@ -115,4 +115,30 @@ cudaError_t launch_mod_grad(const double* R, int64_t ldR, const uint8_t* res, in
                             const int* expo_m, const int* expo_r, int NQ, int64_t nov, const double* D,
                             const GradGroup& gg, double* dR, int64_t lddR, double* dD, bool first,
                             cudaStream_t stream);
+// ---- block columns of Cholesky factors (log-det trailing updates)
+// One matrix: its factor's columns are converted panel by panel; a block column gets the products of
+// all panels before it at once (K up to the order), so that it is read and written once.
+struct ModMat {
+  CUtensorMap mA, mB;  // planes as 128- and 256-row boxes
+  double* A;
+  int64_t ld;
+  int8_t* planes;  // [modulus][row][pitch]
+  uint8_t* res;    // [modulus][column of the block][ldo]
+  int* expo;       // powers of two of the rows
+  int n, pitch, ldo;
+};
+struct ModCholArgs {
+  int col0, nb, K, ntj;
+  int* err;
+};
+size_t mod_chol_bytes(int n, int nb, size_t* planes, size_t* res);  // of one matrix
+cudaError_t mod_chol_fill(PFN_cuTensorMapEncodeTiled_v12000 encode, ModMat& m, double* A, int64_t ld, int n, int nb,
+                          uint8_t* base);
+cudaError_t launch_mod_chol_expo(const ModMat* mats, int nmat, int nmax, cudaStream_t stream);
+// Planes of the factored columns c0 .. c0 + nb - 1, rows row0 and below.
+cudaError_t launch_mod_chol_planes(const ModMat* mats, int nmat, int nmax, int row0, int c0, int nb,
+                                   cudaStream_t stream);
+// A(i, j) -= sum_{k < K} L(i, k) L(j, k) for i >= j, col0 <= j < col0 + nb.
+cudaError_t launch_mod_chol_update(const ModMat* mats, int nmat, int nmax, int col0, int nb, int K, int* err,
+                                   cudaStream_t stream);
 }  // namespace rpa
