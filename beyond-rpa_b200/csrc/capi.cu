@@ -453,10 +453,9 @@ bool try_ensure(DevBuf& b, size_t bytes) {
 int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t planesA, int rowsA, int8_t* pb,
                 int64_t planesB, int rowsB, int64_t K, int nz, bool tri, uint8_t* out, int64_t ldo) {
   const int64_t pitch = rpa::mod_pitch(K);
-  CUtensorMap mA, mB, mBh;
+  CUtensorMap mA, mB;
   if (rpa::mod_map(h->encode, &mA, pa, K, rowsA, planesA, pitch, 128) != cudaSuccess ||
-      rpa::mod_map(h->encode, &mB, pb, K, rowsB, planesB, pitch, 256) != cudaSuccess ||
-      rpa::mod_map(h->encode, &mBh, pb, K, rowsB, planesB, pitch, 128) != cudaSuccess)
+      rpa::mod_map(h->encode, &mB, pb, K, rowsB, planesB, pitch, 128) != cudaSuccess)
     return fail(h, RPA_ERR_CUDA, "cuTensorMapEncodeTiled failed for residue planes");
   RPA_CUDA(h, rpa::mod_plan(a, rowsA, rowsB, K, nz, tri));
   a.zplanesA = planesA > rpa::kModCount ? rpa::kModCount : 0;
@@ -473,7 +472,7 @@ int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t pla
     RPA_CUDA(h, cudaMemsetAsync(h->syncBuf.p, 0, (size_t)words * sizeof(int), h->stream));
     a.sync = static_cast<int*>(h->syncBuf.p);
   }
-  RPA_CUDA(h, rpa::launch_modgemm(mA, mB, mBh, a, h->num_sms, h->stream));
+  RPA_CUDA(h, rpa::launch_modgemm(mA, mB, a, h->num_sms, h->stream));
   return RPA_OK;
 }
 

@@ -17,7 +17,8 @@
 //
 //  * mod_cols_kernel: operands whose K index is contiguous (column-major K x rows)
 //  * mod_pi_kernel:   X_k(Q, ai) = sqrt(alpha c_k(ai)) R(Q, ai), transposed to ai-contiguous rows
-//  * modgemm_kernel:  residues of C, 15 int8 products per tile
+//  * modgemm_pair_kernel: residues of C, 15 int8 products per tile, tiles of 256 x 256 on CTA pairs
+//  * modgemm_chol_kernel: the same for block columns of Cholesky factors
 //  * mod_*crt*:       C from its residues
 #include <algorithm>
 #include <utility>
@@ -329,49 +330,8 @@ __device__ __forceinline__ uint64_t desc_k_sw128(uint32_t addr) {
 // One tile of one modulus: operand rows j0 .. (128 lanes) and i0 .. (ni columns) of planes pa and pb.
 struct MgUnit {
   int m, j0, i0, ni, pa, pb;
-  bool live;
   uint8_t* out;  // residues of (j0, i0)
   int nj;        // rows of the tile that are stored
-};
-
-// Persistent launch over (batch, modulus, tile), tiles of one plane next to one another.
-struct MgFull {
-  const CUtensorMap *mA, *mB, *mBh;
-  const ModGemmArgs& a;
-  __device__ __forceinline__ int begin() const { return blockIdx.x; }
-  __device__ __forceinline__ int end() const { return a.nunits; }
-  __device__ __forceinline__ int step() const { return gridDim.x; }
-  __device__ __forceinline__ int nch() const { return a.nch; }
-  __device__ __forceinline__ int64_t ldo() const { return a.ldo; }
-  __device__ __forceinline__ MgUnit get(int u) const {
-    MgUnit x;
-    const int zm = u / a.ntiles, t = u - zm * a.ntiles;
-    const int z = zm / kModCount;
-    x.m = zm - z * kModCount;
-    int ti, tj;
-    if (a.tri) {  // ti-major: tile (ti, tj) with tj <= 2 ti + 1 (only i >= j is kept)
-      ti = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-      while ((ti + 1) * (ti + 2) <= t) ++ti;
-      while (ti * (ti + 1) > t) --ti;
-      tj = t - ti * (ti + 1);
-    } else {
-      tj = t / a.nti;
-      ti = t - tj * a.nti;
-    }
-    x.j0 = tj * MG_TM;
-    x.i0 = ti * MG_TN;
-    x.ni = MG_TN;
-    if (a.tri && tj == 2 * ti + 1) {  // the first 128 columns lie above the diagonal
-      x.i0 += MG_TM;
-      x.ni = MG_TM;
-    }
-    x.pa = z * a.zplanesA + x.m;
-    x.pb = z * a.zplanesB + x.m;
-    x.live = true;
-    x.nj = a.rowsA - x.j0;
-    x.out = a.out + (int64_t)zm * a.out_plane + (int64_t)x.j0 * a.ldo + x.i0;
-    return x;
-  }
 };
 
 // Block column of a batch of Cholesky factors: a CTA takes one tile of one matrix and a third of the
@@ -403,7 +363,6 @@ struct MgChol {
     }
     x.j0 = a.col0 + tj * MG_TM;
     x.i0 = a.col0 + i0;
-    x.live = true;
     x.nj = min(MG_TM, min(a.nb, mat->n - a.col0) - tj * MG_TM);
     x.out = mat->res + (int64_t)m * a.nb * mat->ldo + (int64_t)(tj * MG_TM) * mat->ldo + i0;
     return x;
@@ -420,10 +379,29 @@ __device__ __forceinline__ bool mg_wait_count(const int* c, int target) {
   return false;
 }
 
+// Residues of 64 accumulator columns (one row per lane) added to those in w, four to a word:
+// r = acc mod p in [0, p].
+__device__ __forceinline__ void mod_drain(uint32_t taddr, int p, int mg, uint32_t (&w)[16]) {
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    float v[32];
+    tmem_ld_32x32b_x32(taddr + (uint32_t)(half * 32), v);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      uint32_t r[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int acc = __float_as_int(v[4 * t + e]) + (int)((w[half * 8 + t] >> (8 * e)) & 255u);
+        r[e] = (uint32_t)(acc - (__mulhi(acc, mg) >> 6) * p);
+      }
+      w[half * 8 + t] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+    }
+  }
+}
+
 template <class Src>
 __device__ __forceinline__ void modgemm_body(const Src& src, const CUtensorMap* tmA, const CUtensorMap* tmB,
-                                             const CUtensorMap* tmBh, int* sync, int sync_every, int* err,
-                                             const ModReduce& red) {
+                                             const CUtensorMap* tmBh, int* err, const ModReduce& red) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + MG_STAGES * MG_STAGE);
@@ -459,21 +437,12 @@ __device__ __forceinline__ void modgemm_body(const Src& src, const CUtensorMap* 
       tma_prefetch_desc(tmB);
       int stage = 0;
       uint32_t phase = 0, issued = 0, issued_par = 0;
-      bool ok = true, sync_wait = true;
-      const int nmile = sync ? (src.nch() + sync_every - 1) / sync_every : 0;
+      bool ok = true;
       for (int u = src.begin(); u < src.end() && ok; u += src.step()) {
         const MgUnit x = src.get(u);
-        const int wave = sync ? (u - (int)blockIdx.x) / (int)gridDim.x : 0;
-        const int members = min((int)gridDim.x, src.end() - wave * (int)gridDim.x);
         const CUtensorMap* mb = x.ni == MG_TN ? tmB : tmBh;
         const uint32_t bytes = (uint32_t)(MG_TM + x.ni) * MG_TK;
         for (int ch = 0; ch < src.nch(); ++ch) {
-          if (sync && ch % sync_every == 0) {
-            const int mi = ch / sync_every;
-            int* row = sync + (int64_t)wave * nmile;
-            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(row + mi) : "memory");
-            if (sync_wait && mi >= 2) sync_wait = mg_wait_count(row + mi - 2, members);
-          }
           if (!mbar_wait(&empty[stage], phase ^ 1u, err, kDevTimeoutTmaEmpty)) {
             ok = false;
             break;
@@ -560,22 +529,7 @@ __device__ __forceinline__ void modgemm_body(const Src& src, const CUtensorMap* 
         }
         tc_fence_after();
         if (col0 < x.ni) {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            float v[32];
-            tmem_ld_32x32b_x32(
-                tmem_base + (uint32_t)(b * MG_TN + col0 + half * 32) + ((uint32_t)(quarter * 32) << 16), v);
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              uint32_t r[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int acc = __float_as_int(v[4 * t + e]) + (int)((w[half * 8 + t] >> (8 * e)) & 255u);
-                r[e] = (uint32_t)(acc - (__mulhi(acc, mg) >> 6) * p);
-              }
-              w[half * 8 + t] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
-            }
-          }
+          mod_drain(tmem_base + (uint32_t)(b * MG_TN + col0) + ((uint32_t)(quarter * 32) << 16), p, mg, w);
         }
         tc_fence_before();
         __syncwarp();
@@ -599,17 +553,260 @@ __device__ __forceinline__ void modgemm_body(const Src& src, const CUtensorMap* 
 }
 
 __global__ void __launch_bounds__(MG_THREADS, 1)
-    modgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const __grid_constant__ CUtensorMap tmBh, const ModGemmArgs a, const ModReduce red) {
-  modgemm_body(MgFull{&tmA, &tmB, &tmBh, a}, &tmA, &tmB, &tmBh, a.sync, a.sync_every, a.err, red);
-}
-
-__global__ void __launch_bounds__(MG_THREADS, 1)
     modgemm_chol_kernel(const ModMat* __restrict__ mats, const ModCholArgs a, const ModReduce red) {
   const ModMat* mat = mats + blockIdx.y;
   MgChol src{mat, a, (int)blockIdx.x / MG_GROUPS, (int)blockIdx.x % MG_GROUPS};
   if (!src.any()) return;  // CTA-uniform
-  modgemm_body(src, &mat->mA, &mat->mB, &mat->mA, nullptr, 1, a.err, red);
+  modgemm_body(src, &mat->mA, &mat->mB, &mat->mA, a.err, red);
+}
+
+// ------------------------------------------------------------------ CTA pairs
+// The full and triangular products as 256 x 256 tiles on pairs of SMs (cta_group::2): each CTA loads
+// 128 rows of either operand and accumulates 128 of the tile's rows, so that a k step moves 32 KB per
+// CTA for the work that takes 48 KB of one CTA.  One int8 tile of 128 x 256 asks L2 for 96 bytes per
+// clock and SM, and the tensor pipe of the one-CTA kernel was 76 % busy waiting for them.
+// The even CTA issues every MMA; its `full` barriers count the bytes of both CTAs, `empty` and
+// `acc_full` are signalled in both by multicast commits, `acc_empty` collects both epilogues.
+constexpr int M2_STAGES = 6;
+constexpr int M2_STAGE = 2 * MG_ABYTES;
+constexpr int M2_SMEM = M2_STAGES * M2_STAGE + 1024 + 256;
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The even CTA's copy of a shared-memory object of this CTA.
+__device__ __forceinline__ uint32_t leader_addr(const void* p) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+  return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const void* tmap, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+      "%3, %4}], [%5];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void mma_s8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Arrive on the barrier at this offset in both CTAs once the MMAs issued so far have completed.
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+
+struct PairUnit {
+  int m, j0, i0, pa, pb, zm;
+};
+__device__ __forceinline__ PairUnit pair_unit(int u, const ModGemmArgs& a) {
+  PairUnit x;
+  int ti, tj, z;
+  if (a.tri) {  // (batch, modulus, tile), ti-major, tj <= ti
+    const int zm = u / a.ntiles, t = u - zm * a.ntiles;
+    z = zm / kModCount;
+    x.m = zm - z * kModCount;
+    ti = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+    while (ti * (ti + 1) / 2 > t) --ti;
+    tj = t - ti * (ti + 1) / 2;
+  } else {  // (modulus, tj, batch, ti): the rows of a shared first operand stay in L2 for every batch
+    ti = u % a.nti;
+    int q = u / a.nti;
+    z = q % a.nz;
+    q /= a.nz;
+    tj = q % a.ntj;
+    x.m = q / a.ntj;
+  }
+  x.zm = z * kModCount + x.m;
+  x.j0 = tj * 256;
+  x.i0 = ti * 256;
+  x.pa = z * a.zplanesA + x.m;
+  x.pb = z * a.zplanesB + x.m;
+  return x;
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
+    modgemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                        const ModGemmArgs a, const ModReduce red) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + M2_STAGES * M2_STAGE);
+  uint64_t* empty = full + M2_STAGES;
+  uint64_t* acc_full = empty + M2_STAGES;
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* drain = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < M2_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 32);
+    }
+    mbar_init(drain, 1);
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ------------------------------------------------------------ producer: this CTA's halves
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
+      int stage = 0;
+      uint32_t phase = 0, issued = 0, issued_par = 0;
+      bool ok = true, sync_wait = rank == 0;
+      const int nmile = a.sync && rank == 0 ? (a.nch + a.sync_every - 1) / a.sync_every : 0;
+      for (int u = pair; u < a.nunits && ok; u += npairs) {
+        const PairUnit x = pair_unit(u, a);
+        const int wave = (u - pair) / npairs;
+        const int members = min(npairs, a.nunits - wave * npairs);
+        for (int ch = 0; ch < a.nch; ++ch) {
+          if (nmile && ch % a.sync_every == 0) {
+            const int mi = ch / a.sync_every;
+            int* row = a.sync + (int64_t)wave * nmile;
+            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(row + mi) : "memory");
+            if (sync_wait && mi >= 2) sync_wait = mg_wait_count(row + mi - 2, members);
+          }
+          if (!mbar_wait(&empty[stage], phase ^ 1u, a.err, kDevTimeoutTmaEmpty)) {
+            ok = false;
+            break;
+          }
+          if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * M2_STAGE);
+          uint8_t* st = smem + stage * M2_STAGE;
+          const uint32_t bar = leader_addr(&full[stage]);
+          tma_load_3d_pair(st, &tmA, bar, ch * MG_TK, x.j0 + rank * MG_TM, x.pa);
+          tma_load_3d_pair(st + MG_ABYTES, &tmB, bar, ch * MG_TK, x.i0 + rank * MG_TM, x.pb);
+          issued |= 1u << stage;
+          issued_par = (issued_par & ~(1u << stage)) | (phase << stage);
+          if (++stage == M2_STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      // every issued load has landed (the even CTA counts the bytes of both) and been consumed before the
+      // shared memory goes: both CTAs meet at the cluster barrier below
+      for (int s = 0; s < M2_STAGES; ++s)
+        if (issued & (1u << s)) {
+          if (rank == 0) mbar_wait(&full[s], (issued_par >> s) & 1u, a.err, kDevTimeoutDrain);
+          mbar_wait(&empty[s], (issued_par >> s) & 1u, a.err, kDevTimeoutDrain);
+        }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      // ------------------------------------------------------------ MMA issuer (even CTA)
+      constexpr uint32_t idesc = idesc_s8_s32(256, 256);
+      int stage = 0, it = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int u = pair; u < a.nunits && ok; u += npairs) {
+        for (int c0 = 0; c0 < a.nch && ok; c0 += MG_SEG, ++it) {
+          const int b = it & 1;
+          if (!mbar_wait(&acc_empty[b], (uint32_t)((it >> 1) & 1) ^ 1u, a.err, kDevTimeoutAccEmpty)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d = tmem_base + (uint32_t)(b * 256);
+          const int c1 = min(a.nch, c0 + MG_SEG);
+          for (int ch = c0; ch < c1; ++ch) {
+            if (!mbar_wait(&full[stage], phase, a.err, kDevTimeoutTmaFull)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(smem + stage * M2_STAGE), sb = sa + MG_ABYTES;
+#pragma unroll
+            for (int kk = 0; kk < MG_TK / 32; ++kk)
+              mma_s8_pair(d, desc_k_sw128(sa + kk * 32), desc_k_sw128(sb + kk * 32), idesc,
+                          (ch > c0 || kk > 0) ? 1u : 0u);
+            commit_pair(&empty[stage]);
+            if (++stage == M2_STAGES) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+          if (!ok) break;
+          commit_pair(&acc_full[b]);
+        }
+      }
+      // every issued MMA must complete before TMEM is freed
+      commit_pair(drain);
+      mbar_wait(drain, 0, a.err, kDevTimeoutDrain);
+    }
+  } else {
+    // -------------------------------------------------------------- epilogue (both CTAs: 128 rows each)
+    const int quarter = warp & 3;
+    const int col0 = ((warp - 2) >> 2) * 64;
+    const uint32_t release[2] = {leader_addr(&acc_empty[0]), leader_addr(&acc_empty[1])};
+    int it = 0;
+    bool ok = true;
+    for (int u = pair; u < a.nunits && ok; u += npairs) {
+      const PairUnit x = pair_unit(u, a);
+      const int p = red.p[x.m];
+      const int mg = red.magic[x.m];
+      uint32_t w[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w[i] = 0;
+      for (int c0 = 0; c0 < a.nch; c0 += MG_SEG, ++it) {
+        const int b = it & 1;
+        if (!mbar_wait(&acc_full[b], (uint32_t)((it >> 1) & 1), a.err, kDevTimeoutAccFull)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        mod_drain(tmem_base + (uint32_t)(b * 256 + col0) + ((uint32_t)(quarter * 32) << 16), p, mg, w);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(release[b]);
+      }
+      if (!ok) break;
+      const int j = x.j0 + rank * MG_TM + quarter * 32 + lane;
+      if (j < a.rowsA) {
+        uint4* dst = reinterpret_cast<uint4*>(a.out + (int64_t)x.zm * a.out_plane + (int64_t)j * a.ldo + x.i0 + col0);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) dst[t] = make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs are done with each other's barriers and with the accumulators
+  tc_fence_after();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
 }
 
 // Power of two of every row of a Cholesky factor, known beforehand: ||L_i||^2 = A_ii.
@@ -860,20 +1057,18 @@ cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, in
 
 int64_t mod_sync_words(const ModGemmArgs& a, int num_sms) {
   if (a.sync_every <= 0) return 0;
-  const int grid = std::min(a.nunits, num_sms);
-  return grid <= 0 ? 0 : (int64_t)((a.nunits + grid - 1) / grid) * ((a.nch + a.sync_every - 1) / a.sync_every);
+  const int pairs = std::min(a.nunits, num_sms / 2);
+  return pairs <= 0 ? 0 : (int64_t)((a.nunits + pairs - 1) / pairs) * ((a.nch + a.sync_every - 1) / a.sync_every);
 }
 
 cudaError_t mod_plan(ModGemmArgs& a, int rowsA, int rowsB, int64_t K, int nz, bool tri) {
   a.rowsA = rowsA;
   a.nch = (int)((K + MG_TK - 1) / MG_TK);
   a.tri = tri ? 1 : 0;
-  a.nti = (rowsB + MG_TN - 1) / MG_TN;
-  const int ntj = (rowsA + MG_TM - 1) / MG_TM;
-  int64_t tiles = (int64_t)a.nti * ntj;
-  if (tri) {  // tiles (ti, tj <= min(2 ti + 1, ntj - 1)): the enumeration is ti-major, so the cut is at its end
-    tiles = (int64_t)a.nti * (a.nti + 1) - (2 * a.nti > ntj ? 1 : 0);
-  }
+  a.nti = (rowsB + 255) / 256;
+  a.ntj = (rowsA + 255) / 256;
+  a.nz = nz;
+  const int64_t tiles = tri ? (int64_t)a.nti * (a.nti + 1) / 2 : (int64_t)a.nti * a.ntj;
   const int64_t units = tiles * kModCount * nz;
   if (units > INT32_MAX) return cudaErrorInvalidValue;
   a.ntiles = (int)tiles;
@@ -881,12 +1076,12 @@ cudaError_t mod_plan(ModGemmArgs& a, int rowsA, int rowsB, int64_t K, int nz, bo
   return cudaSuccess;
 }
 
-cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmBh,
-                           const ModGemmArgs& a, int num_sms, cudaStream_t stream) {
+cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const ModGemmArgs& a, int num_sms,
+                           cudaStream_t stream) {
   if (a.nunits <= 0) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(modgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM);
+  cudaError_t e = cudaFuncSetAttribute(modgemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, M2_SMEM);
   if (e != cudaSuccess) return e;
-  modgemm_kernel<<<std::min(a.nunits, num_sms), MG_THREADS, MG_SMEM, stream>>>(tmA, tmB, tmBh, a, tables().red);
+  modgemm_pair_kernel<<<2 * std::min(a.nunits, num_sms / 2), MG_THREADS, M2_SMEM, stream>>>(tmA, tmB, a, tables().red);
   ++g_launches;
   return cudaGetLastError();
 }

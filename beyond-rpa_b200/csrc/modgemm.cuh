@@ -77,7 +77,7 @@ inline int64_t mod_pitch(int64_t K) { return (K + 127) / 128 * 128; }
 struct ModGemmArgs {
   int rowsA;
   int nch;  // 128-wide k chunks
-  int nti, ntiles, nunits, tri;
+  int nti, ntj, nz, ntiles, nunits, tri;  // 256 x 256 tiles
   int zplanesA, zplanesB;  // planes between batches of each operand (0: shared)
   uint8_t* out;            // [z][modulus][j][i], i contiguous
   int64_t out_plane, ldo;  // bytes between planes; between j (a multiple of 256)
@@ -103,8 +103,9 @@ cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, con
                           cudaStream_t stream);
 cudaError_t mod_plan(ModGemmArgs& a, int rowsA, int rowsB, int64_t K, int nz, bool tri);
 int64_t mod_sync_words(const ModGemmArgs& a, int num_sms);
-cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmBh,
-                           const ModGemmArgs& a, int num_sms, cudaStream_t stream);
+// tmA, tmB: the operands' planes as boxes of 128 rows (mod_map).
+cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const ModGemmArgs& a, int num_sms,
+                           cudaStream_t stream);
 cudaError_t launch_mod_crt_lower(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo, int n, int batch,
                                  double* C, int64_t ldc, int64_t strideC, cudaStream_t stream);
 cudaError_t launch_mod_crt_full(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo_i, const int* expo_j,
