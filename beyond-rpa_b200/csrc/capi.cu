@@ -2722,7 +2722,7 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   std::vector<std::pair<int, int>> plist;
   for (int j = 0; j < no; ++j)
     for (int i = j; i < no; ++i) plist.push_back({i, j});
-  const size_t per_pair = 3 * nvv * 8 + (rpa::syevd_workspace_bytes(nv, 2) - rpa::syevd_workspace_bytes(nv, 1));
+  const size_t per_pair = 3 * nvv * 8 + (rpa::syevd_workspace_bytes(nv, 3) - rpa::syevd_workspace_bytes(nv, 2));
   const int bmax = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)plist.size(),
                                                                (int64_t)((size_t)4 << 30) / (int64_t)per_pair));
   RPA_CUDA(h, ensure(h->jD, (size_t)(std::max(8 * no, bmax) + 8) * sizeof(rpa::GemmF64Args) +

@@ -2,12 +2,14 @@
 // (src/linear-algebra/real_linalg.f90:1501-1559), which calls LAPACK's
 // divide-and-conquer dsyevd.  Same three stages, each shaped for the B200:
 //
-//  1. Householder reduction to tridiagonal form T = Q_H^T A Q_H (lower), in
-//     panels of kNB columns: one cooperative launch per panel (per column: the
+//  1. Householder reduction to tridiagonal form T = Q_H^T A Q_H (lower): in
+//     shared memory, one CTA per matrix, up to order kSmallN; above it in
+//     panels of kNB columns, one cooperative launch per panel (per column: the
 //     deferred update from the panel's V/W, the reflector, the matrix-vector
-//     product with the trailing matrix); batches of matrices take a cluster
-//     kernel and a matrix-vector kernel per column.  After each panel the
-//     trailing matrix is updated by two FP64 DMMA GEMMs (A -= V W^T + W V^T).
+//     product with the trailing matrix), the trailing matrix then being
+//     updated by one FP64 DMMA GEMM of depth 2 kNB (A -= [V W] [W V]^T).
+//     Batches of larger matrices take a cluster kernel and a matrix-vector
+//     kernel per column and two GEMMs per panel.
 //  2. Divide and conquer on T (Cuppen's tearing, rank-one merges):
 //     leaves of <= 32 rows are solved by cyclic Jacobi, one warp per leaf;
 //     every merge sorts the poles, deflates small z components and close
@@ -260,6 +262,8 @@ __global__ void __launch_bounds__(256) trailing_gemv_kernel(const double* A, int
 //      products V_c^T v, W_c^T v as further columns of the same product, one warp per column. [barrier]
 // Over a matrix of order 2304 on B200 a column takes 9.7 us on average, against 17 us for the cluster step and the
 // matrix-vector product as two launches (13.5 us and 3 us, each bound by its own latencies).
+// Wp = [W | V] and VW = [V | W] (2 kNB columns each): the two operands of the rank-2 update of the
+// trailing matrix, which is then one product of depth 64 instead of two of depth 32.
 // The kernel is launched cooperatively (every CTA is resident) and its barrier waits are bounded.
 constexpr int kPT = 512;  // threads per CTA
 
@@ -301,8 +305,8 @@ __device__ bool grid_barrier(GridBarrier& g) {
 }
 
 __global__ void __launch_bounds__(kPT, 1)
-    panel_kernel(double* A, int n, double* V, double* Wp, int p, int nb, double* y, double* dots, double* part,
-                 double* tau, double* d, double* e, GridBarrier bar) {
+    panel_kernel(double* A, int n, double* V, double* Wp, double* VW, int p, int nb, double* y, double* dots,
+                 double* part, double* tau, double* d, double* e, GridBarrier bar) {
   extern __shared__ __align__(16) double panel_v[];  // v of the current column, by row
   __shared__ double red[33];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -351,7 +355,7 @@ __global__ void __launch_bounds__(kPT, 1)
       if (i > 0) {
         vr = panel_v[r];
         w = tj * (yr - warp_sum(vrc * s2 + wrc * s1)) + alpha * vr;
-        if (lane == 0) Wp[r + ld * (i - 1)] = w;
+        if (lane == 0) Wp[r + ld * (i - 1)] = VW[r + ld * (kNB + i - 1)] = w;
       }
       if (col) {
         const double a = ar - warp_sum(vrc * wjc + wrc * vjc) - (vr * wj + w * vj);
@@ -378,7 +382,10 @@ __global__ void __launch_bounds__(kPT, 1)
     for (int r = j + 1 + t; r < n; r += kPT) panel_v[r] = r == j + 1 ? 1.0 : __ldcg(A + r + ld * j) * scale;
     __syncthreads();
     double* vg = V + ld * j;
-    for (int r = cta * kPT + t; r < n; r += G * kPT) vg[r] = r > j ? panel_v[r] : 0.0;
+    for (int r = cta * kPT + t; r < n; r += G * kPT) {
+      const double v = r > j ? panel_v[r] : 0.0;
+      vg[r] = Wp[r + ld * (kNB + i)] = VW[r + ld * i] = v;
+    }
     if (cta == 0 && t == 0) {
       tau[j] = tj;
       d[j] = __ldcg(A + j + ld * j);
@@ -415,6 +422,77 @@ __global__ void __launch_bounds__(kPT, 1)
     }
     if (!grid_barrier(bar)) return;
   }
+}
+
+// ---- small matrices (n <= kSmallN): the whole reduction of one matrix in one CTA, in shared memory
+// Both triangles are kept, so that rows read as columns.  Per column three CTA barriers and about
+// 3 m^2 FP64 operations; norms and the scalar p^T v are taken by every warp for itself.  136 matrices of
+// order 128: 0.52 ms in one launch, against 9.1 ms of a cluster and a matrix-vector launch per
+// column (131 and 127 launches of 62 and 7.5 us).
+constexpr int kSmallN = 160;
+__host__ __device__ constexpr int small_pitch(int n) { return n | 1; }
+constexpr size_t small_smem(int n) { return sizeof(double) * ((size_t)n * small_pitch(n) + 2 * (size_t)n); }
+
+__global__ void __launch_bounds__(512) small_reduce_kernel(double* A, int n, int64_t mstride, double* V, double* tau,
+                                                           double* d, double* e) {
+  extern __shared__ __align__(16) double small_a[];
+  const int P = small_pitch(n);
+  double* v = small_a + (size_t)n * P;
+  double* pr = v + n;  // A v
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int64_t z = blockIdx.x, ld = n;
+  A += mstride * z;
+  V += mstride * z;
+  tau += n * z;
+  d += n * z;
+  e += n * z;
+  for (int i = t; i < n * n; i += 512) small_a[(i / n) * P + i % n] = A[i];
+  __syncthreads();
+  for (int j = 0; j + 1 < n; ++j) {
+    const double* x = small_a + j * P;
+    double s2 = 0.0;
+    for (int r = j + 2 + lane; r < n; r += 32) s2 = fma(x[r], x[r], s2);
+    s2 = warp_sum(s2);
+    const double a1 = x[j + 1];
+    double beta = a1, tj = 0.0, scale = 0.0;
+    if (s2 != 0.0) {
+      beta = -copysign(sqrt(a1 * a1 + s2), a1);
+      tj = (beta - a1) / beta;
+      scale = 1.0 / (a1 - beta);
+    }
+    if (t < n) {
+      const double vr = t <= j ? 0.0 : t == j + 1 ? 1.0 : x[t] * scale;
+      v[t] = vr;
+      V[t + ld * j] = vr;
+    }
+    if (t == 0) {
+      tau[j] = tj;
+      d[j] = x[j];
+      e[j] = beta;
+    }
+    __syncthreads();
+    for (int r = j + 1 + warp; r < n; r += 16) {
+      double s = 0.0;
+      for (int c = j + 1 + lane; c < n; c += 32) s = fma(small_a[r * P + c], v[c], s);
+      s = warp_sum(s);
+      if (lane == 0) pr[r] = s;
+    }
+    __syncthreads();
+    double pv = 0.0;
+    for (int r = j + 1 + lane; r < n; r += 32) pv = fma(pr[r], v[r], pv);
+    const double g = 0.5 * tj * tj * warp_sum(pv);
+    // A -= v w^T + w v^T, w = tau p - g v: lanes along the columns, warps along the rows
+    for (int c = j + 1 + lane; c < n; c += 32) {
+      const double vc = v[c], wc = fma(tj, pr[c], -g * vc);
+      for (int r = j + 1 + warp; r < n; r += 16) {
+        const double vr = v[r], wr = fma(tj, pr[r], -g * vr);
+        double* a = small_a + r * P + c;
+        *a -= fma(vr, wc, wr * vc);
+      }
+    }
+    __syncthreads();
+  }
+  if (t == 0) A[(n - 1) * (ld + 1)] = small_a[(n - 1) * P + n - 1];
 }
 
 // ---------------------------------------------------------------- stage 3: back-transformation
@@ -911,9 +989,10 @@ size_t syevd_workspace_bytes(int n, int nmat) {
   const size_t nn = (size_t)n * n, B = (size_t)std::max(nmat, 1);
   size_t b = 0;
   b += 3 * align256(B * nn * 8);                    // V (Householder vectors), Qp, Uk
-  b += align256(B * n * kNB * 8);                   // Wp
+  b += align256(B * n * kNB * 8 * (B == 1 ? 2 : 1));  // Wp
+  b += align256(B == 1 ? (size_t)n * 2 * kNB * 8 : 0);  // VW
   b += 2 * align256(B * kNB * n * 8);               // Y, Y2
-  b += 2 * align256(B * kNB * kNB * 8);             // G, T
+  b += 2 * align256((B == 1 ? (size_t)n / kNB + 1 : B) * kNB * kNB * 8);  // G, T
   b += align256(std::max((size_t)16 * kNB * n, (size_t)64 * kNB * kNB) * 8);  // split-K partials (one matrix)
   b += 6 * align256(B * n * 8);                     // y, tau, d, e, zhat, D
   b += align256(B * 2 * n * 8) + align256(B * 2 * n * 4);  // sort keys
@@ -947,11 +1026,13 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
   double* V = (double*)take(B * nn * 8);
   double* Qp = (double*)take(B * nn * 8);
   double* Uk = (double*)take(B * nn * 8);
-  double* Wp = (double*)take(B * n * kNB * 8);
+  double* Wp = (double*)take(B * n * kNB * 8 * (nmat == 1 ? 2 : 1));
+  double* VW = (double*)take(nmat == 1 ? (size_t)n * 2 * kNB * 8 : 0);
   double* Y = (double*)take(B * kNB * n * 8);
   double* Y2 = (double*)take(B * kNB * n * 8);
-  double* Gm = (double*)take(B * kNB * kNB * 8);
-  double* Tb = (double*)take(B * kNB * kNB * 8);
+  const size_t nblk = nmat == 1 ? (size_t)n / kNB + 1 : B;  // one matrix: every panel's, else every matrix's
+  double* Gm = (double*)take(nblk * kNB * kNB * 8);
+  double* Tb = (double*)take(nblk * kNB * kNB * 8);
   double* Pk = (double*)take(std::max((size_t)16 * kNB * n, (size_t)64 * kNB * kNB) * 8);
   double* y = (double*)take(B * n * 8);
   double* tau = (double*)take(B * n * 8);
@@ -1007,7 +1088,7 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
   SY_CHECK(cudaGetDevice(&dev));
   SY_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const size_t vbytes = (size_t)n * 8;
-  bool coop = nmat == 1 && vbytes <= 200 * 1024;
+  bool coop = nmat == 1 && n > kSmallN && vbytes <= 200 * 1024;
   if (coop) {
     SY_CHECK(cudaFuncSetAttribute(panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vbytes));
     SY_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, panel_kernel, kPT, vbytes));
@@ -1019,11 +1100,18 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
   bar.err = err_dev;
   SY_CHECK(cudaMemsetAsync(err_dev, 0, sizeof(int), stream));
   SY_CHECK(cudaMemsetAsync(bar_dev, 0, sizeof(unsigned), stream));
-  for (int p = 0; p <= n - 2; p += kNB) {
+  if (n >= 2 && n <= kSmallN) {
+    SY_CHECK(cudaFuncSetAttribute(small_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)small_smem(kSmallN)));
+    small_reduce_kernel<<<nmat, 512, small_smem(n), stream>>>(A, n, ms, V, tau, d, e);
+    ++g_launches;
+    SY_CHECK(cudaGetLastError());
+  }
+  for (int p = 0; n > kSmallN && p <= n - 2; p += kNB) {
     int nb = std::min(kNB, n - 1 - p);
     if (coop) {
       double *dots = pk_dots, *part = pk_part;
-      void* args[] = {&A, (void*)&n, &V, &Wp, &p, &nb, &y, &dots, &part, &tau, &d, &e, &bar};
+      void* args[] = {&A, (void*)&n, &V, &Wp, &VW, &p, &nb, &y, &dots, &part, &tau, &d, &e, &bar};
       SY_CHECK(cudaLaunchCooperativeKernel((const void*)panel_kernel, dim3(bar.ctas), dim3(kPT), args, vbytes, stream));
       ++g_launches;
       bar.target += 2u * (unsigned)nb * bar.ctas;
@@ -1042,7 +1130,11 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
     }
     SY_CHECK(cudaGetLastError());
     const int pe = p + nb;
-    if (pe < n) {
+    if (pe < n && coop && nb == kNB) {
+      const int mt = n - pe;
+      SY_CHECK(launch_gemm_f64(gemm_args(mt, mt, 2 * kNB, VW + pe, 1, ld, Wp + pe, ld, 1, A + pe + ld * pe, ld, -1.0, 1.0),
+                               stream));
+    } else if (pe < n) {
       const int mt = n - pe;
       // A(pe:, pe:) -= V W^T + W V^T   (panel columns p..p+nb-1)
       SY_CHECK(launch_gemm_f64(batched(gemm_args(mt, mt, nb, V + pe + ld * p, 1, ld, Wp + pe, ld, 1, A + pe + ld * pe,
@@ -1127,6 +1219,18 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
 
   // ---- stage 3: Z <- Q_H Z, panels in reverse order
   const int last_p = ((n - 2) / kNB) * kNB;
+  // One matrix: G = V_b^T V_b and T of every full panel in one launch each (the columns of V are zero
+  // above their panel); per panel they took 18 us for T alone, a chain of 32 steps on one warp
+  const int nfull = nmat == 1 ? (n - 1) / kNB : 0;
+  if (nfull > 0) {
+    GemmF64Args gg = gemm_args(kNB, kNB, n, V, ld, 1, V, 1, ld, Gm, kNB, 1.0, 0.0);
+    gg.batch = nfull;
+    gg.sA = gg.sB = (int64_t)kNB * ld;
+    gg.sC = kNB * kNB;
+    SY_CHECK(launch_gemm_f64(gg, stream));
+    build_t_kernel<<<nfull, 32, 0, stream>>>(Gm, tau, kNB, Tb, kNB);
+    ++g_launches;
+  }
   for (int p = n >= 2 ? last_p : -1; p >= 0; p -= kNB) {
     const int nb = std::min(kNB, n - 1 - p);
     const int mr = n - 1 - p;  // rows p+1 .. n-1
@@ -1144,11 +1248,14 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
       gg = batched(gg, ms, ms, (int64_t)kNB * kNB);
       gy = batched(gy, ms, ms, (int64_t)kNB * n);
     }
-    SY_CHECK(launch_gemm_f64(gg, stream));
-    build_t_kernel<<<nmat, 32, 0, stream>>>(Gm, tau + p, nb, Tb, n);
-    ++g_launches;
+    double* Tp = nmat == 1 ? Tb + (size_t)(p / kNB) * kNB * kNB : Tb;
+    if (p / kNB >= nfull) {
+      SY_CHECK(launch_gemm_f64(gg, stream));
+      build_t_kernel<<<nmat, 32, 0, stream>>>(Gm, tau + p, nb, Tp, n);
+      ++g_launches;
+    }
     SY_CHECK(launch_gemm_f64(gy, stream));
-    SY_CHECK(launch_gemm_f64(batched(gemm_args(nb, n, nb, Tb, 1, kNB, Y, 1, kNB, Y2, kNB, 1.0, 0.0),
+    SY_CHECK(launch_gemm_f64(batched(gemm_args(nb, n, nb, Tp, 1, kNB, Y, 1, kNB, Y2, kNB, 1.0, 0.0),
                                      (int64_t)kNB * kNB, (int64_t)kNB * n, (int64_t)kNB * n),
                              stream));
     SY_CHECK(launch_gemm_f64(batched(gemm_args(mr, n, nb, Vb, 1, ld, Y2, 1, kNB, Z + (p + 1), ld, -1.0, 1.0), ms,

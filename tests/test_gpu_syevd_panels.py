@@ -1,13 +1,14 @@
-"""The eigensolver's panel reduction (one cooperative launch per 32 columns) at its edges."""
+"""The eigensolver's reduction to tridiagonal form at its edges: in shared memory up to order 160, above in
+panels of 32 columns (one cooperative launch each)."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-@pytest.mark.parametrize("n", [2, 3, 15, 16, 17, 31, 32, 33, 34, 64, 65, 97, 400])
+@pytest.mark.parametrize("n", [2, 3, 16, 17, 33, 64, 97, 159, 160, 161, 192, 193, 194, 225, 400])
 @pytest.mark.parametrize("kind", ["random", "graded", "diagonal", "banded"])
 def test_panel_reduction_edges(handle, n, kind):
-    # sizes around the 32-column panels and the 16 rows per CTA; columns with nothing below the
+    # sizes around the two forms' border and the 32-column panels; columns with nothing below the
     # diagonal (no reflector) in the diagonal and banded matrices.  Backward stability: residual and
     # loss of orthogonality a small multiple of n 2^-53 of the norm
     rng = np.random.default_rng(n)
