@@ -260,7 +260,8 @@ __global__ void __launch_bounds__(256) trailing_gemv_kernel(const double* A, int
 //      its lanes; partial sums of the column's norm.                                      [barrier]
 //   2. reflector of column j; v into shared memory; y = A v over the trailing columns and the dot
 //      products V_c^T v, W_c^T v as further columns of the same product, one warp per column. [barrier]
-// Over a matrix of order 2304 on B200 a column takes 9.7 us on average, against 17 us for the cluster step and the
+// Over a matrix of order 2304 on B200 a column takes 9.1 us on average (9.7 us with full fences
+// around the barriers and the column read after the sums), against 17 us for the cluster step and the
 // matrix-vector product as two launches (13.5 us and 3 us, each bound by its own latencies).
 // Wp = [W | V] and VW = [V | W] (2 kNB columns each): the two operands of the rank-2 update of the
 // trailing matrix, which is then one product of depth 64 instead of two of depth 32.
@@ -279,8 +280,9 @@ __device__ bool grid_barrier(GridBarrier& g) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
+    // release and acquire at GPU scope by this thread, with the CTA barriers around them, order the other
+    // threads' accesses too (a full fence on top costs half a microsecond)
     g.target += g.ctas;
-    __threadfence();
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.count) : "memory");
     const unsigned long long t0 = globaltimer_ns();
     int good = 1;
@@ -295,7 +297,6 @@ __device__ bool grid_barrier(GridBarrier& g) {
         break;
       }
     }
-    __threadfence();
     ok = good;
   } else {
     g.target += g.ctas;
@@ -368,10 +369,18 @@ __global__ void __launch_bounds__(kPT, 1)
     if (t == 0) part[cta] = ps;
     if (!grid_barrier(bar)) return;
     // ---- 2. reflector of column j
-    double sg = 0.0;
-    for (int c = t; c < G; c += kPT) sg += __ldcg(part + c);
-    const double sigma2 = block_sum(sg, red);
+    // the column's entries are on their way while every warp adds up the partial sums
+    constexpr int kPre = 6;
+    double xr[kPre];
+#pragma unroll
+    for (int u = 0; u < kPre; ++u) {
+      const int r = j + 1 + t + u * kPT;
+      xr[u] = r < n ? __ldcg(A + r + ld * j) : 0.0;
+    }
     const double a1 = __ldcg(A + j + 1 + ld * j);
+    double sg = 0.0;
+    for (int c = lane; c < G; c += 32) sg += __ldcg(part + c);
+    const double sigma2 = warp_sum(sg);
     double beta = a1, scale = 0.0;
     tj = 0.0;
     if (sigma2 != 0.0) {
@@ -379,7 +388,12 @@ __global__ void __launch_bounds__(kPT, 1)
       tj = (beta - a1) / beta;
       scale = 1.0 / (a1 - beta);
     }
-    for (int r = j + 1 + t; r < n; r += kPT) panel_v[r] = r == j + 1 ? 1.0 : __ldcg(A + r + ld * j) * scale;
+#pragma unroll
+    for (int u = 0; u < kPre; ++u) {
+      const int r = j + 1 + t + u * kPT;
+      if (r < n) panel_v[r] = r == j + 1 ? 1.0 : xr[u] * scale;
+    }
+    for (int r = j + 1 + t + kPre * kPT; r < n; r += kPT) panel_v[r] = __ldcg(A + r + ld * j) * scale;
     __syncthreads();
     double* vg = V + ld * j;
     for (int r = cta * kPT + t; r < n; r += G * kPT) {
@@ -793,19 +807,17 @@ __global__ void __launch_bounds__(1024) merge_prepare_kernel(const Merge* merges
   sc.rho[mz] = rho;
 }
 
-// Apply the deflation rotations to the merge's block of Q (thread per row) and gather its
-// columns as [non-deflated (k) | deflated] into Qp (n x n, ld n).
-__global__ void merge_gather_kernel(const Merge* merges, double* Q, int64_t ldq, double* Qp_base, DcScratch sc,
-                                    int nfull, int64_t mstride, int nm) {
+// Apply the deflation rotations to the merge's block of Q (thread per row).
+__global__ void merge_rotate_kernel(const Merge* merges, double* Q, int64_t ldq, DcScratch sc, int nfull,
+                                    int64_t mstride, int nm) {
   const Merge M = merges[blockIdx.y];
   const int n = M.n1 + M.n2, s = M.s;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   const int64_t mz = blockIdx.y + (int64_t)nm * blockIdx.z;
   Q += mstride * blockIdx.z;
-  Qp_base += mstride * blockIdx.z;
   sc = sc_at(sc, blockIdx.z, nfull);
-  const int k = sc.cnt[2 * mz], nr = sc.cnt[2 * mz + 1];
+  const int nr = sc.cnt[2 * mz + 1];
   double* row = Q + (int64_t)(s + r) + ldq * s;  // row r of the block: row[ldq * col]
   for (int q = 0; q < nr; ++q) {
     const int64_t a = ldq * sc.rp[s + q], b = ldq * sc.ri[s + q];
@@ -814,9 +826,28 @@ __global__ void merge_gather_kernel(const Merge* merges, double* Q, int64_t ldq,
     row[a] = c * x - sn * y;
     row[b] = sn * x + c * y;
   }
-  double* Qp = Qp_base + M.qp_off;
-  for (int c = 0; c < k; ++c) Qp[r + (int64_t)n * c] = row[ldq * sc.colk[s + c]];
-  for (int c = 0; c < n - k; ++c) Qp[r + (int64_t)n * (k + c)] = row[ldq * sc.coldef[s + c]];
+}
+
+// Gather its columns as [non-deflated (k) | deflated] into Qp (n x n, ld n): 128 rows x kGatherCols columns per CTA (one thread per row over all
+// columns left the top merges with 18 CTAs: 4.6 ms over 35 levels of orders up
+// to 2304, now less than 0.8).
+constexpr int kGatherCols = 32;
+__global__ void merge_gather_kernel(const Merge* merges, const double* Q, int64_t ldq, double* Qp_base, DcScratch sc,
+                                    int nfull, int64_t mstride, int nm, int row_blocks) {
+  const Merge M = merges[blockIdx.y];
+  const int n = M.n1 + M.n2, s = M.s;
+  const int r = ((int)blockIdx.x % row_blocks) * blockDim.x + threadIdx.x;
+  const int c0 = ((int)blockIdx.x / row_blocks) * kGatherCols;
+  if (r >= n || c0 >= n) return;
+  const int64_t mz = blockIdx.y + (int64_t)nm * blockIdx.z;
+  Q += mstride * blockIdx.z;
+  sc = sc_at(sc, blockIdx.z, nfull);
+  const int k = sc.cnt[2 * mz];
+  const double* row = Q + (int64_t)(s + r) + ldq * s;
+  double* Qp = Qp_base + mstride * blockIdx.z + M.qp_off + r;
+  const int c1 = min(n, c0 + kGatherCols);
+#pragma unroll 8
+  for (int c = c0; c < c1; ++c) Qp[(int64_t)n * c] = row[ldq * (c < k ? sc.colk[s + c] : sc.coldef[s + c - k])];
 }
 
 // Roots of 1 + rho sum_i z_i^2 / (d_i - lambda) = 0 by bisection on tau = lambda - d_org, with
@@ -1194,13 +1225,15 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
     const int nm_ = (int)mv.size();
     SY_CHECK(cudaMemcpyAsync(dMerges, mv.data(), mv.size() * sizeof(Merge), cudaMemcpyHostToDevice, stream));
     merge_prepare_kernel<<<dim3(nm_, nmat), 1024, 0, stream>>>(dMerges, D, Z, ld, e, sc, n, ms, nm_);
-    merge_gather_kernel<<<dim3((nmax + 127) / 128, nm_, nmat), 128, 0, stream>>>(dMerges, Z, ld, Qp, sc, n, ms, nm_);
+    const int rb = (nmax + 127) / 128, cb = (nmax + kGatherCols - 1) / kGatherCols;
+    merge_rotate_kernel<<<dim3(rb, nm_, nmat), 128, 0, stream>>>(dMerges, Z, ld, sc, n, ms, nm_);
+    merge_gather_kernel<<<dim3(rb * cb, nm_, nmat), 128, 0, stream>>>(dMerges, Z, ld, Qp, sc, n, ms, nm_, rb);
     secular_kernel<<<dim3((nmax + 7) / 8, nm_, nmat), 256, 0, stream>>>(dMerges, sc, n, nm_);
     lowner_kernel<<<dim3((nmax + 127) / 128, nm_, nmat), 128, 0, stream>>>(dMerges, sc, zhat, n, nm_);
     merge_vectors_kernel<<<dim3(nmax, nm_, nmat), 256, 0, stream>>>(dMerges, sc, zhat, Uk, D, n, ms, nm_);
     copy_deflated_kernel<<<dim3((unsigned)std::min<int64_t>(((int64_t)nmax * nmax + 255) / 256, 1024), nm_, nmat), 256,
                            0, stream>>>(dMerges, Qp, Z, ld, sc.cnt, ms, nm_);
-    g_launches += 6;
+    g_launches += 7;
     SY_CHECK(cudaGetLastError());
     cnt.resize(2 * (size_t)nm_ * nmat);
     SY_CHECK(cudaMemcpyAsync(cnt.data(), sc.cnt, cnt.size() * 4, cudaMemcpyDeviceToHost, stream));
