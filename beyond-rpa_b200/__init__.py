@@ -227,6 +227,24 @@ def _colmajor(x, nrows):
     return _Arg(a.ctypes.data, ld=nrows, owner=a)
 
 
+def _amplitude_buffer(R, nov, n_guess):
+    """Device memory for the amplitudes U of vectors R that are on the device themselves, so that the exchange
+    energy reads them where the T2 solver left them; None (host memory) for host R or when it would take
+    more than a sixteenth of the free device memory, which the solver's own workspace may need."""
+    if not (_is_torch(R) and R.is_cuda):
+        return None
+    import torch
+    cap = int(n_guess if n_guess is not None else min(int(np.ceil(3.0 * int(R.shape[0]))), nov))
+    if cap <= 0 or nov <= 0 or 8 * cap * nov > torch.cuda.mem_get_info(R.device)[0] // 16:
+        return None
+    try:
+        buf = torch.empty((cap, nov), dtype=torch.float64, device=R.device).T
+    except torch.cuda.OutOfMemoryError:
+        return None
+    torch.cuda.current_stream(R.device).synchronize()  # the block's last user may still run; the solver has its own stream
+    return buf
+
+
 class Handle:
     """A librpa_b200 handle bound to one GPU (rpa_b200_create / rpa_b200_destroy)."""
 
@@ -429,7 +447,8 @@ class Handle:
         ex, eig, nts = [], [], []
         for R, eo, ev in active:
             t2 = self.dring_t2(R, eo, ev, x, w, prec=prec, seed=seed, n_guess=n_guess, cutoff_thresh=cutoff_thresh,
-                               cutoff_type=cutoff_type, common_thresh=common)
+                               cutoff_type=cutoff_type, common_thresh=common,
+                               u_out=_amplitude_buffer(R, len(eo) * len(ev), n_guess))
             common = t2["common_thresh"]
             nts.append(t2["NT"])
             eig.append(float(np.sum(t2["EigRPA"])))

@@ -78,6 +78,10 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
 }
 }  // namespace
 
+// Pinned staging: results (4 doubles per frequency, error word, non-finite count) in the first part,
+// orbital energies after it.
+constexpr size_t kPinResults = 4096, kPinBytes = 256 * 1024;
+
 struct rpa_b200_handle {
   int device = 0;
   int num_sms = 0;
@@ -116,7 +120,18 @@ struct rpa_b200_handle {
   int* count_dev = nullptr;  // non-finite counter
   PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   cudaEvent_t ev[5] = {};
-  double timings[6] = {0, 0, 0, 0, 0, 0};
+  mutable double timings[6] = {0, 0, 0, 0, 0, 0};
+  // Events of the last finished call, swapped with the running call's: its times are taken when
+  // rpa_b200_last_timings asks for them (six event queries cost a small call a tenth of its time).
+  struct TimedCall {
+    cudaEvent_t ev[5] = {};
+    std::vector<cudaEvent_t> pool;
+    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> split_ev, tc_ev;
+  };
+  TimedCall done;
+  mutable bool timings_pending = false;
+  // pinned host memory: orbital energies on their way to the device, and small results on theirs back
+  uint8_t* pin = nullptr;
   int64_t launches = 0;
   int seg_chunks = 16;  // 512-column accumulation segments of the tensor-core SYRK
   int sync_every = 32;  // K chunks between the wave-progress milestones of the SYRK (0: off)
@@ -295,10 +310,16 @@ int fetch_small(rpa_b200_handle* h, const double* p, int64_t n, std::vector<doub
   return RPA_OK;
 }
 
+int device_error_status(rpa_b200_handle* h, int err);
+
 int check_device_error(rpa_b200_handle* h) {
   int err = 0;
   RPA_CUDA(h, cudaMemcpyAsync(&err, h->err_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+  return device_error_status(h, err);
+}
+
+int device_error_status(rpa_b200_handle* h, int err) {
   if (err == rpa::kDevNotSPD) return fail(h, RPA_ERR_NOT_SPD, "1+Pi(u) is not positive definite (Cholesky pivot <= 0)");
   if (err != 0) return fail(h, RPA_ERR_TIMEOUT, "device-side bounded wait expired (code %d)", err);
   return RPA_OK;
@@ -355,14 +376,28 @@ int validate_common(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVirt,
 int stage_eps(rpa_b200_handle* h, const Validated& v) {
   RPA_CUDA(h, ensure(h->eps, (size_t)(v.no + v.nv) * 8));
   double* ed = static_cast<double*>(h->eps.p);
-  RPA_CUDA(h, cudaMemcpyAsync(ed, v.eo.data(), (size_t)v.no * 8, cudaMemcpyHostToDevice, h->stream));
-  RPA_CUDA(h, cudaMemcpyAsync(ed + v.no, v.ev.data(), (size_t)v.nv * 8, cudaMemcpyHostToDevice, h->stream));
+  if (kPinResults + (size_t)(v.no + v.nv) * 8 <= kPinBytes) {  // one copy that the host does not wait for
+    double* pe = reinterpret_cast<double*>(h->pin + kPinResults);
+    std::memcpy(pe, v.eo.data(), (size_t)v.no * 8);
+    std::memcpy(pe + v.no, v.ev.data(), (size_t)v.nv * 8);
+    RPA_CUDA(h, cudaMemcpyAsync(ed, pe, (size_t)(v.no + v.nv) * 8, cudaMemcpyHostToDevice, h->stream));
+  } else {
+    RPA_CUDA(h, cudaMemcpyAsync(ed, v.eo.data(), (size_t)v.no * 8, cudaMemcpyHostToDevice, h->stream));
+    RPA_CUDA(h, cudaMemcpyAsync(ed + v.no, v.ev.data(), (size_t)v.nv * 8, cudaMemcpyHostToDevice, h->stream));
+  }
   RPA_CUDA(h, ensure(h->D, (size_t)v.nov * 8));
   RPA_CUDA(h, rpa::launch_dai(ed, ed + v.no, v.no, v.nv, static_cast<double*>(h->D.p), h->stream));
   return RPA_OK;
 }
 
-int stage_R(rpa_b200_handle* h, const Validated& v, const double* R, int64_t ldR, const double** Rd, int64_t* ldd) {
+// defer: the count of non-finite entries is left on its way to *pin_count(h); the caller, who
+// synchronises the stream later, reports it (before any other status).
+int* pin_count(rpa_b200_handle* h) { return reinterpret_cast<int*>(h->pin + kPinResults) - 1; }
+int* pin_error(rpa_b200_handle* h) { return reinterpret_cast<int*>(h->pin + kPinResults) - 2; }
+static_assert(64 * 4 * sizeof(double) + 2 * sizeof(int) <= kPinResults, "results of 64 frequencies fit");
+
+int stage_R(rpa_b200_handle* h, const Validated& v, const double* R, int64_t ldR, const double** Rd, int64_t* ldd,
+            bool defer = false) {
   if (is_device_ptr(R)) {
     *Rd = R;
     *ldd = ldR;
@@ -382,10 +417,10 @@ int stage_R(rpa_b200_handle* h, const Validated& v, const double* R, int64_t ldR
   RPA_CUDA(h, rpa::launch_count_nonfinite_cols(*Rd, *ldd, v.NQ, v.nov, h->count_dev, h->stream));
   int s = stage_eps(h, v);
   if (s != RPA_OK) return s;
-  int cnt = 0;
-  RPA_CUDA(h, cudaMemcpyAsync(&cnt, h->count_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  RPA_CUDA(h, cudaMemcpyAsync(pin_count(h), h->count_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  if (defer) return RPA_OK;
   RPA_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (cnt) return fail(h, RPA_ERR_NONFINITE, "%d non-finite entries in the Cholesky vectors", cnt);
+  if (int cnt = *pin_count(h)) return fail(h, RPA_ERR_NONFINITE, "%d non-finite entries in the Cholesky vectors", cnt);
   return RPA_OK;
 }
 
@@ -971,10 +1006,11 @@ int energy_from_workspace(rpa_b200_handle* h, int NQ, int K, const std::vector<d
   if (cs != RPA_OK) return cs;
   RPA_CUDA(h, rpa::launch_logdet_sum(static_cast<double*>(h->Ldiag.p), NQ, K, ld, h->stream));
   RPA_CUDA(h, cudaEventRecord(h->ev[3], h->stream));
-  std::vector<double> host(4 * (size_t)K);
-  RPA_CUDA(h, cudaMemcpyAsync(host.data(), tr, (size_t)4 * K * 8, cudaMemcpyDeviceToHost, h->stream));
+  const double* host = reinterpret_cast<const double*>(h->pin);
+  RPA_CUDA(h, cudaMemcpyAsync(h->pin, tr, (size_t)4 * K * 8, cudaMemcpyDeviceToHost, h->stream));
+  RPA_CUDA(h, cudaMemcpyAsync(pin_error(h), h->err_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   RPA_CUDA(h, cudaStreamSynchronize(h->stream));
-  int s = check_device_error(h);
+  int s = device_error_status(h, *pin_error(h));
   if (s != RPA_OK) return s;
   dd ec{0.0, 0.0};
   for (int k = 0; k < K; ++k) {
@@ -1246,17 +1282,25 @@ int begin_call(rpa_b200_handle* h) {
 }
 
 void finish_timings(rpa_b200_handle* h) {
-  cudaEventSynchronize(h->ev[4]);
-  h->timings[0] = elapsed(h->ev[0], h->ev[1]);
-  h->timings[1] = elapsed(h->ev[1], h->ev[2]);
-  h->timings[2] = elapsed(h->ev[2], h->ev[3]);
-  h->timings[3] = elapsed(h->ev[3], h->ev[4]);
+  std::swap(h->ev, h->done.ev);
+  std::swap(h->pool, h->done.pool);
+  std::swap(h->tc_ev, h->done.tc_ev);
+  std::swap(h->split_ev, h->done.split_ev);
+  h->timings_pending = true;
+  h->launches = rpa::g_launches;
+}
+
+void take_timings(const rpa_b200_handle* h) {
+  if (!h->timings_pending) return;
+  h->timings_pending = false;
+  const auto& d = h->done;
+  cudaEventSynchronize(d.ev[4]);
+  for (int i = 0; i < 4; ++i) h->timings[i] = elapsed(d.ev[i], d.ev[i + 1]);
   double tc = 0.0, sp = 0.0;
-  for (auto& p : h->tc_ev) tc += elapsed(p.first, p.second);
-  for (auto& p : h->split_ev) sp += elapsed(p.first, p.second);
+  for (auto& p : d.tc_ev) tc += elapsed(p.first, p.second);
+  for (auto& p : d.split_ev) sp += elapsed(p.first, p.second);
   h->timings[4] = tc;
   h->timings[5] = sp;
-  h->launches = rpa::g_launches;
 }
 
 // Handler of the entry points' function-try-blocks: the status of the exception in flight, its
@@ -1301,7 +1345,8 @@ int rpa_b200_create(rpa_b200_handle** handle, int64_t device, int64_t flags) try
       cudaStreamCreateWithFlags(&h->aux[0], cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&h->aux[1], cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&h->aux[2], cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&h->err_dev, sizeof(int)) != cudaSuccess || cudaMalloc(&h->count_dev, sizeof(int)) != cudaSuccess) {
+      cudaMalloc(&h->err_dev, sizeof(int)) != cudaSuccess || cudaMalloc(&h->count_dev, sizeof(int)) != cudaSuccess ||
+      cudaMallocHost(&h->pin, kPinBytes) != cudaSuccess) {
     rpa_b200_destroy(h);  // releases whatever was created (it skips null members)
     return RPA_ERR_CUDA;
   }
@@ -1314,6 +1359,7 @@ int rpa_b200_create(rpa_b200_handle** handle, int64_t device, int64_t flags) try
   if (const char* sg = std::getenv("RPA_B200_SOSEX_SEG")) h->sosex_seg = std::max(1, std::atoi(sg));
   if (const char* rg = std::getenv("RPA_B200_RING_SEG")) h->ring_seg = std::max(1, std::atoi(rg));
   for (auto& e : h->ev) cudaEventCreate(&e);
+  for (auto& e : h->done.ev) cudaEventCreate(&e);
   for (auto& e : h->fork_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   if (const char* la = std::getenv("RPA_B200_LOOKAHEAD")) h->lookahead = std::atoi(la) != 0;
   h->ozaki_slices = rpa::ozaki_slices_default();
@@ -1365,6 +1411,10 @@ int rpa_b200_destroy(rpa_b200_handle* h) try {
   for (auto& e : h->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : h->pool) cudaEventDestroy(e);
+  for (auto& e : h->done.ev)
+    if (e) cudaEventDestroy(e);
+  for (auto& e : h->done.pool) cudaEventDestroy(e);
+  if (h->pin) cudaFreeHost(h->pin);
   for (auto& g : h->chol_graphs) cudaGraphExecDestroy(g.exec);
   for (auto& e : h->fork_ev)
     if (e) cudaEventDestroy(e);
@@ -1412,6 +1462,7 @@ const char* rpa_b200_last_error(const rpa_b200_handle* h) { return h ? h->last_e
 
 int rpa_b200_last_timings(const rpa_b200_handle* h, double* out, int64_t n) try {
   if (!h || !out) return RPA_ERR_INVALID_ARG;
+  take_timings(h);
   for (int64_t i = 0; i < n && i < 6; ++i) out[i] = h->timings[i];
   return RPA_OK;
 } catch (...) {
@@ -1607,10 +1658,13 @@ int rpa_b200_ec(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVirt, con
   }
   const double* Rd;
   int64_t ldd;
-  if ((s = stage_R(h, v, R, ldR, &Rd, &ldd))) return s;
+  if ((s = stage_R(h, v, R, ldR, &Rd, &ldd, true))) return s;
   RPA_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
-  if ((s = build_pi(h, v, Rd, ldd, alpha, prec))) return s;
-  if ((s = energy_from_workspace(h, v.NQ, v.K, v.weights, Ec, Eu))) return s;
+  s = build_pi(h, v, Rd, ldd, alpha, prec);
+  if (s == RPA_OK) s = energy_from_workspace(h, v.NQ, v.K, v.weights, Ec, Eu);
+  RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+  if (int cnt = *pin_count(h)) return fail(h, RPA_ERR_NONFINITE, "%d non-finite entries in the Cholesky vectors", cnt);
+  if (s) return s;
   RPA_CUDA(h, cudaEventRecord(h->ev[4], h->stream));
   finish_timings(h);
   return RPA_OK;
