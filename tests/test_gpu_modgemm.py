@@ -75,7 +75,8 @@ def test_pi_fp64_padded_columns_and_small_workspace(handle, pkg):
     assert np.max(np.abs(capped - ref) / norms(ref)) < 280 * 2.0 ** -53  # 280 sequential FP64 additions
 
 
-@pytest.mark.parametrize("nq,no,nv,k", [(127, 2, 64, 2), (128, 2, 64, 2), (193, 4, 33, 3), (257, 5, 77, 17), (321, 3, 64, 5)])
+@pytest.mark.parametrize("nq,no,nv,k", [(127, 2, 64, 2), (128, 2, 64, 2), (193, 4, 33, 3), (257, 5, 77, 17), (321, 3, 64, 5),
+                                        (1100, 8, 32, 35)])
 def test_gradient_fp64(handle, nq, no, nv, k):
     # dE/dR and dE/de against the FP64 oracle: 1 + Pi has eigenvalues in [1, 1.8], so inverse and
     # products lose a few roundings of sqrt(NQ) terms; 1e-13 of the largest entry bounds both sides
