@@ -106,6 +106,7 @@ struct rpa_b200_handle {
   DevBuf thZ, thXa, thXi, thYX, thR;  // THC factors, Khatri-Rao block, Cholesky vectors formed from them
   DevBuf jU, jL, jX, jPno, jWork;      // particle-hole corrections: localised T2 vectors, PNOs, scratch
   DevBuf jPack, jQS, jS, jD;           // per-orbital PNO packs, QS slots, S blocks, grouped-GEMM descriptors
+  DevBuf jBat;                         // QS slots, S blocks, G and its products of several pairs
   DevBuf jT, jM, jV, jMap;             // batched PNO stage: T_ij, T T^T, eigenvectors, column map
   DevBuf jSK;                          // split-K partials of the G products
   DevBuf sxR, sxU, sxP;                // split-BF16 exchange: R and U (U2) hi/lo rows, partial sums
@@ -1270,7 +1271,7 @@ int begin_call(rpa_b200_handle* h) {
   if (!h) return RPA_ERR_INVALID_ARG;
   h->last_error.clear();
   g_account = &h->account;
-  h->account.idle = {&h->Xhi, &h->Xlo, &h->gY, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE, &h->mcBuf, &h->bMod};
+  h->account.idle = {&h->Xhi, &h->Xlo, &h->gY, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE, &h->mcBuf, &h->bMod, &h->jBat};
   h->pool_used = 0;
   h->split_ev.clear();
   h->tc_ev.clear();
@@ -1401,7 +1402,7 @@ int rpa_b200_destroy(rpa_b200_handle* h) try {
                     &h->tRU, &h->tSmall, &h->tPerm, &h->bDesc, &h->bRes, &h->gY, &h->gD, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE, &h->mcBuf, &h->mcDesc, &h->bMod,
                     &h->xM, &h->eW, &h->eA, &h->eZ, &h->thZ, &h->thXa, &h->thXi, &h->thYX, &h->thR,
                     &h->jU, &h->jL, &h->jX, &h->jPno, &h->jWork,
-                    &h->jPack, &h->jQS, &h->jS, &h->jD, &h->syncBuf,
+                    &h->jPack, &h->jQS, &h->jS, &h->jD, &h->jBat, &h->syncBuf,
                     &h->jT, &h->jM, &h->jV, &h->jMap, &h->jSK, &h->tune, &h->sxR, &h->sxU, &h->sxP,
                     &h->t2Z, &h->t2M, &h->t2Sync, &h->ozBuf[0], &h->ozBuf[1]})
     release(*b);
@@ -2887,14 +2888,42 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   RPA_CUDA(h, ensure(h->jQS, (size_t)nv * maxcol * 2 * 8));
   RPA_CUDA(h, ensure(h->jSK, std::max((size_t)64 * nvv, (size_t)16 * std::max(nq, ng) * no) * 8));
   RPA_CUDA(h, ensure(h->jS, (size_t)4 * no * std::max<int64_t>(max_n * max_n, 1) * 8));
-  RPA_CUDA(h, ensure(h->jD, (size_t)(8 * no + 8) * sizeof(rpa::GemmF64Args) + (size_t)(8 * no + 16) * sizeof(int)));
 
   // ---- energy terms (rpa_JCTC2024_Gaibj_Gabij_v2)
+  // The pairs of one j run in batches of up to np_max, which share their launches: their S blocks and QS
+  // slots in three grouped GEMMs, the G products in one batched GEMM, everything with the Y and ZYX
+  // factors in products over the columns of all of them (one pair at a time took 19 launches of mostly
+  // less than 20 us; 16 orbitals of 128 virtuals on 1024 points: 21.6 ms instead of 39.9).  Batches are bounded by kJBatchBytes of workspace; without room
+  // for them pairs run one by one in the scratch above.
+  constexpr size_t kJBatchBytes = (size_t)1 << 30;
+  const size_t s_one = (size_t)4 * no * std::max<int64_t>(max_n * max_n, 1), qs_one = (size_t)nv * maxcol;
+  const size_t w_cols = (size_t)std::max<int64_t>(nv, 2 * max_n);
+  const size_t one = 2 * qs_one + s_one + 2 * nvv + 2 * ng * w_cols;  // words of a pair in a batch
+  int64_t ndesc = 0;
+  for (int j = 0; j < no; ++j)
+    for (int i = j; i < no; ++i)
+      for (int k = 0; k < no; ++k)
+        if (pn[(size_t)k + (size_t)no * j] && pn[(size_t)k + (size_t)no * i]) ndesc += i != j ? 8 : 6;
+  RPA_CUDA(h, ensure(h->jD, (size_t)std::max<int64_t>(ndesc, 1) * sizeof(rpa::GemmF64Args) +
+                                (size_t)(ndesc + 3 * npairs) * sizeof(int) + 256));
+  int np_max = (int)std::min<size_t>((size_t)no, kJBatchBytes / (8 * one));
+  if (np_max < 2 || !try_ensure(h->jBat, np_max * one * 8)) np_max = 1;
+  double *QSall = static_cast<double*>(h->jQS.p), *Sall = static_cast<double*>(h->jS.p), *Gall = Gg;
+  double *W1 = Wx, *W2 = Wy;
+  size_t w_room = (size_t)nv;  // columns of W1 and of W2
+  if (np_max > 1) {
+    QSall = static_cast<double*>(h->jBat.p);
+    Sall = QSall + np_max * 2 * qs_one;
+    Gall = Sall + np_max * s_one;
+    W1 = Gall + np_max * 2 * nvv;
+    w_room = np_max * w_cols;
+    W2 = W1 + ng * w_room;
+  }
   const double c2b = -2.0, c2c = -2.0, c2d = 2.0, c2g = -4.0, c2h = -4.0, c2i = 2.0, c2j = 2.0;
   auto slot = [&](int64_t pair, int term) { return part + (size_t)(5 * pair + term) * rpa::kDotPartials; };
   auto G = [&](const rpa::GemmF64Args& g) { return rpa::launch_gemm_f64(g, h->stream); };
-  // grouped-GEMM descriptors of every pair, built once and uploaded in one copy: the k sum of a
-  // pair is one grouped launch for its S blocks and two for its QS slots
+  // grouped-GEMM descriptors of every batch, built once and uploaded in one copy: the k sums of a
+  // batch are one grouped launch for its S blocks and two for its QS slots
   struct GroupRef {
     int64_t desc, start;
     int nprob, ntiles;
@@ -2904,9 +2933,6 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   std::vector<int> all_start;
   std::vector<GroupRef> groups;
   {
-    double* QSg = static_cast<double*>(h->jQS.p);
-    double* QSb = QSg + (size_t)nv * maxcol;
-    double* Sbase = static_cast<double*>(h->jS.p);
     auto add_group = [&](const std::vector<rpa::GemmF64Args>& v) {
       GroupRef gr{(int64_t)all_desc.size(), (int64_t)all_start.size(), (int)v.size(), 0, true, true};
       if (!v.empty()) {
@@ -2922,61 +2948,63 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
       groups.push_back(gr);
     };
     for (int j = 0; j < no; ++j)
-      for (int i = j; i < no; ++i) {
+      for (int i0 = j; i0 < no; i0 += np_max) {
+        const int np = std::min(np_max, no - i0);
         std::vector<rpa::GemmF64Args> sp, q1, q2;
-        size_t soff = 0;
-        const double* pj = pack + (size_t)nv * pack_off[j];
-        const double* pi_ = pack + (size_t)nv * pack_off[i];
-        for (int k = 0; k < no; ++k) {
-          const int nkj = pn[(size_t)k + (size_t)no * j], nki = pn[(size_t)k + (size_t)no * i];
-          if (nkj == 0 || nki == 0) continue;
-          const double* kj[2] = {pj + (size_t)nv * kcol[(size_t)j * no + k], nullptr};
-          kj[1] = kj[0] + (size_t)nv * nkj;
-          const double* ki[2] = {pi_ + (size_t)nv * kcol[(size_t)i * no + k], nullptr};
-          ki[1] = ki[0] + (size_t)nv * nki;
-          int Pki, Qki, Pik, Qik, Pkj, Qkj, Pjk, Qjk;
-          if (k >= i) { Pki = 0; Qki = 1; Pik = 1; Qik = 0; } else { Pki = 1; Qki = 0; Pik = 0; Qik = 1; }
-          if (k >= j) { Pkj = 0; Qkj = 1; Pjk = 1; Qjk = 0; } else { Pkj = 1; Qkj = 0; Pjk = 0; Qjk = 1; }
-          double* S_jk_ki = Sbase + soff;
-          double* S_jk_ik = S_jk_ki + (size_t)nkj * nki;
-          double* S_kj_ki = S_jk_ik + (size_t)nkj * nki;
-          double* S_kj_ik = S_kj_ki + (size_t)nkj * nki;
-          soff += 4 * (size_t)nkj * nki;
-          sp.push_back(gemm_g(nkj, nki, nv, kj[Qjk], nv, true, ki[Pki], nv, false, S_jk_ki, nkj));
-          sp.push_back(gemm_g(nkj, nki, nv, kj[Qjk], nv, true, ki[Pik], nv, false, S_jk_ik, nkj));
-          sp.push_back(gemm_g(nkj, nki, nv, kj[Qkj], nv, true, ki[Pki], nv, false, S_kj_ki, nkj));
-          sp.push_back(gemm_g(nkj, nki, nv, kj[Qkj], nv, true, ki[Pik], nv, false, S_kj_ik, nkj));
-          const size_t c0 = (size_t)kcol[(size_t)j * no + k];
-          double* qg[2] = {QSg + (size_t)nv * c0, QSg + (size_t)nv * (c0 + nkj)};
-          double* qb[2] = {QSb + (size_t)nv * c0, QSb + (size_t)nv * (c0 + nkj)};
-          // alpha ki[q] S^T (+ beta slot)
-          auto qs = [&](double* dst, int q, const double* S, double alpha, double beta) {
-            return gemm_g(nv, nkj, nki, ki[q], nv, false, S, nkj, true, dst, nv, alpha, beta);
-          };
-          if (i != j) {
-            q1.push_back(qs(qg[Pjk], Qki, S_jk_ki, 2.0 * c2g, 0.0));
-            q2.push_back(qs(qg[Pjk], Qik, S_jk_ik, c2i + c2j, 1.0));
-            q1.push_back(qs(qg[Pkj], Qik, S_kj_ik, 2.0 * c2h, 0.0));
-            q2.push_back(qs(qg[Pkj], Qki, S_kj_ki, c2i + c2j, 1.0));
-            q1.push_back(qs(qb[Pkj], Qik, S_kj_ik, 2.0 * c2d, 0.0));
-            q2.push_back(qs(qb[Pkj], Qki, S_kj_ki, c2b + c2c, 1.0));
-            q1.push_back(qs(qb[Pjk], Qik, S_jk_ik, c2b + c2c, 0.0));
-          } else {
-            q1.push_back(qs(qg[Pjk], Qki, S_jk_ki, c2g, 0.0));
-            q2.push_back(qs(qg[Pjk], Qik, S_jk_ik, c2i + c2j, 1.0));
-            q1.push_back(qs(qg[Pkj], Qik, S_kj_ik, c2h, 0.0));
-            q1.push_back(qs(qb[Pkj], Qik, S_kj_ik, c2d, 0.0));  // the other slot of 2b..2d stays zero
-            q2.push_back(qs(qb[Pkj], Qki, S_kj_ki, c2b + c2c, 1.0));
+        for (int i = i0; i < i0 + np; ++i) {
+          // slots of the batch: QSg of its pairs, then QSb
+          double* QSg = QSall + (size_t)(i - i0) * qs_one;
+          double* QSb = QSall + (size_t)(np + i - i0) * qs_one;
+          double* Sbase = Sall + (size_t)(i - i0) * s_one;
+          size_t soff = 0;
+          const double* pj = pack + (size_t)nv * pack_off[j];
+          const double* pi_ = pack + (size_t)nv * pack_off[i];
+          for (int k = 0; k < no; ++k) {
+            const int nkj = pn[(size_t)k + (size_t)no * j], nki = pn[(size_t)k + (size_t)no * i];
+            if (nkj == 0 || nki == 0) continue;
+            const double* kj[2] = {pj + (size_t)nv * kcol[(size_t)j * no + k], nullptr};
+            kj[1] = kj[0] + (size_t)nv * nkj;
+            const double* ki[2] = {pi_ + (size_t)nv * kcol[(size_t)i * no + k], nullptr};
+            ki[1] = ki[0] + (size_t)nv * nki;
+            int Pki, Qki, Pik, Qik, Pkj, Qkj, Pjk, Qjk;
+            if (k >= i) { Pki = 0; Qki = 1; Pik = 1; Qik = 0; } else { Pki = 1; Qki = 0; Pik = 0; Qik = 1; }
+            if (k >= j) { Pkj = 0; Qkj = 1; Pjk = 1; Qjk = 0; } else { Pkj = 1; Qkj = 0; Pjk = 0; Qjk = 1; }
+            // S = [P | Q](kj)^T [P | Q](ki) in one product; its four blocks by the halves of either side
+            double* S = Sbase + soff;
+            const int64_t lds = 2 * (int64_t)nkj;
+            const double *S_jk_ki = S + Qjk * nkj + lds * Pki * nki, *S_jk_ik = S + Qjk * nkj + lds * Pik * nki,
+                         *S_kj_ki = S + Qkj * nkj + lds * Pki * nki, *S_kj_ik = S + Qkj * nkj + lds * Pik * nki;
+            soff += 4 * (size_t)nkj * nki;
+            sp.push_back(gemm_g(2 * nkj, 2 * nki, nv, kj[0], nv, true, ki[0], nv, false, S, lds));
+            const size_t c0 = (size_t)kcol[(size_t)j * no + k];
+            double* qg[2] = {QSg + (size_t)nv * c0, QSg + (size_t)nv * (c0 + nkj)};
+            double* qb[2] = {QSb + (size_t)nv * c0, QSb + (size_t)nv * (c0 + nkj)};
+            // alpha ki[q] S^T (+ beta slot)
+            auto qs = [&](double* dst, int q, const double* Sb, double alpha, double beta) {
+              return gemm_g(nv, nkj, nki, ki[q], nv, false, Sb, lds, true, dst, nv, alpha, beta);
+            };
+            if (i != j) {
+              q1.push_back(qs(qg[Pjk], Qki, S_jk_ki, 2.0 * c2g, 0.0));
+              q2.push_back(qs(qg[Pjk], Qik, S_jk_ik, c2i + c2j, 1.0));
+              q1.push_back(qs(qg[Pkj], Qik, S_kj_ik, 2.0 * c2h, 0.0));
+              q2.push_back(qs(qg[Pkj], Qki, S_kj_ki, c2i + c2j, 1.0));
+              q1.push_back(qs(qb[Pkj], Qik, S_kj_ik, 2.0 * c2d, 0.0));
+              q2.push_back(qs(qb[Pkj], Qki, S_kj_ki, c2b + c2c, 1.0));
+              q1.push_back(qs(qb[Pjk], Qik, S_jk_ik, c2b + c2c, 0.0));
+            } else {
+              q1.push_back(qs(qg[Pjk], Qki, S_jk_ki, c2g, 0.0));
+              q2.push_back(qs(qg[Pjk], Qik, S_jk_ik, c2i + c2j, 1.0));
+              q1.push_back(qs(qg[Pkj], Qik, S_kj_ik, c2h, 0.0));
+              q1.push_back(qs(qb[Pkj], Qik, S_kj_ik, c2d, 0.0));  // the other slot of 2b..2d stays zero
+              q2.push_back(qs(qb[Pkj], Qki, S_kj_ki, c2b + c2c, 1.0));
+            }
           }
         }
-
         add_group(sp);
         add_group(q1);
         add_group(q2);
       }
   }
-  RPA_CUDA(h, ensure(h->jD, std::max<size_t>(all_desc.size(), 1) * sizeof(rpa::GemmF64Args) +
-                                std::max<size_t>(all_start.size(), 1) * sizeof(int) + 256));
   rpa::GemmF64Args* dprob = static_cast<rpa::GemmF64Args*>(h->jD.p);
   int* dstart = reinterpret_cast<int*>(static_cast<char*>(h->jD.p) +
                                        ((std::max<size_t>(all_desc.size(), 1) * sizeof(rpa::GemmF64Args) + 255) & ~(size_t)255));
@@ -2985,8 +3013,9 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
                                 cudaMemcpyHostToDevice, h->stream));
   RPA_CUDA(h, cudaMemcpyAsync(dstart, all_start.data(), all_start.size() * sizeof(int), cudaMemcpyHostToDevice,
                               h->stream));
-  int64_t pair = 0;
+  int64_t pair = 0, batch = 0;
   std::vector<std::pair<int, int>> pair_ij;
+  constexpr int64_t kSlot = rpa::kDotPartials, kPair = 5 * kSlot;
   for (int j = 0; j < no; ++j) {
     const double* xj = Xd + (int64_t)ldx * j;
     // ZYX(k, b) = sum_g Z(g, k) X(g, j) Y(g, b); ZYX(g, b) = Z ZYX(k, b)
@@ -3005,52 +3034,74 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
     g2.kscale = xj;
     RPA_CUDA(h, narrow(g2));
     RPA_CUDA(h, narrow(gemm_g(ng, no - j, nq, Zd, ldz, false, zkj, nq, false, zgj, ng)));
-    for (int i = j; i < no; ++i, ++pair) {
-      pair_ij.push_back({i, j});
-      const double* xi = Xd + (int64_t)ldx * i;
-      const double *zk = zkj + (size_t)nq * (i - j), *zg = zgj + (size_t)ng * (i - j);
-      RPA_CUDA(h, rpa::launch_dot_partials(zk, nq, zk, nq, nq, 1, nullptr, slot(pair, 4), h->stream));
-      // S1a, S1b of the pair (i, j)
-      const int nij = pn[(size_t)i + (size_t)no * j];
-      if (nij > 0) {
-        const double* P = pno + poff[(size_t)i + (size_t)no * j];
-        const double* Q = P + (size_t)nv * nij;
-        for (int t = 0; t < 2; ++t) {  // t = 0: S1b (Y Q, ZYX P); t = 1: S1a (Y P, ZYX Q)
-          rpa::GemmF64Args gx = gemm_g(ng, nij, nv, Yd, ldy, false, t == 0 ? Q : P, nv, false, Wx, ng);
-          gx.rowscale = xi;
-          RPA_CUDA(h, G(gx));
-          RPA_CUDA(h, G(gemm_g(ng, nij, nv, ZYXg, ng, false, t == 0 ? P : Q, nv, false, Wy, ng)));
-          RPA_CUDA(h, rpa::launch_dot_partials(Wx, ng, Wy, ng, ng, nij, nullptr, slot(pair, t == 0 ? 1 : 0),
-                                               h->stream));
+    const int ncj = ncol[j];
+    const double* pj = pack + (size_t)nv * pack_off[j];
+    for (int i0 = j; i0 < no; i0 += np_max, ++batch) {
+      const int np = std::min(np_max, no - i0);
+      const double* x0 = Xd + (int64_t)ldx * i0;
+      const double *zk = zkj + (size_t)nq * (i0 - j), *zg = zgj + (size_t)ng * (i0 - j);
+      RPA_CUDA(h, rpa::launch_dot_partials(zk, nq, nq, zk, nq, nq, nq, 1, nullptr, 0, slot(pair, 4), kPair, np,
+                                           h->stream));
+      // S1a, S1b of the pairs: sum_g X(g, i) (Y Q)(g, n) (ZYX P)(g, n) and the same with P and Q exchanged;
+      // [P | Q] of the batch's pairs are columns c0 .. c1 - 1 of orbital j's pack
+      const int* kc = kcol.data() + (size_t)j * no;
+      const int c0 = kc[i0], c1 = i0 + np < no ? kc[i0 + np] : ncj;
+      const bool whole = (size_t)(c1 - c0) <= w_room;
+      if (whole && c1 > c0) {
+        RPA_CUDA(h, G(gemm_g(ng, c1 - c0, nv, Yd, ldy, false, pj + (size_t)nv * c0, nv, false, W1, ng)));
+        RPA_CUDA(h, G(gemm_g(ng, c1 - c0, nv, ZYXg, ng, false, pj + (size_t)nv * c0, nv, false, W2, ng)));
+      }
+      for (int i = i0; i < i0 + np; ++i) {
+        pair_ij.push_back({i, j});
+        const int n = pn[(size_t)i + (size_t)no * j];
+        if (n == 0) continue;
+        const double* xi = Xd + (int64_t)ldx * i;
+        double* s1b = slot(pair + (i - i0), 1);  // S1a is the slot before it
+        if (whole) {
+          const int64_t half = (int64_t)ng * n, off = (int64_t)ng * (kc[i] - c0);
+          RPA_CUDA(h, rpa::launch_dot_partials(W1 + off + half, ng, -half, W2 + off, ng, half, ng, n, xi, 0, s1b, -kSlot,
+                                               2, h->stream));
+        } else {  // one pair whose 2 n columns do not fit at once
+          const double* P = pj + (size_t)nv * kc[i];
+          const double* Q = P + (size_t)nv * n;
+          for (int t = 0; t < 2; ++t) {
+            RPA_CUDA(h, G(gemm_g(ng, n, nv, Yd, ldy, false, t == 0 ? Q : P, nv, false, W1, ng)));
+            RPA_CUDA(h, G(gemm_g(ng, n, nv, ZYXg, ng, false, t == 0 ? P : Q, nv, false, W2, ng)));
+            RPA_CUDA(h, rpa::launch_dot_partials(W1, ng, 0, W2, ng, 0, ng, n, xi, 0, s1b - t * kSlot, 0, 1, h->stream));
+          }
         }
       }
       // G(ba; ji) for 2g..2j and G(bj; ai) for 2b..2d: the k sum becomes one GEMM over the
       // packed PNO blocks of orbital j against per-k QS slots (zero where a pair has no PNOs)
-      const int ncj = ncol[j];
-      const double* pj = pack + (size_t)nv * pack_off[j];
-      double* QSg = static_cast<double*>(h->jQS.p);
-      double* QSb = QSg + (size_t)nv * maxcol;
-      RPA_CUDA(h, cudaMemsetAsync(QSg, 0, (size_t)nv * maxcol * 2 * 8, h->stream));
+      RPA_CUDA(h, cudaMemsetAsync(QSall, 0, 2 * np * qs_one * 8, h->stream));
       for (int gi = 0; gi < 3; ++gi) {
-        const GroupRef& gr = groups[(size_t)3 * pair + gi];
+        const GroupRef& gr = groups[(size_t)3 * batch + gi];
         RPA_CUDA(h, rpa::launch_gemm_f64_grouped_dev(dprob + gr.desc, dstart + gr.start, gr.nprob, gr.ntiles,
                                                      gr.am, gr.bn, h->stream));
       }
-      // the G products have few output tiles and K = sum_k 2 Nkj: split K (about 600 CTA slots)
-      for (int t = 0; t < 2; ++t) {
-        rpa::GemmF64Args gk = gemm_g(nv, nv, ncj, pj, nv, false, t == 0 ? QSg : QSb, nv, true, t == 0 ? Gg : Gb, nv,
-                                     1.0, 0.0);
-        gk.splitk = std::max(1, std::min({64, ncj / 256, 600 / std::max(1, rpa::gemm_f64_tiles(gk))}));
-        gk.work = static_cast<double*>(h->jSK.p);
+      // the G products have few output tiles and K = sum_k 2 Nkj: one by one K is split (about 600 CTA slots;
+      // 21 us per product of 128 x 128 with K of some thousands), six and more run as one batch (about 100 us)
+      rpa::GemmF64Args gk = gemm_g(nv, nv, ncj, pj, nv, false, QSall, nv, true, Gall, nv, 1.0, 0.0);
+      const int tiles = std::max(1, rpa::gemm_f64_tiles(gk));
+      if (np >= 3 || 2 * np * tiles >= 2 * h->num_sms) {
+        gk.batch = 2 * np;
+        gk.sA = 0;
+        gk.sB = (int64_t)qs_one;
+        gk.sC = (int64_t)nvv;
         RPA_CUDA(h, G(gk));
+      } else {
+        gk.splitk = std::max(1, std::min({64, ncj / 256, 600 / tiles}));
+        gk.work = static_cast<double*>(h->jSK.p);
+        for (int t = 0; t < 2 * np; ++t, gk.B += qs_one, gk.C += nvv) RPA_CUDA(h, G(gk));
       }
-      // Tr V G: sum_ga Y(g,a) ZXX(g) (Y G)(g,a)  and  sum_ga (ZYX G)(g,a) X(g,i) Y(g,a)
-      rpa::GemmF64Args gg = gemm_g(ng, nv, nv, Yd, ldy, false, Gg, nv, false, Wg, ng);
-      gg.rowscale = zg;
-      RPA_CUDA(h, G(gg));
-      RPA_CUDA(h, rpa::launch_dot_partials(Yd, ldy, Wg, ng, ng, nv, nullptr, slot(pair, 2), h->stream));
-      RPA_CUDA(h, G(gemm_g(ng, nv, nv, ZYXg, ng, false, Gb, nv, false, Wg, ng)));
-      RPA_CUDA(h, rpa::launch_dot_partials(Wg, ng, Yd, ldy, ng, nv, xi, slot(pair, 3), h->stream));
+      // Tr V G: sum_ga ZXX(g) Y(g,a) (Y G)(g,a)  and  sum_ga X(g,i) Y(g,a) (ZYX G)(g,a)
+      RPA_CUDA(h, G(gemm_g(ng, np * nv, nv, Yd, ldy, false, Gall, nv, false, W1, ng)));
+      RPA_CUDA(h, rpa::launch_dot_partials(W1, ng, (int64_t)ng * nv, Yd, ldy, 0, ng, nv, zg, ng, slot(pair, 2), kPair, np,
+                                           h->stream));
+      RPA_CUDA(h, G(gemm_g(ng, np * nv, nv, ZYXg, ng, false, Gall + np * nvv, nv, false, W2, ng)));
+      RPA_CUDA(h, rpa::launch_dot_partials(W2, ng, (int64_t)ng * nv, Yd, ldy, 0, ng, nv, x0, ldx, slot(pair, 3), kPair,
+                                           np, h->stream));
+      pair += np;
     }
   }
   RPA_CUDA(h, cudaEventRecord(h->ev[3], h->stream));

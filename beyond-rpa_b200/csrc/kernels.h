@@ -343,8 +343,10 @@ cudaError_t launch_hadamard(const double* A, int64_t lda, const double* B, int64
                             double* C, int64_t ldc, cudaStream_t stream);
 // out[0 .. kDotPartials) = per-CTA partial sums of sum_{r,c} w(r) A(r,c) B(r,c) (w may be nullptr).
 constexpr int kDotPartials = 64;
-cudaError_t launch_dot_partials(const double* A, int64_t lda, const double* B, int64_t ldb, int rows, int cols,
-                                const double* w, double* out, cudaStream_t stream);
+// batch of them: element strides sA, sB, sw, sOut.
+cudaError_t launch_dot_partials(const double* A, int64_t lda, int64_t sA, const double* B, int64_t ldb, int64_t sB,
+                                int rows, int cols, const double* w, int64_t sw, double* out, int64_t sOut, int batch,
+                                cudaStream_t stream);
 // YX(g, a + nv*ii) = Xa(g, a) Xi(g, i0 + ii) for ii < ni (YX: ngrid x nv*ni, ld ngrid).
 // YX(g, c) = Xa(g, a) Xi(g, i) for the ai columns ai0 .. ai0 + ncols - 1 (ai = a + nv i), ld ngrid.
 cudaError_t launch_khatri_rao_cols(const double* Xa, int64_t ldXa, const double* Xi, int64_t ldXi, int ngrid, int nv,

@@ -363,9 +363,15 @@ __global__ void hadamard_kernel(const double* A, int64_t lda, const double* B, i
 // Partial sums of sum_{r,c} w(r) A(r,c) B(r,c) (w optional): kDotBlocks CTAs each write one
 // partial to out[blockIdx.x]; the caller adds them in a fixed order.
 constexpr int kDotBlocks = kDotPartials;
-__global__ void __launch_bounds__(256) dot_partials_kernel(const double* A, int64_t lda, const double* B, int64_t ldb,
-                                                           int rows, int cols, const double* w, double* out) {
+__global__ void __launch_bounds__(256) dot_partials_kernel(const double* A, int64_t lda, int64_t sA, const double* B,
+                                                           int64_t ldb, int64_t sB, int rows, int cols,
+                                                           const double* w, int64_t sw, double* out, int64_t sOut) {
   __shared__ double red[256];
+  const int64_t z = blockIdx.y;
+  A += sA * z;
+  B += sB * z;
+  if (w) w += sw * z;
+  out += sOut * z;
   const int64_t total = (int64_t)rows * cols;
   double acc = 0.0;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -598,9 +604,11 @@ cudaError_t launch_hadamard(const double* A, int64_t lda, const double* B, int64
   return cudaGetLastError();
 }
 
-cudaError_t launch_dot_partials(const double* A, int64_t lda, const double* B, int64_t ldb, int rows, int cols,
-                                const double* w, double* out, cudaStream_t stream) {
-  dot_partials_kernel<<<kDotBlocks, 256, 0, stream>>>(A, lda, B, ldb, rows, cols, w, out);
+cudaError_t launch_dot_partials(const double* A, int64_t lda, int64_t sA, const double* B, int64_t ldb, int64_t sB,
+                                int rows, int cols, const double* w, int64_t sw, double* out, int64_t sOut, int batch,
+                                cudaStream_t stream) {
+  dot_partials_kernel<<<dim3(kDotBlocks, (unsigned)batch), 256, 0, stream>>>(A, lda, sA, B, ldb, sB, rows, cols, w, sw,
+                                                                             out, sOut);
   ++g_launches;
   return cudaGetLastError();
 }
