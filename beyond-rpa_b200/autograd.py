@@ -3,7 +3,7 @@
 The forward pass calls rpa_b200_ec (Pi(u) on the tensor cores, FP64 log-det)
 and keeps only its inputs; the backward pass calls rpa_b200_ec_grad, which
 recomputes Pi(u) per frequency instead of storing all of them and applies
-((1+Pi)^{-1} - 1) to R by FP64 triangular solves.  Gradients flow to R
+((1+Pi)^{-1} - 1) to R in FP64-accurate products.  Gradients flow to R
 ((NQ, nov) column-major view) and to the occupied / virtual orbital energies.
 """
 from __future__ import annotations

@@ -1995,7 +1995,8 @@ int rpa_b200_exchange_sosex(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
 // ((S Y + Y S)_mn = mu_m + mu_n in the eigenbasis), and the antisymmetric part 2 U_mn (A_n - A_m),
 // which is small because |A| << 1; the residual-correction iteration
 //   X <- X + Q [(Q^T (A - B^T X - X B) Q)_mn / (mu_m + mu_n)] Q^T
-// contracts by about three orders of magnitude per step.  All matrix products are FP64 DMMA GEMMs.
+// contracts by about three orders of magnitude per step.  The matrix products are FP64 GEMMs (residue products
+// where they pay).
 int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVirt, const double* R,
                             int64_t ldR, const double* OccEnergies, const double* VirtEnergies, int64_t NVecsT2,
                             const double* U, int64_t ldU, const double* A, int64_t Prec, double* Ex, double* X,
@@ -2448,7 +2449,7 @@ static int stage_matrix(rpa_b200_handle* h, DevBuf& buf, const double* A, int64_
 }
 
 // R = Z^T (Xa * Xi) into Rout (device, NQ x nov, ld ldR): Khatri-Rao blocks of whole occupied
-// orbitals (<= ~1 GB each) and one FP64 DMMA GEMM per block.
+// orbitals (<= ~1 GB each) and one FP64 GEMM per block.
 static int form_thc_r(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOcc, int64_t NVirt, const double* Zd, int64_t ldz,
                const double* Xad, int64_t ldxa, const double* Xid, int64_t ldxi, double* Rout, int64_t ldR) {
   const int64_t per_occ = NGrid * NVirt;
@@ -2516,7 +2517,7 @@ int rpa_b200_thc_r(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOcc, 
 
 // Split-BF16 Pi build straight from THC factors, the way rpa_THC_PiU_BlockAlgo forms and
 // contracts R block by block (src/rpa/rpa_THC.f90:285-340, 374-403): the ai columns are taken in
-// pieces; for each piece the Khatri-Rao block YX = Xa * Xi of its columns, one FP64 DMMA GEMM
+// pieces; for each piece the Khatri-Rao block YX = Xa * Xi of its columns, one FP64 GEMM
 // R_piece = Z^T YX, the scale/split pass into piece-sized bf16 operands and the tensor-core SYRK
 // adding the piece into Pi (FP64).  Neither the whole R nor the whole split operands are held:
 // the device holds one piece of each (the piece width is sized to h->thc_piece_bytes).  The exact

@@ -48,11 +48,12 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// 1 / d and 1 / sqrt(d) to about an ulp.  The hardware estimates (error 2^-20 or better) take one
-// third-order Newton step each: with e = 1 - d r, 1 / d = r (1 + e + e^2 + ...); with e = 1 - d y^2,
-// 1 / sqrt(d) = y (1 + e / 2 + 3 e^2 / 8 + ...), the rest of both series being below 2^-60.  Only the
-// reciprocal is on the chain of pivots.  Pivots near the ends of the exponent range take the library
-// functions; one that is not positive counts as 1 and is reported.
+// 1 / d and 1 / sqrt(d) to about an ulp.  The hardware estimates (error 2^-20 or better) take one step of
+// Householder's iteration of order 3 each, the binomial series in the residual: with e = 1 - d r,
+// 1 / d = r (1 + e + e^2 + ...); with e = 1 - d y^2, 1 / sqrt(d) = y (1 + e / 2 + 3 e^2 / 8 + ...), the
+// rest of both series being below 2^-60.  Only the reciprocal is on the chain of pivots.  Pivots near
+// the ends of the exponent range take the library functions; one that is not positive counts as 1 and
+// is reported.
 __device__ __forceinline__ void pivot_inverses(double& d, double& rd, double& ri, bool& bad) {
   if (!(d > 1e-290 && d < 1e290)) {
     if (!(d > 0.0)) {

@@ -65,7 +65,9 @@ typedef enum rpa_status {
 } rpa_status;
 
 /* Precision of the Pi(u) contraction. */
-#define RPA_PREC_FP64 0      /* plain FP64 (FP64 tensor-core DMMA)                 */
+#define RPA_PREC_FP64 0      /* FP64 accuracy: int8 residue products (exact integers,
+                                operands rounded at 2^-58 of their row norm), or FP64
+                                tensor-core DMMA for small shapes                  */
 #define RPA_PREC_SPLIT_BF16 1 /* X = hi + lo (bf16), 3 tcgen05 products, FP32 acc,
                                  exact FP64 diagonal                               */
 
@@ -236,7 +238,8 @@ int rpa_b200_mbe_energy(int64_t NBody, const double* E, double* Eint);
  *   dE/dR(:,ai) = sum_u w_u/(2 pi) 2 alpha c_u(ai) ((1+Pi_u)^{-1} - 1) R(:,ai),
  *   dE/dD(ai)   = sum_u w_u/(2 pi) alpha R(:,ai)^T ((1+Pi_u)^{-1} - 1) R(:,ai) dc_u/dD,
  * c_u = D/(D^2+u^2).  Pi(u) is recomputed (prec as in rpa_b200_ec) and
- * factorised; (1+Pi_u)^{-1} R comes from two batched triangular solves in FP64.
+ * factorised; (1+Pi_u)^{-1} R comes from the factor's inverse in FP64-accurate products
+ * (two batched triangular solves in FP64 where the workspace cap leaves no room).
  * dR/dOcc/dVirt may be host or device pointers (dOcc/dVirt may be NULL).
  */
 int rpa_b200_ec_grad(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVirt, const double* R, int64_t ldR,
