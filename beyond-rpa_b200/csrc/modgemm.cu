@@ -717,13 +717,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
           }
         }
       }
-      // every issued load has landed (the even CTA counts the bytes of both) and been consumed before the
-      // shared memory goes: both CTAs meet at the cluster barrier below
+      // every issued load has landed (the even CTA counts the bytes of both) before the shared memory goes:
+      // both CTAs meet at the cluster barrier below
+      if (rank == 0) {
+        for (int s = 0; s < M2_STAGES; ++s)
+          if (issued & (1u << s) && !mbar_wait(&full[s], (issued_par >> s) & 1u, a.err, kDevTimeoutDrain)) break;
+      }
       for (int s = 0; s < M2_STAGES; ++s)
-        if (issued & (1u << s)) {
-          if (rank == 0) mbar_wait(&full[s], (issued_par >> s) & 1u, a.err, kDevTimeoutDrain);
-          mbar_wait(&empty[s], (issued_par >> s) & 1u, a.err, kDevTimeoutDrain);
-        }
+        if (issued & (1u << s)) mbar_wait(&empty[s], (issued_par >> s) & 1u, a.err, kDevTimeoutTmaEmpty);
+      // the last commit arrives in both CTAs: the odd one's shared memory must outlive its arrival too
+      if (rank != 0) mbar_wait(drain, 0, a.err, kDevTimeoutDrain);
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {

@@ -58,14 +58,15 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 // Slow path of the bounded wait (kept out of line so that the fast path of
-// the hot loops needs no extra registers).
+// the hot loops needs no extra registers).  A drain (copies or MMAs in flight at exit) goes on to
+// its own limit when another wait has failed: its work must not outlive the CTA.
 static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, int* err, int code,
                                                    unsigned long long limit_ns = kWaitLimitNs) {
   const unsigned long long t0 = globaltimer_ns();
   uint32_t it = 0;
   while (!mbar_try_wait(bar, parity)) {
     if ((++it & 255u) == 0u) {
-      if (*reinterpret_cast<volatile int*>(err) != 0) return false;
+      if (code != kDevTimeoutDrain && *reinterpret_cast<volatile int*>(err) != 0) return false;
       if (globaltimer_ns() - t0 > limit_ns) {
         atomicCAS(err, 0, code);
         return false;
@@ -75,7 +76,7 @@ static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parit
   return true;
 }
 // Bounded wait: returns false (and records `code` in *err) when the wait limit
-// expires or another thread already recorded an error.
+// expires or another thread already recorded an error (drains look at the limit alone).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, int code) {
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, err, code);
