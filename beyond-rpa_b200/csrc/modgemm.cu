@@ -557,6 +557,10 @@ __global__ void __launch_bounds__(MG_THREADS, 1)
   const ModMat* mat = mats + blockIdx.y;
   MgChol src{mat, a, (int)blockIdx.x / MG_GROUPS, (int)blockIdx.x % MG_GROUPS};
   if (!src.any()) return;  // CTA-uniform
+  if (threadIdx.x == 0) {  // the producer
+    tensormap_acquire(&mat->mA);
+    tensormap_acquire(&mat->mB);
+  }
   modgemm_body(src, &mat->mA, &mat->mB, &mat->mA, a.err, red);
 }
 

@@ -86,6 +86,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
+// A tensor map in global memory that the host has copied there (over an earlier one, as a descriptor array
+// that is filled again for another shape): its contents are read through the tensormap proxy, which this
+// thread has to be told to look at memory again before its first use.
+__device__ __forceinline__ void tensormap_acquire(const void* tmap) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(tmap))
+               : "memory");
+}
 // 3-D tiled bulk tensor load global -> shared, completion via mbarrier tx count.
 __device__ __forceinline__ void tma_load_3d(void* dst, const void* tmap, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(

@@ -82,6 +82,7 @@ __device__ __forceinline__ void named_barrier(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
+template <bool kMapsInMemory>
 __device__ __forceinline__ void scale_split_body(const double* __restrict__ R, int64_t ldR, int NQ, int64_t nov,
                                                  const double* __restrict__ D, const FreqGroup& fg, double alpha,
                                                  const CUtensorMap* tm_hi, const CUtensorMap* tm_lo,
@@ -203,6 +204,10 @@ __device__ __forceinline__ void scale_split_body(const double* __restrict__ R, i
     }
   } else if (lane == 0) {
     // store thread: one bulk tensor store per 64-column box of each full stage
+    if (kMapsInMemory) {
+      tensormap_acquire(tm_hi);
+      tensormap_acquire(tm_lo);
+    }
     tma_prefetch_desc(tm_hi);
     tma_prefetch_desc(tm_lo);
     uint32_t it = 0;
@@ -259,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 2) scale_split_kernel(
     const double* __restrict__ R, int64_t ldR, int NQ, int64_t nov, const double* __restrict__ D, FreqGroup fg,
     double alpha, const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo,
     double* __restrict__ diag_part, int64_t ai_per_split, int split0, int* err) {
-  scale_split_body(R, ldR, NQ, nov, D, fg, alpha, &tm_hi, &tm_lo, diag_part, ai_per_split, blockIdx.x,
+  scale_split_body<false>(R, ldR, NQ, nov, D, fg, alpha, &tm_hi, &tm_lo, diag_part, ai_per_split, blockIdx.x,
                    split0 + (int)blockIdx.y, err);
 }
 
@@ -268,7 +273,7 @@ __global__ void __launch_bounds__(kThreads, 2) scale_split_multi_kernel(const Sp
                                                                         const int4* __restrict__ work, int* err) {
   const int4 w = work[blockIdx.x];
   const SplitJob& j = jobs[w.x];
-  scale_split_body(j.R, j.ldR, j.NQ, j.nov, j.D, j.fg, j.alpha, &j.tm_hi, &j.tm_lo, j.diag_part, j.ai_per_split,
+  scale_split_body<true>(j.R, j.ldR, j.NQ, j.nov, j.D, j.fg, j.alpha, &j.tm_hi, &j.tm_lo, j.diag_part, j.ai_per_split,
                    w.y, w.z, err);
 }
 

@@ -82,6 +82,7 @@ struct Unit {
 
 // Single instance: tensor maps are kernel parameters, units are decoded.
 struct SingleSource {
+  static constexpr bool kMapsInMemory = false;
   const CUtensorMap* maps[4];
   SyrkTcArgs a;
   int nblocks, ntm, nchunks, nunits;
@@ -109,6 +110,7 @@ struct SingleSource {
 
 // Many instances: per-instance descriptors (tensor maps in global memory) and a work list.
 struct MultiSource {
+  static constexpr bool kMapsInMemory = true;
   const SyrkInst* insts;
   const uint4* work;  // (instance, k, tm, tn)
   int nunits;
@@ -143,6 +145,7 @@ struct MultiSource {
 // General GEMM: tensor maps are kernel parameters; units (tm, tn) over the full tile grid,
 // tm-major (consecutive units share an A band).
 struct GemmSource {
+  static constexpr bool kMapsInMemory = false;
   const CUtensorMap* maps[4];
   GemmSplitArgs a;
   int ntn, nchunks, nunits;
@@ -235,7 +238,10 @@ __device__ __forceinline__ void syrk_body(const Source& src, int* err, const int
       for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
         const Unit x = src.get(u);
         if (x.map[0] != last) {
-          for (int i = 0; i < 4; ++i) tma_prefetch_desc(x.map[i]);
+          for (int i = 0; i < 4; ++i) {
+            if (Source::kMapsInMemory) tensormap_acquire(x.map[i]);
+            tma_prefetch_desc(x.map[i]);
+          }
           last = x.map[0];
         }
         const int wave = (u - (int)blockIdx.x) / (int)gridDim.x;

@@ -18,3 +18,31 @@ def test_short_launches_back_to_back(handle):
     for it in range(400):
         s, r = systems[it & 1], ref[it & 1]
         assert np.array_equal(handle.pi_u(s.R, s.eps_o, s.eps_v, x, prec="fp64"), r)
+
+
+def _pi(n, k, seed):
+    rng = np.random.default_rng(seed)
+    X = rng.standard_normal((k, n, 64)) * 0.05
+    return X @ X.transpose(0, 2, 1)
+
+
+def test_descriptors_rewritten_in_place(pkg):
+    # tensor maps in descriptor arrays that every new shape fills again at the same address (log-det blocks,
+    # split pass and SYRK of a batch): each call must see its own.  Fresh handles give the same bits.
+    x, w = O.casimir_polder(2, 0.8)
+    pis = [_pi(n, 2, n) for n in (1300, 1452, 1281)]
+    sets = [[(s.R, s.eps_o, s.eps_v, x, w) for s in (O.make_system(nq, no, nv, nq, decay=30.0, lam0=0.8)
+                                                     for nq, no, nv in shapes)]
+            for shapes in ([(200, 4, 60), (1537, 3, 100)], [(1545, 4, 70), (190, 5, 66)], [(210, 3, 50), (180, 6, 30)])]
+    ref_e, ref_b = [], []
+    for pi, t in zip(pis, sets):
+        with pkg.Handle(0) as h:
+            h.set_autotune(False)
+            ref_e.append(h.ec_from_pi(pi, np.ones(2))[1])
+            ref_b.append(h.ec_batched(t, prec="split")[0])
+    with pkg.Handle(0) as h:
+        h.set_autotune(False)
+        for it in range(12):
+            i = (it * 2 + it // 3) % 3
+            assert np.array_equal(h.ec_from_pi(pis[i], np.ones(2))[1], ref_e[i])
+            assert np.array_equal(h.ec_batched(sets[i], prec="split")[0], ref_b[i])
