@@ -513,36 +513,48 @@ int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t pla
 }
 
 // One FP64 product on the FP64 tensor pipe, or by residues where that is the faster: the pipe's
-// 28 TFLOP/s against 15 int8 products at 2.4 POP/s, the conversion of both operands (3 TB/s of
-// planes), the residues of C written and read, and the extra launches.  1.2: the estimate's margin.
+// 28 TFLOP/s against 15 int8 products at 2.4 POP/s, the sizes of both operands along K and their conversion
+// (5.5 TB/s read, 3 TB/s of planes), the residues of C written and read, and the extra launches.  1.2: the
+// estimate's margin.
 bool mod_pays(int64_t M, int64_t N, int64_t K) {
   const double flops = 2.0 * (double)M * (double)N * (double)K;
   return M >= 128 && N >= 128 && K >= 128 &&
-         flops * (1.0 / 28e12 - 15.0 / 2.4e15) > 1.2 * (5e-12 * (double)(M + N) * (double)K + 1e-11 * (double)M * (double)N + 25e-6);
+         flops * (1.0 / 28e12 - 15.0 / 2.4e15) > 1.2 * (6.5e-12 * (double)(M + N) * (double)K + 1e-11 * (double)M * (double)N + 33e-6);
 }
 
 int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30) {
-  const bool plain = g.batch == 1 && g.splitk <= 1 && (!g.kscale || g.b_k == 1) && !g.rowscale && (g.a_m == 1 || g.a_k == 1) &&
-                     (g.b_n == 1 || g.b_k == 1);
+  const bool plain = g.batch == 1 && g.splitk <= 1 && !g.rowscale && (g.a_m == 1 || g.a_k == 1) && (g.b_n == 1 || g.b_k == 1);
   if (plain && g.K <= INT32_MAX && mod_pays(g.M, g.N, g.K)) {
     const size_t NM = rpa::kModCount;
     const int64_t pitch = rpa::mod_pitch(g.K), ldo = ((int64_t)g.M + 255) / 256 * 256;
     // C is formed in blocks of columns whose planes and residues fit the budget
     const int64_t nmax = (int64_t)(budget / (NM * (size_t)(pitch + ldo))) / 128 * 128;
     const int64_t nb = std::min<int64_t>(g.N, nmax);
+    // an operand times its own transpose needs no balance along K
+    const bool same = g.A == g.B && g.a_m == g.b_n && g.a_k == g.b_k && g.M == g.N && !g.kscale;
+    const size_t kw = same ? 0 : (size_t)g.K;
     if (nb >= std::min<int64_t>(g.N, 128) && try_ensure(h->mA, NM * g.M * (size_t)pitch) &&
         try_ensure(h->mB, NM * nb * (size_t)pitch) && try_ensure(h->mC, NM * nb * (size_t)ldo) &&
-        try_ensure(h->mE, ((size_t)g.M + nb) * sizeof(int))) {
+        try_ensure(h->mE, kw * 24 + ((size_t)g.M + nb) * sizeof(int))) {
       int8_t *pa = static_cast<int8_t*>(h->mA.p), *pb = static_cast<int8_t*>(h->mB.p);
-      int *ea = static_cast<int*>(h->mE.p), *eb = ea + g.M;
-      if (g.a_k == 1) RPA_CUDA(h, rpa::launch_mod_cols(g.A, g.a_m, 0, (int)g.K, g.M, 1, pa, ea, h->stream));
-      else RPA_CUDA(h, rpa::launch_mod_rows(g.A, g.a_k, g.M, g.K, pa, ea, h->stream));
+      double *fa = nullptr, *fb = nullptr;  // factors of column k
+      int* ea = static_cast<int*>(h->mE.p);
+      if (!same) {
+        fa = static_cast<double*>(h->mE.p);
+        fb = fa + g.K;
+        int* sizes = reinterpret_cast<int*>(fb + g.K);
+        ea = sizes + 2 * g.K;
+        RPA_CUDA(h, rpa::launch_mod_balance(g.A, g.a_m, g.a_k, g.M, g.B, g.b_n, g.b_k, g.N, g.K, g.kscale, sizes, fa, fb,
+                                            h->stream));
+      }
+      int* eb = ea + g.M;
+      if (g.a_k == 1) RPA_CUDA(h, rpa::launch_mod_cols(g.A, g.a_m, 0, (int)g.K, g.M, 1, pa, ea, h->stream, 0.0, fa));
+      else RPA_CUDA(h, rpa::launch_mod_rows(g.A, g.a_k, g.M, g.K, fa, pa, ea, h->stream));
       for (int64_t n0 = 0; n0 < g.N; n0 += nb) {
         const int64_t n = std::min<int64_t>(nb, g.N - n0);
         if (g.b_k == 1)
-          RPA_CUDA(h, rpa::launch_mod_cols(g.B + n0 * g.b_n, g.b_n, 0, (int)g.K, n, 1, pb, eb, h->stream, 0.0,
-                                           g.kscale));
-        else RPA_CUDA(h, rpa::launch_mod_rows(g.B + n0, g.b_k, (int)n, g.K, pb, eb, h->stream));
+          RPA_CUDA(h, rpa::launch_mod_cols(g.B + n0 * g.b_n, g.b_n, 0, (int)g.K, n, 1, pb, eb, h->stream, 0.0, fb));
+        else RPA_CUDA(h, rpa::launch_mod_rows(g.B + n0, g.b_k, (int)n, g.K, fb, pb, eb, h->stream));
         rpa::ModGemmArgs a{};
         if (int s = mod_product(h, a, pb, NM, (int)n, pa, NM, g.M, g.K, 1, false, static_cast<uint8_t*>(h->mC.p), ldo))
           return s;

@@ -135,6 +135,47 @@ __global__ void __launch_bounds__(256) mod_cols_kernel(const double* __restrict_
   }
 }
 
+// ---- sizes of two operands along K
+// A product whose operands are graded against each other along K (large entries of a where those of b
+// are small) would lose what the rows' own powers of two round away: 2^-58 of a row norm is much for a
+// small entry that meets a large one.  Column k of a is therefore multiplied by 2^h and column k of b by
+// 2^-h, exactly, so that their largest entries agree; then a' = a S, b' = b S^-1 (S diagonal, powers of
+// two) give the same integers as a and b.  Sizes are the upper words of the largest magnitudes.
+// K contiguous, entry (r, k) at S[r * ld + k]: a thread per k, 64 rows per CTA.
+constexpr int kSizeRows = 64;
+__global__ void __launch_bounds__(256) mod_ksize_cols_kernel(const double* __restrict__ S, int64_t ld, int64_t rows,
+                                                             int64_t K, int* __restrict__ size) {
+  const int64_t k = (int64_t)blockIdx.y * 256 + threadIdx.x;
+  if (k >= K) return;
+  const int64_t r0 = (int64_t)blockIdx.x * kSizeRows, r1 = min(rows, r0 + kSizeRows);
+  int m = 0;
+#pragma unroll 8
+  for (int64_t r = r0; r < r1; ++r) m = max(m, __double2hiint(__ldg(S + r * ld + k)) & 0x7fffffff);
+  atomicMax(size + k, m);
+}
+// Rows contiguous, entry (r, k) at S[r + k * ld]: a warp per k.
+__global__ void __launch_bounds__(256) mod_ksize_rows_kernel(const double* __restrict__ S, int64_t ld, int64_t rows,
+                                                             int64_t K, int* __restrict__ size) {
+  const int64_t k = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (k >= K) return;
+  int m = 0;
+#pragma unroll 8
+  for (int64_t r = threadIdx.x & 31; r < rows; r += 32) m = max(m, __double2hiint(__ldg(S + r + k * ld)) & 0x7fffffff);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) size[k] = m;
+}
+// The factors of column k: 2^h for a; 2^-h, and the product's own scale of k, for b.
+__global__ void mod_kfactor_kernel(const int* __restrict__ size_a, const int* __restrict__ size_b,
+                                   const double* __restrict__ kscale, int64_t K, double* __restrict__ fa,
+                                   double* __restrict__ fb) {
+  const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (k >= K) return;
+  const double s = kscale ? kscale[k] : 1.0;
+  const int h = mod_balance(size_a[k], size_b[k], kscale ? __double2hiint(s) & 0x7fffffff : 1023 << 20);
+  fa[k] = mod_pow2(h);
+  fb[k] = mod_pow2(-h) * s;
+}
+
 // fac[k * nov + ai] = sqrt(alpha D / (D^2 + u_k^2))
 __global__ void mod_chi_kernel(const double* __restrict__ D, int64_t nov, FreqGroup fg, double alpha,
                                double* __restrict__ fac) {
@@ -208,22 +249,28 @@ __global__ void mod_pi_expo_kernel(const double* __restrict__ part, int nsplit, 
   expo[i] = mod_exponent(s, 0);
 }
 
-// expo[r] of the rows of a column-major (rows x K) matrix: lane = row, eight warps stride over k
+// expo[r] of the rows of a column-major (rows x K) matrix, column k times fac[k] when given: lane = row,
+// eight warps stride over k
 __global__ void __launch_bounds__(256) mod_row_norm_kernel(const double* __restrict__ S, int64_t ld, int rows,
-                                                           int64_t K, int* __restrict__ expo) {
+                                                           int64_t K, const double* __restrict__ fac,
+                                                           int* __restrict__ expo) {
   __shared__ double red[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = blockIdx.x * 32 + lane;
+  auto entry = [&](int64_t k) {
+    const double x = r < rows ? S[r + ld * k] : 0.0;
+    return fac ? x * __ldg(fac + k) : x;
+  };
   auto sum = [&](double f) {
     double s0 = 0.0, s1 = 0.0;
     int64_t k = warp;
     for (; k + 8 < K; k += 16) {
-      const double x = r < rows ? S[r + ld * k] * f : 0.0, y = r < rows ? S[r + ld * (k + 8)] * f : 0.0;
+      const double x = entry(k) * f, y = entry(k + 8) * f;
       s0 = fma(x, x, s0);
       s1 = fma(y, y, s1);
     }
-    if (k < K && r < rows) {
-      const double x = S[r + ld * k] * f;
+    if (k < K) {
+      const double x = entry(k) * f;
       s0 = fma(x, x, s0);
     }
     __syncthreads();
@@ -250,7 +297,7 @@ __global__ void __launch_bounds__(256) mod_row_norm_kernel(const double* __restr
 // NQ 2048, 16384 ai, 16 frequencies).
 constexpr int kPiPitch = 128 + 4;
 constexpr size_t kModPiSmem = sizeof(double) * (32 * kPiPitch + kMaxKgLaunch * 128);
-// kFac false: the rows of R itself (one set of planes, no factors).
+// kFac false: the rows of R itself (one set of planes, no factors); with kg = 1 fac is any factor per column.
 template <bool kFac>
 __global__ void __launch_bounds__(256, 4) mod_pi_kernel(const double* __restrict__ R, int64_t ldR, int NQ, int64_t nov,
                                                         const double* __restrict__ fac, int kg,
@@ -1048,17 +1095,36 @@ cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, con
   return cudaGetLastError();
 }
 
-cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, int8_t* planes, int* expo,
-                            cudaStream_t stream) {
+cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, const double* fac, int8_t* planes,
+                            int* expo, cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
   const int64_t pitch = mod_pitch(K);
-  const cudaError_t e =
-      cudaFuncSetAttribute(mod_pi_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModPiSmem);
-  if (e != cudaSuccess) return e;
-  mod_row_norm_kernel<<<(unsigned)((rows + 31) / 32), 256, 0, stream>>>(S, ld, rows, K, expo);
-  mod_pi_kernel<false><<<dim3((unsigned)((rows + 31) / 32), (unsigned)((pitch + 127) / 128)), 256,
-                         sizeof(double) * 32 * kPiPitch, stream>>>(S, ld, rows, K, nullptr, 1, expo, planes, pitch);
+  mod_row_norm_kernel<<<(unsigned)((rows + 31) / 32), 256, 0, stream>>>(S, ld, rows, K, fac, expo);
+  const dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((pitch + 127) / 128));
+  constexpr size_t smem = sizeof(double) * (32 * kPiPitch + 128);
+  static_assert(smem <= 48 * 1024, "no opt-in needed");
+  if (fac) mod_pi_kernel<true><<<grid, 256, smem, stream>>>(S, ld, rows, K, fac, 1, expo, planes, pitch);
+  else mod_pi_kernel<false><<<grid, 256, smem, stream>>>(S, ld, rows, K, nullptr, 1, expo, planes, pitch);
   g_launches += 2;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mod_balance(const double* A, int64_t a_r, int64_t a_k, int64_t rowsA, const double* B, int64_t b_r,
+                               int64_t b_k, int64_t rowsB, int64_t K, const double* kscale, int* sizes, double* fa,
+                               double* fb, cudaStream_t stream) {
+  if (K <= 0 || rowsA <= 0 || rowsB <= 0) return cudaSuccess;
+  const cudaError_t e = cudaMemsetAsync(sizes, 0, 2 * (size_t)K * sizeof(int), stream);
+  if (e != cudaSuccess) return e;
+  auto size = [&](const double* S, int64_t s_r, int64_t s_k, int64_t rows, int* out) {
+    if (s_k == 1)
+      mod_ksize_cols_kernel<<<dim3((unsigned)((rows + kSizeRows - 1) / kSizeRows), (unsigned)((K + 255) / 256)), 256, 0,
+                              stream>>>(S, s_r, rows, K, out);
+    else mod_ksize_rows_kernel<<<(unsigned)((K + 7) / 8), 256, 0, stream>>>(S, s_k, rows, K, out);
+  };
+  size(A, a_r, a_k, rowsA, sizes);
+  size(B, b_r, b_k, rowsB, sizes + K);
+  mod_kfactor_kernel<<<(unsigned)((K + 255) / 256), 256, 0, stream>>>(sizes, sizes + K, kscale, K, fa, fb);
+  g_launches += 3;
   return cudaGetLastError();
 }
 

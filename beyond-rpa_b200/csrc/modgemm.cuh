@@ -46,6 +46,15 @@ __device__ __forceinline__ double mod_pow2(int e) {
   return __longlong_as_double((long long)(1023 + e) << 52);
 }
 
+// h such that 2^h a and 2^-h b are of the same size, from the upper words of the magnitudes of a, b and a
+// factor of b (zero or denormal ones count as 2^-1023).  No scaling where one is not finite.
+__host__ __device__ __forceinline__ int mod_balance(int a, int b, int fb) {
+  const int ea = a >> 20, eb = (b >> 20) + (fb >> 20) - 1023;
+  if (ea >= 2047 || (b >> 20) >= 2047 || (fb >> 20) >= 2047) return 0;
+  const int h = (eb - ea) >> 1;
+  return h < -1000 ? -1000 : h > 1000 ? 1000 : h;
+}
+
 // Integers from four neighbouring columns of residues (one byte each, planes apart), as doubles
 // rounded once: sum_i r_i W_i mod P in (-P/2, P/2).
 __device__ __forceinline__ void mod_crt4(const uint8_t* src, int64_t plane, const ModCrt& crt, double (&c)[4]) {
@@ -94,9 +103,15 @@ cudaError_t mod_map(PFN_cuTensorMapEncodeTiled_v12000 encode, CUtensorMap* m, vo
 cudaError_t launch_mod_cols(const double* S, int64_t ld, int64_t strideS, int K, int64_t rows, int batch,
                             int8_t* planes, int* expo, cudaStream_t stream, double shift = 0.0,
                             const double* ks = nullptr);
-// Residue planes [modulus][row][pitch] of the rows of S (rows x K, column-major).
-cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, int8_t* planes, int* expo,
-                            cudaStream_t stream);
+// Residue planes [modulus][row][pitch] of the rows of S (rows x K, column-major), column k times fac[k] when
+// fac is given.
+cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, const double* fac, int8_t* planes,
+                            int* expo, cudaStream_t stream);
+// fa[k], fb[k]: factors that bring column k of both operands to the same size (mod_balance), fb times
+// kscale[k] when given.  Entry (r, k) of an operand at S[r * s_r + k * s_k], one stride 1; sizes: 2 K ints.
+cudaError_t launch_mod_balance(const double* A, int64_t a_r, int64_t a_k, int64_t rowsA, const double* B, int64_t b_r,
+                               int64_t b_k, int64_t rowsB, int64_t K, const double* kscale, int* sizes, double* fa,
+                               double* fb, cudaStream_t stream);
 // Residue planes [k][modulus][Q][pitch] of X_k; fac: fg.n * nov doubles, part: nsplit * fg.n * NQ.
 cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, const double* D, const FreqGroup& fg,
                           double alpha, double* fac, double* part, int nsplit, int* expo, int8_t* planes,

@@ -71,6 +71,15 @@ typedef enum rpa_status {
 #define RPA_PREC_SPLIT_BF16 1 /* X = hi + lo (bf16), 3 tcgen05 products, FP32 acc,
                                  exact FP64 diagonal                               */
 
+/* Large FP64 products of the other entry points (rpa_b200_thc_r, rpa_b200_ec_thc,
+ * rpa_b200_dring_t2, rpa_b200_exchange_mbpt3, rpa_b200_piu_basis,
+ * rpa_b200_project_basis, rpa_b200_jctc2024) also run as int8 residue products:
+ * the sums are exact, and the entries of both operands are rounded at 2^-58 of
+ * the norm of their row of the product.  Both are first scaled along the summed
+ * index by powers of two that make their largest entries equal, so a product
+ * does not depend on how a scale is shared between its operands (THC: Z(g, :)
+ * against X(g, :)).                                                          */
+
 typedef struct rpa_b200_handle rpa_b200_handle;
 
 /* Create / destroy a handle bound to one GPU (`device` = CUDA ordinal).

@@ -46,3 +46,26 @@ def test_descriptors_rewritten_in_place(pkg):
             i = (it * 2 + it // 3) % 3
             assert np.array_equal(h.ec_from_pi(pis[i], np.ones(2))[1], ref_e[i])
             assert np.array_equal(h.ec_batched(sets[i], prec="split")[0], ref_b[i])
+
+
+@pytest.mark.parametrize("sd", [0.0, 2.0, 4.0])
+def test_thc_vectors_from_graded_factors(handle, sd):
+    # R(k, ai) = sum_g Z(g, k) Xa(g, a) Xi(g, i) does not change when grid points of Z are scaled by t(g) and
+    # those of Xa by 1 / t(g) (log-normal t: sizes e^-3sd .. e^3sd and more), nor may its accuracy.  Powers of two
+    # give the same bits; any t leaves the error below 16 units of 2^-53 of the sum of magnitudes, the rounding of
+    # operands of even size (FP64 sums of 2500 terms stay within 2500).
+    ng, nq, no, nv = 2500, 801, 12, 126
+    Z, Xa, Xi, _, _ = O.make_thc_factors(ng, nq, no, nv, 5)
+    rng = np.random.default_rng(17)
+    t = np.exp(sd * rng.standard_normal(ng))
+    two = np.exp2(np.rint(np.log2(t)))
+    R = handle.thc_r(Z, Xa, Xi)
+    assert np.array_equal(handle.thc_r(Z * two[:, None], Xa / two[:, None], Xi), R)
+    Zs, Xs = Z * t[:, None], Xa / t[:, None]
+    got = handle.thc_r(Zs, Xs, Xi)
+    k = rng.integers(0, nq, 24)
+    ai = rng.integers(0, no * nv, 40)
+    a = Zs[:, k].astype(np.longdouble)
+    b = (Xs[:, ai % nv].astype(np.longdouble) * Xi[:, ai // nv])
+    ref, size = a.T @ b, np.abs(a).T @ np.abs(b)
+    assert np.max(np.abs(got[np.ix_(k, ai)] - ref) / size) < 16 * 2.0 ** -53
