@@ -3756,7 +3756,10 @@ static int grad_trsm(rpa_b200_handle* h, const Validated& v, const double* Rd, i
 // The same by explicit inverses: V = L^-1, M_k = V^T V - 1 = (1 + Pi_k)^{-1} - 1, and M_k R as
 // residue products on the int8 tensor cores (R is converted once for all frequencies), accumulated
 // straight from the residues.  1 + Pi_k has eigenvalues >= 1, so ||V|| <= 1 and the inverse is as
-// accurate as the two solves.  Returns 1 (nothing done) for small orders or without memory.
+// accurate as the two solves.  M_k is formed from V - 1, not from V: Cholesky vectors are graded (their rows
+// fall off), entries of M_k then fall off in both indices, and V^T V - 1 would leave them with the absolute error
+// of the ones on the diagonal (rows of dR 1e-8 of the largest lost 8 of their 14 digits).
+// Returns 1 (nothing done) for small orders or without memory.
 // NQ 2560, 30720 ai, 16 frequencies: the solves took 390 ms (GEMM updates at 35 TFLOP/s 305 ms,
 // diagonal blocks 83 ms).
 static int grad_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t ldd, double alpha, double* dRd,
@@ -3786,13 +3789,13 @@ static int grad_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, in
   int* er = em + (size_t)v.K * n;
   const int64_t nn = (int64_t)n * n;
   RPA_CUDA(h, rpa::launch_tri_inverse(L, n, nn, V, n, nn, n, v.K, h->stream));
-  RPA_CUDA(h, rpa::launch_mod_cols(V, n, nn, n, n, v.K, mp, em, h->stream));
+  RPA_CUDA(h, rpa::launch_mod_cols(V, n, nn, n, n, v.K, mp, em, h->stream, 1.0));
   rpa::ModGemmArgs a{};
   int s;
   if ((s = mod_product(h, a, mp, v.K * NM, n, mp, v.K * NM, n, n, v.K, true, res, ldo))) return s;
-  RPA_CUDA(h, rpa::launch_mod_crt_lower(res, a.out_plane, ldo, em, n, v.K, L, n, nn, h->stream));
+  RPA_CUDA(h, rpa::launch_mod_crt_lower(res, a.out_plane, ldo, em, n, v.K, L, n, nn, h->stream, V));
   RPA_CUDA(h, rpa::launch_symmetrize(L, n, nn, n, v.K, h->stream));
-  RPA_CUDA(h, rpa::launch_mod_cols(L, n, nn, n, n, v.K, mp, em, h->stream, 1.0));
+  RPA_CUDA(h, rpa::launch_mod_cols(L, n, nn, n, n, v.K, mp, em, h->stream));
   RPA_CUDA(h, rpa::launch_mod_cols(Rd, ldd, 0, n, nov, 1, rp, er, h->stream));
   for (int g0 = 0; g0 < v.K; g0 += grp) {
     const int nb = std::min(grp, v.K - g0);

@@ -917,11 +917,14 @@ __global__ void __launch_bounds__(256) mod_chol_crt_kernel(const ModMat* __restr
 }
 
 // ------------------------------------------------------------------ C from its residues
-// Lower triangles Pi_z(i, j), i >= j (column-major, ld NQ): four consecutive i per thread.
+// Lower triangles Pi_z(i, j), i >= j (column-major, ld NQ): four consecutive i per thread.  With V (lower
+// triangles, as C): the residues are those of (V - 1)^T (V - 1), and C = V^T V - 1 is put together without the
+// cancellation: V + V^T - 2 + (V - 1)^T (V - 1).
 __global__ void __launch_bounds__(256) mod_crt_lower_kernel(const uint8_t* __restrict__ res, int64_t plane,
                                                             int64_t ldo, const ModCrt crt,
                                                             const int* __restrict__ expo, int n,
-                                                            double* __restrict__ C, int64_t ldc, int64_t strideC) {
+                                                            double* __restrict__ C, int64_t ldc, int64_t strideC,
+                                                            const double* __restrict__ V) {
   const int z = blockIdx.z, j = blockIdx.y;
   const int i0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (i0 + 3 < j || i0 >= n) return;
@@ -929,11 +932,14 @@ __global__ void __launch_bounds__(256) mod_crt_lower_kernel(const uint8_t* __res
   double c[4];
   mod_crt4(src, plane, crt, c);
   const double sj = mod_pow2(-expo[(int64_t)z * n + j]);
-  double* dst = C + (int64_t)z * strideC + (int64_t)j * ldc;
+  const int64_t off = (int64_t)z * strideC + (int64_t)j * ldc;
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int i = i0 + e;
-    if (i >= j && i < n) dst[i] = c[e] * mod_pow2(-expo[(int64_t)z * n + i]) * sj;
+    if (i < j || i >= n) continue;
+    double x = c[e] * mod_pow2(-expo[(int64_t)z * n + i]) * sj;
+    if (V) x += i == j ? 2.0 * (V[off + i] - 1.0) : V[off + i];
+    C[off + i] = x;
   }
 }
 
@@ -1160,9 +1166,9 @@ cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const
 }
 
 cudaError_t launch_mod_crt_lower(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo, int n, int batch,
-                                 double* C, int64_t ldc, int64_t strideC, cudaStream_t stream) {
+                                 double* C, int64_t ldc, int64_t strideC, cudaStream_t stream, const double* V) {
   mod_crt_lower_kernel<<<dim3((unsigned)((n + 1023) / 1024), (unsigned)n, (unsigned)batch), 256, 0, stream>>>(
-      res, plane, ldo, tables().crt, expo, n, C, ldc, strideC);
+      res, plane, ldo, tables().crt, expo, n, C, ldc, strideC, V);
   ++g_launches;
   return cudaGetLastError();
 }

@@ -121,8 +121,10 @@ int64_t mod_sync_words(const ModGemmArgs& a, int num_sms);
 // tmA, tmB: the operands' planes as boxes of 128 rows (mod_map).
 cudaError_t launch_modgemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const ModGemmArgs& a, int num_sms,
                            cudaStream_t stream);
+// V (optional, leading dimension and stride of C): C = V^T V - 1 from the residues of (V - 1)^T (V - 1).
 cudaError_t launch_mod_crt_lower(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo, int n, int batch,
-                                 double* C, int64_t ldc, int64_t strideC, cudaStream_t stream);
+                                 double* C, int64_t ldc, int64_t strideC, cudaStream_t stream,
+                                 const double* V = nullptr);
 cudaError_t launch_mod_crt_full(const uint8_t* res, int64_t plane, int64_t ldo, const int* expo_i, const int* expo_j,
                                 int ni, int64_t nj, double* C, int64_t ldc, double alpha, double beta,
                                 cudaStream_t stream);

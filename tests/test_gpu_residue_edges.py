@@ -69,3 +69,44 @@ def test_thc_vectors_from_graded_factors(handle, sd):
     b = (Xs[:, ai % nv].astype(np.longdouble) * Xi[:, ai // nv])
     ref, size = a.T @ b, np.abs(a).T @ np.abs(b)
     assert np.max(np.abs(got[np.ix_(k, ai)] - ref) / size) < 16 * 2.0 ** -53
+
+
+def _graded_grad(handle, nq, no, nv, k, span):
+    # rows of R from 1 down to e^-span, as pivoted Cholesky vectors fall off
+    rng = np.random.default_rng(nq)
+    nov = no * nv
+    R = np.asfortranarray(rng.standard_normal((nq, nov)) * 0.05 * np.exp(-np.linspace(0, span, nq))[:, None])
+    eo, ev = np.sort(rng.uniform(-1.0, -0.5, no)), np.sort(rng.uniform(0.1, 2.0, nv))
+    x, w = O.casimir_polder(k, 0.8)
+    _, dR, dO, dV = handle.ec_grad(R, eo, ev, x, w, prec="fp64")
+    return R, eo, ev, x, w, dR
+
+
+@pytest.mark.parametrize("nq, span, sample", [(200, 0.0, 200), (200, 20.0, 200), (330, 30.0, 330)])
+def test_gradient_rows_of_graded_vectors(handle, nq, span, sample):
+    # every row of dE/dR against its own size: (1 + Pi)^-1 - 1 = -X (1 + X^T X)^-1 X^T is graded as R is, and
+    # so are the errors of a factorization of 1 + Pi and of its solves: nq roundings of 2^-53 per row, four-fold
+    # for the two triangular factors and the two products.  Reference: the small side, 80-bit.
+    R, eo, ev, x, w, dR = _graded_grad(handle, nq, 2, 64, 2, span)
+    d = O.dai(eo, ev).astype(np.longdouble)
+    Rl = R.astype(np.longdouble)
+    ref = np.zeros(R.shape, np.longdouble)
+    for u, f in zip(x, w):
+        c = d / (d * d + np.longdouble(u) ** 2)
+        X = Rl * np.sqrt(4.0 * c)[None, :]
+        B = np.eye(R.shape[1], dtype=np.longdouble) + X.T @ X
+        # (1 + X X^T)^-1 X = X B^-1; solve by Cholesky in 80 bits
+        n = B.shape[0]
+        L = np.zeros_like(B)
+        for j in range(n):
+            L[j:, j] = B[j:, j] - L[j:, :j] @ L[j, :j]
+            L[j:, j] /= np.sqrt(L[j, j])
+        Y = X.copy()  # rows times L^-T, then L^-1
+        for j in range(n):
+            Y[:, j] = (Y[:, j] - Y[:, :j] @ L[j, :j]) / L[j, j]
+        for j in range(n - 1, -1, -1):
+            Y[:, j] = (Y[:, j] - Y[:, j + 1:] @ L[j + 1:, j]) / L[j, j]
+        # dE/dR = w / (2 pi) 2 alpha c ((1 + Pi)^-1 - 1) R: X column a is sqrt(4 c_a) R column a
+        ref += f / (2 * np.pi) * 2.0 * np.sqrt(4.0 * c)[None, :] * (Y - X)
+    err = np.linalg.norm((dR - ref).astype(float), axis=1) / np.linalg.norm(ref.astype(float), axis=1)
+    assert np.max(err) < 16 * nq * 2.0 ** -53
