@@ -151,6 +151,7 @@ struct rpa_b200_handle {
     int nb2, tile_w;
     int oz;  // digits of the int8 trailing updates (0: DMMA)
     const void* mod;  // descriptors of the residue updates (null: DMMA); their contents are the call's
+    bool unit_shift;  // of the residue updates (rpa::ModChol)
     cudaGraphExec_t exec;
     int64_t launches;
   };
@@ -960,14 +961,16 @@ const rpa::OzakiWork* ozaki_for(rpa_b200_handle* h, int n, int nmat, const rpa::
   return &h->ozw;
 }
 
-int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, int nmat, double* Ldiag) {
+int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, int nmat, double* Ldiag,
+             bool unit_shift = false) {
   if (int ts = tune_single(h, n, nmat)) return ts;
   const rpa::LogdetPlan plan = plan_for(h, n);
   const rpa::OzakiWork* oz = ozaki_for(h, n, nmat, plan);
   rpa::ModChol mc;
   if (int ms = mod_chol_for(h, A, ld, stride, n, nmat, &mc)) return ms;
+  mc.unit_shift = unit_shift && mc.mats;
   for (auto& g : h->chol_graphs) {
-    if (g.mod == mc.mats && g.A == A && g.ld == ld && g.stride == stride && g.n == n && g.nmat == nmat && g.Ldiag == Ldiag &&
+    if (g.mod == mc.mats && g.unit_shift == mc.unit_shift && g.A == A && g.ld == ld && g.stride == stride && g.n == n && g.nmat == nmat && g.Ldiag == Ldiag &&
         g.stream == h->stream && g.nb2 == plan.nb2 && g.tile_w == plan.tile_w && g.oz == (oz ? oz->S : 0)) {
       RPA_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
       rpa::g_launches += g.launches;
@@ -991,7 +994,8 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
         h->chol_graphs.erase(h->chol_graphs.begin());
       }
       h->chol_graphs.push_back(
-          {A, ld, stride, n, nmat, Ldiag, h->stream, plan.nb2, plan.tile_w, oz ? oz->S : 0, mc.mats, exec, count});
+          {A, ld, stride, n, nmat, Ldiag, h->stream, plan.nb2, plan.tile_w, oz ? oz->S : 0, mc.mats, mc.unit_shift,
+           exec, count});
       RPA_CUDA(h, cudaGraphLaunch(exec, h->stream));
       rpa::g_launches += count;
       return RPA_OK;
@@ -1007,7 +1011,8 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
 }
 
 // Energy from the lower triangles of K matrices Pi_k stored in h->Pi (ld = NQ).
-int energy_from_workspace(rpa_b200_handle* h, int NQ, int K, const std::vector<double>& w, double* Ec, double* Eu) {
+int energy_from_workspace(rpa_b200_handle* h, int NQ, int K, const std::vector<double>& w, double* Ec, double* Eu,
+                          bool unit_shift = false) {
   double* Pi = static_cast<double*>(h->Pi.p);
   RPA_CUDA(h, ensure(h->Ldiag, (size_t)K * NQ * 8));
   RPA_CUDA(h, ensure(h->ddbuf, (size_t)4 * K * 8));
@@ -1015,7 +1020,7 @@ int energy_from_workspace(rpa_b200_handle* h, int NQ, int K, const std::vector<d
   double* ld = tr + 2 * K;
   RPA_CUDA(h, rpa::launch_trace_shift(Pi, NQ, (int64_t)NQ * NQ, NQ, K, nullptr, tr, h->stream));
   RPA_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
-  int cs = cholesky(h, Pi, NQ, (int64_t)NQ * NQ, NQ, K, static_cast<double*>(h->Ldiag.p));
+  int cs = cholesky(h, Pi, NQ, (int64_t)NQ * NQ, NQ, K, static_cast<double*>(h->Ldiag.p), unit_shift);
   if (cs != RPA_OK) return cs;
   RPA_CUDA(h, rpa::launch_logdet_sum(static_cast<double*>(h->Ldiag.p), NQ, K, ld, h->stream));
   RPA_CUDA(h, cudaEventRecord(h->ev[3], h->stream));
@@ -1709,7 +1714,8 @@ int rpa_b200_dring_t2(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVir
   RPA_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
   if ((s = build_pi(h, v, Rd, ldd, alpha, prec))) return s;
   double ec = 0.0;
-  if ((s = energy_from_workspace(h, v.NQ, v.K, v.weights, &ec, nullptr))) return s;  // leaves L_k in h->Pi
+  // leaves L_k in h->Pi; the split form's Pi is semidefinite to 2^-16 only
+  if ((s = energy_from_workspace(h, v.NQ, v.K, v.weights, &ec, nullptr, prec == RPA_PREC_FP64))) return s;
   if (Ec) *Ec = ec;
 
   T2Ctx c;
@@ -3827,7 +3833,7 @@ int rpa_b200_ec_grad(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVirt
   // recompute Pi(u) for every frequency and factor 1 + Pi(u) (the energy comes out on the way)
   if ((s = build_pi(h, v, Rd, ldd, alpha, prec))) return s;
   double ec = 0.0;
-  if ((s = energy_from_workspace(h, v.NQ, v.K, v.weights, &ec, nullptr))) return s;
+  if ((s = energy_from_workspace(h, v.NQ, v.K, v.weights, &ec, nullptr, prec == RPA_PREC_FP64))) return s;
   if (Ec) *Ec = ec;
   const int n = v.NQ;
   const int64_t nov = v.nov;

@@ -215,6 +215,7 @@ cudaError_t launch_ozaki_update(const OzakiWork& w, int buf, double* A, int64_t 
 struct ModMat;
 struct ModChol {
   const ModMat* mats = nullptr;
+  bool unit_shift = false;  // the matrices are 1 + P with P positive semidefinite to rounding
 };
 // Outer block of the factorization under residue updates: a multiple of 128, at most 256 (the residue
 // buffers hold that many columns); 0 when the plan's block is none.

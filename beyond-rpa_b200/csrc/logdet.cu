@@ -604,7 +604,7 @@ cudaError_t launch_cholesky_lower(double* A, int64_t ld, int64_t stride, int n, 
   const int nb2 = use_mod ? mod_chol_block(plan.nb2) : plan.nb2;
   if (cudaError_t e0 = panel_smem_optin()) return e0;
   if (use_mod)
-    if (cudaError_t e0 = launch_mod_chol_expo(mc->mats, nmat, n, stream)) return e0;
+    if (cudaError_t e0 = launch_mod_chol_expo(mc->mats, nmat, n, mc->unit_shift, stream)) return e0;
   int obuf = 0;  // digit-plane buffer of the current outer block (alternates: the rest of block t's
                  // update may still read its planes while block t+1 is sliced)
   LookaheadState st{la, stream};
@@ -681,7 +681,7 @@ cudaError_t launch_logdet_varlen(const MatDesc* mats, int nmat, int nmax, int* e
   if (e != cudaSuccess) return e;
   const bool use_mod = mc && mc->mats && mod_chol_block(plan.nb2) > 0;
   const int nb2 = use_mod ? mod_chol_block(plan.nb2) : plan.nb2;
-  if (use_mod && (e = launch_mod_chol_expo(mc->mats, nmat, nmax, stream)) != cudaSuccess) return e;
+  if (use_mod && (e = launch_mod_chol_expo(mc->mats, nmat, nmax, mc->unit_shift, stream)) != cudaSuccess) return e;
   LookaheadState st{la, stream};
   if ((e = st.begin(stream)) != cudaSuccess) return e;
   const cudaStream_t S = st.S;

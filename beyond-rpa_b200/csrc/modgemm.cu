@@ -863,11 +863,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
 }
 
-// Power of two of every row of a Cholesky factor, known beforehand: ||L_i||^2 = A_ii.
-__global__ void mod_chol_expo_kernel(const ModMat* __restrict__ mats) {
+// Power of two of every row of a Cholesky factor, known beforehand: ||L_i||^2 = A_ii.  The products take the
+// entries left of the diagonal only; for A = 1 + P, P positive semidefinite, L_ii^2 >= 1 and their norm is
+// at most A_ii - 1, which keeps the digits of rows with small P_ii (graded Cholesky vectors).  The
+// factorization's own rounding, n 2^-53 A_ii, is added fourfold.
+__global__ void mod_chol_expo_kernel(const ModMat* __restrict__ mats, int unit_shift) {
   const ModMat& m = mats[blockIdx.y];
   const int i = blockIdx.x * 256 + threadIdx.x;
-  if (i < m.n) m.expo[i] = mod_exponent(m.A[i + m.ld * (int64_t)i], 0);
+  if (i >= m.n) return;
+  double s2 = m.A[i + m.ld * (int64_t)i];
+  if (unit_shift) s2 = fmax(s2 - 1.0, 0.0) + 4.0 * m.n * 1.1102230246251565e-16 * s2;
+  m.expo[i] = mod_exponent(s2, 0);
 }
 
 // Planes of columns c0 .. c0 + nb - 1 (nb a multiple of 128), rows row0 .. n - 1, of the factors: the
@@ -1216,8 +1222,9 @@ cudaError_t mod_chol_fill(PFN_cuTensorMapEncodeTiled_v12000 encode, ModMat& m, d
   return e == cudaSuccess ? mod_map(encode, &m.mB, m.planes, n, n, kModCount, m.pitch, MG_TN) : e;
 }
 
-cudaError_t launch_mod_chol_expo(const ModMat* mats, int nmat, int nmax, cudaStream_t stream) {
-  mod_chol_expo_kernel<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)nmat), 256, 0, stream>>>(mats);
+cudaError_t launch_mod_chol_expo(const ModMat* mats, int nmat, int nmax, bool unit_shift, cudaStream_t stream) {
+  mod_chol_expo_kernel<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)nmat), 256, 0, stream>>>(mats,
+                                                                                                unit_shift ? 1 : 0);
   ++g_launches;
   return cudaGetLastError();
 }

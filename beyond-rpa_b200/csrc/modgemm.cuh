@@ -152,7 +152,7 @@ struct ModCholArgs {
 size_t mod_chol_bytes(int n, int nb, size_t* planes, size_t* res);  // of one matrix
 cudaError_t mod_chol_fill(PFN_cuTensorMapEncodeTiled_v12000 encode, ModMat& m, double* A, int64_t ld, int n, int nb,
                           uint8_t* base);
-cudaError_t launch_mod_chol_expo(const ModMat* mats, int nmat, int nmax, cudaStream_t stream);
+cudaError_t launch_mod_chol_expo(const ModMat* mats, int nmat, int nmax, bool unit_shift, cudaStream_t stream);
 // Planes of the factored columns c0 .. c0 + nb - 1, rows row0 and below.
 cudaError_t launch_mod_chol_planes(const ModMat* mats, int nmat, int nmax, int row0, int c0, int nb,
                                    cudaStream_t stream);
