@@ -134,6 +134,7 @@ struct rpa_b200_handle {
   // pinned host memory: orbital energies on their way to the device, and small results on theirs back
   uint8_t* pin = nullptr;
   int64_t launches = 0;
+  int selftest_error = 0;  // device error word that every check sees (RPA_B200_SELFTEST_DEVICE_ERROR; tests)
   int seg_chunks = 16;  // 512-column accumulation segments of the tensor-core SYRK
   int sync_every = 32;  // K chunks between the wave-progress milestones of the SYRK (0: off)
   DevBuf syncBuf;       // milestone counters of the SYRK waves
@@ -220,6 +221,7 @@ int finite_or_fail(rpa_b200_handle* h, std::initializer_list<double> xs, const c
     cudaError_t e_ = (call);                                                                                \
     if (e_ != cudaSuccess) {                                                                                \
       if (e_ == cudaErrorMemoryAllocation) return fail(h, RPA_ERR_OOM, "%s: %s", #call, cudaGetErrorString(e_)); \
+      if (e_ == cudaErrorLaunchTimeout) return fail(h, RPA_ERR_TIMEOUT, "device-side bounded wait expired (%s)", #call); \
       return fail(h, RPA_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_));                                \
     }                                                                                                       \
   } while (0)
@@ -322,6 +324,7 @@ int check_device_error(rpa_b200_handle* h) {
 }
 
 int device_error_status(rpa_b200_handle* h, int err) {
+  if (err == 0) err = h->selftest_error;
   if (err == rpa::kDevNotSPD) return fail(h, RPA_ERR_NOT_SPD, "1+Pi(u) is not positive definite (Cholesky pivot <= 0)");
   if (err != 0) return fail(h, RPA_ERR_TIMEOUT, "device-side bounded wait expired (code %d)", err);
   return RPA_OK;
@@ -1379,6 +1382,7 @@ int rpa_b200_create(rpa_b200_handle** handle, int64_t device, int64_t flags) try
   for (auto& e : h->ev) cudaEventCreate(&e);
   for (auto& e : h->done.ev) cudaEventCreate(&e);
   for (auto& e : h->fork_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+  if (const char* de = std::getenv("RPA_B200_SELFTEST_DEVICE_ERROR")) h->selftest_error = std::atoi(de);
   if (const char* la = std::getenv("RPA_B200_LOOKAHEAD")) h->lookahead = std::atoi(la) != 0;
   h->ozaki_slices = rpa::ozaki_slices_default();
   {
@@ -2135,9 +2139,11 @@ int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
       g2.beta = 1.0;
       if (int gs = gemm64(h, g2)) return gs;
       if ((s = sqnorm(Res, r2))) return s;
-      if (!std::isfinite(r2) || r2 > 1e4 * a2)
+      if (!std::isfinite(r2) || r2 > 1e4 * a2) {
+        if ((s = check_device_error(h))) return s;
         return fail(h, RPA_ERR_NOT_CONVERGED, "MBPT3 Lyapunov iteration diverged (|res|/|A| = %.3e)",
                     std::sqrt(r2 / a2));
+      }
       if (r2 <= 1e-26 * a2) {
         converged = true;
         break;
@@ -2157,14 +2163,18 @@ int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
       int nbad = 0;
       RPA_CUDA(h, cudaMemcpyAsync(&nbad, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
       RPA_CUDA(h, cudaStreamSynchronize(h->stream));
-      if (nbad)
+      if (nbad) {
+        if ((s = check_device_error(h))) return s;
         return fail(h, RPA_ERR_NOT_CONVERGED,
                     "MBPT3 Lyapunov solve: symmetric part of B is not positive definite (%d pairs)", nbad);
+      }
     }
   }
-  if (!converged)
+  if (!converged) {
+    if ((s = check_device_error(h))) return s;
     return fail(h, RPA_ERR_NOT_CONVERGED, "MBPT3 Lyapunov iteration did not converge (|res|/|A| = %.3e)",
                 std::sqrt(r2 / a2));
+  }
 
   // Tr(XK): W_ij from U, W_ji from U X
   if (int gs = gemm64(h, gemm_nn((int)nov, NT, NT, Ud, ldu, Xd, NT, UX, nov))) return gs;
@@ -2190,7 +2200,7 @@ int rpa_b200_exchange_mbpt3(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_
                                     cudaMemcpyDeviceToHost, h->stream));
   }
   RPA_CUDA(h, cudaEventRecord(h->ev[4], h->stream));
-  RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+  if ((s = check_device_error(h))) return s;  // also synchronises the stream
   dd acc{split_sum, 0.0};
   for (double x : hp) acc = rpa::dd_add(acc, x);
   if ((s = finite_or_fail(h, {acc.hi}, "MBPT3 exchange energy"))) return s;
@@ -2354,7 +2364,9 @@ int rpa_b200_piu_basis(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVi
         RPA_CUDA(h, cudaMemcpyAsync(piv.data(), h->Ldiag.p, (size_t)n * 8, cudaMemcpyDeviceToHost, h->stream));
         RPA_CUDA(h, cudaStreamSynchronize(h->stream));
         const auto mm = std::minmax_element(piv.begin(), piv.end());
-        if (check_device_error(h) != RPA_OK || !(*mm.first > 0.5) || !(*mm.second < 2.0))
+        s = check_device_error(h);
+        if (s == RPA_ERR_TIMEOUT) return s;
+        if (s != RPA_OK || !(*mm.first > 0.5) || !(*mm.second < 2.0))
           return fail(h, RPA_ERR_NOT_SPD, "random Pi basis: Pi G is numerically rank deficient (CholeskyQR)");
         RPA_CUDA(h, cudaMemcpyAsync(Gd, Yt, nn * 8, cudaMemcpyDeviceToDevice, h->stream));  // Gd <- Q^T
       }
@@ -2364,7 +2376,7 @@ int rpa_b200_piu_basis(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVi
       RPA_CUDA(h, cudaMemcpyAsync(Th.data(), S, nn * 8, cudaMemcpyDeviceToHost, h->stream));
       RPA_CUDA(h, cudaMemcpyAsync(Qh.data(), Yt, nn * 8, cudaMemcpyDeviceToHost, h->stream));
       RPA_CUDA(h, rpa::launch_transpose(Yt, n, n, n, Gd, n, h->stream));  // G = Q
-      RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+      if ((s = check_device_error(h))) return s;  // also synchronises the stream
       for (int p = 0; p < n; ++p) {
         dd acc{0.0, 0.0};
         for (int k = 0; k < n; ++k) acc = rpa::dd_add(acc, Th[(size_t)p + (size_t)n * k] * Qh[(size_t)p + (size_t)n * k]);
@@ -2437,6 +2449,7 @@ int rpa_b200_project_basis(rpa_b200_handle* h, int64_t NQ, int64_t NVecs, int64_
   if (int gs = gemm64(h, gemm_tn((int)NVecs, (int)nov, NQ, Gd, ldg, Rd, ldr, out, ldo))) return gs;
   RPA_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
   RPA_CUDA(h, cudaEventRecord(h->ev[3], h->stream));
+  if ((s = check_device_error(h))) return s;
   if ((s = screen_result(h, out, ldo, NVecs, nov, "the projected Cholesky vectors"))) return s;
   if (!dev_out)
     RPA_CUDA(h, cudaMemcpy2DAsync(Rp, (size_t)ldRp * 8, out, (size_t)NVecs * 8, (size_t)NVecs * 8, (size_t)nov,
@@ -2521,6 +2534,7 @@ int rpa_b200_thc_r(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOcc, 
   if ((s = form_thc_r(h, NGrid, NQ, NOcc, NVirt, Zd, ldz, Xad, ldxa, Xid, ldxi, Rd, ldr))) return s;
   RPA_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
   RPA_CUDA(h, cudaEventRecord(h->ev[3], h->stream));
+  if ((s = check_device_error(h))) return s;
   if ((s = screen_result(h, Rd, ldr, NQ, nov, "the formed Cholesky vectors"))) return s;
   if (!dev)
     RPA_CUDA(h, cudaMemcpy2DAsync(R, (size_t)ldR * 8, Rd, (size_t)NQ * 8, (size_t)NQ * 8, (size_t)nov,
@@ -2608,7 +2622,7 @@ int build_pi_thc(rpa_b200_handle* h, const Validated& v, int64_t NGrid, const do
   }
   int cnt = 0;
   RPA_CUDA(h, cudaMemcpyAsync(&cnt, h->count_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+  if ((s = check_device_error(h))) return s;  // also synchronises the stream
   if (cnt) return fail(h, RPA_ERR_NONFINITE, "%d non-finite entries in the Cholesky vectors formed from the THC factors",
                        cnt);
   return RPA_OK;
@@ -2650,6 +2664,7 @@ int rpa_b200_ec_thc(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOcc,
   RPA_CUDA(h, ensure(h->thR, (size_t)NQ * nov * 8));
   double* Rd = static_cast<double*>(h->thR.p);
   if ((s = form_thc_r(h, NGrid, NQ, NOcc, NVirt, Zd, ldz, Xad, ldxa, Xid, ldxi, Rd, NQ))) return s;
+  if ((s = check_device_error(h))) return s;  // the energy call clears the error word
   return rpa_b200_ec(h, NQ, NOcc, NVirt, Rd, NQ, OccEnergies, VirtEnergies, NFreqs, Freqs, FreqWeights, alpha, prec,
                      Ec, Eu);
 } catch (...) {
@@ -3127,7 +3142,7 @@ int rpa_b200_jctc2024(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   std::vector<double> ph((size_t)nslot * rpa::kDotPartials);
   RPA_CUDA(h, cudaMemcpyAsync(ph.data(), part, ph.size() * 8, cudaMemcpyDeviceToHost, h->stream));
   RPA_CUDA(h, cudaEventRecord(h->ev[4], h->stream));
-  RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+  if ((s = check_device_error(h))) return s;  // also synchronises the stream
   auto total = [&](int64_t p, int term) {
     dd acc{0.0, 0.0};
     const double* q = ph.data() + (size_t)(5 * p + term) * rpa::kDotPartials;

@@ -110,3 +110,45 @@ def test_gradient_rows_of_graded_vectors(handle, nq, span):
         ref += f / (2 * np.pi) * 2.0 * np.sqrt(4.0 * c)[None, :] * (Y - X)
     err = np.linalg.norm((dR - ref).astype(float), axis=1) / np.linalg.norm(ref.astype(float), axis=1)
     assert np.max(err) < 16 * nq * 2.0 ** -53
+
+
+def test_every_call_reports_an_expired_device_wait(pkg, monkeypatch):
+    # the error word of the device as every check of it sees it: a call that does not look at it before it
+    # answers would return RPA_OK with whatever an unfinished product left
+    ng, nq, no, nv = 120, 30, 4, 10
+    Z, Xa, Xi, eo, ev = O.make_thc_factors(ng, nq, no, nv, 9)
+    s = O.make_system(40, no, nv, 3, decay=10.0, lam0=0.8)
+    x, w = O.casimir_polder(4, 0.8)
+    pi = O.pi_matrices(s.R, s.eps_o, s.eps_v, x)
+    U, _ = np.linalg.qr(np.random.default_rng(2).standard_normal((no * nv, 8)))
+    A = -0.1 * np.linspace(0.2, 1.0, 8)
+    G = np.eye(40)[:, :20]
+    calls = {
+        "thc_r": lambda h: h.thc_r(Z, Xa, Xi),
+        "ec_thc fp64": lambda h: h.ec_thc(Z, Xa, Xi, eo, ev, x, w, prec="fp64"),
+        "ec_thc split": lambda h: h.ec_thc(Z, Xa, Xi, eo, ev, x, w, prec="split"),
+        "project_basis": lambda h: h.project_basis(G, s.R),
+        "piu_basis random": lambda h: h.piu_basis(s.R, s.eps_o, s.eps_v, 0.1, basis="random"),
+        "piu_basis eigen": lambda h: h.piu_basis(s.R, s.eps_o, s.eps_v, 0.1, basis="eigen"),
+        "dring_t2": lambda h: h.dring_t2(s.R, s.eps_o, s.eps_v, x, w),
+        "mbpt3 fp64": lambda h: h.exchange_mbpt3(s.R, s.eps_o, s.eps_v, U, A, prec="fp64"),
+        "mbpt3 split": lambda h: h.exchange_mbpt3(s.R, s.eps_o, s.eps_v, U, A, prec="split"),
+        "sosex split": lambda h: h.exchange_sosex(s.R, no, nv, U, A, prec="split"),
+        "jctc2024": lambda h: h.jctc2024(Z, Xi, Xa, U, A),
+        "pi_u": lambda h: h.pi_u(s.R, s.eps_o, s.eps_v, x, prec="fp64"),
+        "ec fp64": lambda h: h.ec_rpa(s.R, s.eps_o, s.eps_v, x, w, prec="fp64"),
+        "ec split": lambda h: h.ec_rpa(s.R, s.eps_o, s.eps_v, x, w, prec="split"),
+        "ec_from_pi": lambda h: h.ec_from_pi(pi, w),
+        "ec_grad": lambda h: h.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="fp64"),
+        "ec_batched": lambda h: h.ec_batched([(s.R, s.eps_o, s.eps_v, x, w)] * 2, prec="split"),
+    }
+    with pkg.Handle(0) as h:
+        for call in calls.values():
+            call(h)  # each of them is sound as it stands
+    monkeypatch.setenv("RPA_B200_SELFTEST_DEVICE_ERROR", "103")
+    with pkg.Handle(0) as h:
+        h.set_autotune(False)
+        for name, call in calls.items():
+            with pytest.raises(pkg.RPAError) as err:
+                call(h)
+            assert err.value.status == pkg.RPA_ERR_TIMEOUT, name
