@@ -36,11 +36,15 @@ struct DevBuf {
 // (rpa_b200_set_workspace_limit; 0 = none).  Every workspace allocation of a call goes through
 // dev_alloc / dev_free below, which charge the handle whose call is running on this thread.
 // idle: buffers of the handle that hold nothing between calls and that the running call has not asked
-// for yet; an allocation that finds no room frees them and tries again.
+// for yet; an allocation that finds no room frees them and tries again.  spent: buffers that the
+// running call has filled and no longer needs (give_back); they go the same way for an allocation
+// that the call cannot do without.  Optional workspace does not take them: two optional buffers that do not fit
+// together would otherwise be freed and allocated in turn by every call.
 struct WorkspaceAccount {
   size_t used = 0;
   size_t limit = 0;
-  std::vector<DevBuf*> idle;
+  std::vector<DevBuf*> idle, spent;
+  cudaStream_t stream = nullptr;  // of the running call
 };
 namespace {
 thread_local WorkspaceAccount* g_account = nullptr;
@@ -63,18 +67,24 @@ void dev_free(void* p, size_t bytes) {
   if (a) a->used = a->used > bytes ? a->used - bytes : 0;
 }
 
-cudaError_t dev_alloc(void** p, size_t bytes) {
+cudaError_t dev_alloc(void** p, size_t bytes, bool optional = false) {
   cudaError_t e = dev_alloc_once(p, bytes);
   WorkspaceAccount* a = g_account;
-  if (e != cudaErrorMemoryAllocation || !a || a->idle.empty()) return e;
-  cudaGetLastError();
-  for (DevBuf* b : a->idle) {
-    dev_free(b->p, b->bytes);
-    b->p = nullptr;
-    b->bytes = 0;
+  if (!a) return e;
+  for (auto* list : {&a->idle, &a->spent}) {
+    if (e != cudaErrorMemoryAllocation || (optional && list == &a->spent)) break;
+    if (list->empty()) continue;
+    cudaGetLastError();
+    cudaStreamSynchronize(a->stream);  // kernels of this call may still read what was given back
+    for (DevBuf* b : *list) {
+      dev_free(b->p, b->bytes);
+      b->p = nullptr;
+      b->bytes = 0;
+    }
+    list->clear();
+    e = dev_alloc_once(p, bytes);
   }
-  a->idle.clear();
-  return dev_alloc_once(p, bytes);
+  return e;
 }
 }  // namespace
 
@@ -134,6 +144,8 @@ struct rpa_b200_handle {
   // pinned host memory: orbital energies on their way to the device, and small results on theirs back
   uint8_t* pin = nullptr;
   int64_t launches = 0;
+  int gemm64_form = -1;     // FP64 products: 0 DMMA, 1 residues, -1 the faster (RPA_B200_GEMM64_RESIDUES)
+  size_t gemm64_bytes = 0;  // planes and residues of a block of columns (RPA_B200_GEMM64_BYTES; 0: the call's)
   int selftest_error = 0;  // device error word that every check sees (RPA_B200_SELFTEST_DEVICE_ERROR; tests)
   int seg_chunks = 16;  // 512-column accumulation segments of the tensor-core SYRK
   int sync_every = 32;  // K chunks between the wave-progress milestones of the SYRK (0: off)
@@ -239,11 +251,10 @@ int screen_result(rpa_b200_handle* h, const double* A, int64_t ld, int64_t rows,
   return RPA_OK;
 }
 
-cudaError_t ensure(DevBuf& b, size_t bytes) {
-  if (g_account) {
-    auto& idle = g_account->idle;
-    idle.erase(std::remove(idle.begin(), idle.end(), &b), idle.end());
-  }
+cudaError_t ensure(DevBuf& b, size_t bytes, bool optional = false) {
+  if (g_account)
+    for (auto* list : {&g_account->idle, &g_account->spent})
+      list->erase(std::remove(list->begin(), list->end(), &b), list->end());
   if (b.bytes >= bytes && b.p) return cudaSuccess;
   if (b.p) {
     dev_free(b.p, b.bytes);
@@ -251,8 +262,29 @@ cudaError_t ensure(DevBuf& b, size_t bytes) {
     b.bytes = 0;
   }
   if (bytes == 0) bytes = 256;
-  cudaError_t e = dev_alloc(&b.p, bytes);
+  cudaError_t e = dev_alloc(&b.p, bytes, optional);
   if (e == cudaSuccess) b.bytes = bytes;
+  return e;
+}
+
+// The running call no longer needs what it has put into these buffers.
+void give_back(rpa_b200_handle* h, std::initializer_list<DevBuf*> bufs) {
+  for (DevBuf* b : bufs)
+    if (b->p) h->account.spent.push_back(b);
+}
+
+// Device bytes that allocations of the running call can have: free memory and what idle and spent
+// buffers hold; with own, also the buffers about to be replaced.
+cudaError_t available_bytes(rpa_b200_handle* h, std::initializer_list<DevBuf*> own, size_t* out) {
+  size_t free_b = 0, total_b = 0;
+  const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+  std::vector<DevBuf*> bufs(own);
+  bufs.insert(bufs.end(), h->account.idle.begin(), h->account.idle.end());
+  bufs.insert(bufs.end(), h->account.spent.begin(), h->account.spent.end());
+  std::sort(bufs.begin(), bufs.end());
+  bufs.erase(std::unique(bufs.begin(), bufs.end()), bufs.end());
+  for (DevBuf* b : bufs) free_b += b->bytes;
+  *out = free_b;
   return e;
 }
 
@@ -458,14 +490,13 @@ int choose_kg(rpa_b200_handle* h, const Validated& v, int64_t pitch) {
   const size_t perFreq = (size_t)v.NQ * pitch * 2 * 2;  // hi + lo
   const int kmax = std::min(v.K, rpa::kMaxKgLaunch);
   if (h->Xhi.bytes >= (size_t)kmax * v.NQ * pitch * 2 && h->Xlo.bytes >= (size_t)kmax * v.NQ * pitch * 2) return kmax;
-  size_t freeB = 0, totalB = 0;
-  cudaError_t e = cudaMemGetInfo(&freeB, &totalB);
+  size_t avail = 0;
+  cudaError_t e = available_bytes(h, {&h->Xhi, &h->Xlo}, &avail);
   if (e != cudaSuccess) {
     fail(h, RPA_ERR_CUDA, "CUDA error %s", cudaGetErrorString(e));
     return -RPA_ERR_CUDA;
   }
-  const size_t have = h->Xhi.bytes + h->Xlo.bytes;
-  const size_t budget = (size_t)((double)(freeB + have) * 0.7);
+  const size_t budget = (size_t)((double)avail * 0.7);
   return (int)std::min<size_t>((size_t)kmax, std::max<size_t>(1, budget / perFreq));
 }
 
@@ -484,7 +515,7 @@ int prepare_sync(rpa_b200_handle* h, int NQ, int kg, int64_t nov_part, int** out
 // Allocates workspace that the caller can do without: false (no error left behind) when the device or
 // the caller's workspace cap has no room for it.
 bool try_ensure(DevBuf& b, size_t bytes) {
-  if (ensure(b, bytes) == cudaSuccess) return true;
+  if (ensure(b, bytes, true) == cudaSuccess) return true;
   cudaGetLastError();
   return false;
 }
@@ -507,8 +538,7 @@ int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t pla
   a.sync = nullptr;
   a.sync_every = h->sync_every;
   const int64_t words = rpa::mod_sync_words(a, h->num_sms);
-  if (words > 0) {
-    RPA_CUDA(h, ensure(h->syncBuf, (size_t)words * sizeof(int)));
+  if (words > 0 && try_ensure(h->syncBuf, (size_t)words * sizeof(int))) {
     RPA_CUDA(h, cudaMemsetAsync(h->syncBuf.p, 0, (size_t)words * sizeof(int), h->stream));
     a.sync = static_cast<int*>(h->syncBuf.p);
   }
@@ -527,8 +557,10 @@ bool mod_pays(int64_t M, int64_t N, int64_t K) {
 }
 
 int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30) {
+  if (h->gemm64_bytes) budget = h->gemm64_bytes;
   const bool plain = g.batch == 1 && g.splitk <= 1 && !g.rowscale && (g.a_m == 1 || g.a_k == 1) && (g.b_n == 1 || g.b_k == 1);
-  if (plain && g.K <= INT32_MAX && mod_pays(g.M, g.N, g.K)) {
+  const bool pays = h->gemm64_form < 0 ? mod_pays(g.M, g.N, g.K) : h->gemm64_form != 0;
+  if (plain && pays && g.M > 0 && g.N > 0 && g.K > 0 && g.K <= INT32_MAX) {
     const size_t NM = rpa::kModCount;
     const int64_t pitch = rpa::mod_pitch(g.K), ldo = ((int64_t)g.M + 255) / 256 * 256;
     // C is formed in blocks of columns whose planes and residues fit the budget
@@ -565,6 +597,7 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
         RPA_CUDA(h, rpa::launch_mod_crt_full(a.out, a.out_plane, ldo, ea, eb, g.M, n, g.C + n0 * g.ldc, g.ldc, g.alpha,
                                              g.beta, h->stream));
       }
+      give_back(h, {&h->mA, &h->mB, &h->mC, &h->mE});
       return RPA_OK;
     }
     for (DevBuf* b : {&h->mA, &h->mB, &h->mC, &h->mE}) release(*b);
@@ -617,6 +650,7 @@ int build_pi_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, int64
     RPA_CUDA(h, cudaEventRecord(e2, h->stream));
     h->tc_ev.push_back({e1, e2});
   }
+  give_back(h, {&h->Xhi, &h->Xlo, &h->diag_part});
   return RPA_OK;
 }
 
@@ -695,6 +729,7 @@ int build_pi(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t l
     RPA_CUDA(h, cudaEventRecord(e2, h->stream));
     h->tc_ev.push_back({e1, e2});
   }
+  give_back(h, {&h->Xhi, &h->Xlo});
   return RPA_OK;
 }
 
@@ -804,6 +839,7 @@ int build_pi_pipelined(rpa_b200_handle* h, const Validated& v, const double* Rh,
     RPA_CUDA(h, cudaEventRecord(e2, h->stream));
     h->tc_ev.push_back({e1, e2});
   }
+  give_back(h, {&h->Xhi, &h->Xlo});
   return RPA_OK;
 }
 
@@ -914,7 +950,7 @@ int tune_single(rpa_b200_handle* h, int n, int nmat) {
   if (!h->autotune || n < 512 || h->logdet_plans.count(plan_bucket(n))) return RPA_OK;
   for (int m = nmat; m >= 1; m = m > 4 ? 4 : 0) {
     void* tmp = nullptr;
-    if (dev_alloc(&tmp, (size_t)m * n * n * 8) != cudaSuccess) {
+    if (dev_alloc(&tmp, (size_t)m * n * n * 8, true) != cudaSuccess) {
       cudaGetLastError();
       continue;
     }
@@ -942,8 +978,7 @@ const rpa::OzakiWork* ozaki_for(rpa_b200_handle* h, int n, int nmat, const rpa::
   for (DevBuf& b : h->ozBuf)
     if (b.bytes < bytes) {
       cudaStreamSynchronize(h->stream);
-      if (ensure(b, bytes) != cudaSuccess) {
-        cudaGetLastError();
+      if (!try_ensure(b, bytes)) {
         h->ozw.S = 0;
         return nullptr;  // no room: DMMA updates
       }
@@ -977,6 +1012,7 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
         g.stream == h->stream && g.nb2 == plan.nb2 && g.tile_w == plan.tile_w && g.oz == (oz ? oz->S : 0)) {
       RPA_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
       rpa::g_launches += g.launches;
+      give_back(h, {&h->mcBuf});
       return RPA_OK;
     }
   }
@@ -1001,6 +1037,7 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
            exec, count});
       RPA_CUDA(h, cudaGraphLaunch(exec, h->stream));
       rpa::g_launches += count;
+      give_back(h, {&h->mcBuf});
       return RPA_OK;
     }
     if (graph) cudaGraphDestroy(graph);
@@ -1010,6 +1047,7 @@ int cholesky(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, i
   }
   // capture unavailable on this stream: launch the same kernels directly
   RPA_CUDA(h, rpa::launch_cholesky_lower(A, ld, stride, n, nmat, Ldiag, h->err_dev, h->stream, plan, nullptr, oz, &mc));
+  give_back(h, {&h->mcBuf});
   return RPA_OK;
 }
 
@@ -1291,6 +1329,8 @@ int begin_call(rpa_b200_handle* h) {
   if (!h) return RPA_ERR_INVALID_ARG;
   h->last_error.clear();
   g_account = &h->account;
+  h->account.stream = h->stream;
+  h->account.spent.clear();
   h->account.idle = {&h->Xhi, &h->Xlo, &h->gY, &h->gM, &h->mA, &h->mB, &h->mC, &h->mE, &h->mcBuf, &h->bMod, &h->jBat};
   h->pool_used = 0;
   h->split_ev.clear();
@@ -1382,6 +1422,8 @@ int rpa_b200_create(rpa_b200_handle** handle, int64_t device, int64_t flags) try
   for (auto& e : h->ev) cudaEventCreate(&e);
   for (auto& e : h->done.ev) cudaEventCreate(&e);
   for (auto& e : h->fork_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+  if (const char* gf = std::getenv("RPA_B200_GEMM64_RESIDUES")) h->gemm64_form = std::atoi(gf) != 0;
+  if (const char* gb = std::getenv("RPA_B200_GEMM64_BYTES")) h->gemm64_bytes = (size_t)std::max(0ll, std::atoll(gb));
   if (const char* de = std::getenv("RPA_B200_SELFTEST_DEVICE_ERROR")) h->selftest_error = std::atoi(de);
   if (const char* la = std::getenv("RPA_B200_LOOKAHEAD")) h->lookahead = std::atoi(la) != 0;
   h->ozaki_slices = rpa::ozaki_slices_default();
@@ -1735,8 +1777,8 @@ int rpa_b200_dring_t2(rpa_b200_handle* h, int64_t NQ, int64_t NOcc, int64_t NVir
   }
   const int G = (int)GuessNVecs;
   const int64_t nov = v.nov;
-  size_t freeB = 0, totalB = 0;
-  RPA_CUDA(h, cudaMemGetInfo(&freeB, &totalB));
+  size_t freeB = 0;
+  RPA_CUDA(h, available_bytes(h, {}, &freeB));
   const size_t zAll = (size_t)v.K * v.NQ * nov * 8;
   const size_t fixed = (size_t)nov * G * 8 * 3 + (size_t)G * G * 8 * 2;
   c.z_resident = zAll + fixed < (size_t)(0.8 * (double)(freeB + h->tZ.bytes));
@@ -2620,6 +2662,7 @@ int build_pi_thc(rpa_b200_handle* h, const Validated& v, int64_t NGrid, const do
     RPA_CUDA(h, cudaEventRecord(e2, h->stream));
     h->tc_ev.push_back({e1, e2});
   }
+  give_back(h, {&h->Xhi, &h->Xlo});
   int cnt = 0;
   RPA_CUDA(h, cudaMemcpyAsync(&cnt, h->count_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   if ((s = check_device_error(h))) return s;  // also synchronises the stream
@@ -3269,11 +3312,9 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
     release(h->Xhi);
     release(h->Xlo);
   }
-  size_t freeB = 0, totalB = 0;
-  RPA_CUDA(h, cudaMemGetInfo(&freeB, &totalB));
-  // buffers that ensure() below may free and reallocate count as available
-  const size_t have = h->Xhi.bytes + h->Xlo.bytes + h->Pi.bytes + h->Ldiag.bytes + h->bMod.bytes;
-  const size_t budget = h->batch_bytes > 0 ? h->batch_bytes : (size_t)(0.6 * (double)(freeB + have));
+  size_t avail = 0;  // buffers that ensure() below may free and reallocate count as available
+  RPA_CUDA(h, available_bytes(h, {&h->Xhi, &h->Xlo, &h->Pi, &h->Ldiag, &h->bMod}, &avail));
+  const size_t budget = h->batch_bytes > 0 ? h->batch_bytes : (size_t)(0.6 * (double)avail);
   std::vector<std::pair<int, int>> batches;  // [b0, b1)
   {
     size_t acc = 0;
@@ -3326,8 +3367,6 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
   RPA_CUDA(h, ensure(h->Ldiag, 2 * smallStride + 256));
   RPA_CUDA(h, ensure(h->bDesc, desc_off.back() + 256));
   RPA_CUDA(h, ensure(h->bRes, res_off.back() * 8 + 256));
-  // without room for the planes the log-det's updates stay on DMMA
-  const bool mod_ld = maxMod > 0 && try_ensure(h->bMod, maxMod);
 
   // wave-milestone counters of every batch's multi-instance SYRK, allocated once for the call
   std::vector<int64_t> sync_off(batches.size() + 1, 0);
@@ -3345,6 +3384,8 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
     sync_off[b + 1] = sync_off[b] + words;
   }
   if (sync_off.back() > 0) RPA_CUDA(h, ensure(h->syncBuf, (size_t)sync_off.back() * sizeof(int)));
+  // last, what the call can do without: without room for the planes the log-det's updates stay on DMMA
+  const bool mod_ld = maxMod > 0 && try_ensure(h->bMod, maxMod);
   // graph cache key: shapes, pointers and workspace addresses of this call
   uint64_t key = 1469598103934665603ull;
   auto mix = [&](uint64_t x) { key = (key ^ x) * 1099511628211ull; };
@@ -3751,10 +3792,10 @@ static int grad_trsm(rpa_b200_handle* h, const Validated& v, const double* Rd, i
                      int64_t lddr, double* dD) {
   const int n = v.NQ;
   const int64_t nov = v.nov;
-  size_t freeB = 0, totalB = 0;
-  RPA_CUDA(h, cudaMemGetInfo(&freeB, &totalB));
+  size_t avail = 0;
+  RPA_CUDA(h, available_bytes(h, {&h->gY}, &avail));
   const size_t perK = (size_t)n * nov * 8;
-  int grp = (int)std::max<size_t>(1, std::min<size_t>(16, (size_t)(0.5 * (double)(freeB + h->gY.bytes)) / perK));
+  int grp = (int)std::max<size_t>(1, std::min<size_t>(16, (size_t)(0.5 * (double)avail) / perK));
   grp = std::min(grp, v.K);
   RPA_CUDA(h, ensure(h->gY, perK * grp));
   double* Y = static_cast<double*>(h->gY.p);
@@ -3795,11 +3836,23 @@ static int grad_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, in
   const size_t b_rp = NM * nov * (size_t)pitch, b_rr = NM * nov * (size_t)ldo;  // R's planes; residues of M_k R
   // h->Xhi: planes of V, then of M; h->Xlo: residues; h->gY: V, then the planes of R
   const int grp = (int)std::min<size_t>(std::min(v.K, 16), std::max<size_t>(1, 2 * kModBudget / b_rr));
-  if (!try_ensure(h->Xhi, v.K * b_mp) || !try_ensure(h->gY, std::max(v.K * b_sq, b_rp)) ||
-      !try_ensure(h->Xlo, std::max(v.K * b_mr, grp * b_rr)) ||
-      !try_ensure(h->gM, ((size_t)v.K * n + nov) * sizeof(int))) {
-    for (DevBuf* b : {&h->Xhi, &h->Xlo, &h->gY, &h->gM}) release(*b);  // leave the solves all the room they had
-    return 1;
+  auto room = [&] {
+    return try_ensure(h->Xhi, v.K * b_mp) && try_ensure(h->gY, std::max(v.K * b_sq, b_rp)) &&
+           try_ensure(h->Xlo, std::max(v.K * b_mr, grp * b_rr)) &&
+           try_ensure(h->gM, ((size_t)v.K * n + nov) * sizeof(int));
+  };
+  auto release_all = [&] {
+    RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+    for (DevBuf* b : {&h->Xhi, &h->Xlo, &h->gY, &h->gM, &h->mcBuf}) release(*b);
+    return (int)RPA_OK;
+  };
+  if (!room()) {
+    // the operands of Pi and the planes of its factorization are done with and may be much larger
+    if (int rs = release_all()) return rs;
+    if (!room()) {
+      if (int rs = release_all()) return rs;  // leave the solves all the room they had
+      return 1;
+    }
   }
   double* L = static_cast<double*>(h->Pi.p);
   double* V = static_cast<double*>(h->gY.p);

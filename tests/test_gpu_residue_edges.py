@@ -152,3 +152,56 @@ def test_every_call_reports_an_expired_device_wait(pkg, monkeypatch):
             with pytest.raises(pkg.RPAError) as err:
                 call(h)
             assert err.value.status == pkg.RPA_ERR_TIMEOUT, name
+
+
+def _caps(pkg, call, monkeypatch, steps=24):
+    """The call at caps from the least it runs with up to all it asks for: results, none of them refused."""
+    def run(limit):
+        with pkg.Handle(0) as h:
+            h.set_autotune(False)
+            h.set_workspace_limit(limit)
+            try:
+                out = call(h)
+            except pkg.RPAError as e:
+                assert e.status == pkg.RPA_ERR_OOM
+                return None, h.workspace_bytes()[0]
+            return out, h.workspace_bytes()[0]
+    free, full = run(0)
+    monkeypatch.setenv("RPA_B200_GEMM64_RESIDUES", "0")
+    lo, hi = 0, full
+    while hi - lo > max(full // 512, 4096):  # the least cap, products on DMMA
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if run(mid)[0] is not None else (mid, hi)
+    monkeypatch.setenv("RPA_B200_GEMM64_RESIDUES", "1")
+    out = []
+    for c in np.linspace(hi, full, steps):
+        r, used = run(int(c))
+        assert r is not None, "refused at a cap of %d bytes, %d suffice" % (c, hi)
+        assert used <= c
+        out.append(r)
+    return free, out
+
+
+@pytest.mark.parametrize("what", ["ec", "grad", "t2", "batch"])
+def test_optional_planes_never_cost_a_call_its_room(pkg, monkeypatch, what):
+    # workspace caps at which some of the residue planes fit: what the call needs afterwards must still find
+    # its room, whatever the planes took first.  The forms differ by their rounding only (tolerances as in
+    # the tests of each form).
+    monkeypatch.setenv("RPA_B200_GEMM64_RESIDUES", "1")
+    nq, no, nv = (1540, 2, 70) if what == "batch" else (260, 4, 70)
+    s = O.make_system(nq, no, nv, 9, decay=nq / 8.0, lam0=0.8)
+    x, w = O.casimir_polder(3, 0.8)
+    guess = np.random.default_rng(4).standard_normal((no * nv, 90))
+    if what == "ec":
+        call = lambda h: np.array([h.ec_rpa(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")[0]])
+    elif what == "grad":
+        call = lambda h: h.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")[1]
+    elif what == "t2":
+        call = lambda h: h.dring_t2(s.R, s.eps_o, s.eps_v, x, w, guess=guess, cutoff_thresh=1e-6)["A"]
+    else:
+        call = lambda h: h.ec_batched([(s.R, s.eps_o, s.eps_v, x, w)] * 2, prec="fp64")[0]
+    free, out = _caps(pkg, call, monkeypatch, steps=10 if what == "batch" else 24)
+    tol = 1e-12 if what != "t2" else 1e-9  # T2: eigenvalues of a Rayleigh-Ritz step, both forms in FP64
+    for r in out:
+        assert r.shape == free.shape
+        assert np.max(np.abs(r - free)) < tol * np.max(np.abs(free))
