@@ -560,7 +560,7 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
   if (h->gemm64_bytes) budget = h->gemm64_bytes;
   const bool plain = g.batch == 1 && g.splitk <= 1 && !g.rowscale && (g.a_m == 1 || g.a_k == 1) && (g.b_n == 1 || g.b_k == 1);
   const bool pays = h->gemm64_form < 0 ? mod_pays(g.M, g.N, g.K) : h->gemm64_form != 0;
-  if (plain && pays && g.M > 0 && g.N > 0 && g.K > 0 && g.K <= INT32_MAX) {
+  if (plain && pays && g.M > 0 && g.N > 0 && g.K > 0 && g.K <= rpa::kModMaxK && rpa::mod_units_fit(g.M, g.N, 1, false)) {
     const size_t NM = rpa::kModCount;
     const int64_t pitch = rpa::mod_pitch(g.K), ldo = ((int64_t)g.M + 255) / 256 * 256;
     // C is formed in blocks of columns whose planes and residues fit the budget
@@ -611,7 +611,7 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
 int build_pi_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t ldR, double alpha) {
   const int NQ = v.NQ;
   const int64_t nov = v.nov;
-  if (NQ < kModMinNQ || nov < kModMinK) return 1;
+  if (NQ < kModMinNQ || nov < kModMinK || NQ > rpa::kModMaxOrder || nov > rpa::kModMaxK) return 1;
   const int64_t pitch = rpa::mod_pitch(nov), ldo = (NQ + 255) / 256 * 256;
   const size_t perA = (size_t)rpa::kModCount * NQ * pitch, perC = (size_t)rpa::kModCount * NQ * ldo;
   // a few GiB of planes per group keep the tensor cores busy and leave the memory to the other buffers
@@ -3828,7 +3828,9 @@ static int grad_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, in
                     int64_t lddr, double* dD) {
   const int n = v.NQ;
   const int64_t nov = v.nov;
-  if (n < kModMinNQ || nov < kModMinK) return 1;
+  if (n < kModMinNQ || nov < kModMinK || n > rpa::kModMaxOrder ||
+      !rpa::mod_units_fit(nov, n, std::min(v.K, 16), false))
+    return 1;
   const size_t NM = rpa::kModCount;
   const int64_t pitch = rpa::mod_pitch(n), ldo = (n + 255) / 256 * 256;
   const size_t b_sq = (size_t)n * n * 8;                        // one matrix

@@ -79,6 +79,15 @@ __device__ __forceinline__ void mod_crt4(const uint8_t* src, int64_t plane, cons
   }
 }
 
+// Limits of the residue form, for the callers to keep to (beyond them the FP64 pipe takes over): summed
+// lengths and orders that the conversions and the recombination put in a grid's second dimension, and tiles
+// counted in 32 bits.
+constexpr int64_t kModMaxK = (int64_t)65535 * 128;
+constexpr int kModMaxOrder = 65535;
+inline bool mod_units_fit(int64_t rowsA, int64_t rowsB, int64_t nz, bool tri) {
+  const double ti = (double)((rowsB + 255) / 256), tj = (double)((rowsA + 255) / 256);
+  return (tri ? ti * (ti + 1.0) / 2.0 : ti * tj) * kModCount * (double)nz < 2147483647.0;
+}
 inline int64_t mod_pitch(int64_t K) { return (K + 127) / 128 * 128; }
 
 // One launch: residues of C(i, j) = sum_k a(j, k) b(i, k) for nz batches, j < rowsA (lanes),

@@ -205,3 +205,25 @@ def test_optional_planes_never_cost_a_call_its_room(pkg, monkeypatch, what):
     for r in out:
         assert r.shape == free.shape
         assert np.max(np.abs(r - free)) < tol * np.max(np.abs(free))
+
+
+def test_more_pairs_than_a_grid_dimension_holds(handle):
+    # 128-wide chunks of ai beyond 65535: the FP64 pipe forms Pi (8.6 GB of vectors).  Sums of 8.4e6 products
+    # of either sign, each rounded at 2^-53 of the partial sum, on both sides: 1e-11 of the norms is
+    # 1e5 roundings, far above the sqrt(8.4e6) = 3e3 that independent ones leave.
+    import torch
+    no, nv, nq = 2049, 4096, 128
+    assert no * nv > 65535 * 128
+    g = torch.Generator(device="cuda").manual_seed(1)
+    Rt = torch.randn((no * nv, nq), dtype=torch.float64, device="cuda", generator=g) * 1e-2
+    eo, ev = np.sort(np.linspace(-2.0, -0.5, no)), np.sort(np.linspace(0.1, 3.0, nv))
+    got = handle.pi_u(Rt.T, eo, ev, np.array([0.7]), prec="fp64")[0]
+    d = torch.from_numpy((ev[None, :] - eo[:, None]).ravel()).cuda()
+    c = 4.0 * d / (d * d + 0.49)
+    ref = torch.zeros((nq, nq), dtype=torch.float64, device="cuda")
+    for a in range(0, no * nv, 1 << 20):
+        blk = Rt[a:a + (1 << 20)]
+        ref += blk.T @ (blk * c[a:a + (1 << 20), None])
+    n = torch.sqrt(torch.diagonal(ref))
+    ref, n = ref.cpu().numpy(), n.cpu().numpy()
+    assert np.max(np.abs(got - ref) / (n[:, None] * n[None, :])) < 1e-11
