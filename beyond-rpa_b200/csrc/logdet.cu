@@ -91,8 +91,13 @@ __device__ __forceinline__ void factor_panel(double* S, double* inv, int p, bool
     double d = __shfl_sync(0xffffffffu, v, row & 31), rd, ri;
     const double xp = low ? x0[j] : x1[j];
     pivot_inverses(d, rd, ri, bad);
-    // the next pivot, in its lane: a - x^2 / d
-    if (j + 1 < kPC) v = fma(-(xp * xp), rd, low ? x0[j + 1] : x1[j + 1]);
+    // the next pivot, in its lane: a - x^2 / d; where x^2 would leave the exponent range, a - (x / sqrt(d))^2
+    if (j + 1 < kPC) {
+      const double xx = xp * xp, a = low ? x0[j + 1] : x1[j + 1];
+      const bool far = lane == ((row + 1) & 31) && xp != 0.0 && !(xx > 1e-290 && xx < 1e290);
+      const double l = xp * ri;
+      v = __any_sync(0xffffffffu, far) ? fma(-l, l, a) : fma(-xx, rd, a);
+    }
     const double l0 = lane > row ? x0[j] * ri : 0.0, l1 = lane + 32 > row ? x1[j] * ri : 0.0;
     const double lp = low ? l0 : l1;
     col[j * kLP] = lane == row ? d * ri : l0;

@@ -227,3 +227,28 @@ def test_more_pairs_than_a_grid_dimension_holds(handle):
     n = torch.sqrt(torch.diagonal(ref))
     ref, n = ref.cpu().numpy(), n.cpu().numpy()
     assert np.max(np.abs(got - ref) / (n[:, None] * n[None, :])) < 1e-11
+
+
+@pytest.mark.parametrize("scale", [1e140, 1e180, 1e280])
+def test_log_det_of_very_large_pi(handle, scale):
+    # squares of the off-diagonal entries leave the exponent range, the factorization does not: ln det is lost in
+    # E(u) = ln det - Tr, which is -Tr to one rounding
+    n = 130
+    rng = np.random.default_rng(7)
+    X = rng.standard_normal((2, n, n + 10)) / n
+    pi = (X @ X.transpose(0, 2, 1)) * scale
+    _, eu = handle.ec_from_pi(pi, np.ones(2))
+    tr = np.trace(pi, axis1=1, axis2=2)
+    assert np.all(np.abs(eu + tr) <= 2.0 ** -50 * tr)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-40, 1e-50, 1e30])
+def test_random_basis_does_not_depend_on_the_size_of_pi(handle, scale):
+    # CholeskyQR of Pi G: entries of its Gram matrix from 1e-200 to 1e120
+    s = O.make_system(90, 4, 40, 3, decay=30.0, lam0=0.8)
+    guess = np.random.default_rng(8).standard_normal((90, 90))
+    ref, _, tr0 = handle.piu_basis(s.R, s.eps_o, s.eps_v, 0.1, target_error=0.0, basis="random", guess=guess)
+    two = np.exp2(np.rint(np.log2(scale)))  # exact
+    G, _, tr = handle.piu_basis(s.R * two, s.eps_o, s.eps_v, 0.1, target_error=0.0, basis="random", guess=guess)
+    assert abs(tr - tr0 * two * two) <= 1e-14 * tr
+    assert np.max(np.abs(np.abs(np.sum(G * ref, axis=0)) - 1.0)) < 1e-8
