@@ -10,6 +10,7 @@
 // A non-positive pivot is reported as an error, never as a NaN energy.
 #include <algorithm>
 
+#include <atomic>
 #include <cstdlib>
 
 #include "modgemm.cuh"
@@ -324,19 +325,22 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_varlen_kernel(const MatDesc
   trsm_panel_body(md.A, md.ld, md.n, j0, blockIdx.x, md.Ldiag);
 }
 
-// Shared-memory opt-in of the panel kernels (> 48 KB), once per process.
+// Shared-memory opt-in of the panel kernels (> 48 KB), once per device of the process.
 cudaError_t panel_smem_optin() {
-  static const cudaError_t e = [] {
-    cudaError_t r = cudaFuncSetAttribute(trsm_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem);
-    if (r == cudaSuccess)
-      r = cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem);
-    if (r == cudaSuccess)
-      r = cudaFuncSetAttribute(potrf_varlen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem);
-    if (r == cudaSuccess)
-      r = cudaFuncSetAttribute(trsm_varlen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem);
-    return r;
-  }();
-  return e;
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  cudaError_t r = cudaGetDevice(&dev);
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (r != cudaSuccess || (done.load() & bit)) return r;
+  r = cudaFuncSetAttribute(trsm_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem);
+  if (r == cudaSuccess)
+    r = cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem);
+  if (r == cudaSuccess)
+    r = cudaFuncSetAttribute(potrf_varlen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem);
+  if (r == cudaSuccess)
+    r = cudaFuncSetAttribute(trsm_varlen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem);
+  if (r == cudaSuccess) done.fetch_or(bit);
+  return r;
 }
 
 // Deterministic block reduction of double-double values (blockDim = 256).

@@ -1119,9 +1119,11 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
   SY_CHECK(cudaGetDevice(&dev));
   SY_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const size_t vbytes = (size_t)n * 8;
-  bool coop = nmat == 1 && n > kSmallN && vbytes <= 200 * 1024;
+  constexpr size_t kPanelSmem = 200 * 1024;
+  bool coop = nmat == 1 && n > kSmallN && vbytes <= kPanelSmem;
   if (coop) {
-    SY_CHECK(cudaFuncSetAttribute(panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vbytes));
+    // the attribute is the function's, for all threads: always its largest value
+    SY_CHECK(cudaFuncSetAttribute(panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem));
     SY_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, panel_kernel, kPT, vbytes));
     coop = fit > 0;
   }

@@ -252,3 +252,28 @@ def test_random_basis_does_not_depend_on_the_size_of_pi(handle, scale):
     G, _, tr = handle.piu_basis(s.R * two, s.eps_o, s.eps_v, 0.1, target_error=0.0, basis="random", guess=guess)
     assert abs(tr - tr0 * two * two) <= 1e-14 * tr
     assert np.max(np.abs(np.abs(np.sum(G * ref, axis=0)) - 1.0)) < 1e-8
+
+
+def test_eigensolvers_of_several_threads(pkg):
+    # handles of their own, orders with other shared-memory sizes: the limit of a kernel is the process's
+    import threading
+    rng = np.random.default_rng(11)
+    mats = [(lambda a: a + a.T)(rng.standard_normal((n, n))) for n in (170, 700, 301)]
+    ref = [np.linalg.eigvalsh(a) for a in mats]
+    failed = []
+
+    def work(a, r):
+        try:
+            with pkg.Handle(0) as h:
+                for _ in range(25):
+                    w, _ = h.syevd(a)
+                    assert np.max(np.abs(w - r)) < 64 * len(r) * 2.0 ** -53 * np.max(np.abs(r))
+        except Exception as e:  # noqa: BLE001
+            failed.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=t) for t in zip(mats, ref)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
