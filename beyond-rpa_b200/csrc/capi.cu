@@ -144,7 +144,9 @@ struct rpa_b200_handle {
   // pinned host memory: orbital energies on their way to the device, and small results on theirs back
   uint8_t* pin = nullptr;
   int64_t launches = 0;
-  int gemm64_form = -1;     // FP64 products: 0 DMMA, 1 residues, -1 the faster (RPA_B200_GEMM64_RESIDUES)
+  // FP64 products, Pi(u) and the gradient (and the log-det's updates from their usual orders on): 0 DMMA,
+  // 1 residues, -1 the faster (RPA_B200_RESIDUES)
+  int residues = -1;
   size_t gemm64_bytes = 0;  // planes and residues of a block of columns (RPA_B200_GEMM64_BYTES; 0: the call's)
   int selftest_error = 0;  // device error word that every check sees (RPA_B200_SELFTEST_DEVICE_ERROR; tests)
   int seg_chunks = 16;  // 512-column accumulation segments of the tensor-core SYRK
@@ -520,6 +522,9 @@ bool try_ensure(DevBuf& b, size_t bytes) {
   return false;
 }
 
+// The form of an FP64 product: what the rule for its sizes says, unless the handle is told.
+bool by_residues(const rpa_b200_handle* h, bool rule) { return h->residues < 0 ? rule : h->residues != 0; }
+
 // Residues of one product, from operand planes already on the device (pa: rowsA rows, pb: rowsB rows of K).
 int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t planesA, int rowsA, int8_t* pb,
                 int64_t planesB, int rowsB, int64_t K, int nz, bool tri, uint8_t* out, int64_t ldo) {
@@ -559,8 +564,7 @@ bool mod_pays(int64_t M, int64_t N, int64_t K) {
 int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30) {
   if (h->gemm64_bytes) budget = h->gemm64_bytes;
   const bool plain = g.batch == 1 && g.splitk <= 1 && !g.rowscale && (g.a_m == 1 || g.a_k == 1) && (g.b_n == 1 || g.b_k == 1);
-  const bool pays = h->gemm64_form < 0 ? mod_pays(g.M, g.N, g.K) : h->gemm64_form != 0;
-  if (plain && pays && g.M > 0 && g.N > 0 && g.K > 0 && g.K <= rpa::kModMaxK && rpa::mod_units_fit(g.M, g.N, 1, false)) {
+  if (plain && by_residues(h, mod_pays(g.M, g.N, g.K)) && g.M > 0 && g.N > 0 && g.K > 0 && g.K <= rpa::kModMaxK && rpa::mod_units_fit(g.M, g.N, 1, false)) {
     const size_t NM = rpa::kModCount;
     const int64_t pitch = rpa::mod_pitch(g.K), ldo = ((int64_t)g.M + 255) / 256 * 256;
     // C is formed in blocks of columns whose planes and residues fit the budget
@@ -611,7 +615,7 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
 int build_pi_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t ldR, double alpha) {
   const int NQ = v.NQ;
   const int64_t nov = v.nov;
-  if (NQ < kModMinNQ || nov < kModMinK || NQ > rpa::kModMaxOrder || nov > rpa::kModMaxK) return 1;
+  if (!by_residues(h, NQ >= kModMinNQ && nov >= kModMinK) || NQ > rpa::kModMaxOrder || nov > rpa::kModMaxK) return 1;
   const int64_t pitch = rpa::mod_pitch(nov), ldo = (NQ + 255) / 256 * 256;
   const size_t perA = (size_t)rpa::kModCount * NQ * pitch, perC = (size_t)rpa::kModCount * NQ * ldo;
   // a few GiB of planes per group keep the tensor cores busy and leave the memory to the other buffers
@@ -861,7 +865,7 @@ rpa::LogdetPlan plan_for(const rpa_b200_handle* h, int n) {
 // those on the device): {nullptr} for small orders or without memory (the updates stay on DMMA).
 int mod_chol_for(rpa_b200_handle* h, double* A, int64_t ld, int64_t stride, int n, int nmat, rpa::ModChol* out) {
   out->mats = nullptr;
-  if (n < kModCholMin || h->ozaki_slices) return RPA_OK;
+  if (n < kModCholMin || h->ozaki_slices || h->residues == 0) return RPA_OK;
   size_t pb, rb;
   const size_t per = rpa::mod_chol_bytes(n, 256, &pb, &rb);
   if (!try_ensure(h->mcBuf, per * nmat) || !try_ensure(h->mcDesc, sizeof(rpa::ModMat) * nmat)) {
@@ -1422,7 +1426,7 @@ int rpa_b200_create(rpa_b200_handle** handle, int64_t device, int64_t flags) try
   for (auto& e : h->ev) cudaEventCreate(&e);
   for (auto& e : h->done.ev) cudaEventCreate(&e);
   for (auto& e : h->fork_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-  if (const char* gf = std::getenv("RPA_B200_GEMM64_RESIDUES")) h->gemm64_form = std::atoi(gf) != 0;
+  if (const char* rs = std::getenv("RPA_B200_RESIDUES")) h->residues = std::atoi(rs) != 0;
   if (const char* gb = std::getenv("RPA_B200_GEMM64_BYTES")) h->gemm64_bytes = (size_t)std::max(0ll, std::atoll(gb));
   if (const char* de = std::getenv("RPA_B200_SELFTEST_DEVICE_ERROR")) h->selftest_error = std::atoi(de);
   if (const char* la = std::getenv("RPA_B200_LOOKAHEAD")) h->lookahead = std::atoi(la) != 0;
@@ -3305,7 +3309,7 @@ static int ec_batched_groups(rpa_b200_handle* h, int64_t ninst, const rpa_instan
     per[i].pib = (size_t)v[i].K * v[i].NQ * v[i].NQ * 8;
     per[i].smallb = (size_t)v[i].K * v[i].NQ * 8 * (2 + per[i].plan.nsplit) + 64 * (size_t)v[i].K;
     size_t pb, rb;
-    per[i].modb = v[i].NQ >= kModCholMinBatch && !h->ozaki_slices ? rpa::mod_chol_bytes(v[i].NQ, 256, &pb, &rb) : 0;
+    per[i].modb = v[i].NQ >= kModCholMinBatch && !h->ozaki_slices && h->residues != 0 ? rpa::mod_chol_bytes(v[i].NQ, 256, &pb, &rb) : 0;
   }
   if (prec == RPA_PREC_FP64) {  // the bf16 operands are not used: give their memory to Pi
     RPA_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -3828,7 +3832,7 @@ static int grad_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, in
                     int64_t lddr, double* dD) {
   const int n = v.NQ;
   const int64_t nov = v.nov;
-  if (n < kModMinNQ || nov < kModMinK || n > rpa::kModMaxOrder ||
+  if (!by_residues(h, n >= kModMinNQ && nov >= kModMinK) || n > rpa::kModMaxOrder ||
       !rpa::mod_units_fit(nov, n, std::min(v.K, 16), false))
     return 1;
   const size_t NM = rpa::kModCount;

@@ -167,12 +167,12 @@ def _caps(pkg, call, monkeypatch, steps=24):
                 return None, h.workspace_bytes()[0]
             return out, h.workspace_bytes()[0]
     free, full = run(0)
-    monkeypatch.setenv("RPA_B200_GEMM64_RESIDUES", "0")
+    monkeypatch.setenv("RPA_B200_RESIDUES", "0")
     lo, hi = 0, full
-    while hi - lo > max(full // 512, 4096):  # the least cap, products on DMMA
+    while hi - lo > max(full // 512, 4096):  # the least cap, everything on DMMA
         mid = (lo + hi) // 2
         lo, hi = (lo, mid) if run(mid)[0] is not None else (mid, hi)
-    monkeypatch.setenv("RPA_B200_GEMM64_RESIDUES", "1")
+    monkeypatch.setenv("RPA_B200_RESIDUES", "1")
     out = []
     for c in np.linspace(hi, full, steps):
         r, used = run(int(c))
@@ -187,7 +187,7 @@ def test_optional_planes_never_cost_a_call_its_room(pkg, monkeypatch, what):
     # workspace caps at which some of the residue planes fit: what the call needs afterwards must still find
     # its room, whatever the planes took first.  The forms differ by their rounding only (tolerances as in
     # the tests of each form).
-    monkeypatch.setenv("RPA_B200_GEMM64_RESIDUES", "1")
+    monkeypatch.setenv("RPA_B200_RESIDUES", "1")
     nq, no, nv = (1540, 2, 70) if what == "batch" else (260, 4, 70)
     s = O.make_system(nq, no, nv, 9, decay=nq / 8.0, lam0=0.8)
     x, w = O.casimir_polder(3, 0.8)
@@ -277,3 +277,103 @@ def test_eigensolvers_of_several_threads(pkg):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.fixture
+def forms(pkg, monkeypatch):
+    """Two handles whose FP64 products run by residues (in blocks of 128 columns) and on DMMA, at any size."""
+    hs = []
+    for form in ("1", "0"):
+        monkeypatch.setenv("RPA_B200_RESIDUES", form)
+        monkeypatch.setenv("RPA_B200_GEMM64_BYTES", str(15 * (384 + 512) * 128))
+        hs.append(pkg.Handle(0))
+    yield hs
+    for h in hs:
+        h.close()
+
+
+def _long_error(got, a, b):
+    """Largest error of got = a^T b against 80 bits, relative to the norms of the two rows."""
+    al, bl = a.astype(np.longdouble), b.astype(np.longdouble)
+    n = np.sqrt(np.sum(al * al, axis=0))[:, None] * np.sqrt(np.sum(bl * bl, axis=0))[None, :]
+    n[n == 0] = 1
+    return float(np.max(np.abs(got - al.T @ bl) / n))
+
+
+@pytest.mark.parametrize("nq, nvec, nov", [(1, 1, 1), (31, 7, 130), (128, 128, 256), (129, 127, 257), (300, 250, 391),
+                                           (384, 384, 140)])
+def test_projection_by_residues(forms, nq, nvec, nov):
+    # R' = G^T R, both operands contiguous along the summed index; blocks of 128 columns of R'.  Operands are rounded
+    # at 2^-58 of their norms and the result once at 2^-53: 4 2^-53 of the norms.  Columns of zeros, of
+    # very different size, and one whose squares leave the exponent range.
+    rng = np.random.default_rng(nq + nov)
+    G, R = rng.standard_normal((nq, nvec)), np.asfortranarray(rng.standard_normal((nq, nov)))
+    R *= np.exp(rng.uniform(-60, 60, nov))[None, :]
+    R[:, ::17] = 0.0
+    R[:, nov - 1] *= 1e170
+    got = forms[0].project_basis(G, R)
+    assert np.all(got[:, ::17][:, :-1] == 0.0)
+    assert _long_error(got, G, R) < 4 * 2.0 ** -53
+    assert _long_error(forms[1].project_basis(G, R), G, R) < max(nq, 4) * 2.0 ** -53
+
+
+@pytest.mark.parametrize("ng, nq, no, nv", [(1, 1, 1, 1), (130, 33, 3, 50), (257, 200, 5, 61), (384, 129, 2, 64)])
+def test_thc_vectors_by_residues(forms, ng, nq, no, nv):
+    Z, Xa, Xi, _, _ = O.make_thc_factors(ng, nq, no, nv, 5)
+    YX = (Xa.astype(np.longdouble)[:, None, :] * Xi.astype(np.longdouble)[:, :, None]).reshape(ng, no * nv)
+    # the Khatri-Rao entries themselves are rounded at 2^-53
+    assert _long_error(forms[0].thc_r(Z, Xa, Xi), Z, YX) < 6 * 2.0 ** -53
+    assert _long_error(forms[1].thc_r(Z, Xa, Xi), Z, YX) < max(ng, 6) * 2.0 ** -53
+
+
+def test_nan_in_an_operand_is_reported(forms, pkg):
+    rng = np.random.default_rng(3)
+    G, R = rng.standard_normal((140, 130)), np.asfortranarray(rng.standard_normal((140, 150)))
+    for bad in (np.nan, np.inf):
+        R[7, 149] = bad
+        for h in forms:
+            with pytest.raises(pkg.RPAError) as e:
+                h.project_basis(G, R)
+            assert e.value.status == pkg.RPA_ERR_NONFINITE
+
+
+@pytest.mark.parametrize("nq, no, nv, nt", [(60, 3, 21, 30), (137, 4, 70, 129), (200, 5, 52, 140)])
+def test_lyapunov_products_by_residues(forms, nq, no, nv, nt):
+    # every operand order of the products, alpha = -1 with beta = 1, and a scale of the summed index (the orbital
+    # energy differences): both forms solve the same equation to 1e-13 of its right-hand side
+    s = O.make_system(nq, no, nv, nt, decay=nq / 6.0, lam0=0.8)
+    U, _ = np.linalg.qr(np.random.default_rng(nt).standard_normal((no * nv, nt)))
+    A = -np.exp(-np.linspace(1.5, 6.0, nt))
+    out = [h.exchange_mbpt3(s.R, s.eps_o, s.eps_v, U, A, return_x=True) for h in forms]
+    (e0, x0), (e1, x1) = out
+    assert abs(e0 - e1) < 1e-11 * abs(e1)
+    assert np.max(np.abs(x0 - x1)) < 1e-11 * np.max(np.abs(x1))
+
+
+def test_amplitudes_and_basis_by_residues(forms):
+    # T2 eigenvalues (rows contiguous times columns contiguous, both summed indices) and the random basis (an
+    # operand times its own transpose): 1e-10 as in the tests of each against the oracle
+    s = O.make_system(150, 4, 33, 2, decay=25.0, lam0=0.8)
+    x, w = O.casimir_polder(5, 0.8)
+    guess = np.random.default_rng(5).standard_normal((132, 120))
+    t0, t1 = [h.dring_t2(s.R, s.eps_o, s.eps_v, x, w, guess=guess) for h in forms]
+    assert t0["NT"] == t1["NT"]
+    assert np.max(np.abs(t0["A"] - t1["A"])) < 1e-10 * np.max(np.abs(t1["A"]))
+    assert np.max(np.abs(t0["EigRPA"] - t1["EigRPA"])) < 1e-10 * np.max(np.abs(t1["EigRPA"]))
+    g = np.random.default_rng(6).standard_normal((90, 90))
+    s = O.make_system(90, 4, 40, 3, decay=30.0, lam0=0.8)
+    b0, b1 = [h.piu_basis(s.R, s.eps_o, s.eps_v, 0.1, target_error=0.0, basis="random", guess=g)[0] for h in forms]
+    assert np.max(np.abs(np.abs(np.sum(b0 * b1, axis=0)) - 1.0)) < 1e-9
+
+
+@pytest.mark.parametrize("nq, no, nv, k", [(1, 1, 1, 1), (5, 2, 9, 3), (127, 3, 40, 2), (100, 2, 30, 17)])
+def test_small_pi_and_gradient_by_residues(forms, nq, no, nv, k):
+    # below the sizes from which the residue forms are taken, both forms agree with the oracle
+    s = O.make_system(nq, no, nv, nq + k, decay=nq / 4.0 + 1.0, lam0=0.8)
+    x, w = O.casimir_polder(k, 0.8)
+    ref = O.pi_matrices(s.R, s.eps_o, s.eps_v, x)
+    gref = O.ec_grad(s.R, s.eps_o, s.eps_v, x, w)
+    for h in forms:
+        assert np.max(np.abs(h.pi_u(s.R, s.eps_o, s.eps_v, x, prec="fp64") - ref)) < 1e-13 * np.max(np.abs(ref))
+        for a, b in zip(h.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")[1:], gref):
+            assert np.max(np.abs(a - b)) < 1e-13 * np.max(np.abs(b))
