@@ -118,6 +118,7 @@ def load_library(path: str | os.PathLike | None = None):
     lib.rpa_b200_set_workspace_limit.argtypes = [_vp, _i64]
     lib.rpa_b200_workspace_bytes.argtypes = [_vp, _vp, _vp]
     lib.rpa_b200_selftest_wait_timeout.argtypes = [_vp, _dbl]
+    lib.rpa_b200_selftest_pivots.argtypes = [_vp, _i64, _vp, _vp, _vp]
     if path is None:
         _lib = lib
     return lib
@@ -331,6 +332,14 @@ class Handle:
     def selftest_wait_timeout(self, limit_ms=20.0):
         """Run the bounded-wait self-test; returns its status (RPA_ERR_TIMEOUT when detection works)."""
         return int(self.lib.rpa_b200_selftest_wait_timeout(self._h, float(limit_ms)))
+
+    def selftest_pivots(self, d):
+        """1 / d and 1 / sqrt(d) as the log-det's factorization forms them (rpa_b200_selftest_pivots)."""
+        d = np.ascontiguousarray(d, dtype=np.float64)
+        inv, inv_sqrt = np.empty_like(d), np.empty_like(d)
+        self._check(self.lib.rpa_b200_selftest_pivots(self._h, d.size, d.ctypes.data, inv.ctypes.data,
+                                                      inv_sqrt.ctypes.data))
+        return inv, inv_sqrt
 
     # ------------------------------------------------------------------ Pi(u)
     def pi_u(self, R, eps_o, eps_v, freqs, alpha=4.0, prec="split", out=None):

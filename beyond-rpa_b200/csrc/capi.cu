@@ -1614,6 +1614,24 @@ int rpa_b200_selftest_wait_timeout(rpa_b200_handle* h, double LimitMs) try {
   return exception_status(h);
 }
 
+int rpa_b200_selftest_pivots(rpa_b200_handle* h, int64_t N, const double* D, double* Inv, double* InvSqrt) try {
+  int s = begin_call(h);
+  if (s != RPA_OK) return s;
+  if ((s = check_arrays(h, {D, Inv, InvSqrt}))) return s;
+  if (N < 1 || N > INT32_MAX || !D || !Inv || !InvSqrt)
+    return fail(h, RPA_ERR_INVALID_ARG, "invalid argument to rpa_b200_selftest_pivots");
+  RPA_CUDA(h, ensure(h->tSmall, (size_t)N * 24));
+  double* d = static_cast<double*>(h->tSmall.p);
+  RPA_CUDA(h, cudaMemcpyAsync(d, D, (size_t)N * 8, cudaMemcpyDefault, h->stream));
+  RPA_CUDA(h, rpa::launch_pivots_selftest(d, N, d + N, d + 2 * N, h->stream));
+  RPA_CUDA(h, cudaMemcpyAsync(Inv, d + N, (size_t)N * 8, cudaMemcpyDefault, h->stream));
+  RPA_CUDA(h, cudaMemcpyAsync(InvSqrt, d + 2 * N, (size_t)N * 8, cudaMemcpyDefault, h->stream));
+  RPA_CUDA(h, cudaStreamSynchronize(h->stream));
+  return RPA_OK;
+} catch (...) {
+  return exception_status(h);
+}
+
 int rpa_b200_set_autotune(rpa_b200_handle* h, int64_t on) try {
   if (!h) return RPA_ERR_INVALID_ARG;
   h->autotune = on != 0;

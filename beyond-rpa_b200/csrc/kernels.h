@@ -236,6 +236,8 @@ cudaError_t launch_dai(const double* eps_o, const double* eps_v, int64_t no, int
 cudaError_t launch_symmetrize(double* A, int64_t ld, int64_t stride, int n, int nmat, cudaStream_t stream);
 // Failure-detection self-test: one bounded wait on an mbarrier nobody arrives on, limit_ns long;
 // it records kDevTimeoutSelfTest in *err when it expires.
+// inv[i], inv_sqrt[i]: what the diagonal blocks of the Cholesky take for 1 / d[i] and 1 / sqrt(d[i]).
+cudaError_t launch_pivots_selftest(const double* d, int64_t n, double* inv, double* inv_sqrt, cudaStream_t stream);
 cudaError_t launch_wait_timeout_selftest(int* err, unsigned long long limit_ns, cudaStream_t stream);
 // Count non-finite entries of a device array (result accumulated into *count).
 cudaError_t launch_count_nonfinite(const double* x, int64_t n, int* count, cudaStream_t stream);

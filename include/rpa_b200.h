@@ -154,6 +154,13 @@ int rpa_b200_workspace_bytes(const rpa_b200_handle* handle, int64_t* Used, int64
 int rpa_b200_selftest_wait_timeout(rpa_b200_handle* handle, double LimitMs);
 
 /*
+ * Arithmetic self-test.  No reference counterpart.  Inv(i) = 1 / D(i) and
+ * InvSqrt(i) = 1 / sqrt(D(i)) as the log-det's factorization forms them for its
+ * pivots (1 and 1 where D(i) is not positive); arrays of length N.
+ */
+int rpa_b200_selftest_pivots(rpa_b200_handle* handle, int64_t N, const double* D, double* Inv, double* InvSqrt);
+
+/*
  * Pi(u) matrices:  PiU(:,:,u) = alpha * sum_ai R(:,ai) Chi_u(ai) R(:,ai)^T,
  * Chi_u(ai) = D(ai) / (D(ai)^2 + u^2), D(ai) = VirtEnergies(a) - OccEnergies(i).
  * Replaces rpa_THC_PiU / rpa_THC_PiU_BlockAlgo / rpa_THC_ChiRkai

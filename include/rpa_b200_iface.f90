@@ -315,6 +315,14 @@ module rpa_b200_iface
                   type(c_ptr), value :: handle
                   real(c_double), value :: LimitMs          ! returns RPA_ERR_TIMEOUT when detection works
             end function
+            integer(c_int) function rpa_b200_selftest_pivots(handle, N, D, Inv, InvSqrt) &
+                  bind(C, name="rpa_b200_selftest_pivots")
+                  import :: c_int, c_int64_t, c_double, c_ptr
+                  type(c_ptr), value :: handle
+                  integer(c_int64_t), value :: N
+                  real(c_double), dimension(*), intent(in) :: D
+                  real(c_double), dimension(*), intent(out) :: Inv, InvSqrt
+            end function
       end interface
 
 contains

@@ -377,3 +377,23 @@ def test_small_pi_and_gradient_by_residues(forms, nq, no, nv, k):
         assert np.max(np.abs(h.pi_u(s.R, s.eps_o, s.eps_v, x, prec="fp64") - ref)) < 1e-13 * np.max(np.abs(ref))
         for a, b in zip(h.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")[1:], gref):
             assert np.max(np.abs(a - b)) < 1e-13 * np.max(np.abs(b))
+
+
+def test_pivot_inverses(handle):
+    # 1 / d and 1 / sqrt(d) of the diagonal blocks against the correctly rounded ones: a truncated series below
+    # 2^-58.6 and two roundings, so within 2^-52 of the value; both sides of the switch to the library
+    # functions, denormals, and pivots that are not positive
+    rng = np.random.default_rng(13)
+    m = np.concatenate([rng.uniform(1.0, 4.0, 60000), 1.0 + 2.0 ** -52 * np.arange(64), 4.0 - 2.0 ** -51 * np.arange(1, 64)])
+    d = np.ldexp(m, rng.integers(-1020, 1021, m.size))
+    edges = [x * (1.0 + 2.0 ** -52 * i) for x in (1e-290, 1e290) for i in range(-200, 200)]
+    d = np.concatenate([d, m, edges, [1.0, 2.0, 0.5, 2.0 ** -1022, 2.0 ** 1022, 1.7e308]])
+    inv, inv_sqrt = handle.selftest_pivots(d)
+    dl = d.astype(np.longdouble)
+    for got, ref in ((inv, 1 / dl), (inv_sqrt, 1 / np.sqrt(dl))):
+        normal = ref > 2.3e-308  # 1 / d of the largest d is denormal
+        err = np.abs(got - ref) / ref
+        assert np.max(err[normal]) < 2.0 ** -52
+        assert np.max(np.abs(got - ref)[~normal], initial=0.0) <= 2.0 ** -1074
+    inv, inv_sqrt = handle.selftest_pivots(np.array([0.0, -1.0, -np.inf, np.nan]))
+    assert np.all(inv == 1.0) and np.all(inv_sqrt == 1.0)
