@@ -199,9 +199,11 @@ namespace {
 
 const double kPi = 3.14159265358979323846;
 
-// Residue products (modgemm.cu) pay off from here on; below, the DMMA kernels are as fast.
-constexpr int kModMinNQ = 128;
-constexpr int64_t kModMinK = 128;
+// Gradients whose inverses and products run by residues (modgemm.cu) from here on, the smallest measured (order
+// 64, 128 pairs, 1 and 16 frequencies: 1027 -> 252 and 475 -> 292 us per call; order 1024, 512 pairs: 2839 -> 1283,
+// 4082 -> 2611).
+constexpr int kModGradMinNQ = 64;
+constexpr int64_t kModGradMinK = 128;
 // Orders from which the log-det's trailing updates run by residues: one system (16 matrices) 1100 0.75
 // -> 0.72 ms, 1387 1.10 -> 1.00, 2048 2.47 -> 2.11, 4096 13.4 -> 8.8; batches, whose many small
 // matrices fill the FP64 pipe (60 matrices): 1280 2.21 -> 2.24, 1408 2.71 -> 2.74, 1792 4.89 -> 4.57,
@@ -553,12 +555,28 @@ int mod_product(rpa_b200_handle* h, rpa::ModGemmArgs& a, int8_t* pa, int64_t pla
 
 // One FP64 product on the FP64 tensor pipe, or by residues where that is the faster: the pipe's
 // 28 TFLOP/s against 15 int8 products at 2.4 POP/s, the sizes of both operands along K and their conversion
-// (5.5 TB/s read, 3 TB/s of planes), the residues of C written and read, and the extra launches.  1.2: the
-// estimate's margin.
+// (5.5 TB/s read, 3 TB/s of planes), the residues of C written and read, and the extra launches; 1.1: the
+// estimate's margin.  THC vectors, K x M x N, DMMA / residues in us per call: 800^3 149 / 186, 1000^3 179 / 179,
+// 1200^3 246 / 210, 2048^3 695 / 346; 8000 x 500 x 500 559 / 394, 512 x 700 x 6000 248 / 253, 512 x 700 x 12000
+// 419 / 378, 256 x 4000 x 4000 393 / 400, 1024 x 1024 x 4096 398 / 277.
 bool mod_pays(int64_t M, int64_t N, int64_t K) {
-  const double flops = 2.0 * (double)M * (double)N * (double)K;
+  const double m = (double)M, n = (double)N, k = (double)K;
   return M >= 128 && N >= 128 && K >= 128 &&
-         flops * (1.0 / 28e12 - 15.0 / 2.4e15) > 1.2 * (6.5e-12 * (double)(M + N) * (double)K + 1e-11 * (double)M * (double)N + 33e-6);
+         2.0 * m * n * k * (1.0 / 28e12 - 15.0 / 2.4e15) > 1.1 * (6.5e-12 * (m + n) * k + 1.5e-11 * m * n + 33e-6);
+}
+
+// FP64 Pi(u) of K frequencies: the scaled SYRK sums over the pairs in one chain per 64 x 64 tile, 0.075 us a pair
+// while every tile has its SM and 0.33 ns a tile and pair (25 TFLOP/s) when the GPU is full; the residue form has
+// its launches, the tiles' own time and the planes.  Microseconds per call, scaled SYRK / residues, K = 1 and 16:
+// NQ 128, 512 pairs 125 / 124 and 128 / 203; 128, 4096 387 / 151 and 405 / 266; 384, 4096 406 / 167 and 655 / 449;
+// 512, 128 95 / 125 and 129 / 244; 512, 512 125 / 126 and 196 / 256; 512, 4096 404 / 172 and 838 / 511;
+// 64, 4096 381 / 151 and 404 / 256 (nothing smaller measured).
+bool mod_pi_pays(int64_t NQ, int64_t nov, int64_t K) {
+  const double a = (double)nov, k = (double)K, s = (double)((NQ + 63) / 64), t = (double)((NQ + 255) / 256);
+  const double tiles = k * s * (s + 1.0) / 2.0;
+  const double syrk = a * (tiles <= 148.0 ? 0.075 : std::max(0.065 + 2.1e-4 * tiles, 3.3e-4 * tiles));
+  const double mod = 35.0 + k * (3.0 + 0.75 * t * (t + 1.0)) + a * (0.004 + 9e-6 * (double)NQ * k);
+  return NQ >= 64 && syrk > 1.1 * mod;
 }
 
 int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30) {
@@ -615,7 +633,7 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
 int build_pi_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t ldR, double alpha) {
   const int NQ = v.NQ;
   const int64_t nov = v.nov;
-  if (!by_residues(h, NQ >= kModMinNQ && nov >= kModMinK) || NQ > rpa::kModMaxOrder || nov > rpa::kModMaxK) return 1;
+  if (!by_residues(h, mod_pi_pays(NQ, nov, v.K)) || NQ > rpa::kModMaxOrder || nov > rpa::kModMaxK) return 1;
   const int64_t pitch = rpa::mod_pitch(nov), ldo = (NQ + 255) / 256 * 256;
   const size_t perA = (size_t)rpa::kModCount * NQ * pitch, perC = (size_t)rpa::kModCount * NQ * ldo;
   // a few GiB of planes per group keep the tensor cores busy and leave the memory to the other buffers
@@ -3850,7 +3868,7 @@ static int grad_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, in
                     int64_t lddr, double* dD) {
   const int n = v.NQ;
   const int64_t nov = v.nov;
-  if (!by_residues(h, n >= kModMinNQ && nov >= kModMinK) || n > rpa::kModMaxOrder ||
+  if (!by_residues(h, n >= kModGradMinNQ && nov >= kModGradMinK) || n > rpa::kModMaxOrder ||
       !rpa::mod_units_fit(nov, n, std::min(v.K, 16), false))
     return 1;
   const size_t NM = rpa::kModCount;
