@@ -199,15 +199,24 @@ namespace {
 
 const double kPi = 3.14159265358979323846;
 
+// FP64 Pi(u) by residue products (modgemm.cu) from here on.  The line is one of accuracy, not of time: an entry is
+// within 1e-16 of the norms of its rows at any number of pairs, where the FP64 pipe's sum of 385 pairs is off
+// by 2.1e-15 and of 768 by 3.0e-15.  Microseconds per call, scaled SYRK / residues, 1 and 16 frequencies: NQ 128,
+// 128 pairs 96 / 128 and 98 / 196, 512 pairs 125 / 124 and 128 / 203, 4096 387 / 151 and 405 / 266; NQ 512, 128
+// pairs 95 / 125 and 129 / 244, 512 125 / 126 and 196 / 256, 4096 404 / 172 and 838 / 511; so below some
+// 1000 pairs a call takes up to 0.1 ms longer.
+constexpr int kModPiMinNQ = 128;
+constexpr int64_t kModPiMinK = 128;
 // Gradients whose inverses and products run by residues (modgemm.cu) from here on, the smallest measured (order
 // 64, 128 pairs, 1 and 16 frequencies: 1027 -> 252 and 475 -> 292 us per call; order 1024, 512 pairs: 2839 -> 1283,
 // 4082 -> 2611).
 constexpr int kModGradMinNQ = 64;
 constexpr int64_t kModGradMinK = 128;
-// Orders from which the log-det's trailing updates run by residues: one system (16 matrices) 1100 0.75
-// -> 0.72 ms, 1387 1.10 -> 1.00, 2048 2.47 -> 2.11, 4096 13.4 -> 8.8; batches, whose many small
-// matrices fill the FP64 pipe (60 matrices): 1280 2.21 -> 2.24, 1408 2.71 -> 2.74, 1792 4.89 -> 4.57,
-// 2304 9.45 -> 7.89.
+// Orders from which the log-det's trailing updates run by residues.  One system, DMMA / residues in us for 1, 4 and
+// 16 matrices: 1100 590 / 613, 637 / 650, 826 / 829; 1200 640 / 651, 684 / 694, 900 / 893; 1279 728 / 739, 781 / 807,
+// 1095 / 1041; 1290 719 / 733, 781 / 789, 1105 / 1090; 1387 800 / 808, 872 / 880, 1280 / 1207; 1536 817 / 827,
+// 912 / 920, 1357 / 1298; 2048 (16 matrices) 2470 / 2110, 4096 13.4 / 8.8 ms.  Batches, whose many small matrices
+// fill the FP64 pipe (60 matrices, ms): 1280 2.21 / 2.24, 1408 2.71 / 2.74, 1792 4.89 / 4.57, 2304 9.45 / 7.89.
 constexpr int kModCholMin = 1280;
 constexpr int kModCholMinBatch = 1536;
 constexpr size_t kModBudget = (size_t)4 << 30;  // device bytes of one group of residue planes
@@ -565,20 +574,6 @@ bool mod_pays(int64_t M, int64_t N, int64_t K) {
          2.0 * m * n * k * (1.0 / 28e12 - 15.0 / 2.4e15) > 1.1 * (6.5e-12 * (m + n) * k + 1.5e-11 * m * n + 33e-6);
 }
 
-// FP64 Pi(u) of K frequencies: the scaled SYRK sums over the pairs in one chain per 64 x 64 tile, 0.075 us a pair
-// while every tile has its SM and 0.33 ns a tile and pair (25 TFLOP/s) when the GPU is full; the residue form has
-// its launches, the tiles' own time and the planes.  Microseconds per call, scaled SYRK / residues, K = 1 and 16:
-// NQ 128, 512 pairs 125 / 124 and 128 / 203; 128, 4096 387 / 151 and 405 / 266; 384, 4096 406 / 167 and 655 / 449;
-// 512, 128 95 / 125 and 129 / 244; 512, 512 125 / 126 and 196 / 256; 512, 4096 404 / 172 and 838 / 511;
-// 64, 4096 381 / 151 and 404 / 256 (nothing smaller measured).
-bool mod_pi_pays(int64_t NQ, int64_t nov, int64_t K) {
-  const double a = (double)nov, k = (double)K, s = (double)((NQ + 63) / 64), t = (double)((NQ + 255) / 256);
-  const double tiles = k * s * (s + 1.0) / 2.0;
-  const double syrk = a * (tiles <= 148.0 ? 0.075 : std::max(0.065 + 2.1e-4 * tiles, 3.3e-4 * tiles));
-  const double mod = 35.0 + k * (3.0 + 0.75 * t * (t + 1.0)) + a * (0.004 + 9e-6 * (double)NQ * k);
-  return NQ >= 64 && syrk > 1.1 * mod;
-}
-
 int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30) {
   if (h->gemm64_bytes) budget = h->gemm64_bytes;
   const bool plain = g.batch == 1 && g.splitk <= 1 && !g.rowscale && (g.a_m == 1 || g.a_k == 1) && (g.b_n == 1 || g.b_k == 1);
@@ -633,7 +628,7 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
 int build_pi_mod(rpa_b200_handle* h, const Validated& v, const double* Rd, int64_t ldR, double alpha) {
   const int NQ = v.NQ;
   const int64_t nov = v.nov;
-  if (!by_residues(h, mod_pi_pays(NQ, nov, v.K)) || NQ > rpa::kModMaxOrder || nov > rpa::kModMaxK) return 1;
+  if (!by_residues(h, NQ >= kModPiMinNQ && nov >= kModPiMinK) || NQ > rpa::kModMaxOrder || nov > rpa::kModMaxK) return 1;
   const int64_t pitch = rpa::mod_pitch(nov), ldo = (NQ + 255) / 256 * 256;
   const size_t perA = (size_t)rpa::kModCount * NQ * pitch, perC = (size_t)rpa::kModCount * NQ * ldo;
   // a few GiB of planes per group keep the tensor cores busy and leave the memory to the other buffers

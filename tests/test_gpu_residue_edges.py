@@ -5,7 +5,6 @@ import numpy as np
 import pytest
 
 from oracle import rpa_oracle as O
-from tests.test_gpu_modgemm import SHAPES, norms, pi_long
 
 pytestmark = pytest.mark.gpu
 
@@ -398,25 +397,3 @@ def test_pivot_inverses(handle):
         assert np.max(np.abs(got - ref)[~normal], initial=0.0) <= 2.0 ** -1074
     inv, inv_sqrt = handle.selftest_pivots(np.array([0.0, -1.0, -np.inf, np.nan]))
     assert np.all(inv == 1.0) and np.all(inv_sqrt == 1.0)
-
-
-@pytest.mark.parametrize("nq, no, nv, k", SHAPES)
-def test_pi_entries_by_residues(forms, nq, no, nv, k):
-    # the tile and chunk edges of the residue form, which the sizes alone would leave to the FP64 pipe
-    s = O.make_system(nq, no, nv, 7 * nq + k, decay=nq / 8.0, lam0=0.8)
-    x, _ = O.casimir_polder(k, 0.8)
-    keep = list(range(k)) if k <= 3 else [0, k // 2, k - 1]
-    ref = pi_long(s, np.asarray(x)[keep])
-    got = forms[0].pi_u(s.R, s.eps_o, s.eps_v, x, prec="fp64")[keep]
-    assert np.max(np.abs(got - ref) / norms(ref)) < 16 * 2.0 ** -53
-
-
-@pytest.mark.parametrize("nq, no, nv, k, form", [(128, 2, 64, 1, 1), (384, 4, 128, 16, 1), (200, 8, 60, 4, 1),
-                                                 (128, 16, 128, 1, 0), (300, 32, 128, 16, 0), (64, 16, 256, 2, 0)])
-def test_form_of_pi_by_size(forms, handle, nq, no, nv, k, form):
-    # few pairs or many: whichever form is the faster (both are deterministic, and differ in their last bits)
-    s = O.make_system(nq, no, nv, nq, decay=nq / 8.0, lam0=0.8)
-    x, _ = O.casimir_polder(k, 0.8)
-    a, b = [h.pi_u(s.R, s.eps_o, s.eps_v, x, prec="fp64") for h in forms]
-    assert not np.array_equal(a, b)
-    assert np.array_equal(handle.pi_u(s.R, s.eps_o, s.eps_v, x, prec="fp64"), (a, b)[form])
