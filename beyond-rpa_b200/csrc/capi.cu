@@ -574,7 +574,10 @@ bool mod_pays(int64_t M, int64_t N, int64_t K) {
          2.0 * m * n * k * (1.0 / 28e12 - 15.0 / 2.4e15) > 1.1 * (6.5e-12 * (m + n) * k + 1.5e-11 * m * n + 33e-6);
 }
 
-int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30) {
+// b_factors: the two factors of a B that is their Khatri-Rao product (without kscale), whose sizes along K then
+// come from them (537 MB of B at NGrid 4096, 16384 pairs: 0.1 ms).
+int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_t)2 << 30,
+           const rpa::ModOperand* b_factors = nullptr) {
   if (h->gemm64_bytes) budget = h->gemm64_bytes;
   const bool plain = g.batch == 1 && g.splitk <= 1 && !g.rowscale && (g.a_m == 1 || g.a_k == 1) && (g.b_n == 1 || g.b_k == 1);
   if (plain && by_residues(h, mod_pays(g.M, g.N, g.K)) && g.M > 0 && g.N > 0 && g.K > 0 && g.K <= rpa::kModMaxK && rpa::mod_units_fit(g.M, g.N, 1, false)) {
@@ -588,7 +591,7 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
     const size_t kw = same ? 0 : (size_t)g.K;
     if (nb >= std::min<int64_t>(g.N, 128) && try_ensure(h->mA, NM * g.M * (size_t)pitch) &&
         try_ensure(h->mB, NM * nb * (size_t)pitch) && try_ensure(h->mC, NM * nb * (size_t)ldo) &&
-        try_ensure(h->mE, kw * 24 + ((size_t)g.M + nb) * sizeof(int))) {
+        try_ensure(h->mE, kw * 28 + ((size_t)g.M + nb) * sizeof(int))) {
       int8_t *pa = static_cast<int8_t*>(h->mA.p), *pb = static_cast<int8_t*>(h->mB.p);
       double *fa = nullptr, *fb = nullptr;  // factors of column k
       int* ea = static_cast<int*>(h->mE.p);
@@ -596,9 +599,10 @@ int gemm64(rpa_b200_handle* h, const rpa::GemmF64Args& g, size_t budget = (size_
         fa = static_cast<double*>(h->mE.p);
         fb = fa + g.K;
         int* sizes = reinterpret_cast<int*>(fb + g.K);
-        ea = sizes + 2 * g.K;
-        RPA_CUDA(h, rpa::launch_mod_balance(g.A, g.a_m, g.a_k, g.M, g.B, g.b_n, g.b_k, g.N, g.K, g.kscale, sizes, fa, fb,
-                                            h->stream));
+        ea = sizes + 3 * g.K;
+        const rpa::ModOperand a{g.A, g.a_m, g.a_k, g.M}, b{g.B, g.b_n, g.b_k, g.N};
+        RPA_CUDA(h, rpa::launch_mod_balance(a, b_factors ? b_factors[0] : b, b_factors ? b_factors + 1 : nullptr, g.K,
+                                            g.kscale, sizes, fa, fb, h->stream));
       }
       int* eb = ea + g.M;
       if (g.a_k == 1) RPA_CUDA(h, rpa::launch_mod_cols(g.A, g.a_m, 0, (int)g.K, g.M, 1, pa, ea, h->stream, 0.0, fa));
@@ -2566,9 +2570,11 @@ static int form_thc_r(rpa_b200_handle* h, int64_t NGrid, int64_t NQ, int64_t NOc
   double* YX = static_cast<double*>(h->thYX.p);
   for (int64_t i0 = 0; i0 < NOcc; i0 += ib) {
     const int64_t ni = std::min(ib, NOcc - i0);
+    const rpa::ModOperand factors[2] = {{Xad, ldxa, 1, NVirt}, {Xid + ldxi * i0, ldxi, 1, ni}};
     RPA_CUDA(h, rpa::launch_khatri_rao(Xad, ldxa, Xid, ldxi, (int)NGrid, (int)NVirt, (int)i0, (int)ni, YX, h->stream));
-    if (int gs = gemm64(h, gemm_tn((int)NQ, (int)(NVirt * ni), NGrid, Zd, ldz, YX, NGrid,
-                                             Rout + ldR * (i0 * NVirt), ldR))) return gs;
+    if (int gs = gemm64(h, gemm_tn((int)NQ, (int)(NVirt * ni), NGrid, Zd, ldz, YX, NGrid, Rout + ldR * (i0 * NVirt), ldR),
+                        (size_t)2 << 30, factors))
+      return gs;
   }
   return RPA_OK;
 }
@@ -2659,9 +2665,12 @@ int build_pi_thc(rpa_b200_handle* h, const Validated& v, int64_t NGrid, const do
   for (int64_t a0 = 0; a0 < nov; a0 += w) {
     const int64_t wp = std::min(w, nov - a0);
     const bool first = a0 == 0, last = a0 + wp == nov;
+    const int64_t i0 = a0 / v.nv, i1 = (a0 + wp - 1) / v.nv;  // occupied orbitals of the piece
+    const rpa::ModOperand factors[2] = {{Xad, ldxa, 1, v.nv}, {Xid + ldxi * i0, ldxi, 1, i1 - i0 + 1}};
     cudaEvent_t e0 = pool_event(h), e1 = pool_event(h), e2 = pool_event(h);
     RPA_CUDA(h, rpa::launch_khatri_rao_cols(Xad, ldxa, Xid, ldxi, (int)NGrid, (int)v.nv, a0, wp, YX, h->stream));
-    if (int gs = gemm64(h, gemm_tn(NQ, (int)wp, NGrid, Zd, ldz, YX, NGrid, Rp, NQ), h->thc_piece_bytes / 2)) return gs;
+    if (int gs = gemm64(h, gemm_tn(NQ, (int)wp, NGrid, Zd, ldz, YX, NGrid, Rp, NQ), h->thc_piece_bytes / 2, factors))
+      return gs;
     RPA_CUDA(h, rpa::launch_count_nonfinite(Rp, (int64_t)NQ * wp, h->count_dev, h->stream));
     const rpa::SplitPlan plan = rpa::plan_scale_split(NQ, wp, h->num_sms);
     RPA_CUDA(h, ensure(h->diag_part, (size_t)plan.nsplit * K * NQ * 8));

@@ -166,12 +166,13 @@ __global__ void __launch_bounds__(256) mod_ksize_rows_kernel(const double* __res
 }
 // The factors of column k: 2^h for a; 2^-h, and the product's own scale of k, for b.
 __global__ void mod_kfactor_kernel(const int* __restrict__ size_a, const int* __restrict__ size_b,
-                                   const double* __restrict__ kscale, int64_t K, double* __restrict__ fa,
-                                   double* __restrict__ fb) {
+                                   const int* __restrict__ size_b2, const double* __restrict__ kscale, int64_t K,
+                                   double* __restrict__ fa, double* __restrict__ fb) {
   const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (k >= K) return;
   const double s = kscale ? kscale[k] : 1.0;
-  const int h = mod_balance(size_a[k], size_b[k], kscale ? __double2hiint(s) & 0x7fffffff : 1023 << 20);
+  const int s2 = size_b2 ? size_b2[k] : kscale ? __double2hiint(s) & 0x7fffffff : 1023 << 20;
+  const int h = mod_balance(size_a[k], size_b[k], s2);
   fa[k] = mod_pow2(h);
   fb[k] = mod_pow2(-h) * s;
 }
@@ -1121,22 +1122,24 @@ cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, co
   return cudaGetLastError();
 }
 
-cudaError_t launch_mod_balance(const double* A, int64_t a_r, int64_t a_k, int64_t rowsA, const double* B, int64_t b_r,
-                               int64_t b_k, int64_t rowsB, int64_t K, const double* kscale, int* sizes, double* fa,
-                               double* fb, cudaStream_t stream) {
-  if (K <= 0 || rowsA <= 0 || rowsB <= 0) return cudaSuccess;
-  const cudaError_t e = cudaMemsetAsync(sizes, 0, 2 * (size_t)K * sizeof(int), stream);
+cudaError_t launch_mod_balance(const ModOperand& a, const ModOperand& b, const ModOperand* b2, int64_t K,
+                               const double* kscale, int* sizes, double* fa, double* fb, cudaStream_t stream) {
+  if (K <= 0 || a.rows <= 0 || b.rows <= 0) return cudaSuccess;
+  const cudaError_t e = cudaMemsetAsync(sizes, 0, 3 * (size_t)K * sizeof(int), stream);
   if (e != cudaSuccess) return e;
-  auto size = [&](const double* S, int64_t s_r, int64_t s_k, int64_t rows, int* out) {
-    if (s_k == 1)
-      mod_ksize_cols_kernel<<<dim3((unsigned)((rows + kSizeRows - 1) / kSizeRows), (unsigned)((K + 255) / 256)), 256, 0,
-                              stream>>>(S, s_r, rows, K, out);
-    else mod_ksize_rows_kernel<<<(unsigned)((K + 7) / 8), 256, 0, stream>>>(S, s_k, rows, K, out);
+  auto size = [&](const ModOperand& x, int* out) {
+    if (x.s_k == 1)
+      mod_ksize_cols_kernel<<<dim3((unsigned)((x.rows + kSizeRows - 1) / kSizeRows), (unsigned)((K + 255) / 256)), 256,
+                              0, stream>>>(x.S, x.s_r, x.rows, K, out);
+    else mod_ksize_rows_kernel<<<(unsigned)((K + 7) / 8), 256, 0, stream>>>(x.S, x.s_k, x.rows, K, out);
+    ++g_launches;
   };
-  size(A, a_r, a_k, rowsA, sizes);
-  size(B, b_r, b_k, rowsB, sizes + K);
-  mod_kfactor_kernel<<<(unsigned)((K + 255) / 256), 256, 0, stream>>>(sizes, sizes + K, kscale, K, fa, fb);
-  g_launches += 3;
+  size(a, sizes);
+  size(b, sizes + K);
+  if (b2) size(*b2, sizes + 2 * K);
+  mod_kfactor_kernel<<<(unsigned)((K + 255) / 256), 256, 0, stream>>>(sizes, sizes + K, b2 ? sizes + 2 * K : nullptr,
+                                                                     kscale, K, fa, fb);
+  ++g_launches;
   return cudaGetLastError();
 }
 

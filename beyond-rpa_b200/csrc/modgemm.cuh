@@ -116,11 +116,15 @@ cudaError_t launch_mod_cols(const double* S, int64_t ld, int64_t strideS, int K,
 // fac is given.
 cudaError_t launch_mod_rows(const double* S, int64_t ld, int rows, int64_t K, const double* fac, int8_t* planes,
                             int* expo, cudaStream_t stream);
-// fa[k], fb[k]: factors that bring column k of both operands to the same size (mod_balance), fb times
-// kscale[k] when given.  Entry (r, k) of an operand at S[r * s_r + k * s_k], one stride 1; sizes: 2 K ints.
-cudaError_t launch_mod_balance(const double* A, int64_t a_r, int64_t a_k, int64_t rowsA, const double* B, int64_t b_r,
-                               int64_t b_k, int64_t rowsB, int64_t K, const double* kscale, int* sizes, double* fa,
-                               double* fb, cudaStream_t stream);
+// fa[k], fb[k]: factors that bring column k of operands a and b to the same size (mod_balance), fb times
+// kscale[k] when given.  With b2, column k of the second operand is made of products of entries of column k of b and of
+// b2 (a Khatri-Rao product, of which only the factors are read).  sizes: 3 K ints.
+struct ModOperand {
+  const double* S;  // entry (r, k) at S[r * s_r + k * s_k], one stride 1
+  int64_t s_r, s_k, rows;
+};
+cudaError_t launch_mod_balance(const ModOperand& a, const ModOperand& b, const ModOperand* b2, int64_t K,
+                               const double* kscale, int* sizes, double* fa, double* fb, cudaStream_t stream);
 // Residue planes [k][modulus][Q][pitch] of X_k; fac: fg.n * nov doubles, part: nsplit * fg.n * NQ.
 cudaError_t launch_mod_pi(const double* R, int64_t ldR, int NQ, int64_t nov, const double* D, const FreqGroup& fg,
                           double alpha, double* fac, double* part, int nsplit, int* expo, int8_t* planes,
