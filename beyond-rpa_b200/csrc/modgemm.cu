@@ -10,7 +10,10 @@
 // its 15 residues (Chinese remainder theorem).  Each residue is one int8 x int8 -> int32 matrix
 // product of tcgen05 (kind::i8), exact as long as K <= 65536 per accumulation.  The only errors
 // are the rounding of the operands (0.5 units of 2^-58 of the row norm) and one rounding of C, less
-// than a chain of K FP64 additions leaves (tests/test_gpu_modgemm.py compares both).
+// than a chain of K FP64 additions leaves (tests/test_gpu_modgemm.py compares both).  The rounding is
+// relative to the row, not to the entry: operands that may be graded against each other along K are
+// brought to the same sizes first (launch_mod_balance); in X X^T, (V - 1)^T (V - 1), M R and L L^T both
+// carry the same grading.
 //
 // On B200 the int8 pipe sustains 3.9 POP/s (random operands from shared memory, M 128 x N 256), so
 // 15 products cost what 260 TFLOP/s of FP64 would, against 37 TFLOP/s of the FP64 pipe.

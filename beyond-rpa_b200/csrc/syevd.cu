@@ -1112,9 +1112,10 @@ cudaError_t syevd_batched(double* A, int n, int nmat, double* Z, void* work, siz
     return g;
   };
 
-  // ---- stage 1: tridiagonal reduction (one 8-CTA cluster per matrix per column step)
-  // One matrix whose column fits in shared memory: a cooperative launch per panel; batches (the small
-  // matrices of many pairs): a cluster per matrix and column step.
+  // ---- stage 1: tridiagonal reduction
+  // Orders up to kSmallN: one CTA per matrix, in shared memory.  One larger matrix whose column fits in
+  // shared memory: a cooperative launch per panel.  Else (batches of larger matrices): an 8-CTA cluster per
+  // matrix and column step.
   int dev = 0, sms = 0, fit = 0;
   SY_CHECK(cudaGetDevice(&dev));
   SY_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

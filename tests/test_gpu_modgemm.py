@@ -1,5 +1,6 @@
 """Residue products on the int8 tensor cores (modgemm.cu): the FP64 form of Pi(u) and the adjoint's
-back-contraction, at the edges of their 128 x 256 tiles, 128-wide K chunks and frequency groups.
+back-contraction, at the edges of their 256 x 256 tiles (128 rows per CTA of a pair), 128-wide K chunks and
+frequency groups.
 
 Tolerances.  Operand rows are rounded to 2^-58 of their 2-norm, so an entry of Pi is off by at most
   0.5 sqrt(nov) 2^-57 2 ||X_Q|| ||X_P||  (rounding)  +  2^-53 |Pi_QP|  (one rounding of the result)
@@ -13,7 +14,7 @@ from oracle import rpa_oracle as O
 
 pytestmark = pytest.mark.gpu
 
-# NQ, NOcc, NVirt, K: tile edges (128, 256 rows), K chunks (128 ai), one and several frequency groups
+# NQ, NOcc, NVirt, K: tile edges (128, 256, 512 rows), K chunks (128 ai), one and several frequency groups
 SHAPES = [(128, 2, 64, 1), (129, 4, 33, 2), (255, 3, 43, 3), (256, 2, 64, 17), (257, 5, 77, 2), (385, 3, 64, 5),
           (513, 2, 65, 33), (640, 6, 128, 4)]
 

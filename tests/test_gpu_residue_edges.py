@@ -397,3 +397,22 @@ def test_pivot_inverses(handle):
         assert np.max(np.abs(got - ref)[~normal], initial=0.0) <= 2.0 ** -1074
     inv, inv_sqrt = handle.selftest_pivots(np.array([0.0, -1.0, -np.inf, np.nan]))
     assert np.all(inv == 1.0) and np.all(inv_sqrt == 1.0)
+
+
+def test_energy_from_factors_in_pieces(pkg, monkeypatch):
+    # pieces of 128 pairs that begin and end inside an occupied orbital: each piece's vectors as a residue
+    # product, balanced over the orbitals it covers, against the vectors formed whole on the FP64 pipe
+    ng, nq, no, nv = 300, 150, 5, 61
+    Z, Xa, Xi, eo, ev = O.make_thc_factors(ng, nq, no, nv, 21)
+    t = np.exp(3.0 * np.random.default_rng(22).standard_normal(ng))[:, None]
+    x, w = O.casimir_polder(4, 0.8)
+    monkeypatch.setenv("RPA_B200_RESIDUES", "0")
+    with pkg.Handle(0) as h:
+        R = h.thc_r(Z, Xa, Xi)
+        ref = h.ec_rpa(R, eo, ev, x, w, prec="split")[0]
+    monkeypatch.setenv("RPA_B200_RESIDUES", "1")
+    monkeypatch.setenv("RPA_B200_THC_PIECE_BYTES", "1")
+    monkeypatch.setenv("RPA_B200_GEMM64_BYTES", str(15 * (384 + 256) * 128))
+    with pkg.Handle(0) as h:
+        ec = h.ec_thc(Z * t, Xa / t, Xi, eo, ev, x, w, prec="split")[0]
+    assert abs(ec - ref) < 1e-6  # split products in pieces against the whole, as in the pieces' own test
