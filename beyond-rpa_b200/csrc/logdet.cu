@@ -63,7 +63,7 @@ __device__ __forceinline__ void pivot_inverses(double& d, double& rd, double& ri
       bad = true;
       d = 1.0;
     }
-    rd = 1.0 / d;
+    rd = fmin(1.0 / d, 1.7976931348623157e308);  // finite: it meets entries that are zero
     ri = rsqrt(d);
     return;
   }
