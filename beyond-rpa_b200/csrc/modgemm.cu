@@ -266,19 +266,22 @@ __global__ void __launch_bounds__(256) mod_row_norm_kernel(const double* __restr
     return fac ? x * __ldg(fac + k) : x;
   };
   auto sum = [&](double f) {
-    double s0 = 0.0, s1 = 0.0;
+    // eight entries and factors on their way at a time
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
     int64_t k = warp;
-    for (; k + 8 < K; k += 16) {
-      const double x = entry(k) * f, y = entry(k + 8) * f;
-      s0 = fma(x, x, s0);
-      s1 = fma(y, y, s1);
+    for (; k + 56 < K; k += 64) {
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = entry(k + 8 * u) * f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s[u & 3] = fma(x[u], x[u], s[u & 3]);
     }
-    if (k < K) {
+    for (; k < K; k += 8) {
       const double x = entry(k) * f;
-      s0 = fma(x, x, s0);
+      s[0] = fma(x, x, s[0]);
     }
     __syncthreads();
-    red[warp][lane] = s0 + s1;
+    red[warp][lane] = (s[0] + s[1]) + (s[2] + s[3]);
     __syncthreads();
     double t = 0.0;
 #pragma unroll
