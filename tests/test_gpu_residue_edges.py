@@ -182,7 +182,7 @@ def _caps(pkg, call, monkeypatch, steps=24):
     return free, out
 
 
-@pytest.mark.parametrize("what", ["ec", "grad", "t2", "batch"])
+@pytest.mark.parametrize("what", ["ec", "grad", "grad split", "t2", "batch"])
 def test_optional_planes_never_cost_a_call_its_room(pkg, monkeypatch, what):
     # workspace caps at which some of the residue planes fit: what the call needs afterwards must still find
     # its room, whatever the planes took first.  The forms differ by their rounding only (tolerances as in
@@ -196,6 +196,8 @@ def test_optional_planes_never_cost_a_call_its_room(pkg, monkeypatch, what):
         call = lambda h: np.array([h.ec_rpa(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")[0]])
     elif what == "grad":
         call = lambda h: h.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="fp64")[1]
+    elif what == "grad split":
+        call = lambda h: h.ec_grad(s.R, s.eps_o, s.eps_v, x, w, prec="split")[1]
     elif what == "t2":
         call = lambda h: h.dring_t2(s.R, s.eps_o, s.eps_v, x, w, guess=guess, cutoff_thresh=1e-6)["A"]
     else:
