@@ -83,8 +83,9 @@ typedef enum rpa_status {
 typedef struct rpa_b200_handle rpa_b200_handle;
 
 /* Create / destroy a handle bound to one GPU (`device` = CUDA ordinal).
- * The handle owns a stream, a grow-only device workspace and the TMA
- * descriptors.  flags: reserved, pass 0.                                    */
+ * The handle owns a stream, a device workspace that is kept between calls
+ * (buffers that hold nothing are freed where an allocation finds no room) and the
+ * TMA descriptors.  flags: reserved, pass 0.                                    */
 int rpa_b200_create(rpa_b200_handle** handle, int64_t device, int64_t flags);
 int rpa_b200_destroy(rpa_b200_handle* handle);
 const char* rpa_b200_status_string(int status);
