@@ -231,12 +231,16 @@ def _colmajor(x, nrows):
 def _amplitude_buffer(R, nov, n_guess):
     """Device memory for the amplitudes U of vectors R that are on the device themselves, so that the exchange
     energy reads them where the T2 solver left them; None (host memory) for host R or when it would take
-    more than a sixteenth of the free device memory, which the solver's own workspace may need."""
+    more than a sixteenth of the free device memory, which the solver's own workspace may need.  Below a
+    gigabyte it does not ask (the query can hold the host up for 100 ms while other processes use the
+    driver); should the solver then find no room, its caller takes the buffer back."""
     if not (_is_torch(R) and R.is_cuda):
         return None
     import torch
     cap = int(n_guess if n_guess is not None else min(int(np.ceil(3.0 * int(R.shape[0]))), nov))
-    if cap <= 0 or nov <= 0 or 8 * cap * nov > torch.cuda.mem_get_info(R.device)[0] // 16:
+    if cap <= 0 or nov <= 0:
+        return None
+    if 8 * cap * nov > 1 << 30 and 8 * cap * nov > torch.cuda.mem_get_info(R.device)[0] // 16:
         return None
     try:
         buf = torch.empty((cap, nov), dtype=torch.float64, device=R.device).T
@@ -455,9 +459,21 @@ class Handle:
         common = -1.0
         ex, eig, nts = [], [], []
         for R, eo, ev in active:
-            t2 = self.dring_t2(R, eo, ev, x, w, prec=prec, seed=seed, n_guess=n_guess, cutoff_thresh=cutoff_thresh,
-                               cutoff_type=cutoff_type, common_thresh=common,
-                               u_out=_amplitude_buffer(R, len(eo) * len(ev), n_guess))
+            def solve(u_out):
+                return self.dring_t2(R, eo, ev, x, w, prec=prec, seed=seed, n_guess=n_guess,
+                                     cutoff_thresh=cutoff_thresh, cutoff_type=cutoff_type, common_thresh=common,
+                                     u_out=u_out)
+            buf, t2 = _amplitude_buffer(R, len(eo) * len(ev), n_guess), None
+            try:
+                t2 = solve(buf)
+            except RPAError as e:
+                if buf is None or e.status != RPA_ERR_OOM:
+                    raise
+            if t2 is None:  # the amplitudes go to the host, their device memory to the solver
+                import torch
+                buf = None
+                torch.cuda.empty_cache()
+                t2 = solve(None)
             common = t2["common_thresh"]
             nts.append(t2["NT"])
             eig.append(float(np.sum(t2["EigRPA"])))
